@@ -35,11 +35,15 @@ class VisionPlan:
 
     @staticmethod
     def build(grids, cfg: VisionConfig, device) -> "VisionPlan":
-        cu, mx = positions.vision_segments(grids)
-        if ops.tables_on_device(device) and len(grids) and np.prod(grids, axis=-1).any():
+        g = np.asarray(grids, dtype=np.int64).reshape(-1, 3)
+        merge = cfg.spatial_merge_size
+        # the tables are in merge-block order: an image with patches has whole blocks only
+        if (g < 0).any() or (g[g.prod(1) != 0, 1:] % merge).any():
+            raise ValueError(f"image sizes (frames, height, width in patches) must be multiples of {merge} patches: {g.tolist()}")
+        cu, mx = positions.vision_segments(g)
+        if ops.tables_on_device(device) and g.prod(1).any():
             # the tables are functions of the grids alone: made on the device; the grids travel, and the sine and cosine of every row
             # or column times every frequency, as numpy rounds them
-            g = np.asarray(grids, dtype=np.int64).reshape(-1, 3)
             first = np.concatenate(([0], np.cumsum(g.prod(1))))
             fr = np.arange(g[:, 1:].max(), dtype=np.float32)[:, None] * _inv_freq(cfg.head_dim // 2)
             trig = np.stack((np.cos(fr), np.sin(fr)), -1).astype(np.float32, copy=False)  # [coordinate, frequency, 2]
@@ -48,8 +52,7 @@ class VisionPlan:
             small = both[trig.size:]
             images = small[:4 * len(g)].view(-1, 4)
             side = int(round(cfg.num_position_embeddings ** 0.5))
-            cos, sin, idx, wt = ops.vision_plan(images, both[:trig.size].view(torch.float32), trig.shape[1], side, cfg.spatial_merge_size,
-                                                int(first[-1]))
+            cos, sin, idx, wt = ops.vision_plan(images, both[:trig.size].view(torch.float32), trig.shape[1], side, merge, int(first[-1]))
             return VisionPlan(small[4 * len(g):], mx, cos, sin, idx, wt, images)
         coords = positions.vision_rot_coords(grids, cfg.spatial_merge_size)
         half = cfg.head_dim // 2

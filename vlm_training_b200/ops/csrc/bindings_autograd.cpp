@@ -738,8 +738,8 @@ struct PosEmbed : torch::autograd::Function<PosEmbed> {
                             reinterpret_cast<uintptr_t>(g.data_ptr()) % 16 == 0;
       if (in_place) check_storage(g);
       Tensor out = in_place ? g : torch::empty_like(table);
-      vlmt_pos_embed_bwd(dy.data_ptr(), saved[1].data_ptr<int>(), (int)saved[1].size(0), (int)c->n_q, (int)c->n_kv, out.data_ptr(), in_place,
-                         (int)table.size(1), cur_stream());
+      vlmt_pos_embed_bwd(dy.data_ptr(), saved[1].data_ptr<int>(), (int)saved[1].size(0), (int)c->n_q, (int)c->n_kv, dy.size(0), out.data_ptr(),
+                         in_place, (int)table.size(1), cur_stream());
       tick(1);
       if (in_place) c->t[0]->report(); else dt = out;
     }
@@ -779,7 +779,7 @@ std::vector<Tensor> rope_tables(const Tensor& pos, const Tensor& inv_freq, int64
 std::vector<Tensor> vision_plan(const Tensor& images, const Tensor& trig, int64_t nf, int64_t side, int64_t merge, int64_t n) {
   TORCH_CHECK(images.is_cuda() && images.scalar_type() == at::kInt && images.is_contiguous() && images.dim() == 2 && images.size(1) == 4 &&
               trig.scalar_type() == at::kFloat && trig.is_contiguous() && trig.is_cuda() && nf > 0 && trig.numel() > 0 && trig.numel() % (2 * nf) == 0 &&
-              (uintptr_t)trig.data_ptr() % 8 == 0);
+              (uintptr_t)trig.data_ptr() % 8 == 0 && side > 0 && merge > 0 && images.size(0) > 0);
   c10::cuda::CUDAGuard guard(images.device());
   auto fo = trig.options();
   Tensor c = torch::empty({n, 4 * nf}, fo), s = torch::empty({n, 4 * nf}, fo), index = torch::empty({4, n}, fo.dtype(at::kLong)),

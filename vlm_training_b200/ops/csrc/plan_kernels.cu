@@ -34,7 +34,7 @@ __device__ __forceinline__ Cell cell_of(int i, int count, int side, double step)
   // double products rounded once to float, the last point exactly side - 1: the same table positions as the host's numpy form
   const float x = i > 0 && i == count - 1 ? (float)(side - 1) : (float)__dmul_rn((double)i, step);
   Cell c;
-  c.lo = (int)x;
+  c.lo = min((int)x, side - 1);
   c.hi = min(c.lo + 1, side - 1);
   c.frac = x - (float)c.lo;
   return c;
@@ -54,9 +54,11 @@ __global__ void vision_plan_kernel(const int* __restrict__ images, int n_img, co
   const int h = images[4 * lo + 1], w = images[4 * lo + 2];
   const int r = (int)((n - images[4 * lo + 3]) % ((long)h * w)), mm = merge * merge;
   const int block = r / mm, in = r % mm, wb = w / merge;
-  const int row = (block / wb) * merge + in / merge, col = (block % wb) * merge + in % merge;
+  // sides are multiples of `merge` (checked on the host); clamped, so that no other size reaches beyond the tables
+  const int row = min(max(wb ? (block / wb) * merge + in / merge : 0, 0), coords - 1);
+  const int col = min(wb ? (block % wb) * merge + in % merge : 0, coords - 1);
   for (int k = lane; k < 2 * nf; k += 32) {   // channels: nf row angles, nf column angles, both again
-    const float2 cs = trig[(long)min(k < nf ? row : col, coords - 1) * nf + (k < nf ? k : k - nf)];
+    const float2 cs = trig[(long)(k < nf ? row : col) * nf + (k < nf ? k : k - nf)];
     cosv[n * 4 * nf + k] = cosv[n * 4 * nf + 2 * nf + k] = cs.x;
     sinv[n * 4 * nf + k] = sinv[n * 4 * nf + 2 * nf + k] = cs.y;
   }
@@ -111,7 +113,7 @@ __global__ void __launch_bounds__(256) pos_embed_fwd_kernel(const uint4* __restr
 // One block per table cell.  The patches that read a cell form a small rectangle of every image (rows and columns whose position lies
 // within one cell of it), so the gradient is a gather in fixed order: no sort, no atomics, every dy row read by four cells.
 __global__ void __launch_bounds__(256) pos_embed_bwd_kernel(const uint4* __restrict__ dy, const int* __restrict__ images, int n_img, int side,
-                                                            int merge, uint4* __restrict__ dtable, int accumulate, int dv) {
+                                                            int merge, long N, uint4* __restrict__ dtable, int accumulate, int dv) {
   const int cr = blockIdx.x / side, cc = blockIdx.x % side;
   for (int v = threadIdx.x; v < dv; v += blockDim.x) {
     float a[8];
@@ -136,7 +138,7 @@ __global__ void __launch_bounds__(256) pos_embed_bwd_kernel(const uint4* __restr
           if (wc == 0.f) continue;
           const long at = first + ((long)(i / merge) * (w / merge) + j / merge) * merge * merge + (i % merge) * merge + j % merge;
           const float wt = wr * wc;
-          for (int f = 0; f < frames; ++f) {
+          for (int f = 0; f < frames && at + (long)f * h * w < N; ++f) {
             float g[8];
             unpack8(dy[(at + (long)f * h * w) * dv + v], g);
 #pragma unroll
@@ -174,9 +176,9 @@ void vlmt_pos_embed_fwd(const void* x, const void* table, const long* pe_index, 
   pos_embed_fwd_kernel<<<(unsigned)((N * (D / 8) + 255) / 256), 256, 0, st>>>((const uint4*)x, (const uint4*)table, pe_index, pe_weight, (uint4*)out,
                                                                               N, D / 8);
 }
-void vlmt_pos_embed_bwd(const void* dy, const int* images, int n_img, int side, int merge, void* dtable, int accumulate, int D,
+void vlmt_pos_embed_bwd(const void* dy, const int* images, int n_img, int side, int merge, long N, void* dtable, int accumulate, int D,
                         cudaStream_t st) {
   const int dv = D / 8, threads = dv >= 256 ? 256 : (dv + 31) / 32 * 32;
-  pos_embed_bwd_kernel<<<side * side, threads, 0, st>>>((const uint4*)dy, images, n_img, side, merge, (uint4*)dtable, accumulate, dv);
+  pos_embed_bwd_kernel<<<side * side, threads, 0, st>>>((const uint4*)dy, images, n_img, side, merge, N, (uint4*)dtable, accumulate, dv);
 }
 }

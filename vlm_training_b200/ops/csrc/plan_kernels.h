@@ -17,8 +17,9 @@ void vlmt_vision_plan(const int* images, int n_img, const float* trig, int coord
                       float* sinv, long* pe_index, float* pe_weight, cudaStream_t st);
 // out[n] = x[n] + bf16(sum_c pe_weight[c, n] * table[pe_index[c, n]]), rows of D bf16 (D a multiple of 8)
 void vlmt_pos_embed_fwd(const void* x, const void* table, const long* pe_index, const float* pe_weight, void* out, long N, int D, cudaStream_t st);
-// gradient of the table [side * side, D]: stored in, or (accumulate) added to, the bf16 `dtable`
-void vlmt_pos_embed_bwd(const void* dy, const int* images, int n_img, int side, int merge, void* dtable, int accumulate, int D, cudaStream_t st);
+// gradient of the table [side * side, D] from dy [N, D]: stored in, or (accumulate) added to, the bf16 `dtable`
+void vlmt_pos_embed_bwd(const void* dy, const int* images, int n_img, int side, int merge, long N, void* dtable, int accumulate, int D,
+                        cudaStream_t st);
 #ifdef __cplusplus
 }
 #endif
