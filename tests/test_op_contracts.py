@@ -32,3 +32,72 @@ def test_position_indices_stay_in_the_table():
     trig = torch.ones(37 * 4 * 2, device=DEV)
     index = ops.vision_plan(images, trig, 4, 48, 2, 113)[2]
     assert int(index.min()) >= 0 and int(index.max()) < 48 * 48
+
+
+_T, _H, _N = 256, 128, 384
+_ROWS = torch.arange(_T)
+# name -> (op of (x, parameters), parameter shapes, width of x)
+_PARAM_OPS = {
+    "linear": (lambda x, p: ops.linear(x, p["w"], p["b"]), dict(w=(_N, _H), b=(_N,)), _H),
+    "norm_linear": (lambda x, p: ops.rms_norm_linear(x, p["nw"], p["w"]), dict(nw=(_H,), w=(_N, _H)), _H),
+    "norm_linear_residual": (lambda x, p: ops.rms_norm_linear(x, p["nw"], p["w"], residual=_rand(_T, _H, seed=5)), dict(nw=(_H,), w=(_N, _H)), _H),
+    "ln_linear": (lambda x, p: ops.layer_norm_linear(x, p["nw"], p["nb"], p["w"], p["b"]), dict(nw=(_H,), nb=(_H,), w=(_N, _H), b=(_N,)), _H),
+    "gelu_linear": (lambda x, p: ops.gelu_linear(x, p["w"], p["b"]), dict(w=(_N, _H), b=(_N,)), _H),
+    "swiglu_linear": (lambda x, p: ops.swiglu_linear(x, p["w"]), dict(w=(_N, _H)), 2 * _H),
+    "rms_norm": (lambda x, p: ops.rms_norm(x, p["nw"]), dict(nw=(_H,)), _H),
+    "layer_norm": (lambda x, p: ops.layer_norm(x, p["nw"], p["nb"]), dict(nw=(_H,), nb=(_H,)), _H),
+    "rms_norm_gated": (lambda x, p: ops.rms_norm_gated(x, _rand(_T, _H, seed=6), p["nw"]), dict(nw=(_H,)), _H),
+    "qkv_norm_rope": (lambda x, p: ops.qkv_norm_rope(x, 2, 1, 128, p["qw"], p["kw"], _rand(_T, 128, seed=7).float(), _rand(_T, 128, seed=8).float())[:3],
+                      dict(qw=(128,), kw=(128,)), 512),
+    "loss": (lambda x, p: ops.linear_cross_entropy(x, p["w"], (_ROWS * 7 % _N).to(DEV), 64, grad_in_place=True)[0], dict(w=(_N, _H)), _H),
+    "experts": (lambda x, p: ops.moe_experts(x, p["gu"], p["dn"], torch.full((_T, 2), 0.5, device=DEV, dtype=torch.bfloat16),
+                                             torch.stack((_ROWS % 4, (_ROWS + 1) % 4), 1).to(DEV)), dict(gu=(4, 256, _H), dn=(4, _H, 128)), _H),
+}
+_TAGGED = {name: shapes for name, (_, shapes, _) in _PARAM_OPS.items()}
+
+
+def _leaves(name, tag=None, grad=0.0, fp8=False, resharded=False):
+    """``x`` and the op's parameters; ``tag``: gradients of the parameters land in views of an engine's buffer, which it is called on."""
+    _, shapes, width = _PARAM_OPS[name]
+    x = _rand(_T, width, seed=1).requires_grad_()
+    params = {}
+    for i, (k, shape) in enumerate(shapes.items()):
+        p = params[k] = torch.nn.Parameter(_rand(*shape, scale=0.2, seed=10 + i) + (1.0 if k in ("nw", "qw", "kw") else 0.0))
+        if tag is not None:
+            p.grad = torch.full_like(p, grad)
+            p._vlmt_grad_in_place, p._vlmt_grad_ready = True, tag
+        if fp8:
+            p._vlmt_fp8 = p.dim() == 2
+        if resharded:
+            p._vlmt_resharded = True
+    return x, params
+
+
+def _backward(name, x, params, seed=30, **kw):
+    out = _PARAM_OPS[name][0](x, params)
+    outs = [o for o in (out if isinstance(out, tuple) else (out,)) if o is not None]
+    torch.autograd.backward(outs, [_rand(*o.shape, seed=seed + i, dtype=o.dtype) if o.dim() else torch.full_like(o, 1.7) for i, o in enumerate(outs)], **kw)
+
+
+@gpu
+@pytest.mark.parametrize("name,form", [(n, "") for n in _PARAM_OPS] + [("linear", "fp8"), ("linear", "resharded"), ("norm_linear", "resharded"),
+                                                                       ("norm_linear_residual", "resharded"), ("ln_linear", "resharded")])
+def test_a_parameter_is_reported_ready_after_its_last_read(name, form):
+    """The engine may enqueue the update of a parameter (and store it into the peers' memory) as soon as its gradient is reported: the
+    callback here overwrites the parameter on the current stream, and the gradient of ``x`` must not change."""
+    kw = {form: True} if form else {}
+    x0, plain = _leaves(name, **kw)
+    _backward(name, x0, plain)
+    seen = []
+
+    def overwrite(p):
+        seen.append(id(p))
+        p.data.fill_(float("nan"))
+
+    x1, tagged = _leaves(name, overwrite, **kw)
+    _backward(name, x1, tagged)
+    assert torch.equal(x0.grad, x1.grad)
+    for k, p in tagged.items():
+        assert torch.equal(p.grad, plain[k].grad), k
+        assert seen.count(id(p)) == (1 if id(p) in seen else 0), k
+    assert seen

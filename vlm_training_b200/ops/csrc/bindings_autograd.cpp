@@ -90,8 +90,10 @@ Tensor mm(const Tensor& a, const Tensor& b, bool a_mn, bool b_mn, const Tensor& 
   tick(1);
   return out;
 }
-// dW[N, K] = dY^T[N, M] . X[M, K]
-Tensor weight_grad(const Tensor& dy, const Tensor& x, const Target& t) {
+// dW[N, K] = dY^T[N, M] . X[M, K].  A parameter is reported only when every kernel of the backward pass that reads it has been
+// enqueued: its bucket's update may run on another stream, or in a peer's kernel, from that moment on.
+Tensor weight_grad(const Tensor& dy, const Tensor& x, const Target& t, bool& report) {
+  report = false;
   if (t) {
     Tensor g = t->param.grad();
     if (g.defined() && g.scalar_type() == at::kBFloat16 && g.dim() == 2 && g.size(0) == dy.size(1) && g.size(1) == x.size(1) &&
@@ -99,11 +101,18 @@ Tensor weight_grad(const Tensor& dy, const Tensor& x, const Target& t) {
       check_storage(g);
       gemm(dy, x, g, true, true, c10::nullopt, 0, true, c10::nullopt);
       tick(1);
-      t->report();
+      report = true;
       return Tensor();
     }
   }
   return mm(dy, x, true, true);
+}
+// for a function whose last read of the weight has been enqueued
+Tensor weight_grad(const Tensor& dy, const Tensor& x, const Target& t) {
+  bool report;
+  Tensor dw = weight_grad(dy, x, t, report);
+  if (report) t->report();
+  return dw;
 }
 // where the gradient of a 1-D parameter goes: added to a tagged .grad, or a new tensor of the parameter's type
 struct VecGrad {
@@ -246,10 +255,12 @@ struct NormLinear : torch::autograd::Function<NormLinear> {
       dx = dr;
     } else {
       Tensor dy = rows_of(grads[0]);
-      if (c->need[3]) dw = weight_grad(dy, rmsnorm_fwd(r, c10::nullopt, nw, c->eps, c->offset)[0], c->t[1]);
+      bool report = false;   // the weight is read once more, by d(normalised rows)
+      if (c->need[3]) dw = weight_grad(dy, rmsnorm_fwd(r, c10::nullopt, nw, c->eps, c->offset)[0], c->t[1], report);
       auto b = rmsnorm_bwd_partial(mm(dy, w, false, true), r, nw, rstd, dr.defined() ? OptTensor(dr.contiguous()) : OptTensor(), c->offset);
       dx = b[0];
       tick(2);
+      if (report) c->t[1]->report();
       if (c->need[2]) {
         VecGrad g(nw, c->t[0]);
         sum_rows(b[1].data_ptr<float>(), nullptr, b[1].size(1), b[1].size(0), b[1].size(1), g, nullptr);
@@ -299,9 +310,11 @@ struct LnLinear : torch::autograd::Function<LnLinear> {
     const Tensor &x = saved[0], &lw = saved[1], &mean = saved[2], &rstd = saved[3], &w = saved[4];
     Tensor lb = c->n_q ? saved[5] : Tensor(), b = c->n_kv ? saved[5 + c->n_q] : Tensor();
     Tensor dy = rows_of(grads[0]), dlw, dlb, dw, db;
-    if (c->need[3]) dw = weight_grad(dy, layernorm_fwd(x, lw, opt(lb), c->eps)[0], c->t[2]);
+    bool report = false;   // the weight is read once more, by d(normalised rows)
+    if (c->need[3]) dw = weight_grad(dy, layernorm_fwd(x, lw, opt(lb), c->eps)[0], c->t[2], report);
     auto r = layernorm_bwd_partial(mm(dy, w, false, true), x, lw, mean, rstd);
     tick(2);
+    if (report) c->t[2]->report();
     if (c->need[1] || c->need[2]) {
       VecGrad gw(lw, c->need[1] ? c->t[0] : Target());
       const int rows = r[1].size(0), cols = r[1].size(1);

@@ -145,18 +145,25 @@ def _grad_target(w):
     return w if (_WGRAD_IN_PLACE and getattr(w, "_vlmt_grad_in_place", False)) else None
 
 
-def _wgrad(dy2, x2, param=None, alpha=None):
+def _report(param):
+    """The engine's gradient-ready hook of a tagged parameter, called by hand because autograd has nothing to accumulate.  The update
+    may run at once on another stream or in a peer's kernel: every kernel that reads the parameter must have been enqueued."""
+    ready = getattr(param, "_vlmt_grad_ready", None)
+    if ready is not None:
+        ready(param)
+
+
+def _wgrad(dy2, x2, param=None, alpha=None, report=True):
     """dW[N,K] = dY^T[N,M] . X[M,K].  For a tagged parameter the GEMM adds the product into ``param.grad`` from its
     epilogue (TMA reduce-add) and autograd gets ``None``: no separate accumulation pass over the gradient, no temporary.
-    The engine's gradient-ready hook is called by hand because autograd has nothing to accumulate."""
+    ``report=False``: kernels that read the parameter are still to come; the caller reports it behind them if it gets ``None``."""
     if param is not None:
         g = param.grad
         if (g is not None and g.dtype == torch.bfloat16 and g.dim() == 2 and g.shape == (dy2.shape[1], x2.shape[1])
                 and g.stride(1) == 1 and g.stride(0) % 8 == 0 and g.data_ptr() % 16 == 0):
             _gemm(dy2, x2, a_mn=True, b_mn=True, out=g, accumulate=True, alpha=alpha)
-            ready = getattr(param, "_vlmt_grad_ready", None)
-            if ready is not None:
-                ready(param)
+            if report:
+                _report(param)
             return None
     return _gemm(dy2, x2, a_mn=True, b_mn=True, alpha=alpha)
 
@@ -299,9 +306,11 @@ class _NormLinear(torch.autograd.Function):
         eps, offset, has_res = ctx.cfg
         dy2 = _as_gemm_operand(dy)
         h = _C.rmsnorm_fwd(r, None, norm_w, eps, offset)[0]  # recompute the normalised activation
-        dw = _wgrad(dy2, h, ctx.w_param)
+        dw = _wgrad(dy2, h, ctx.w_param, report=False)
         del h
         dh = _gemm(dy2, w, b_mn=True)
+        if dw is None:
+            _report(ctx.w_param)
         dx, dnw = _C.rmsnorm_bwd(dh, r, norm_w, rstd, dr.contiguous() if dr is not None else None, offset)
         _tick(3)
         dnw = dnw.to(norm_w.dtype)
@@ -343,9 +352,11 @@ class _LNLinear(torch.autograd.Function):
         x, ln_w, ln_b, mean, rstd, w = ctx.saved_tensors
         dy2 = _as_gemm_operand(dy)
         h = _C.layernorm_fwd(x, ln_w, ln_b, ctx.eps)[0]
-        dw = _wgrad(dy2, h, ctx.w_param)
+        dw = _wgrad(dy2, h, ctx.w_param, report=False)
         del h
         dh = _gemm(dy2, w, b_mn=True)
+        if dw is None:
+            _report(ctx.w_param)
         dx, dlw, dlb = _C.layernorm_bwd(dh, x, ln_w, mean, rstd)
         db = None
         if ctx.has_bias:
@@ -488,8 +499,10 @@ class _LinearCrossEntropy(torch.autograd.Function):
         if ctx.keep_logits:
             dl, hidden, weight = ctx.saved_tensors
             alpha = g_loss.float()
-            dw = _wgrad(dl, hidden, ctx.w_param, alpha=alpha) if hidden is not None else None   # dW = alpha dL^T . H
+            dw = _wgrad(dl, hidden, ctx.w_param, alpha=alpha, report=False) if hidden is not None else None   # dW = alpha dL^T . H
             dh = _gemm(dl, weight, b_mn=True, alpha=alpha) if weight is not None else None       # dH = alpha dL . W
+            if hidden is not None and dw is None:
+                _report(ctx.w_param)
             return dh, dw, None, None, None, None, None
         dh, dw = ctx.saved_tensors
         if dh is not None:

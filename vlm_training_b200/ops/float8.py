@@ -123,9 +123,7 @@ class _LinearFp8(torch.autograd.Function):
                     and g.stride(0) % 8 == 0 and g.data_ptr() % 16 == 0):
                 # added into the optimizer's gradient bucket by the GEMM's epilogue; autograd has nothing to accumulate
                 C.gemm_fp8(d8t, x8t, g, rd, rx, E5M2, E4M3, True)
-                ready = getattr(param, "_vlmt_grad_ready", None)
-                if ready is not None:
-                    ready(param)
+                cu._report(param)
             else:
                 dw = torch.empty(ctx.w_shape, dtype=torch.bfloat16, device=dy.device)
                 C.gemm_fp8(d8t, x8t, dw, rd, rx, E5M2, E4M3, False)

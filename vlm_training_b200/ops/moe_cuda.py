@@ -58,8 +58,8 @@ class _GroupedLinear(torch.autograd.Function):
             cu._tick()
             if g is None:
                 dw = dw.view(E, N, K)
-            elif (ready := getattr(param, "_vlmt_grad_ready", None)) is not None:
-                ready(param)
+            else:
+                cu._report(param)
         return dx, dw, None
 
 
