@@ -101,3 +101,37 @@ def test_a_parameter_is_reported_ready_after_its_last_read(name, form):
         assert torch.equal(p.grad, plain[k].grad), k
         assert seen.count(id(p)) == (1 if id(p) in seen else 0), k
     assert seen
+
+
+# tiles with an odd number of 64-column slabs (N mod 256 up to 64, or 129 to 192) that are followed by more work of the same block or pair,
+# and an epilogue that lags (one or two blocks of K): the next item's first slab reuses the staging buffer of this item's last one
+@gpu
+@pytest.mark.parametrize("M,N,K", [(40000, 576, 64), (40000, 448, 128), (40000, 64, 64), (20000, 192, 64)])
+@pytest.mark.parametrize("accumulate", [False, True])
+def test_gemm_epilogue_with_odd_slabs(M, N, K, accumulate):
+    from vlm_training_b200.ops import cuda as cu
+
+    a, b, base = _rand(M, K, seed=1), _rand(N, K, seed=2), _rand(M, N, seed=3)
+    out = base.clone()
+    cu._gemm(a, b, out=out, accumulate=accumulate)
+    want = a.float() @ b.float().t() + (base.float() if accumulate else 0.0)
+    torch.testing.assert_close(out.float(), want, atol=0.1 if accumulate else 1e-2, rtol=1.6e-2 if accumulate else 8e-3)   # one or two bf16 roundings
+    cu.check_status()
+
+
+@gpu
+@pytest.mark.parametrize("M,N,K", [(40000, 576, 128), (40000, 64, 128), (128 * 16, 192, 128)])
+@pytest.mark.parametrize("accumulate", [False, True])
+def test_fp8_gemm_epilogue_with_odd_slabs(M, N, K, accumulate):
+    from vlm_training_b200.ops import cuda as cu
+    from vlm_training_b200.ops.float8 import E4M3
+
+    a8, _, ra = cu._C.fp8_quantize(_rand(M, K, seed=1), E4M3, True, False)
+    b8, _, rb = cu._C.fp8_quantize(_rand(N, K, seed=2), E4M3, True, False)
+    base = _rand(M, N, seed=3)
+    out = base.clone()
+    cu._C.gemm_fp8(a8, b8, out, ra, rb, E4M3, E4M3, accumulate)
+    f8 = torch.float8_e4m3fn
+    want = (a8.view(f8).float() @ b8.view(f8).float().t()) * (ra[1] * rb[1]) + (base.float() if accumulate else 0.0)
+    torch.testing.assert_close(out.float(), want, atol=0.1 if accumulate else 2e-2, rtol=1.6e-2 if accumulate else 8e-3)
+    cu.check_status()

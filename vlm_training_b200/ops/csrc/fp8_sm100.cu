@@ -262,6 +262,7 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
     const int q = warp & 3;  // TMEM lane quarter this warp may read
     const float scale = p.rec_a[1] * p.rec_b[1];
     int it = 0;
+    uint32_t slab = 0;   // runs across items (see gemm_sm100.cu)
     bool ok = true;
     for (int item = blockIdx.x; item < num_items && ok; item += gridDim.x, ++it) {
       const int tile = item % num_tiles;
@@ -278,7 +279,7 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
       for (int c = 0; c < BN / 64; ++c) {
         const int col0 = n0 + c * 64;
         if (col0 >= p.N) break;
-        uint8_t* buf = stage + (c & 1) * 4096;
+        uint8_t* buf = stage + (slab++ & 1) * 4096;
         if (lane == 0) tma_store_wait_read<1>();  // the store issued two slabs ago has finished reading this buffer
         __syncwarp();
 #pragma unroll

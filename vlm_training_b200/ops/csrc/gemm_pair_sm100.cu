@@ -178,6 +178,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
     const float alpha = FP8 ? p.rec_a[1] * p.rec_b[1] : p.alpha != nullptr ? __ldg(p.alpha) : 1.f;
     uint8_t* out = smem + kOutOffset + q * 8192;
     int it = 0;
+    uint32_t slab = 0;   // runs across items (see gemm_sm100.cu)
     for (int item = pair; item < num_items; item += pairs, ++it) {
       const int tile = p.k_splits > 1 ? item % num_tiles : item;
       int tm, tn;
@@ -191,8 +192,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
       for (int c = 0; c < BN / 64; ++c) {
         const int col0 = n0 + c * 64;
         if (col0 >= p.N || row0 >= p.M) break;
-        uint8_t* buf = out + (c & 1) * 4096;
-        if (lane == 0) tma_store_wait_read<1>();
+        uint8_t* buf = out + (slab++ & 1) * 4096;
+        if (lane == 0) tma_store_wait_read<1>();   // the store issued two slabs ago has finished reading this buffer
         __syncwarp();
 #pragma unroll
         for (int h = 0; h < 2; ++h) {

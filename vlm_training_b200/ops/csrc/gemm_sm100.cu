@@ -475,6 +475,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
     const int q = warp & 3;  // TMEM lane quarter this warp may read
     const float alpha = p.alpha != nullptr ? __ldg(p.alpha) : 1.f;
     int it = 0;
+    uint32_t slab = 0;   // runs across items: a tile may have an odd number of slabs, and its last store may still be reading its buffer
     bool ok = true;
     for (int item = blockIdx.x; item < num_items && ok; item += gridDim.x, ++it) {
       const int tile = p.cluster > 1 ? item / p.cluster : p.k_splits > 1 ? item % num_tiles : item;
@@ -517,7 +518,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
         for (int c = 0; c < BN / 64; ++c) {
           const int col0 = n0 + c * 64;
           if (col0 >= p.N || (empty_group && p.accumulate)) break;
-          uint8_t* buf = stage + (c & 1) * 4096;
+          uint8_t* buf = stage + (slab++ & 1) * 4096;
           if (lane == 0) tma_store_wait_read<1>();  // the store issued two slabs ago has finished reading this buffer
           __syncwarp();
 #pragma unroll
