@@ -135,3 +135,43 @@ def test_fp8_gemm_epilogue_with_odd_slabs(M, N, K, accumulate):
     want = (a8.view(f8).float() @ b8.view(f8).float().t()) * (ra[1] * rb[1]) + (base.float() if accumulate else 0.0)
     torch.testing.assert_close(out.float(), want, atol=0.1 if accumulate else 2e-2, rtol=1.6e-2 if accumulate else 8e-3)
     cu.check_status()
+
+
+# weight gradients with few tiles and a long K, which may be cut over K: the head of the smallest presets with a full row, and two in between
+@gpu
+@pytest.mark.parametrize("V,H,T", [(8192, 512, 8192), (32000, 256, 4096), (1024, 256, 4100), (9, 64, 64)])
+def test_loss_adds_its_weight_gradient_with_one_rounding(V, H, T):
+    """In a tagged ``.grad`` (fp32 sums, rounded once, added once): bit for bit the gradient that autograd gets without a tag; an earlier
+    micro-batch in the buffer stays; the callback fires once per pass and autograd adds nothing."""
+    V = (V + 7) // 8 * 8
+    tgt = (torch.arange(T) * 13 % V).to(DEV)
+    tgt[::5] = -100
+
+    def grads(w, seed, scale):
+        h = _rand(T, H, scale=0.5, seed=seed).requires_grad_()
+        loss, n = ops.linear_cross_entropy(h, w, tgt, 1000, grad_in_place=True)
+        (loss * (scale / n)).backward()
+        return h
+
+    plain = torch.nn.Parameter(_rand(V, H, scale=0.05, seed=3))
+    parts = []
+    for seed, scale in ((1, 1.0), (2, 1.7)):
+        plain.grad = None
+        h = grads(plain, seed, scale)
+        parts.append((plain.grad.clone(), h.grad))
+    tagged = torch.nn.Parameter(plain.detach().clone())
+    seen = []
+    tagged.grad = torch.zeros_like(tagged)
+    tagged._vlmt_grad_in_place, tagged._vlmt_grad_ready = True, lambda p: seen.append(id(p))
+    assert torch.equal(grads(tagged, 1, 1.0).grad, parts[0][1])
+    assert torch.equal(tagged.grad, parts[0][0])
+    assert torch.equal(grads(tagged, 2, 1.7).grad, parts[1][1])
+    # the second sum is rounded to bf16 and added, or (split over a cluster) added in fp32: the forms differ by the rounding of the second
+    # part (2^-9 of it) and of the total in each form (2^-9 each)
+    total = parts[0][0].float() + parts[1][0].float()
+    assert bool(((tagged.grad.float() - total).abs() <= 2.0 ** -8 * (parts[1][0].float().abs() + total.abs())).all())
+    assert seen == [id(tagged)] * 2
+    # against 32 bits: bf16 logits and d(logits) (2^-8 each), one rounding of the sum
+    hr, wr = _rand(T, H, scale=0.5, seed=1).float(), plain.detach().float().requires_grad_()
+    torch.nn.functional.cross_entropy((hr @ wr.t()).to(torch.bfloat16).float(), tgt, ignore_index=-100).backward()
+    assert float((parts[0][0].float() - wr.grad).norm() / wr.grad.norm()) < 1e-2

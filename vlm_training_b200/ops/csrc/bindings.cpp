@@ -42,7 +42,7 @@ static Tensor status_tensor() {
 // ------------------------------------------------------------------ GEMM
 // out[M,N] (+)= a * b^T (see gemm_sm100.h for the layout flags)
 void gemm(const Tensor& a, const Tensor& b, Tensor& out, bool a_mn, bool b_mn, const c10::optional<Tensor>& bias, int64_t epilogue,
-          bool accumulate, const c10::optional<Tensor>& alpha) {
+          bool accumulate, const c10::optional<Tensor>& alpha, bool one_sum) {
   check_bf16(a, "a"); check_bf16(b, "b");
   TORCH_CHECK(a.dim() == 2 && b.dim() == 2 && out.dim() == 2);
   TORCH_CHECK(a.stride(1) == 1 && b.stride(1) == 1 && out.stride(1) == 1, "innermost strides must be 1");
@@ -64,7 +64,8 @@ void gemm(const Tensor& a, const Tensor& b, Tensor& out, bool a_mn, bool b_mn, c
   }
   Tensor st = status_tensor();
   int r = vlmt_gemm_bf16(a.data_ptr(), b.data_ptr(), d_bf16, d_f32, optptr(bias), M, N, K, (int)a.stride(0), (int)b.stride(0),
-                         (int)out.stride(0), a_mn, b_mn, (int)epilogue, accumulate, alpha_p, st.data_ptr<int>(), num_sms(), cur_stream());
+                         (int)out.stride(0), a_mn, b_mn, (int)epilogue, accumulate, alpha_p, one_sum, st.data_ptr<int>(), num_sms(),
+                         cur_stream());
   TORCH_CHECK(r == 0, "vlmt_gemm_bf16 failed with code ", r);
 }
 
@@ -549,7 +550,7 @@ namespace py = pybind11;
 PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   using namespace vlmt;
   m.def("gemm", &gemm, py::arg("a"), py::arg("b"), py::arg("out"), py::arg("a_mn"), py::arg("b_mn"), py::arg("bias"), py::arg("epilogue"),
-        py::arg("accumulate"), py::arg("alpha") = py::none());
+        py::arg("accumulate"), py::arg("alpha") = py::none(), py::arg("one_sum") = false);
   m.def("memset_zero_", [](Tensor& t) {
     TORCH_CHECK(t.is_cuda() && t.is_contiguous(), "memset_zero_: a contiguous CUDA tensor is required");
     c10::cuda::CUDAGuard guard(t.device());

@@ -783,6 +783,7 @@ namespace {
 // Everything one launch needs besides the plain GEMM arguments; passed explicitly down to the launcher.
 struct GemmExtras {
   const float* alpha = nullptr;   // device scalar factor of the product
+  bool one_sum = false;           // no parts of K added to a bf16 D one by one
   // GEMM -> reduce-scatter: output rows owned by rank o (blocks of rs_rows) are stored into rs_dst[o]
   int rs_world = 0, rs_rows = 0;
   void* const* rs_dst = nullptr;
@@ -958,7 +959,7 @@ int gemm_launch(const void* A, const void* B, void* D, float* Dacc32, const void
   p.alpha = x.alpha;
   p.epilogue = epilogue; p.accumulate = accumulate; p.status = status;
   p.k_splits = p.cluster = plan.splits; p.kb_per_split = plan.kb_per;
-  if (plan.splits == 1 && accumulate && p.tma_store && x.grp_mode == 0 && x.rs_world == 0 && x.ag_world == 0 && bias == nullptr && epilogue == GEMM_EPI_NONE &&
+  if (plan.splits == 1 && accumulate && !x.one_sum && p.tma_store && x.grp_mode == 0 && x.rs_world == 0 && x.ag_world == 0 && bias == nullptr && epilogue == GEMM_EPI_NONE &&
       Dacc32 == nullptr && split_k_enabled()) {
     // few output tiles and a long K: cut K so that the work items fill whole waves of SMs (at least 1024 of K per part)
     const long tiles = (long)((M + BM - 1) / BM) * ((N + (bn256 ? 256 : 128) - 1) / (bn256 ? 256 : 128));
@@ -1027,9 +1028,9 @@ int gemm_launch(const void* A, const void* B, void* D, float* Dacc32, const void
 
 extern "C" int vlmt_gemm_bf16(const void* A, const void* B, void* D, float* Dacc32, const void* bias, int M, int N, int K,
                               int lda, int ldb, int ldd, int a_mn_major, int b_mn_major, int epilogue, int accumulate,
-                              const float* alpha, int* status, int num_sms, cudaStream_t stream) {
+                              const float* alpha, int one_sum, int* status, int num_sms, cudaStream_t stream) {
   GemmExtras x;
-  x.alpha = alpha;
+  x.alpha = alpha; x.one_sum = one_sum;
   return gemm_launch(A, B, D, Dacc32, bias, M, N, K, lda, ldb, ldd, a_mn_major, b_mn_major, epilogue, accumulate, x, status, num_sms,
                      stream);
 }

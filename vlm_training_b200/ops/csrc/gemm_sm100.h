@@ -13,10 +13,11 @@ extern "C" {
 // b_mn_major: B is stored [K, N];                    else [N, K].
 // Dacc32 != null: write/accumulate fp32 results there instead of bf16 D.
 // alpha != null: device scalar that multiplies the product (before bias, activation and the addition to D).
+// one_sum: all of K in one fp32 sum, rounded once, whatever `accumulate` says (else a long K may be added to a bf16 D in parts).
 // Returns 0 or a CUDA / encode error code; device-side timeouts land in *status.
 int vlmt_gemm_bf16(const void* A, const void* B, void* D, float* Dacc32, const void* bias, int M, int N, int K, int lda,
-                   int ldb, int ldd, int a_mn_major, int b_mn_major, int epilogue, int accumulate, const float* alpha, int* status,
-                   int num_sms, cudaStream_t stream);
+                   int ldb, int ldd, int a_mn_major, int b_mn_major, int epilogue, int accumulate, const float* alpha, int one_sum,
+                   int* status, int num_sms, cudaStream_t stream);
 // Same GEMM (A K-major; B K-major or MN-major) whose output rows go to `world` destinations: rows owned by rank o
 // (blocks of rows_per_rank, a multiple of 128) are stored into dst[o], typically peer memory.
 int vlmt_gemm_bf16_rs_push(const void* A, const void* B, void* const* dst, int world, int rows_per_rank, int M, int N, int K, int lda,

@@ -92,8 +92,10 @@ def validate_row_indices(cu_seqlens, n_tokens: int, image_rows=None, experts=Non
 
 
 # ------------------------------------------------------------------------------- GEMM
-def _gemm(a, b, a_mn=False, b_mn=False, bias=None, epilogue=0, out=None, accumulate=False, out_dtype=torch.bfloat16, alpha=None):
-    """``out (+)= alpha * op(a) op(b)^T``; ``alpha``: one fp32 value on the device."""
+def _gemm(a, b, a_mn=False, b_mn=False, bias=None, epilogue=0, out=None, accumulate=False, out_dtype=torch.bfloat16, alpha=None,
+          one_sum=False):
+    """``out (+)= alpha * op(a) op(b)^T``; ``alpha``: one fp32 value on the device.  ``one_sum``: the sum over K is rounded once; else
+    an accumulated product with few output tiles and a long K may be added to a bf16 ``out`` in parts."""
     M = a.shape[1] if a_mn else a.shape[0]
     N = b.shape[1] if b_mn else b.shape[0]
     if out is None:
@@ -110,7 +112,7 @@ def _gemm(a, b, a_mn=False, b_mn=False, bias=None, epilogue=0, out=None, accumul
     if b.untyped_storage().size() == 0 or out.untyped_storage().size() == 0:
         # a sharded parameter (or its gradient bucket) whose storage is released: an error here, never a kernel on freed memory
         raise RuntimeError("GEMM operand without storage: a sharded parameter was used outside the forward / backward of its unit")
-    _C.gemm(a, b, out, a_mn, b_mn, bias, epilogue, accumulate, alpha)
+    _C.gemm(a, b, out, a_mn, b_mn, bias, epilogue, accumulate, alpha, one_sum)
     _tick()
     return out
 
@@ -153,7 +155,7 @@ def _report(param):
         ready(param)
 
 
-def _wgrad(dy2, x2, param=None, alpha=None, report=True):
+def _wgrad(dy2, x2, param=None, alpha=None, report=True, one_sum=False):
     """dW[N,K] = dY^T[N,M] . X[M,K].  For a tagged parameter the GEMM adds the product into ``param.grad`` from its
     epilogue (TMA reduce-add) and autograd gets ``None``: no separate accumulation pass over the gradient, no temporary.
     ``report=False``: kernels that read the parameter are still to come; the caller reports it behind them if it gets ``None``."""
@@ -161,7 +163,7 @@ def _wgrad(dy2, x2, param=None, alpha=None, report=True):
         g = param.grad
         if (g is not None and g.dtype == torch.bfloat16 and g.dim() == 2 and g.shape == (dy2.shape[1], x2.shape[1])
                 and g.stride(1) == 1 and g.stride(0) % 8 == 0 and g.data_ptr() % 16 == 0):
-            _gemm(dy2, x2, a_mn=True, b_mn=True, out=g, accumulate=True, alpha=alpha)
+            _gemm(dy2, x2, a_mn=True, b_mn=True, out=g, accumulate=True, alpha=alpha, one_sum=one_sum)
             if report:
                 _report(param)
             return None
@@ -499,7 +501,8 @@ class _LinearCrossEntropy(torch.autograd.Function):
         if ctx.keep_logits:
             dl, hidden, weight = ctx.saved_tensors
             alpha = g_loss.float()
-            dw = _wgrad(dl, hidden, ctx.w_param, alpha=alpha, report=False) if hidden is not None else None   # dW = alpha dL^T . H
+            # dW = alpha dL^T . H, summed over all rows in fp32 as the chunk by chunk form does
+            dw = _wgrad(dl, hidden, ctx.w_param, alpha=alpha, report=False, one_sum=True) if hidden is not None else None
             dh = _gemm(dl, weight, b_mn=True, alpha=alpha) if weight is not None else None       # dH = alpha dL . W
             if hidden is not None and dw is None:
                 _report(ctx.w_param)
