@@ -175,3 +175,21 @@ def test_loss_adds_its_weight_gradient_with_one_rounding(V, H, T):
     hr, wr = _rand(T, H, scale=0.5, seed=1).float(), plain.detach().float().requires_grad_()
     torch.nn.functional.cross_entropy((hr @ wr.t()).to(torch.bfloat16).float(), tgt, ignore_index=-100).backward()
     assert float((parts[0][0].float() - wr.grad).norm() / wr.grad.norm()) < 1e-2
+
+
+@gpu
+def test_loss_with_a_frozen_head_keeps_nothing_of_vocabulary_size():
+    T, H, V = 2048, 1024, 32768
+    w, tgt = _rand(V, H, scale=0.05, seed=3), (torch.arange(T) * 13 % V).to(DEV)
+    grads = []
+    for frozen in (False, True):
+        h = _rand(T, H, scale=0.5, seed=1).requires_grad_()
+        w.requires_grad_(not frozen)
+        torch.cuda.synchronize()
+        before = torch.cuda.memory_allocated()
+        loss, _ = ops.linear_cross_entropy(h, w, tgt, 512)
+        held = torch.cuda.memory_allocated() - before
+        loss.backward()
+        grads.append(h.grad)
+    assert held <= 2 * T * H + (1 << 20)   # the hidden state's gradient
+    torch.testing.assert_close(grads[0].float(), grads[1].float(), atol=1e-4, rtol=1.6e-2)   # chunks of rows may sum K in another order

@@ -455,8 +455,8 @@ class _LinearCrossEntropy(torch.autograd.Function):
     gradient summed over the chunks ``4 V H``.  While the former is the smaller one (T up to 2 H) it is what is kept, and
     backward runs ONE product per gradient over all rows, scaled by the upstream gradient in the GEMM's epilogue: the weight
     gradient goes straight into ``.grad`` with a single rounding, without the fp32 buffer's fill, its read-modify-write per
-    chunk, and the passes that scale, convert and add it (T = 8192, V = 151936, H = 4096: 4 ms of 27).  Longer rows
-    form both gradients chunk by chunk in the forward pass, so nothing of size T x V ever exists."""
+    chunk, and the passes that scale, convert and add it (T = 8192, V = 151936, H = 4096: 4 ms of 27).  Longer rows, and a
+    weight without a gradient, form what is needed chunk by chunk in the forward pass, so nothing of size T x V ever exists."""
 
     @staticmethod
     def forward(ctx, hidden, weight, targets, chunk, ignore_index, grad_scale, w_param):
@@ -468,7 +468,7 @@ class _LinearCrossEntropy(torch.autograd.Function):
         losses = torch.empty(T, dtype=torch.float32, device=hidden.device)
         targets = targets.contiguous()
         ctx.w_dtype, ctx.w_param = weight.dtype, w_param
-        ctx.keep_logits = 2 * T * V <= max(4 * V * H, _KEEP_LOGITS_BYTES)
+        ctx.keep_logits = need_dw and 2 * T * V <= max(4 * V * H, _KEEP_LOGITS_BYTES)
         n_valid = (targets != ignore_index).sum()
         ctx.mark_non_differentiable(n_valid)
         if ctx.keep_logits:
@@ -478,7 +478,7 @@ class _LinearCrossEntropy(torch.autograd.Function):
                 _gemm(hidden[s:e], weight_c, out=dl[s:e])
                 losses[s:e] = _C.ce_fwd_bwd_(dl[s:e], targets[s:e], grad_scale, ignore_index)
                 _tick()
-            ctx.save_for_backward(dl, hidden if need_dw else None, weight_c if need_dh else None)
+            ctx.save_for_backward(dl, hidden, weight_c if need_dh else None)
             return losses.sum(), n_valid
         dh = torch.empty_like(hidden) if need_dh else None
         dw = torch.zeros(V, H, dtype=torch.float32, device=hidden.device) if need_dw else None
@@ -502,9 +502,9 @@ class _LinearCrossEntropy(torch.autograd.Function):
             dl, hidden, weight = ctx.saved_tensors
             alpha = g_loss.float()
             # dW = alpha dL^T . H, summed over all rows in fp32 as the chunk by chunk form does
-            dw = _wgrad(dl, hidden, ctx.w_param, alpha=alpha, report=False, one_sum=True) if hidden is not None else None
+            dw = _wgrad(dl, hidden, ctx.w_param, alpha=alpha, report=False, one_sum=True)
             dh = _gemm(dl, weight, b_mn=True, alpha=alpha) if weight is not None else None       # dH = alpha dL . W
-            if hidden is not None and dw is None:
+            if dw is None:
                 _report(ctx.w_param)
             return dh, dw, None, None, None, None, None
         dh, dw = ctx.saved_tensors
