@@ -193,3 +193,26 @@ def test_loss_with_a_frozen_head_keeps_nothing_of_vocabulary_size():
         grads.append(h.grad)
     assert held <= 2 * T * H + (1 << 20)   # the hidden state's gradient
     torch.testing.assert_close(grads[0].float(), grads[1].float(), atol=1e-4, rtol=1.6e-2)   # chunks of rows may sum K in another order
+
+
+@gpu
+def test_rotary_tables_of_every_accepted_form_of_positions():
+    """Four rows of positions (text and three axes), a single row, a batch dimension, and frequencies that are learned."""
+    from vlm_training_b200.ops import reference as ref
+
+    section, T = [24, 20, 20], 50
+    inv = 1.0 / (1e6 ** (torch.arange(0, 128, 2, device=DEV).float() / 128))
+    pos = torch.randint(0, 4000, (4, T), generator=torch.Generator().manual_seed(0)).to(DEV)
+    for rows in (pos[:3], pos, pos.t().contiguous().t()[:3]):
+        want = ref.mrope_cos_sin(rows, inv, section)
+        assert all(torch.equal(a, b) for a, b in zip(ops.rope_tables(rows, inv, section), want))
+    f = pos[:1][0].float().unsqueeze(-1) * inv
+    want = (torch.cat((f, f), -1).cos(), torch.cat((f, f), -1).sin())
+    for rows in (pos[:1], pos[:3], pos):
+        assert all(torch.equal(a, b) for a, b in zip(ops.rope_tables(rows, inv), want))
+    batch = pos.view(1, 4, T)
+    assert all(torch.equal(a[0], b) for a, b in zip(ops.rope_tables(batch, inv), want))
+    learned = inv.clone().requires_grad_()
+    cos, _ = ops.rope_tables(pos[:1], learned)
+    cos.sum().backward()
+    assert learned.grad is not None and bool(learned.grad.abs().sum() > 0)

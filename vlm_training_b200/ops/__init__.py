@@ -265,10 +265,14 @@ def vision_plan(images, trig, freqs: int, side: int, merge: int, n: int):
 
 def rope_tables(position_ids, inv_freq, mrope_section=None):
     """fp32 cos / sin ``[T, R]`` from ``position_ids`` (``[3, T]`` interleaved multi-axis or ``[1, T]``)."""
-    if _use_cuda(position_ids) and position_ids.dtype == torch.int64:   # the kernel's type; others take the general form
+    # what the kernel takes: int64 [1 or 3, T] (without sections any number of rows, the first counts), frequencies without a gradient
+    if (_use_cuda(position_ids) and position_ids.dtype == torch.int64 and position_ids.dim() == 2
+            and (mrope_section is None or position_ids.shape[0] in (1, 3))
+            and inv_freq.dim() == 1 and not (torch.is_grad_enabled() and inv_freq.requires_grad)):
         return _cu().rope_tables(position_ids, inv_freq, mrope_section)
     if mrope_section is not None:
-        return ref.mrope_cos_sin(position_ids.expand(3, -1), inv_freq, mrope_section, torch.float32)
+        pos = position_ids.expand(3, *position_ids.shape[1:]) if position_ids.shape[0] == 1 else position_ids
+        return ref.mrope_cos_sin(pos, inv_freq, mrope_section, torch.float32)
     f = position_ids[0].float().unsqueeze(-1) * inv_freq.float()
     emb = torch.cat((f, f), -1)
     return emb.cos(), emb.sin()

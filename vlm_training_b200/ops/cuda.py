@@ -653,7 +653,7 @@ def vision_plan(images, trig, freqs, side, merge, n):
 
 def rope_tables(position_ids, inv_freq, mrope_section=None):
     sec = mrope_section if mrope_section is not None else (0, 0, 0)
-    pos = position_ids if position_ids.shape[0] in (1, 3) and mrope_section is not None else position_ids[:1]
+    pos = position_ids if mrope_section is not None else position_ids[:1]
     return _C.rope_tables(pos.contiguous(), _f32(inv_freq), int(sec[1]), int(sec[2]))
 
 
