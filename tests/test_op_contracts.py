@@ -216,3 +216,30 @@ def test_rotary_tables_of_every_accepted_form_of_positions():
     cos, _ = ops.rope_tables(pos[:1], learned)
     cos.sum().backward()
     assert learned.grad is not None and bool(learned.grad.abs().sum() > 0)
+
+
+# a table with rows behind the last square or of a larger square, a transposed one, an index table with a gap
+@gpu
+@pytest.mark.parametrize("form", ["longer", "larger", "strided", "index"])
+def test_position_embedding_forms_outside_the_kernel(form):
+    import dataclasses
+
+    from vlm_training_b200.models.config import VisionConfig
+    from vlm_training_b200.models.vision import VisionPlan
+
+    cfg = VisionConfig(hidden_size=64, num_heads=2, num_position_embeddings=2310, spatial_merge_size=2)
+    plan = VisionPlan.build([[1, 4, 6], [1, 8, 2]], cfg, DEV)
+    x = _rand(40, 64, seed=1)
+    table = _rand({"longer": 2310, "larger": 2500}.get(form, 2304), 64, seed=2)
+    if form == "strided":
+        table = table.t().contiguous().t()
+    if form == "index":
+        plan = dataclasses.replace(plan, pe_index=plan.pe_index.t().contiguous().t())
+    got, want = [], []
+    for out, p in ((got, plan), (want, dataclasses.replace(plan, images=None))):
+        t = table.detach().clone(memory_format=torch.preserve_format).requires_grad_()
+        y = ops.pos_embed_add(x, t, p, 2)
+        y.backward(torch.ones_like(y))
+        out += [y, t.grad]
+    assert torch.equal(got[0], want[0])
+    torch.testing.assert_close(got[1].float(), want[1].float(), atol=2e-2, rtol=1.6e-2)

@@ -32,6 +32,7 @@ class VisionPlan:
     pe_index: torch.Tensor  # int64 [4, N]
     pe_weight: torch.Tensor  # fp32 [4, N]
     images: torch.Tensor | None = None  # GPU: int32 [n_img, 4], frames / height / width / first patch of every image
+    side: int = 0  # GPU: rows (and columns) of the position table the plan was built for
 
     @staticmethod
     def build(grids, cfg: VisionConfig, device) -> "VisionPlan":
@@ -53,7 +54,7 @@ class VisionPlan:
             images = small[:4 * len(g)].view(-1, 4)
             side = int(round(cfg.num_position_embeddings ** 0.5))
             cos, sin, idx, wt = ops.vision_plan(images, both[:trig.size].view(torch.float32), trig.shape[1], side, merge, int(first[-1]))
-            return VisionPlan(small[4 * len(g):], mx, cos, sin, idx, wt, images)
+            return VisionPlan(small[4 * len(g):], mx, cos, sin, idx, wt, images, side)
         coords = positions.vision_rot_coords(grids, cfg.spatial_merge_size)
         half = cfg.head_dim // 2
         fr = coords[:, :, None].astype(np.float32) * _inv_freq(half)[None, None, :]  # [N, 2, half/2]

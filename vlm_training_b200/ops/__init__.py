@@ -280,11 +280,16 @@ def rope_tables(position_ids, inv_freq, mrope_section=None):
 
 def pos_embed_add(x, table, plan, merge: int):
     """``x + sum_c plan.pe_weight[c] * table[plan.pe_index[c]]`` (the vision tower's resampled position embedding)."""
-    if _use_cuda(x) and plan.images is not None and x.dtype == torch.bfloat16 and x.shape[1] % 8 == 0 and table.dtype == torch.bfloat16 \
-            and x.data_ptr() % 16 == 0 and table.data_ptr() % 16 == 0:   # 16-byte loads
+    index, weight = plan.pe_index, plan.pe_weight
+    # what the kernels take: bf16 rows read 16 bytes at a time, the square table that the plan was built for, one row of x per patch
+    if (_use_cuda(x) and plan.images is not None and x.dtype == torch.bfloat16 and table.dtype == torch.bfloat16 and x.dim() == 2
+            and x.shape[1] % 8 == 0 and x.shape[1] == table.shape[1] and x.shape[0] == index.shape[1] and table.is_contiguous()
+            and table.shape[0] == plan.side ** 2 and index.is_contiguous() and weight.is_contiguous()
+            and index.dtype == torch.int64 and weight.dtype == torch.float32 and not weight.requires_grad
+            and x.data_ptr() % 16 == 0 and table.data_ptr() % 16 == 0):
         return _cu().pos_embed_add(x, table, plan, merge)
-    pe = table[plan.pe_index]  # [4, N, hidden]
-    return x + (pe.float() * plan.pe_weight.unsqueeze(-1)).sum(0).to(x.dtype)
+    pe = table[index]  # [4, N, hidden]
+    return x + (pe.float() * weight.unsqueeze(-1)).sum(0).to(x.dtype)
 
 
 def embedding(ids, weight):

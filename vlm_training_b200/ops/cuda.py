@@ -658,7 +658,7 @@ def rope_tables(position_ids, inv_freq, mrope_section=None):
 
 
 def pos_embed_add(x, table, plan, merge):
-    return _C.op_pos_embed(x, table, plan.pe_index, plan.pe_weight, plan.images, int(round(table.shape[0] ** 0.5)), merge)
+    return _C.op_pos_embed(x, table, plan.pe_index, plan.pe_weight, plan.images, plan.side, merge)
 
 
 # ------------------------------------------------------------------------------- optimizer
