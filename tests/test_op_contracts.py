@@ -243,3 +243,23 @@ def test_position_embedding_forms_outside_the_kernel(form):
         out += [y, t.grad]
     assert torch.equal(got[0], want[0])
     torch.testing.assert_close(got[1].float(), want[1].float(), atol=2e-2, rtol=1.6e-2)
+
+
+def _sparse_inputs(lens, Hq=8, Hkv=1, D=256, seed=0):
+    T = sum(lens)
+    q, k, v = (_rand(T, h, D, seed=seed + i) for i, h in enumerate((Hq, Hkv, Hkv)))
+    index = [_rand(T, 4, 64, seed=seed + 3), _rand(T, 64, seed=seed + 4), _rand(T, 4, seed=seed + 5)]
+    return q, k, v, index, [0] + torch.tensor(lens).cumsum(0).tolist()
+
+
+# documents up to 16 times the selected keys (masked) and beyond (gathered); boundaries on the host, as 64-bit values, with a gap between them, absent
+@gpu
+@pytest.mark.parametrize("lens", [[300, 40], [2200]])
+@pytest.mark.parametrize("form", ["host", "int64", "gap", "absent"])
+def test_sparse_attention_takes_boundaries_of_any_form(lens, form):
+    topk = 64 if len(lens) > 1 else 128
+    q, k, v, index, bounds = _sparse_inputs(lens)
+    cu = torch.tensor(bounds, dtype=torch.int32, device=DEV)
+    want = ops.dsa_attention(q, k, v, *index, cu, topk, None, bounds)
+    other = {"host": cu.cpu(), "int64": cu.long(), "gap": torch.stack((cu, cu), 1)[:, 0], "absent": None}[form]
+    assert torch.equal(ops.dsa_attention(q, k, v, *index, other, topk, None, bounds), want)

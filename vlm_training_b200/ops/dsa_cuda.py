@@ -107,6 +107,14 @@ def _native_indexer(idx_q, idx_k) -> bool:
             and idx_q.shape[1:] == (4, 64) and idx_k.shape[-1] == 64 and os.environ.get("VLMT_DSA_INDEXER", "1") != "0")
 
 
+def _device_bounds(cu_seqlens, bounds, device):
+    """The boundaries as the kernels read them; ``cu_seqlens`` may be on the host, of another type or layout, or absent beside the
+    host copy ``bounds``."""
+    if torch.is_tensor(cu_seqlens) and cu_seqlens.device == device and cu_seqlens.numel() == len(bounds):
+        return cu_seqlens.reshape(-1).to(torch.int32).contiguous()
+    return torch.tensor(bounds, dtype=torch.int32).to(device, non_blocking=True)
+
+
 def dsa_attention_cuda(q, k, v, idx_q, idx_k, idx_w, cu_seqlens, topk, scale=None, cu_host=None):
     """``cu_host``: the document boundaries as a host sequence (saves the device read of ``cu_seqlens``)."""
     T, Hq, D = q.shape
@@ -126,7 +134,7 @@ def dsa_attention_cuda(q, k, v, idx_q, idx_k, idx_w, cu_seqlens, topk, scale=Non
         bits = cu._C.dsa_select_bits(iq_c, ik_c, iw_c, bounds, int(topk))
         cu._tick(2 * sum((b - a + _QBLOCK - 1) // _QBLOCK for a, b in zip(bounds[:-1], bounds[1:]) if b - a > topk))
         n = bounds[-1]   # documents end where the packed row ends: tokens behind the last boundary are padding
-        o = _MaskedAttention.apply(q[:n], k[:n], v[:n], cu_seqlens.to(torch.int32), bits[:, :n].contiguous() if n < T else bits, int(topk), float(scale))
+        o = _MaskedAttention.apply(q[:n], k[:n], v[:n], _device_bounds(cu_seqlens, bounds, q.device), bits[:, :n].contiguous() if n < T else bits, int(topk), float(scale))
         return o if n == T else torch.cat((o, q.new_zeros(T - n, Hq, D)), 0)
     # documents end where the packed row ends: tokens behind the last boundary are padding
     outs = []
