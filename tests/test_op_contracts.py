@@ -263,3 +263,20 @@ def test_sparse_attention_takes_boundaries_of_any_form(lens, form):
     want = ops.dsa_attention(q, k, v, *index, cu, topk, None, bounds)
     other = {"host": cu.cpu(), "int64": cu.long(), "gap": torch.stack((cu, cu), 1)[:, 0], "absent": None}[form]
     assert torch.equal(ops.dsa_attention(q, k, v, *index, other, topk, None, bounds), want)
+
+
+@gpu
+@pytest.mark.parametrize("scale", [-0.05, 0.0])
+def test_sparse_attention_with_a_scale_that_is_not_positive(scale):
+    """Against the float32 softmax over the same keys; tolerances: bf16 rounding of P and of the results."""
+    from vlm_training_b200.ops import cuda as cu
+
+    L, topk = 500, 32
+    q, k, v, index, bounds = _sparse_inputs([L], Hq=8, Hkv=1)
+    sel = cu._C.dsa_select(index[0], index[1], index[2].float(), 0, 0, 0, L, topk).long()
+    keep = torch.zeros(L, L + 1, dtype=torch.bool, device=DEV).scatter_(1, torch.where(sel < 0, L, sel), True)[:, :L]
+    o = ops.dsa_attention(q, k, v, *index, torch.tensor(bounds, dtype=torch.int32, device=DEV), topk, scale, bounds)
+    att = torch.einsum("qhd,kd->hqk", q.float(), k[:, 0].float()) * scale
+    want = torch.einsum("hqk,kd->qhd", att.masked_fill(~keep, float("-inf")).softmax(-1), v[:, 0].float())
+    torch.testing.assert_close(o.float(), want, atol=2e-2, rtol=2e-2)
+    cu.check_status()
