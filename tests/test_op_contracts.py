@@ -280,3 +280,26 @@ def test_sparse_attention_with_a_scale_that_is_not_positive(scale):
     want = torch.einsum("hqk,kd->qhd", att.masked_fill(~keep, float("-inf")).softmax(-1), v[:, 0].float())
     torch.testing.assert_close(o.float(), want, atol=2e-2, rtol=2e-2)
     cu.check_status()
+
+
+# masked (equal bit for bit) and gathered (key and value gradients are summed by atomics: fp32 order, one bf16 rounding)
+@gpu
+@pytest.mark.parametrize("topk", [64, 16])
+def test_sparse_attention_never_reads_padding(topk):
+    """Rows behind the last boundary may hold anything; their outputs and gradients are zero.  Inside a document every key and value
+    row has to be finite, selected or not, as the op says."""
+    q, k, v, index, bounds = _sparse_inputs([300, 70], Hq=8, Hkv=1)
+    results = []
+    for fill in (0.0, float("nan"), float("inf")):
+        leaves = []
+        for t in (q, k, v):
+            t = torch.cat((t, torch.full_like(t[:50], fill)), 0).requires_grad_()
+            leaves.append(t)
+        idx = [torch.cat((t, torch.full_like(t[:50], fill)), 0) for t in index]
+        o = ops.dsa_attention(*leaves, *idx, torch.tensor(bounds, dtype=torch.int32, device=DEV), topk, None, bounds)
+        o.backward(_rand(*o.shape, seed=9))
+        results.append([o] + [t.grad for t in leaves])
+    for other in results[1:]:
+        for a, b in zip(results[0], other):
+            torch.testing.assert_close(a, b, atol=0.0 if topk == 64 else 1e-2, rtol=0.0 if topk == 64 else 8e-3)
+    assert all(float(t[370:].abs().sum()) == 0.0 for t in results[0])

@@ -189,7 +189,11 @@ def attention_varlen(q, k, v, cu_seqlens, max_seqlen: int, causal: bool = True, 
 
 
 def dsa_attention(q, k, v, idx_q, idx_k, idx_w, cu_seqlens, topk: int, scale: float | None = None, cu_host=None):
-    """``cu_host``: the document boundaries as a host sequence, if the caller has them (no device read then)."""
+    """``cu_host``: the document boundaries as a host sequence, if the caller has them (no device read then).
+
+    Query, key and value rows inside the documents must be finite: on a GPU a key that a query does not select may still be multiplied
+    by an exact zero, so an infinity or NaN in such a row, or in a neighbouring document's, can make NaN.  Rows behind the last
+    boundary (padding) may hold anything: they are not read, and their outputs and gradients are zero."""
     if _use_cuda(q):
         return _cu().dsa_attention(q, k, v, idx_q, idx_k, idx_w, cu_seqlens, topk, scale, cu_host)
     return ref.dsa_attention(q, k, v, idx_q, idx_k, idx_w, cu_seqlens, topk, scale)
