@@ -53,7 +53,6 @@ _PARAM_OPS = {
     "experts": (lambda x, p: ops.moe_experts(x, p["gu"], p["dn"], torch.full((_T, 2), 0.5, device=DEV, dtype=torch.bfloat16),
                                              torch.stack((_ROWS % 4, (_ROWS + 1) % 4), 1).to(DEV)), dict(gu=(4, 256, _H), dn=(4, _H, 128)), _H),
 }
-_TAGGED = {name: shapes for name, (_, shapes, _) in _PARAM_OPS.items()}
 
 
 def _leaves(name, tag=None, grad=0.0, fp8=False, resharded=False):
@@ -303,3 +302,34 @@ def test_sparse_attention_never_reads_padding(topk):
         for a, b in zip(results[0], other):
             torch.testing.assert_close(a, b, atol=0.0 if topk == 64 else 1e-2, rtol=0.0 if topk == 64 else 8e-3)
     assert all(float(t[370:].abs().sum()) == 0.0 for t in results[0])
+
+
+@gpu
+@pytest.mark.parametrize("name,key,form", [(n, k, "") for n, (_, shapes, _) in _PARAM_OPS.items() for k in shapes] + [("linear", "w", "fp8"), ("norm_linear", "w", "resharded")])
+def test_user_hooks_and_partial_backward_passes_see_tagged_gradients(name, key, form):
+    """A parameter with a tensor hook gets its gradient through autograd; ``autograd.grad`` returns it and adds nothing;
+    ``backward(inputs=...)`` touches only what was asked for."""
+    kw = {form: True} if form else {}
+    x0, plain = _leaves(name, **kw)
+    _backward(name, x0, plain)
+    want = plain[key].grad
+    x1, tagged = _leaves(name, lambda p: None, **kw)
+    p = tagged[key]
+    handle = p.register_hook(lambda g: g * 2)
+    after = []
+    p.register_post_accumulate_grad_hook(lambda q: after.append(q.grad.clone()))
+    _backward(name, x1, tagged)
+    assert torch.equal(p.grad, want * 2)
+    assert len(after) == 1 and torch.equal(after[0], p.grad)
+    handle.remove()
+
+    x2, tagged = _leaves(name, lambda p: None, **kw)
+    out = _PARAM_OPS[name][0](x2, tagged)
+    outs = [o for o in (out if isinstance(out, tuple) else (out,)) if o is not None]
+    cot = [_rand(*o.shape, seed=30 + i, dtype=o.dtype) if o.dim() else torch.full_like(o, 1.7) for i, o in enumerate(outs)]
+    (got,) = torch.autograd.grad(outs, [tagged[key]], cot)
+    assert torch.equal(got, want) and float(tagged[key].grad.abs().sum()) == 0.0
+
+    x3, tagged = _leaves(name, lambda p: None, **kw)
+    _backward(name, x3, tagged, inputs=[x3])
+    assert torch.equal(x3.grad, x0.grad) and float(tagged[key].grad.abs().sum()) == 0.0

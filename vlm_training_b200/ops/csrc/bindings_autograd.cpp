@@ -8,8 +8,10 @@
 // Gradients of parameters whose `.grad` belongs to the optimizer engine (Python attribute `_vlmt_grad_in_place`) are added
 // there by the kernel that forms them: the weight-gradient GEMM's epilogue, or the kernel that sums a norm weight's or
 // bias's partial rows (one rounding, and no conversion, no autograd accumulation launch).  Autograd then gets nothing and the
-// engine's gradient-ready callback (`_vlmt_grad_ready`) is called here.
+// engine's gradient-ready callback (`_vlmt_grad_ready`) is called here.  A parameter with tensor hooks (`register_hook`), and every parameter
+// in a pass that was asked for particular gradients, takes the ordinary way through autograd.
 #include <torch/csrc/autograd/custom_function.h>
+#include <torch/csrc/autograd/graph_task.h>
 #include <torch/extension.h>
 
 #include <atomic>
@@ -67,6 +69,15 @@ Target target_of(const py::object& w) {
   if (ready != nullptr) { Py_INCREF(ready); t->ready = ready; }
   return t;
 }
+// Whether a gradient may be added to `.grad` behind autograd's back.  Not when somebody waits for it on the way: a tensor hook, or
+// `autograd.grad` / `backward(inputs=...)`, whose graph task knows which nodes it executes (`backward()` executes all and names
+// none).  Post-accumulate hooks run either way: autograd accumulates an undefined gradient and calls them.  Called in the backward pass.
+bool may_add(const Tensor& param) {
+  const auto* named = torch::autograd::get_current_graph_task_exec_info();
+  return (named == nullptr || named->empty()) && torch::autograd::impl::hooks(param).empty();
+}
+bool may_add(const Target& t) { return t && may_add(t->param); }
+
 Tensor as_tensor(const py::object& o) { return o.is_none() ? Tensor() : o.cast<Tensor>(); }
 OptTensor opt(const Tensor& t) { return t.defined() ? OptTensor(t) : OptTensor(); }
 Tensor get(const OptTensor& t) { return t.has_value() ? *t : Tensor(); }
@@ -94,7 +105,7 @@ Tensor mm(const Tensor& a, const Tensor& b, bool a_mn, bool b_mn, const Tensor& 
 // enqueued: its bucket's update may run on another stream, or in a peer's kernel, from that moment on.
 Tensor weight_grad(const Tensor& dy, const Tensor& x, const Target& t, bool& report) {
   report = false;
-  if (t) {
+  if (may_add(t)) {
     Tensor g = t->param.grad();
     if (g.defined() && g.scalar_type() == at::kBFloat16 && g.dim() == 2 && g.size(0) == dy.size(1) && g.size(1) == x.size(1) &&
         g.stride(1) == 1 && g.stride(0) % 8 == 0 && reinterpret_cast<uintptr_t>(g.data_ptr()) % 16 == 0) {
@@ -120,7 +131,7 @@ struct VecGrad {
   int mode;
   bool in_place = false, convert = false;
   VecGrad(const Tensor& w, const Target& t) {
-    if (t) {
+    if (may_add(t)) {
       out = t->param.grad();
       if (out.defined() && out.scalar_type() == at::kBFloat16 && out.is_contiguous() && out.numel() == w.numel()) {
         check_storage(out);
@@ -746,7 +757,7 @@ struct PosEmbed : torch::autograd::Function<PosEmbed> {
     if (reinterpret_cast<uintptr_t>(dy.data_ptr()) % 16) dy = dy.clone();
     if (c->need[1]) {
       const Tensor& table = saved[0];
-      Tensor g = c->t[0] ? c->t[0]->param.grad() : Tensor();
+      Tensor g = may_add(c->t[0]) ? c->t[0]->param.grad() : Tensor();
       const bool in_place = g.defined() && g.scalar_type() == at::kBFloat16 && g.is_contiguous() && g.sizes() == table.sizes() &&
                             reinterpret_cast<uintptr_t>(g.data_ptr()) % 16 == 0;
       if (in_place) check_storage(g);
@@ -828,5 +839,6 @@ void bind_autograd(py::module_& m) {
   m.def("rope_tables", &rope_tables);
   m.def("vision_plan", &vision_plan);
   m.def("op_launches", [] { return g_launches.load(); });
+  m.def("may_add_grad", [](const Tensor& param) { return may_add(param); });
   m.def("op_grad_in_place", [](bool on) { g_in_place = on; });
 }

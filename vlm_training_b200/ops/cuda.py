@@ -147,6 +147,12 @@ def _grad_target(w):
     return w if (_WGRAD_IN_PLACE and getattr(w, "_vlmt_grad_in_place", False)) else None
 
 
+def _may_add(param):
+    """Whether the gradient of a tagged parameter may be added to ``.grad`` behind autograd's back: no tensor hooks, and a pass that
+    was not asked for particular gradients.  Called in the backward pass."""
+    return _C.may_add_grad(param)
+
+
 def _report(param):
     """The engine's gradient-ready hook of a tagged parameter, called by hand because autograd has nothing to accumulate.  The update
     may run at once on another stream or in a peer's kernel: every kernel that reads the parameter must have been enqueued."""
@@ -159,7 +165,7 @@ def _wgrad(dy2, x2, param=None, alpha=None, report=True, one_sum=False):
     """dW[N,K] = dY^T[N,M] . X[M,K].  For a tagged parameter the GEMM adds the product into ``param.grad`` from its
     epilogue (TMA reduce-add) and autograd gets ``None``: no separate accumulation pass over the gradient, no temporary.
     ``report=False``: kernels that read the parameter are still to come; the caller reports it behind them if it gets ``None``."""
-    if param is not None:
+    if param is not None and _may_add(param):
         g = param.grad
         if (g is not None and g.dtype == torch.bfloat16 and g.dim() == 2 and g.shape == (dy2.shape[1], x2.shape[1])
                 and g.stride(1) == 1 and g.stride(0) % 8 == 0 and g.data_ptr() % 16 == 0):

@@ -118,7 +118,7 @@ class _LinearFp8(torch.autograd.Function):
             dx = dx.view(ctx.in_shape)
         if need_dw:
             param = ctx.w_param
-            g = param.grad if param is not None else None
+            g = param.grad if param is not None and cu._may_add(param) else None
             if (g is not None and g.dtype == torch.bfloat16 and g.dim() == 2 and tuple(g.shape) == ctx.w_shape and g.stride(1) == 1
                     and g.stride(0) % 8 == 0 and g.data_ptr() % 16 == 0):
                 # added into the optimizer's gradient bucket by the GEMM's epilogue; autograd has nothing to accumulate

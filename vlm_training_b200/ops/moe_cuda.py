@@ -49,7 +49,7 @@ class _GroupedLinear(torch.autograd.Function):
         if ctx.needs_input_grad[1]:
             # dW_e = dY_e^T X_e, added into `.grad` where that is a view of the optimizer engine's buffer (see `cu._wgrad`)
             param, g = ctx.w_param, None
-            if param is not None and param.grad is not None and param.grad.shape == w.shape and param.grad.dtype == torch.bfloat16 \
+            if param is not None and cu._may_add(param) and param.grad is not None and param.grad.shape == w.shape and param.grad.dtype == torch.bfloat16 \
                     and param.grad.is_contiguous() and param.grad.data_ptr() % 16 == 0:
                 g = param.grad.view(E * N, K)
             else:

@@ -174,8 +174,9 @@ class _Domain:
                 self.flat_param[o:o + n].copy_(p.detach().reshape(-1))
                 p.data = self.flat_param[o:o + n].view(p.shape)
                 p.grad = self.flat_grad[o:o + n].view(p.shape)
-                # weight-gradient GEMMs may add into this view directly (ops/cuda.py:_wgrad); valid because every
-                # such parameter enters exactly one linear per forward pass
+                # the kernels that form a gradient of a linear, norm, bias, position table or expert may add into this view directly
+                # (ops/cuda.py:_wgrad, csrc/bindings_autograd.cpp); valid because every such parameter enters exactly one op per
+                # forward pass.  Parameters with tensor hooks get their gradients through autograd.
                 p._vlmt_grad_in_place = True
         # ---- optimizer state on the local shard of every bucket
         self.master, self.exp_avg, self.exp_avg_sq = [], [], []
