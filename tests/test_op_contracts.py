@@ -333,3 +333,16 @@ def test_user_hooks_and_partial_backward_passes_see_tagged_gradients(name, key, 
     x3, tagged = _leaves(name, lambda p: None, **kw)
     _backward(name, x3, tagged, inputs=[x3])
     assert torch.equal(x3.grad, x0.grad) and float(tagged[key].grad.abs().sum()) == 0.0
+
+
+@gpu
+@pytest.mark.parametrize("grad", [True, False])
+@pytest.mark.parametrize("name", list(_PARAM_OPS))
+def test_forward_mode_tangents_are_refused(name, grad):
+    """The ops have no forward-mode derivative: a tangent is refused, never dropped, with and without gradients."""
+    import torch.autograd.forward_ad as fwad
+
+    x, params = _leaves(name)
+    with torch.set_grad_enabled(grad), fwad.dual_level():
+        with pytest.raises(RuntimeError):
+            _PARAM_OPS[name][0](fwad.make_dual(x.detach(), torch.ones_like(x)), params)

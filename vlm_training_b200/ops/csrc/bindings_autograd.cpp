@@ -185,7 +185,13 @@ using CfgPtr = c10::intrusive_ptr<Cfg>;
 void keep(AutogradContext* ctx, const CfgPtr& c) { ctx->saved_data["cfg"] = c10::IValue::make_capsule(c); }
 CfgPtr kept(AutogradContext* ctx) { return c10::static_intrusive_pointer_cast<Cfg>(ctx->saved_data["cfg"].toCapsule()); }
 bool wants(const Tensor& t) { return t.defined() && t.requires_grad(); }
-bool grad_mode() { return c10::GradMode::is_enabled(); }
+// No graph is to be built: gradients are off, and no operand carries a forward-mode tangent (which `Function::apply` refuses and a
+// direct call of the kernels would drop).
+template <typename... T>
+bool no_graph(const T&... operands) {
+  if (c10::GradMode::is_enabled()) return false;
+  return !((operands.defined() && operands._fw_grad(0).defined()) || ...);
+}
 
 // Exceptions of Python hooks on saved tensors (activation checkpointing stops a recomputation with one) keep their type.
 template <typename F>
@@ -227,7 +233,7 @@ struct Linear : torch::autograd::Function<Linear> {
 Tensor op_linear(const Tensor& x, const py::object& w_, const py::object& b_) {
   return guarded([&] {
     Tensor w = w_.cast<Tensor>(), b = as_tensor(b_);
-    if (!grad_mode()) {
+    if (no_graph(x, w, b)) {
       Tensor y = mm(rows_of(x), operand(w), false, false, b);
       if (x.dim() == 2) return y;
       auto out = x.sizes().vec();
@@ -284,7 +290,7 @@ struct NormLinear : torch::autograd::Function<NormLinear> {
 py::object op_norm_linear(const Tensor& x, const py::object& res_, const py::object& nw_, const py::object& w_, double eps, bool offset) {
   return guarded([&]() -> py::object {
     Tensor res = as_tensor(res_), nw = nw_.cast<Tensor>(), w = w_.cast<Tensor>();
-    if (!grad_mode()) {
+    if (no_graph(x, res, nw, w)) {
       auto r = rmsnorm_fwd(x.contiguous(), res.defined() ? OptTensor(res.contiguous()) : OptTensor(), nw, eps, offset);
       tick(1);
       Tensor y = mm(r[0], operand(w), false, false);
@@ -345,7 +351,7 @@ struct LnLinear : torch::autograd::Function<LnLinear> {
 Tensor op_ln_linear(const Tensor& x, const py::object& lw_, const py::object& lb_, const py::object& w_, const py::object& b_, double eps) {
   return guarded([&] {
     Tensor lw = lw_.cast<Tensor>(), lb = as_tensor(lb_), w = w_.cast<Tensor>(), b = as_tensor(b_);
-    if (!grad_mode()) {
+    if (no_graph(x, lw, lb, w, b)) {
       tick(1);
       return mm(layernorm_fwd(x.contiguous(), lw, opt(lb), eps)[0], operand(w), false, false, b);
     }
@@ -383,7 +389,7 @@ struct GeluLinear : torch::autograd::Function<GeluLinear> {
 Tensor op_gelu_linear(const Tensor& pre, const py::object& w_, const py::object& b_, bool tanh_approx) {
   return guarded([&] {
     Tensor w = w_.cast<Tensor>(), b = as_tensor(b_);
-    if (!grad_mode()) {
+    if (no_graph(pre, w, b)) {
       tick(1);
       return mm(gelu_fwd(pre.contiguous(), tanh_approx), operand(w), false, false, b);
     }
@@ -418,7 +424,7 @@ struct SwigluLinear : torch::autograd::Function<SwigluLinear> {
 Tensor op_swiglu_linear(const Tensor& gu, const py::object& w_) {
   return guarded([&] {
     Tensor w = w_.cast<Tensor>();
-    if (!grad_mode()) {
+    if (no_graph(gu, w)) {
       tick(1);
       return mm(swiglu_fwd(gu.contiguous()), operand(w), false, false);
     }
@@ -466,7 +472,7 @@ py::object op_rms_norm(const Tensor& x, const py::object& res_, const py::object
   return guarded([&]() -> py::object {
     Tensor res = as_tensor(res_), w = w_.cast<Tensor>();
     variable_list out;
-    if (!grad_mode()) {
+    if (no_graph(x, res, w)) {
       auto r = rmsnorm_fwd(x.contiguous(), res.defined() ? OptTensor(res.contiguous()) : OptTensor(), w, eps, offset);
       tick(1);
       out = res.defined() ? variable_list{r[0], r[2]} : variable_list{r[0]};
@@ -515,7 +521,7 @@ struct LayerNorm : torch::autograd::Function<LayerNorm> {
 Tensor op_layer_norm(const Tensor& x, const py::object& w_, const py::object& b_, double eps) {
   return guarded([&] {
     Tensor w = w_.cast<Tensor>(), b = as_tensor(b_);
-    if (!grad_mode()) {
+    if (no_graph(x, w, b)) {
       tick(1);
       return layernorm_fwd(x.contiguous(), w, opt(b), eps)[0];
     }
@@ -553,7 +559,7 @@ struct GatedRmsNorm : torch::autograd::Function<GatedRmsNorm> {
 Tensor op_rms_norm_gated(const Tensor& x, const Tensor& z, const py::object& w_, double eps) {
   return guarded([&] {
     Tensor w = w_.cast<Tensor>();
-    if (!grad_mode()) {
+    if (no_graph(x, z, w)) {
       tick(1);
       return rmsnorm_gated_fwd(x.contiguous(), z.contiguous(), w, eps)[0];
     }
@@ -641,7 +647,7 @@ py::tuple op_qkv_norm_rope(const Tensor& qkv, const py::object& qw_, const py::o
                            int64_t n_kv, int64_t D, double eps, bool offset, bool gated) {
   return guarded([&]() -> py::tuple {
     Tensor qw = as_tensor(qw_), kw = as_tensor(kw_);
-    if (!grad_mode()) {
+    if (no_graph(qkv, qw, kw, cosv, sinv)) {
       auto r = qkv_norm_rope_fwd(qkv.contiguous(), n_q, n_kv, D, opt(qw), opt(kw), cosv, sinv, eps, offset, gated);
       tick(1);
       return py::make_tuple(r[0], r[1], r[2], gated ? py::cast(r[4]) : py::object(py::none()));
@@ -671,7 +677,7 @@ struct Rope : torch::autograd::Function<Rope> {
 };
 Tensor op_rope(const Tensor& x, const Tensor& cosv, const Tensor& sinv, int64_t d_out) {
   return guarded([&] {
-    if (!grad_mode()) {
+    if (no_graph(x, cosv, sinv)) {
       tick(1);
       return rope_generic(x, cosv, sinv, false, d_out);
     }
@@ -705,7 +711,7 @@ struct Attention : torch::autograd::Function<Attention> {
 };
 Tensor op_attention(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& cu, int64_t max_seqlen, bool causal, double scale) {
   return guarded([&] {
-    if (!grad_mode()) {
+    if (no_graph(q, k, v)) {
       tick(1);
       return attn_fwd(heads_in_place(q), heads_in_place(k), heads_in_place(v), cu, max_seqlen, causal, scale)[0];
     }

@@ -14,6 +14,7 @@ import os
 
 import numpy as np
 import torch
+import torch.autograd.forward_ad as _fwad
 
 from . import build as _build
 from . import reference as ref
@@ -541,7 +542,8 @@ def linear_cross_entropy(hidden, weight, targets, chunk=1024, ignore_index=-100,
     tagged ``.grad`` by the GEMM itself."""
     if hidden.dtype != torch.bfloat16 or not _tma_ok(hidden, weight) or weight.shape[0] % 8:
         return ref.linear_cross_entropy(hidden, weight, targets, chunk, ignore_index)
-    if not (torch.is_grad_enabled() and (hidden.requires_grad or weight.requires_grad)):
+    # a forward-mode level may be open: `apply` refuses operands with tangents
+    if _fwad._current_level < 0 and not (torch.is_grad_enabled() and (hidden.requires_grad or weight.requires_grad)):
         return _loss_only(hidden, weight, targets, int(chunk), int(ignore_index))
     return _LinearCrossEntropy.apply(hidden, weight, targets, int(chunk), int(ignore_index), float(grad_scale),
                                      _grad_target(weight) if grad_in_place else None)
