@@ -346,3 +346,20 @@ def test_forward_mode_tangents_are_refused(name, grad):
     with torch.set_grad_enabled(grad), fwad.dual_level():
         with pytest.raises(RuntimeError):
             _PARAM_OPS[name][0](fwad.make_dual(x.detach(), torch.ones_like(x)), params)
+
+
+@pytest.mark.multigpu
+def test_position_embedding_runs_on_the_device_of_its_operands():
+    """The current device is another one, and the kernel goes to the operands' device and its stream."""
+    import dataclasses
+
+    from vlm_training_b200.models.config import VisionConfig
+    from vlm_training_b200.models.vision import VisionPlan
+
+    cfg = VisionConfig(hidden_size=64, num_heads=2, num_position_embeddings=2304, spatial_merge_size=2)
+    with torch.cuda.device(0):
+        plan = VisionPlan.build([[1, 4, 6], [1, 8, 2]], cfg, "cuda:1")
+        x, table = _rand(40, 64, seed=1).to("cuda:1").requires_grad_(), _rand(2304, 64, seed=2).to("cuda:1").requires_grad_()
+        y = ops.pos_embed_add(x, table, plan, 2)
+        y.sum().backward()
+        assert torch.equal(y, ops.pos_embed_add(x, table, dataclasses.replace(plan, images=None), 2)) and table.grad is not None

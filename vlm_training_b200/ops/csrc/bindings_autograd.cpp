@@ -155,6 +155,7 @@ struct VecGrad {
 };
 // sums the partial rows of one or two 1-D parameters ([blocks, cols] each with row stride ld) in one launch
 void sum_rows(const float* p0, const float* p1, long ld, int rows, int cols, const VecGrad& g0, const VecGrad* g1) {
+  c10::cuda::CUDAGuard guard(g0.out.device());
   VlmtRowSums a{};
   a.ld = ld;
   a.partial[0] = p0; a.out[0] = g0.out.data_ptr(); a.mode[0] = g0.mode;
@@ -747,6 +748,7 @@ struct RowsUpdate : torch::autograd::Function<RowsUpdate> {
 struct PosEmbed : torch::autograd::Function<PosEmbed> {
   static Tensor forward(AutogradContext* ctx, const Tensor& x, const Tensor& table, const Tensor& index, const Tensor& weight, const Tensor& images,
                         CfgPtr c) {
+    c10::cuda::CUDAGuard guard(x.device());
     Tensor xc = x.contiguous(), out = torch::empty_like(xc);
     vlmt_pos_embed_fwd(xc.data_ptr(), table.data_ptr(), index.data_ptr<int64_t>(), weight.data_ptr<float>(), out.data_ptr(), x.size(0), x.size(1),
                        cur_stream());
@@ -759,6 +761,7 @@ struct PosEmbed : torch::autograd::Function<PosEmbed> {
   static variable_list backward(AutogradContext* ctx, variable_list grads) {
     auto saved = ctx->get_saved_variables();
     auto c = kept(ctx);
+    c10::cuda::CUDAGuard guard(grads[0].device());
     Tensor dy = grads[0].contiguous(), dt;
     if (reinterpret_cast<uintptr_t>(dy.data_ptr()) % 16) dy = dy.clone();
     if (c->need[1]) {
