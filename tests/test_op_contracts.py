@@ -363,3 +363,21 @@ def test_position_embedding_runs_on_the_device_of_its_operands():
         y = ops.pos_embed_add(x, table, plan, 2)
         y.sum().backward()
         assert torch.equal(y, ops.pos_embed_add(x, table, dataclasses.replace(plan, images=None), 2)) and table.grad is not None
+
+
+# bytes beyond what lives before the pass, in units of one [rows, I] bf16: d(activation), which the kernel overwrites with the
+# activation, and d(pre-activation) (two for SwiGLU's pair); the weight gradients land in the tagged .grad
+@gpu
+@pytest.mark.parametrize("name,units", [("gelu", 2), ("swiglu", 3)])
+def test_mlp_backward_peak_memory(name, units):
+    T, I, H = 4096, 8192, 256
+    pre = _rand(T, I * (2 if name == "swiglu" else 1), seed=1).requires_grad_()
+    w = torch.nn.Parameter(_rand(H, I, scale=0.02, seed=2))
+    w.grad, w._vlmt_grad_in_place = torch.zeros_like(w), True
+    y = ops.gelu_linear(pre, w) if name == "gelu" else ops.swiglu_linear(pre, w)
+    g = torch.ones_like(y)
+    torch.cuda.synchronize()
+    before = torch.cuda.memory_allocated()
+    torch.cuda.reset_peak_memory_stats()
+    y.backward(g)
+    assert torch.cuda.max_memory_allocated() - before <= units * T * I * 2 + (4 << 20)

@@ -309,7 +309,7 @@ Tensor swiglu_bwd(const Tensor& dout, const Tensor& gu, Tensor* out) {
   c10::cuda::CUDAGuard guard(gu.device());
   const int I = gu.size(-1) / 2;
   Tensor dgu = torch::empty_like(gu);
-  if (out != nullptr) *out = torch::empty(dout.sizes(), gu.options());
+  if (out != nullptr) *out = dout;
   vlmt_swiglu_bwd(dout.data_ptr(), gu.data_ptr(), dgu.data_ptr(), out != nullptr ? out->data_ptr() : nullptr, gu.numel() / (2 * I), I, cur_stream());
   return dgu;
 }
@@ -340,7 +340,7 @@ Tensor gelu_bwd(const Tensor& dy, const Tensor& x, bool tanh_approx, Tensor* y) 
   check_contig(dy, "dy");
   c10::cuda::CUDAGuard guard(x.device());
   Tensor dx = torch::empty_like(x);
-  if (y != nullptr) *y = torch::empty_like(x);
+  if (y != nullptr) *y = dy;
   vlmt_gelu_bwd(dy.data_ptr(), x.data_ptr(), dx.data_ptr(), y != nullptr ? y->data_ptr() : nullptr, x.numel(), tanh_approx, cur_stream());
   return dx;
 }

@@ -864,8 +864,9 @@ __global__ void swiglu_fwd_kernel(const bf16* __restrict__ gu, bf16* __restrict_
   }
 }
 // `out` (may be null): silu(gate) * up again, for the weight gradient of the linear that follows.  The kernel is bound by memory and has
-// gate and up in registers: a pass of its own for it read them once more (8192 x 12288: 97 + 155 us -> 188 us).
-__global__ void swiglu_bwd_kernel(const bf16* __restrict__ dout, const bf16* __restrict__ gu, bf16* __restrict__ dgu, bf16* __restrict__ out,
+// gate and up in registers: a pass of its own for it read them once more (8192 x 12288: 97 + 155 us -> 188 us).  `out` may be `dout`:
+// each group of 8 is read before it is written, so the activation costs no memory of its own at the peak of the backward pass.
+__global__ void swiglu_bwd_kernel(const bf16* dout, const bf16* __restrict__ gu, bf16* __restrict__ dgu, bf16* out,
                                   long rows, int I) {
   const long nvec = rows * (I >> 3);
   const int vper = I >> 3;
@@ -966,8 +967,8 @@ __global__ void gelu_fwd_kernel(const bf16* __restrict__ x, bf16* __restrict__ y
     reinterpret_cast<uint4*>(y)[v] = pack8(a);
   }
 }
-// `y` (may be null): gelu(x) again, as above for swiglu
-__global__ void gelu_bwd_kernel(const bf16* __restrict__ dy, const bf16* __restrict__ x, bf16* __restrict__ dx, bf16* __restrict__ y, long n8,
+// `y` (may be null, may be `dy`): gelu(x) again, as above for swiglu
+__global__ void gelu_bwd_kernel(const bf16* dy, const bf16* __restrict__ x, bf16* __restrict__ dx, bf16* y, long n8,
                                 int tanh_approx) {
   constexpr int U = 4;
   const long stride = (long)gridDim.x * blockDim.x;

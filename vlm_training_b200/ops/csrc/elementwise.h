@@ -13,7 +13,7 @@ int vlmt_layernorm_bwd(const void* dy, const void* x, const void* w, const float
 void vlmt_rmsnorm_gated_fwd(const void* x, const void* z, const void* w, void* y, float* rstd, int rows, int D, float eps, cudaStream_t st);
 int vlmt_rmsnorm_gated_bwd(const void* dy, const void* x, const void* z, const void* w, const float* rstd, void* dx, void* dz, float* dw_partial, int rows, int D, cudaStream_t st);
 void vlmt_swiglu_fwd(const void* gu, void* out, long rows, int I, cudaStream_t st);
-// out / y may be null: the forward result once more, for a weight gradient
+// out / y: the forward result once more, for a weight gradient; may be null, or dout / dy, which it then replaces
 void vlmt_swiglu_bwd(const void* dout, const void* gu, void* dgu, void* out, long rows, int I, cudaStream_t st);
 void vlmt_sigmoid_mul_fwd(const void* x, const void* gate, void* out, long n, cudaStream_t st);
 void vlmt_sigmoid_mul_bwd(const void* dout, const void* x, const void* gate, void* dx, void* dgate, long n, cudaStream_t st);

@@ -20,11 +20,11 @@ std::vector<Tensor> layernorm_bwd_partial(const Tensor& dy, const Tensor& x, con
 std::vector<Tensor> rmsnorm_gated_fwd(const Tensor& x, const Tensor& z, const Tensor& w, double eps);
 std::vector<Tensor> rmsnorm_gated_bwd_partial(const Tensor& dy, const Tensor& x, const Tensor& z, const Tensor& w, const Tensor& rstd);
 Tensor swiglu_fwd(const Tensor& gu);
-Tensor swiglu_bwd(const Tensor& dout, const Tensor& gu, Tensor* out = nullptr);   // out: swiglu_fwd(gu) from the same pass
+Tensor swiglu_bwd(const Tensor& dout, const Tensor& gu, Tensor* out = nullptr);   // out: swiglu_fwd(gu) from the same pass, in the place of dout
 Tensor sigmoid_mul_fwd(const Tensor& x, const Tensor& gate);
 std::vector<Tensor> sigmoid_mul_bwd(const Tensor& dout, const Tensor& x, const Tensor& gate);
 Tensor gelu_fwd(const Tensor& x, bool tanh_approx);
-Tensor gelu_bwd(const Tensor& dy, const Tensor& x, bool tanh_approx, Tensor* y = nullptr);   // y: gelu_fwd(x) from the same pass
+Tensor gelu_bwd(const Tensor& dy, const Tensor& x, bool tanh_approx, Tensor* y = nullptr);   // y: gelu_fwd(x) from the same pass, in the place of dy
 std::vector<Tensor> qkv_norm_rope_fwd(const Tensor& qkv, int64_t n_q, int64_t n_kv, int64_t D, const OptTensor& qw, const OptTensor& kw,
                                       const Tensor& cosv, const Tensor& sinv, double eps, bool offset, bool gated);
 std::vector<Tensor> qkv_norm_rope_bwd_partial(const Tensor& dq, const Tensor& dk, const Tensor& dv, const OptTensor& dgate, const Tensor& qkv,
