@@ -381,3 +381,13 @@ def test_mlp_backward_peak_memory(name, units):
     torch.cuda.reset_peak_memory_stats()
     y.backward(g)
     assert torch.cuda.max_memory_allocated() - before <= units * T * I * 2 + (4 << 20)
+
+
+@gpu
+def test_expert_gradient_without_storage_is_refused():
+    """A gradient bucket whose storage is released (a sharded unit outside its backward pass): an error, never a kernel on freed memory."""
+    x, params = _leaves("experts", lambda p: None)
+    out = _PARAM_OPS["experts"][0](x, params)
+    params["dn"].grad.untyped_storage().resize_(0)
+    with pytest.raises(RuntimeError):
+        out.backward(torch.ones_like(out))

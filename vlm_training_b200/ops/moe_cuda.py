@@ -51,6 +51,8 @@ class _GroupedLinear(torch.autograd.Function):
             param, g = ctx.w_param, None
             if param is not None and cu._may_add(param) and param.grad is not None and param.grad.shape == w.shape and param.grad.dtype == torch.bfloat16 \
                     and param.grad.is_contiguous() and param.grad.data_ptr() % 16 == 0:
+                if param.grad.untyped_storage().size() == 0:   # a sharded unit's bucket outside its backward pass
+                    raise RuntimeError("expert gradient without storage: a sharded parameter was used outside the backward of its unit")
                 g = param.grad.view(E * N, K)
             else:
                 dw = torch.empty(E * N, K, dtype=w.dtype, device=w.device)
