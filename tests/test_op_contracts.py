@@ -391,3 +391,32 @@ def test_expert_gradient_without_storage_is_refused():
     params["dn"].grad.untyped_storage().resize_(0)
     with pytest.raises(RuntimeError):
         out.backward(torch.ones_like(out))
+
+
+@gpu
+@pytest.mark.parametrize("fp8", [False, True])
+def test_cta_pairs_can_be_switched_off(fp8):
+    """``VLMT_GEMM_PAIR=0`` (read once per process) keeps the pair kernel out of both GEMMs."""
+    import os
+    import subprocess
+    import sys
+
+    code = """
+import torch
+from torch.profiler import ProfilerActivity, profile
+from vlm_training_b200.ops import cuda as cu
+a, b, out = (torch.ones(4096, k, device="cuda", dtype=torch.bfloat16) for k in (256, 256, 4096))
+with profile(activities=[ProfilerActivity.CUDA]) as prof:
+    if %r:
+        a8, _, ra = cu._C.fp8_quantize(a, 0, True, False)
+        cu._C.gemm_fp8(a8, a8, out, ra, ra, 0, 0, False)
+    else:
+        cu._gemm(a, b, out=out)
+    torch.cuda.synchronize()
+assert float(out.float().mean()) == 256.0
+print("pairs" if any("pair" in e.key for e in prof.key_averages()) else "blocks")
+""" % fp8
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    said = [subprocess.run([sys.executable, "-c", code], cwd=root, env={**os.environ, "VLMT_GEMM_PAIR": on}, capture_output=True, text=True).stdout.split()[-1:]
+            for on in ("1", "0")]
+    assert said == [["pairs"], ["blocks"]]

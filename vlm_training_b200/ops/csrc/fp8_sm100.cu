@@ -402,7 +402,7 @@ extern "C" int vlmt_gemm_fp8(const void* A, const void* B, void* D, int M, int N
     }
   }
   // at least one wave of 256 x 256 tiles: CTA pairs (the rule of the bf16 GEMMs); smaller outputs keep the finer tiles
-  if (M > BM && (long)((M + 255) / 256) * ((N + 255) / 256) * p.k_splits >= num_sms / 2)
+  if (M > BM && vlmt_gemm_pair_enabled() && (long)((M + 255) / 256) * ((N + 255) / 256) * p.k_splits >= num_sms / 2)
     return vlmt_gemm_pair_fp8(A, B, D, M, N, K, lda, ldb, ldd, make_idesc_f8(256, BN, a_format, b_format), rec_a, rec_b, accumulate, p.k_splits,
                               p.kb_per_split, status, stream);
   static bool configured = false;

@@ -18,6 +18,7 @@
 
 #include <cuda_runtime.h>
 #include <mutex>
+#include <stdlib.h>
 
 namespace {
 using namespace sm100;
@@ -277,6 +278,11 @@ int launch(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& td, 
   return (int)cudaLaunchKernelEx(&cfg, kern, ta, tb, td, p);
 }
 }  // namespace
+
+extern "C" int vlmt_gemm_pair_enabled() {
+  static const bool on = [] { const char* e = getenv("VLMT_GEMM_PAIR"); return !(e && e[0] == '0'); }();
+  return on;
+}
 
 extern "C" int vlmt_gemm_pair(const void* A, const void* B, void* D, const void* bias, int M, int N, int K, int lda, int ldb, int ldd,
                               int a_mn_major, int b_mn_major, int epilogue, int accumulate, const float* alpha, int k_splits, int kb_per_split,

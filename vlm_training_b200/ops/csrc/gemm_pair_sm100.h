@@ -6,6 +6,7 @@
 #ifdef __cplusplus
 extern "C" {
 #endif
+int vlmt_gemm_pair_enabled();   // 0 with VLMT_GEMM_PAIR=0: every GEMM, bf16 and FP8, on one-block tiles (A/B comparison)
 int vlmt_gemm_pair(const void* A, const void* B, void* D, const void* bias, int M, int N, int K, int lda, int ldb, int ldd, int a_mn_major,
                    int b_mn_major, int epilogue, int accumulate, const float* alpha, int k_splits, int kb_per_split, int* status,
                    cudaStream_t stream);

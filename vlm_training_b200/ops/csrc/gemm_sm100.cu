@@ -806,10 +806,6 @@ struct GemmExtras {
   unsigned* wg_counters = nullptr;
 };
 
-bool pair_enabled() {
-  static const bool on = [] { const char* e = getenv("VLMT_GEMM_PAIR"); return !(e && e[0] == '0'); }();
-  return on;
-}
 bool split_k_enabled() {
   static const bool on = [] { const char* e = getenv("VLMT_GEMM_SPLITK"); return !(e && e[0] == '0'); }();
   return on;
@@ -979,7 +975,7 @@ int gemm_launch(const void* A, const void* B, void* D, float* Dacc32, const void
   }
   // large bf16 outputs go to CTA pairs: at least one wave of 256 x 256 tiles, so the coarser tiles leave no SM idle.  With one row of
   // 128-row tiles half of every pair would have no rows (37 x 24576 x 4096 63.5 us in pairs, 53.3 us without, 1200 x 24576 x 4096 164 and 193).
-  if (plain && M > BM && p.tma_store && p.cluster <= 1 && pair_enabled() &&
+  if (plain && M > BM && p.tma_store && p.cluster <= 1 && vlmt_gemm_pair_enabled() &&
       (long)((M + 255) / 256) * ((N + 255) / 256) * p.k_splits >= num_sms / 2)
     return vlmt_gemm_pair(A, B, D, bias, M, N, K, lda, ldb, ldd, a_mn_major, b_mn_major, epilogue, accumulate, x.alpha, p.k_splits, p.kb_per_split,
                           status, stream);
