@@ -16,6 +16,7 @@
 #include <stdlib.h>
 
 #include "fp8_sm100.h"
+#include "gemm_epilogue.cuh"
 #include "gemm_pair_sm100.h"
 #include "gemm_sm100.h"
 
@@ -155,16 +156,6 @@ __device__ __forceinline__ void umma_f8_ss(uint32_t tmem_d, SmemDesc a, SmemDesc
   }
 }
 
-__device__ __forceinline__ void tile_coords(int tile, int tiles_m, int tiles_n, int& tm, int& tn) {
-  const int per_group = GROUP_M * tiles_n;
-  const int g = tile / per_group;
-  const int first_m = g * GROUP_M;
-  const int gsz = min(GROUP_M, tiles_m - first_m);
-  const int r = tile - g * per_group;
-  tm = first_m + r % gsz;
-  tn = r / gsz;
-}
-
 __global__ void __launch_bounds__(NUM_THREADS, 1)
 gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
                 const __grid_constant__ CUtensorMap tmap_d, Fp8Params p) {
@@ -209,7 +200,7 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
         const int kb_lo = p.k_splits > 1 ? ks * p.kb_per_split : 0;
         const int kb_hi = p.k_splits > 1 ? min(num_kb, kb_lo + p.kb_per_split) : num_kb;
         int tm, tn;
-        tile_coords(tile, tiles_m, tiles_n, tm, tn);
+        tile_coords<GROUP_M>(tile, tiles_m, tiles_n, tm, tn);
         const int m0 = tm * BM, n0 = tn * BN;
         for (int kb = kb_lo; kb < kb_hi; ++kb) {
           if (!mbar_wait(&empty_bar[stage], phase ^ 1, abort_flag, p.status, kErrTimeoutEmpty)) { ok = false; break; }
@@ -267,7 +258,7 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
     for (int item = blockIdx.x; item < num_items && ok; item += gridDim.x, ++it) {
       const int tile = item % num_tiles;
       int tm, tn;
-      tile_coords(tile, tiles_m, tiles_n, tm, tn);
+      tile_coords<GROUP_M>(tile, tiles_m, tiles_n, tm, tn);
       const int acc = it & 1;
       const uint32_t acc_phase = (it >> 1) & 1;
       if (!mbar_wait(&tmem_full[acc], acc_phase, abort_flag, p.status, kErrTimeoutTmemFull)) { ok = false; break; }
@@ -287,16 +278,10 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
           uint32_t r[32];
           tmem_ld_32x32(taddr + c * 64 + h * 32, r);
           tmem_ld_wait();
+          float v[32];
 #pragma unroll
-          for (int t = 0; t < 4; ++t) {
-            uint4 pk;
-            uint32_t* w = reinterpret_cast<uint32_t*>(&pk);
-#pragma unroll
-            for (int j = 0; j < 4; ++j)
-              w[j] = pack_bf16x2(__uint_as_float(r[t * 8 + 2 * j]) * scale, __uint_as_float(r[t * 8 + 2 * j + 1]) * scale);
-            const int ci = h * 4 + t;
-            *reinterpret_cast<uint4*>(buf + lane * 128 + ((ci ^ (lane & 7)) << 4)) = pk;
-          }
+          for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]) * scale;
+          stage_half_slab(buf, lane, h, v);
         }
         fence_async_proxy();
         __syncwarp();

@@ -1,0 +1,54 @@
+// Parts shared by the GEMM kernels (gemm_sm100.cu, gemm_pair_sm100.cu, fp8_sm100.cu): the raster of output tiles and the steps of the
+// epilogue between TMEM and the TMA store of a 64-column slab.
+#pragma once
+#include "gemm_sm100.h"
+#include "sm100.cuh"
+
+namespace sm100 {
+// Tiles in groups of GROUP_M rows of tiles, columns inside a group: the group's rows of A and the B panel they meet share L2.
+template <int GROUP_M>
+__device__ __forceinline__ void tile_coords(int tile, int tiles_m, int tiles_n, int& tm, int& tn) {
+  const int per_group = GROUP_M * tiles_n;
+  const int g = tile / per_group;
+  const int first_m = g * GROUP_M;
+  const int gsz = min(GROUP_M, tiles_m - first_m);
+  const int r = tile - g * per_group;
+  tm = first_m + r % gsz;
+  tn = r / gsz;
+}
+
+__device__ __forceinline__ float gelu_tanh_f(float x) {
+  const float k0 = 0.7978845608028654f, k1 = 0.044715f;
+  float u = k0 * (x + k1 * x * x * x);
+  return 0.5f * x * (1.f + tanhf(u));
+}
+__device__ __forceinline__ float gelu_erf_f(float x) { return 0.5f * x * (1.f + erff(x * 0.7071067811865476f)); }
+
+// 32 columns of a row, from column `col`: bias (or null) and activation (GemmEpilogue)
+__device__ __forceinline__ void bias_activation(float (&v)[32], const __nv_bfloat16* bias, int col, int N, int epilogue) {
+  if (bias != nullptr) {
+#pragma unroll
+    for (int i = 0; i < 32; ++i) if (col + i < N) v[i] += __bfloat162float(bias[col + i]);
+  }
+  if (epilogue == GEMM_EPI_GELU_TANH) {
+#pragma unroll
+    for (int i = 0; i < 32; ++i) v[i] = gelu_tanh_f(v[i]);
+  } else if (epilogue == GEMM_EPI_GELU_ERF) {
+#pragma unroll
+    for (int i = 0; i < 32; ++i) v[i] = gelu_erf_f(v[i]);
+  }
+}
+
+// half `h` of a 64-column slab row (one row per lane) as bf16 into the 128-byte swizzled staging buffer of a TMA store
+__device__ __forceinline__ void stage_half_slab(uint8_t* buf, int lane, int h, const float (&v)[32]) {
+#pragma unroll
+  for (int t = 0; t < 4; ++t) {
+    uint4 pk;
+    pk.x = pack_bf16x2(v[t * 8 + 0], v[t * 8 + 1]);
+    pk.y = pack_bf16x2(v[t * 8 + 2], v[t * 8 + 3]);
+    pk.z = pack_bf16x2(v[t * 8 + 4], v[t * 8 + 5]);
+    pk.w = pack_bf16x2(v[t * 8 + 6], v[t * 8 + 7]);
+    *reinterpret_cast<uint4*>(buf + lane * 128 + (((h * 4 + t) ^ (lane & 7)) << 4)) = pk;
+  }
+}
+}  // namespace sm100

@@ -12,8 +12,8 @@
 //
 // The leader (even rank) issues every MMA; both blocks' loads complete on the leader's "full" barrier; commits arrive on both
 // blocks' "empty" and "accumulator full" barriers; both epilogues arrive on the leader's "accumulator free" barrier.
+#include "gemm_epilogue.cuh"
 #include "gemm_pair_sm100.h"
-#include "gemm_sm100.h"
 #include "sm100.cuh"
 
 #include <cuda_runtime.h>
@@ -44,23 +44,6 @@ struct Params {
   uint32_t idesc;               // FP8: carries the two formats
   int* status;
 };
-
-__device__ __forceinline__ void tile_coords(int tile, int tiles_m, int tiles_n, int& tm, int& tn) {
-  const int per_group = GROUP_M * tiles_n;
-  const int g = tile / per_group;
-  const int first_m = g * GROUP_M;
-  const int gsz = min(GROUP_M, tiles_m - first_m);
-  const int r = tile - g * per_group;
-  tm = first_m + r % gsz;
-  tn = r / gsz;
-}
-
-__device__ __forceinline__ float gelu_tanh_f(float x) {
-  const float k0 = 0.7978845608028654f, k1 = 0.044715f;
-  float u = k0 * (x + k1 * x * x * x);
-  return 0.5f * x * (1.f + tanhf(u));
-}
-__device__ __forceinline__ float gelu_erf_f(float x) { return 0.5f * x * (1.f + erff(x * 0.7071067811865476f)); }
 
 template <bool A_MN, bool B_MN, bool FP8>
 __global__ void __launch_bounds__(NUM_THREADS, 1)
@@ -118,7 +101,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
       for (int item = pair; item < num_items && ok; item += pairs) {
         int tile, kb_lo, kb_hi, tm, tn;
         k_range(item, tile, kb_lo, kb_hi);
-        tile_coords(tile, tiles_m, tiles_n, tm, tn);
+        tile_coords<GROUP_M>(tile, tiles_m, tiles_n, tm, tn);
         const int m0 = (tm * 2 + (int)rank) * BM, n0 = tn * BN + (int)rank * (BN / 2);
         for (int kb = kb_lo; kb < kb_hi; ++kb) {
           if (!mbar_wait(&empty_bar[stage], phase ^ 1, abort_flag, p.status, kErrTimeoutEmpty)) { ok = false; break; }
@@ -183,7 +166,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
     for (int item = pair; item < num_items; item += pairs, ++it) {
       const int tile = p.k_splits > 1 ? item % num_tiles : item;
       int tm, tn;
-      tile_coords(tile, tiles_m, tiles_n, tm, tn);
+      tile_coords<GROUP_M>(tile, tiles_m, tiles_n, tm, tn);
       const int acc = it & 1;
       if (!mbar_wait(&tmem_full[acc], (it >> 1) & 1, abort_flag, p.status, kErrTimeoutTmemFull)) break;
       tc_fence_after();
@@ -204,26 +187,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
           float v[32];
 #pragma unroll
           for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]) * alpha;
-          if (!FP8 && p.bias != nullptr) {
-#pragma unroll
-            for (int i = 0; i < 32; ++i) if (col0 + h * 32 + i < p.N) v[i] += __bfloat162float(p.bias[col0 + h * 32 + i]);
-          }
-          if (!FP8 && p.epilogue == GEMM_EPI_GELU_TANH) {
-#pragma unroll
-            for (int i = 0; i < 32; ++i) v[i] = gelu_tanh_f(v[i]);
-          } else if (!FP8 && p.epilogue == GEMM_EPI_GELU_ERF) {
-#pragma unroll
-            for (int i = 0; i < 32; ++i) v[i] = gelu_erf_f(v[i]);
-          }
-#pragma unroll
-          for (int t = 0; t < 4; ++t) {
-            uint4 pk;
-            pk.x = pack_bf16x2(v[t * 8 + 0], v[t * 8 + 1]);
-            pk.y = pack_bf16x2(v[t * 8 + 2], v[t * 8 + 3]);
-            pk.z = pack_bf16x2(v[t * 8 + 4], v[t * 8 + 5]);
-            pk.w = pack_bf16x2(v[t * 8 + 6], v[t * 8 + 7]);
-            *reinterpret_cast<uint4*>(buf + lane * 128 + (((h * 4 + t) ^ (lane & 7)) << 4)) = pk;
-          }
+          if (!FP8) bias_activation(v, p.bias, col0 + h * 32, p.N, p.epilogue);
+          stage_half_slab(buf, lane, h, v);
         }
         fence_async_proxy();
         __syncwarp();

@@ -23,6 +23,7 @@
 // collective's number into every peer's flag array.  The TMA producer waits (bounded) for a peer's flag before it
 // loads the first tile of that peer's rows from the LOCAL gathered buffer, so remote rows cross NVLink once and the
 // transfer hides behind the own rows' tiles.
+#include "gemm_epilogue.cuh"
 #include "sm100.cuh"
 
 #include <stdlib.h>
@@ -121,23 +122,6 @@ __device__ __forceinline__ int group_of_tile(const int* __restrict__ prefix, int
     if (prefix[mid] <= tm) lo = mid; else hi = mid - 1;
   }
   return lo;
-}
-
-__device__ __forceinline__ float gelu_tanh_f(float x) {
-  const float k0 = 0.7978845608028654f, k1 = 0.044715f;
-  float u = k0 * (x + k1 * x * x * x);
-  return 0.5f * x * (1.f + tanhf(u));
-}
-__device__ __forceinline__ float gelu_erf_f(float x) { return 0.5f * x * (1.f + erff(x * 0.7071067811865476f)); }
-
-__device__ __forceinline__ void tile_coords(int tile, int tiles_m, int tiles_n, int& tm, int& tn) {
-  const int per_group = GROUP_M * tiles_n;
-  const int g = tile / per_group;
-  const int first_m = g * GROUP_M;
-  const int gsz = min(GROUP_M, tiles_m - first_m);
-  const int r = tile - g * per_group;
-  tm = first_m + r % gsz;
-  tn = r / gsz;
 }
 
 __device__ __forceinline__ int ld_acquire_sys_s32(const int* p) {
@@ -279,11 +263,11 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
         }
         if (p.grp_mode == 2) {
           const int g = tile / tiles_per_group;
-          tile_coords(tile - g * tiles_per_group, tiles_m, tiles_n, tm, tn);
+          tile_coords<GROUP_M>(tile - g * tiles_per_group, tiles_m, tiles_n, tm, tn);
           kb_lo = p.grp_prefix[g] * (BM / BK);
           kb_hi = p.grp_prefix[g + 1] * (BM / BK);
         } else {
-          tile_coords(tile, tiles_m, tiles_n, tm, tn);
+          tile_coords<GROUP_M>(tile, tiles_m, tiles_n, tm, tn);
           if (p.grp_mode == 1) b_row = group_of_tile(p.grp_prefix, p.grp_count, tm) * p.grp_b_rows;
         }
         if (AG) { tm += ag_rot; if (tm >= tiles_m) tm -= tiles_m; tn += wg_rot; if (tn >= tiles_n) tn -= tiles_n; }
@@ -483,11 +467,11 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
       bool empty_group = false;   // grp_mode 2: no rows for this group, the accumulator was never written -> zeros
       if (p.grp_mode == 2) {
         const int g = tile / tiles_per_group;
-        tile_coords(tile - g * tiles_per_group, tiles_m, tiles_n, tm, tn);
+        tile_coords<GROUP_M>(tile - g * tiles_per_group, tiles_m, tiles_n, tm, tn);
         d_row0 = g * p.M;
         empty_group = p.grp_prefix[g + 1] == p.grp_prefix[g];
       } else {
-        tile_coords(tile, tiles_m, tiles_n, tm, tn);
+        tile_coords<GROUP_M>(tile, tiles_m, tiles_n, tm, tn);
       }
       if (AG) { tm += ag_rot; if (tm >= tiles_m) tm -= tiles_m; tn += wg_rot; if (tn >= tiles_n) tn -= tiles_n; }
       const int acc = it & 1;
@@ -529,26 +513,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
             float v[32];
 #pragma unroll
             for (int i = 0; i < 32; ++i) v[i] = empty_group ? 0.f : __uint_as_float(r[i]) * alpha;
-            if (p.bias != nullptr) {
-#pragma unroll
-              for (int i = 0; i < 32; ++i) if (col0 + h * 32 + i < p.N) v[i] += __bfloat162float(p.bias[col0 + h * 32 + i]);
-            }
-            if (p.epilogue == GEMM_EPI_GELU_TANH) {
-#pragma unroll
-              for (int i = 0; i < 32; ++i) v[i] = gelu_tanh_f(v[i]);
-            } else if (p.epilogue == GEMM_EPI_GELU_ERF) {
-#pragma unroll
-              for (int i = 0; i < 32; ++i) v[i] = gelu_erf_f(v[i]);
-            }
-#pragma unroll
-            for (int t = 0; t < 4; ++t) {
-              uint4 pk;
-              __nv_bfloat162* p2 = reinterpret_cast<__nv_bfloat162*>(&pk);
-#pragma unroll
-              for (int j = 0; j < 4; ++j) p2[j] = __floats2bfloat162_rn(v[t * 8 + 2 * j], v[t * 8 + 2 * j + 1]);
-              const int ci = h * 4 + t;
-              *reinterpret_cast<uint4*>(buf + lane * 128 + ((ci ^ (lane & 7)) << 4)) = pk;
-            }
+            bias_activation(v, p.bias, col0 + h * 32, p.N, p.epilogue);
+            stage_half_slab(buf, lane, h, v);
           }
           fence_async_proxy();
           __syncwarp();
@@ -575,17 +541,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
           float v[32];
 #pragma unroll
           for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]) * alpha;
-          if (p.bias != nullptr) {
-#pragma unroll
-            for (int i = 0; i < 32; ++i) if (col0 + i < p.N) v[i] += __bfloat162float(p.bias[col0 + i]);
-          }
-          if (p.epilogue == GEMM_EPI_GELU_TANH) {
-#pragma unroll
-            for (int i = 0; i < 32; ++i) v[i] = gelu_tanh_f(v[i]);
-          } else if (p.epilogue == GEMM_EPI_GELU_ERF) {
-#pragma unroll
-            for (int i = 0; i < 32; ++i) v[i] = gelu_erf_f(v[i]);
-          }
+          bias_activation(v, p.bias, col0, p.N, p.epilogue);
           if (p.Dacc32 != nullptr) {
             float* dst = p.Dacc32 + (size_t)row * p.ldd + col0;
             if (col0 + 32 <= p.N && (p.ldd & 3) == 0) {
@@ -640,7 +596,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
   if (p.cluster > 1) {
     // one item per block; every thread of the cluster passes both barriers, also after an abort
     int tm, tn;
-    tile_coords(blockIdx.x / p.cluster, tiles_m, tiles_n, tm, tn);
+    tile_coords<GROUP_M>(blockIdx.x / p.cluster, tiles_m, tiles_n, tm, tn);
     __syncwarp();
     cluster_sync();
     if (!*abort_flag) store_cluster_sum<BN>(smem, p, tm * BM, tn * BN, blockIdx.x % p.cluster, p.alpha != nullptr ? __ldg(p.alpha) : 1.f);
