@@ -287,10 +287,6 @@ std::vector<Tensor> rmsnorm_gated_bwd_partial(const Tensor& dy, const Tensor& x,
                          pw.data_ptr<float>(), rows, D, cur_stream());
   return {dx, dz, pw};
 }
-std::vector<Tensor> rmsnorm_gated_bwd(const Tensor& dy, const Tensor& x, const Tensor& z, const Tensor& w, const Tensor& rstd) {
-  auto r = rmsnorm_gated_bwd_partial(dy, x, z, w, rstd);
-  return {r[0], r[1], sum_partials(r[2])};
-}
 
 // ------------------------------------------------------------------ activations
 Tensor swiglu_fwd(const Tensor& gu) {
@@ -382,14 +378,6 @@ std::vector<Tensor> qkv_norm_rope_bwd_partial(const Tensor& dq, const Tensor& dk
                                  partial.data_ptr<float>(), T, n_q, n_kv, D, R, offset, gated, qw.has_value(), cur_stream());
   TORCH_CHECK(r >= 0, "qkv_norm_rope_bwd failed");
   return {dqkv, partial};
-}
-std::vector<Tensor> qkv_norm_rope_bwd(const Tensor& dq, const Tensor& dk, const Tensor& dv, const c10::optional<Tensor>& dgate,
-                                      const Tensor& qkv, const c10::optional<Tensor>& qw, const c10::optional<Tensor>& kw,
-                                      const Tensor& cosv, const Tensor& sinv, const Tensor& rstd, int64_t n_q, int64_t n_kv, int64_t D,
-                                      bool offset, bool gated) {
-  auto r = qkv_norm_rope_bwd_partial(dq, dk, dv, dgate, qkv, qw, kw, cosv, sinv, rstd, n_q, n_kv, D, offset, gated);
-  Tensor dw = sum_partials(r[1].view({r[1].size(0), 2 * D})).view({2, D});
-  return {r[0], dw[0], dw[1]};
 }
 // generic rotary on a strided [S, H, D] view -> contiguous [S, H, Dout>=D] (zero padded when Dout > D)
 Tensor rope_generic(const Tensor& x, const Tensor& cosv, const Tensor& sinv, bool transpose, int64_t d_out) {
@@ -571,23 +559,16 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("rmsnorm_bwd", &rmsnorm_bwd);
   m.def("layernorm_fwd", &layernorm_fwd);
   m.def("layernorm_bwd", &layernorm_bwd);
-  m.def("rmsnorm_gated_fwd", &rmsnorm_gated_fwd);
-  m.def("rmsnorm_gated_bwd", &rmsnorm_gated_bwd);
   m.def("swiglu_fwd", &swiglu_fwd);
   m.def("swiglu_bwd", [](const Tensor& dout, const Tensor& gu) { return swiglu_bwd(dout, gu); });
-  m.def("sigmoid_mul_fwd", &sigmoid_mul_fwd);
-  m.def("sigmoid_mul_bwd", &sigmoid_mul_bwd);
   m.def("gelu_fwd", &gelu_fwd);
   m.def("gelu_bwd", [](const Tensor& dy, const Tensor& x, bool tanh_approx) { return gelu_bwd(dy, x, tanh_approx); });
   m.def("qkv_norm_rope_fwd", &qkv_norm_rope_fwd);
-  m.def("qkv_norm_rope_bwd", &qkv_norm_rope_bwd);
   m.def("rope_generic", &rope_generic);
   m.def("gdn_gates_fwd", &gdn_gates_fwd);
   m.def("gdn_gates_bwd", &gdn_gates_bwd);
   m.def("conv1d_silu_fwd", &conv1d_silu_fwd);
   m.def("conv1d_silu_bwd", &conv1d_silu_bwd);
-  m.def("rows_update", &rows_update);
-  m.def("rows_gather", &rows_gather);
   m.def("ce_fwd_bwd_", &ce_fwd_bwd_, py::arg("logits"), py::arg("targets"), py::arg("grad_scale"), py::arg("ignore_index"),
         py::arg("want_grad") = true);
   m.def("adamw_", &adamw_);

@@ -210,5 +210,4 @@ void bind_attention(pybind11::module_& m) {
   m.def("dsa_bwd", &dsa_bwd);
   m.def("dsa_supported", [](int64_t D, int64_t rep) { return vlmt_dsa_supported((int)D, (int)rep) != 0; });
   m.def("attn_fwd", &vlmt::attn_fwd);
-  m.def("attn_bwd", &vlmt::attn_bwd);
 }
