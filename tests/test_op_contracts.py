@@ -420,3 +420,15 @@ print("pairs" if any("pair" in e.key for e in prof.key_averages()) else "blocks"
     said = [subprocess.run([sys.executable, "-c", code], cwd=root, env={**os.environ, "VLMT_GEMM_PAIR": on}, capture_output=True, text=True).stdout.split()[-1:]
             for on in ("1", "0")]
     assert said == [["pairs"], ["blocks"]]
+
+
+@gpu
+def test_loss_of_no_rows():
+    """No tokens: a loss of zero, a zero weight gradient and an empty input gradient, with and without a graph."""
+    h, w = _rand(0, 64).requires_grad_(), _rand(128, 64, seed=1).requires_grad_()
+    tgt = torch.empty(0, dtype=torch.int64, device=DEV)
+    loss, n = ops.linear_cross_entropy(h, w, tgt, 32)
+    loss.backward()
+    assert float(loss) == 0.0 and int(n) == 0 and h.grad.shape == (0, 64) and float(w.grad.abs().sum()) == 0.0
+    with torch.no_grad():
+        assert float(ops.linear_cross_entropy(h, w, tgt, 32)[0]) == 0.0

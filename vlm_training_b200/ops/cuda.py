@@ -475,7 +475,7 @@ class _LinearCrossEntropy(torch.autograd.Function):
         losses = torch.empty(T, dtype=torch.float32, device=hidden.device)
         targets = targets.contiguous()
         ctx.w_dtype, ctx.w_param = weight.dtype, w_param
-        ctx.keep_logits = need_dw and 2 * T * V <= max(4 * V * H, _KEEP_LOGITS_BYTES)
+        ctx.keep_logits = need_dw and 0 < 2 * T * V <= max(4 * V * H, _KEEP_LOGITS_BYTES)
         n_valid = (targets != ignore_index).sum()
         ctx.mark_non_differentiable(n_valid)
         if ctx.keep_logits:
