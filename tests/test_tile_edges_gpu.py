@@ -27,7 +27,8 @@ def _close(got, want, atol, rtol, what=""):
                                      f"frac bad {(err > tol).float().mean().item():.4g}"
 
 
-# few output tiles: split over K through the fp32 workspace (odd rows and columns, a last part shorter than the others, one row)
+# few output tiles: K split inside a cluster, whose blocks sum their fp32 parts through shared memory (odd rows and columns, a last part
+# shorter than the others, one row)
 @pytest.mark.parametrize("M,N,K", [(37, 4096, 4096), (1, 520, 2048), (200, 392, 1096), (130, 128, 4104)])
 @pytest.mark.parametrize("layout", ["fwd", "dgrad", "wgrad"])
 def test_gemm_split_over_k(M, N, K, layout):
@@ -40,9 +41,9 @@ def test_gemm_split_over_k(M, N, K, layout):
     want = 0.37 * (ar @ br.t())
     # fp32 accumulation of K products of size about 0.25, then one bf16 rounding (2^-8 of the value)
     tol = dict(atol=2e-2 * (K / 4096) ** 0.5, rtol=8e-3)
-    for first in (True, False):   # the second call finds the counters as the first one left them
-        got = cu._gemm(a, b, a_mn=layout == "wgrad", b_mn=layout != "fwd", bias=bias, alpha=alpha)
-        torch.testing.assert_close(got.float(), want + bias.float(), **tol)
+    got = [cu._gemm(a, b, a_mn=layout == "wgrad", b_mn=layout != "fwd", bias=bias, alpha=alpha) for _ in range(2)]
+    torch.testing.assert_close(got[0].float(), want + bias.float(), **tol)
+    assert torch.equal(got[0], got[1])   # the parts are summed in rank order
     base = _rand(M, N)
     acc = base.clone()
     cu._gemm(a, b, a_mn=layout == "wgrad", b_mn=layout != "fwd", out=acc, accumulate=True, alpha=alpha)

@@ -15,8 +15,8 @@
 // SEL variants (sparse attention): every query of a document longer than `sel_topk` sees only the keys whose bit is set in
 // a selection bit mask (one bit per query and causal key, made by dsa_indexer_sm100.cu).  Every tile up to the diagonal is
 // still computed: gathering a query's 2048 key rows feeds the tensor core 8 query rows at a time and is bound by L2 gather
-// and scatter-add traffic (1.33 ns per query and key, forward + backward, 16 heads), a masked pair costs 0.15 ns, so the
-// dense form wins while documents are shorter than about 16 times the number of selected keys.
+// and scatter-add traffic (1.7 to 2.3 ns per query and key, forward + backward, 16 heads), a masked pair costs 0.10 to 0.15 ns, so
+// the dense form wins while documents are shorter than about 40 times the number of selected keys (the limit in use: ops/dsa_cuda.py).
 //
 // Roles per CTA (192 threads): warp 0 issues TMA loads, one thread of warp 1 issues every MMA, warps 2..5 own one row
 // of the 128-row tile per thread.  Every wait is bounded (sm100::mbar_wait).  No atomics: results are bit-reproducible.
