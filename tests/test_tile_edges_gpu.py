@@ -327,6 +327,12 @@ def test_attention_256_shared_key_tiles(lens, Hq, Hkv, causal):
     for a, b, n in ((q, qr, "dq"), (k, kr, "dk"), (v, vr, "dv")):   # sums over up to Hq / Hkv heads of bf16 products
         _close(a.grad, b.grad, 0.05 * max(1.0, (Hq / Hkv) ** 0.5 / 2), 3e-2, n)
 
+# heads of 256 on CTA pairs: key tiles shared by 4 pairs and by none; an odd number of heads per key head, whose pairs take neighbouring
+# query tiles, with the second one missing, of one row, and full
+@pytest.mark.parametrize("lens,Hq,Hkv,causal", [([1300], 8, 2, True), ([2600], 20, 10, True), ([127, 257, 256], 5, 1, True), ([129, 128], 3, 3, False)])
+def test_attention_256_pairs(lens, Hq, Hkv, causal):
+    test_attention_256_shared_key_tiles(lens, Hq, Hkv, causal)
+
 
 def test_rope_tables_and_position_embedding_outside_the_kernels_forms():
     """Positions that are not int64, and operands off a 16-byte boundary, take the general forms."""

@@ -1,16 +1,21 @@
-// Varlen flash attention for head size 256 (the gated full-attention layers of Qwen3.5) on tcgen05 / TMEM.
+// Varlen flash attention for head size 256 (the gated full-attention layers of Qwen3.5) on tcgen05 / TMEM, on CTA pairs.
 //
-// Head size 256 does not fit the two-query-tile layout of attention_sm100.cu (two [128 x 256] query tiles, two score
-// tiles and two output accumulators exceed both shared and tensor memory), so these kernels work on ONE 128-row tile per
-// CTA against streamed 64-row tiles of the other side, with the score buffers double-buffered in tensor memory so that
-// the tensor core computes the scores of tile j + 1 while the CUDA cores work on tile j:
+// A cluster of two blocks works on one MMA of M = 256 (tcgen05.mma.cta_group::2): each block owns a stationary tile of 128 rows and
+// its accumulator of 256 columns, both stream the same 128-row tiles of the other side.  The B operand of a product is shared: the
+// scores read a streamed tile by rows (each block loads 64 of them, all channels), the accumulations read it by channels (each block
+// loads 128 of them, all rows), so a tile that both kinds of product need comes in twice, by halves.
+// A single block has room for streamed tiles of 64 rows only, whose score products (N = 64) keep the tensor core busy for 70 cycles
+// and use 32 of them.  Against that form, us: 8192 tokens in one document, 16 / 4 heads, forward 540 -> 378, dV 641 -> 368, dK 982 -> 660,
+// dQ 827 -> 580; 12301 tokens in 4 documents with 2048 keys kept, 16 / 2 heads, 445 -> 344, 650 -> 366, 863 -> 617, 653 -> 482.  The
+// forward step takes 2410 cycles of which the tensor core needs 2048, the dQ step 4140 of 3072 (it waits for the first half of dS).
 //
-//   forward   CTA = (128 queries, query head).  S(j) = Q K_j^T (N = 64), online softmax with lazy rescale of the
-//             [128 x 256] fp32 output accumulator in TMEM, O += P(j) V_j with P read from TMEM.
-//   dQ        CTA = (128 queries, query head).  S(j), dP(j) = dO V_j^T, dS = P (dP - delta), dQ += dS(j) K_j.
-//   dK / dV   CTA = (128 keys, kv head), everything transposed (rows = keys), looping over 64-query tiles and the
-//             query heads of the GQA group.  The two accumulators ([128 x 256] fp32 each) plus double-buffered scores
-//             exceed the 512 TMEM columns, so dV and dK are two passes of one templated kernel; each recomputes S^T.
+//   forward   block = (128 queries, query head).  S(j) = Q K_j^T, online softmax with lazy rescale of the [128 x 256] fp32 output
+//             accumulator in TMEM, O += P(j) V_j with P read from TMEM.  Two score buffers: S(j + 1) runs under the softmax of step j.
+//   dQ        block = (128 queries, query head).  S(j), dP(j) = dO V_j^T, dS = P (dP - delta), dQ += dS(j) K_j.
+//             The two blocks of a pair are two query heads of one kv head, or two neighbouring query tiles where a kv head has an odd number.
+//   dK / dV   block = (128 keys, kv head), everything transposed (rows = keys), looping over 128-query tiles and the query heads of
+//             the GQA group; a pair holds neighbouring key tiles.  The two accumulators ([128 x 256] fp32 each) plus scores
+//             exceed the 512 TMEM columns, so dV and dK are two kernels; each recomputes S^T.
 //
 // SEL variants (sparse attention): every query of a document longer than `sel_topk` sees only the keys whose bit is set in
 // a selection bit mask (one bit per query and causal key, made by dsa_indexer_sm100.cu).  Every tile up to the diagonal is
@@ -18,8 +23,9 @@
 // and scatter-add traffic (1.7 to 2.3 ns per query and key, forward + backward, 16 heads), a masked pair costs 0.10 to 0.15 ns, so
 // the dense form wins while documents are shorter than about 40 times the number of selected keys (the limit in use: ops/dsa_cuda.py).
 //
-// Roles per CTA (192 threads): warp 0 issues TMA loads, one thread of warp 1 issues every MMA, warps 2..5 own one row
-// of the 128-row tile per thread.  Every wait is bounded (sm100::mbar_wait).  No atomics: results are bit-reproducible.
+// Roles per block: warp 0 issues TMA loads (both blocks' loads of a tile complete on the barrier of the even one, the leader), one
+// thread of the leader's warp 1 issues every MMA, the compute warps own the rows of their block.  Every wait is bounded
+// (sm100::mbar_wait).  No atomics: results are bit-reproducible.
 #include "attention_sm100.h"
 #include "sm100.cuh"
 
@@ -30,15 +36,14 @@ namespace {
 using namespace sm100;
 
 constexpr int HD = 256;            // head size
-constexpr int BR = 128;            // rows of the stationary tile
-constexpr int BC = 64;             // rows of a streamed tile
-constexpr int THREADS = 192;
+constexpr int BR = 128;            // rows of a block's stationary tile
+constexpr int BC = 128;            // rows of a streamed tile
 constexpr float kLog2e = 1.4426950408889634f;
 constexpr float kLn2 = 0.6931471805599453f;
 constexpr float kRescaleThreshold = 8.f;
-constexpr int kBigTile = BR * HD * 2;     // 65536: a [128 x 256] tile = 4 blocks of [128 rows x 64 channels]
-constexpr int kSmallTile = BC * HD * 2;   // 32768: a [64 x 256] tile = 4 blocks of [64 rows x 64 channels]
-constexpr int kBigBlock = BR * 128, kSmallBlock = BC * 128;   // bytes of one 64-channel block
+constexpr int kBigTile = BR * HD * 2;          // 65536: a stationary tile, 4 blocks of [128 rows x 64 channels]
+constexpr int kHalfTile = BC * HD;             // 32768: half a streamed tile, by rows (4 blocks of [64 rows x 64 channels]) or by channels (2 of [128 x 64])
+constexpr int kBigBlock = BR * 128, kRowBlock = BC / 2 * 128, kChanBlock = BC * 128;   // bytes of one 64-channel block
 
 struct TileInfo {
   int doc_start, doc_len, q0;
@@ -76,19 +81,23 @@ __device__ __forceinline__ uint8_t* align_smem(uint8_t* raw) {
 // k-step kk (16 channels) of a K-major [rows x 256] tile stored as 64-channel blocks of `block_bytes`
 __device__ __forceinline__ uint32_t kmajor_off(int kk, int block_bytes) { return (kk >> 2) * block_bytes + (kk & 3) * 32; }
 
-// D[128 x 64] = A[128 x 256] (K-major, big tile) x B[64 x 256]^T (K-major, small tile): 16 MMAs
-__device__ __forceinline__ void issue_scores(uint32_t dst, SmemDesc a_big, SmemDesc b_small, uint32_t idesc) {
+// D[256 x 128] = A[256 x 256] (K-major, both blocks' stationary tiles) x B[128 x 256]^T (K-major, a streamed tile by rows): 16 MMAs
+__device__ __forceinline__ void issue_scores(uint32_t dst, SmemDesc a_big, SmemDesc b_rows) {
+  constexpr uint32_t idesc = make_idesc_bf16(2 * BR, BC, false, false);
 #pragma unroll
   for (int kk = 0; kk < HD / 16; ++kk) {
-    const SmemDesc a = desc_off(a_big, kmajor_off(kk, kBigBlock)), b = desc_off(b_small, kmajor_off(kk, kSmallBlock));
-    if (kk == 0) umma_ss<0>(dst, a, b, idesc); else umma_ss<1>(dst, a, b, idesc);
+    const SmemDesc a = desc_off(a_big, kmajor_off(kk, kBigBlock)), b = desc_off(b_rows, kmajor_off(kk, kRowBlock));
+    if (kk == 0) umma_ss_pair<0>(dst, a, b, idesc); else umma_ss_pair<1>(dst, a, b, idesc);
   }
 }
-// D[128 x 256] (+)= A[128 x 64] (packed bf16 in TMEM at a_tmem) x B[64 x 256] (small tile read MN-major): 4 MMAs
-__device__ __forceinline__ void issue_accumulate(uint32_t dst, uint32_t a_tmem, SmemDesc b_mn, uint32_t idesc, uint32_t acc) {
+// D[256 x 256] (+)= A[256 x 128] (packed bf16 in TMEM, 64 rows of B at a_lo and 64 at a_hi) x B[128 x 256] (a streamed tile by channels): 8 MMAs
+__device__ __forceinline__ void issue_accumulate(uint32_t dst, uint32_t a_lo, uint32_t a_hi, SmemDesc b_chans, uint32_t acc) {
+  constexpr uint32_t idesc = make_idesc_bf16(2 * BR, HD, false, true);
 #pragma unroll
   for (int kk = 0; kk < BC / 16; ++kk) {
-    if (kk == 0) umma_ts<2>(dst, a_tmem, b_mn, idesc, acc); else umma_ts<1>(dst, a_tmem + kk * 8, desc_off(b_mn, kk * 2048), idesc);
+    const uint32_t a = kk < 4 ? a_lo + kk * 8 : a_hi + (kk - 4) * 8;
+    const SmemDesc b = desc_off(b_chans, kk * 2048);
+    if (kk == 0) umma_ts_pair<2>(dst, a, b, idesc, acc); else umma_ts_pair<1>(dst, a, b, idesc);
   }
 }
 
@@ -101,10 +110,24 @@ struct Params {
   float scale, scale_log2;
   int causal;
   int* status;
-  const uint2* sel;      // SEL: [ceil(L / 64)][T] 64-bit words, word [kt][t] = keys 64 kt .. 64 kt + 63 of t's document kept by query t
+  const uint2* sel;      // SEL: [key tiles of 64][T] 64-bit words, word [kt][t] = keys 64 kt .. 64 kt + 63 of t's document kept by query t
   int sel_topk;          // SEL: documents up to this length keep every causal key and have no words
-  int parts;             // dK / dV: blocks (a cluster) that share a key tile, each with an equal part of the group's query heads
+  int pair_heads;        // forward, dQ: the blocks of a pair are two query heads of one kv head; else two neighbouring query tiles
+  int parts;             // dK / dV: pairs (a cluster) that share two key tiles, each with an equal part of the group's query heads
 };
+
+// The pair of a forward or dQ block: its query tile, its query head, and the steps that both blocks take.
+struct QueryTile { TileInfo ti; int hq, steps; };
+__device__ __forceinline__ QueryTile query_tile(const Params& p, int rank) {
+  const int per_tile = p.pair_heads ? p.Hq / 2 : p.Hq, item = blockIdx.x >> 1, rows = p.pair_heads ? BR : 2 * BR;
+  QueryTile t;
+  t.ti = find_tile(p.cu, p.n_docs, item / per_tile, rows);
+  const int kv_end = p.causal ? min(t.ti.doc_len, t.ti.q0 + rows) : t.ti.doc_len;
+  t.steps = (kv_end + BC - 1) / BC;
+  t.hq = p.pair_heads ? item % per_tile * 2 + rank : item % per_tile;
+  if (!p.pair_heads) t.ti.q0 += rank * BR;   // may lie beyond the document: a block without rows
+  return t;
+}
 
 // 32 x 32 bit transpose across a warp: lane l gets bit l of every lane's word (bit c of the result: lane c)
 __device__ __forceinline__ uint32_t warp_transpose_bits(uint32_t x, int lane) {
@@ -117,15 +140,30 @@ __device__ __forceinline__ uint32_t warp_transpose_bits(uint32_t x, int lane) {
   return x;
 }
 
-__device__ __forceinline__ void load_big(uint8_t* dst, const CUtensorMap* m, uint64_t* bar, int col0, int row0) {
+// loads of one block; `bar`: the leader's barrier (address from cluster_addr)
+__device__ __forceinline__ void load_big(uint8_t* dst, const CUtensorMap* m, uint32_t bar, int col0, int row0) {   // boxes {64, 128}
 #pragma unroll
-  for (int b = 0; b < HD / 64; ++b) tma_load_2d(dst + b * kBigBlock, m, bar, col0 + 64 * b, row0);
+  for (int b = 0; b < HD / 64; ++b) tma_load_2d_pair(dst + b * kBigBlock, m, bar, col0 + 64 * b, row0);
 }
-__device__ __forceinline__ void load_small(uint8_t* dst, const CUtensorMap* m, uint64_t* bar, int col0, int row0) {
+__device__ __forceinline__ void load_rows(uint8_t* dst, const CUtensorMap* m, uint32_t bar, int col0, int row0, int rank) {   // boxes {64, 64}
 #pragma unroll
-  for (int b = 0; b < HD / 64; ++b) tma_load_2d(dst + b * kSmallBlock, m, bar, col0 + 64 * b, row0);
+  for (int b = 0; b < HD / 64; ++b) tma_load_2d_pair(dst + b * kRowBlock, m, bar, col0 + 64 * b, row0 + rank * (BC / 2));
+}
+__device__ __forceinline__ void load_chans(uint8_t* dst, const CUtensorMap* m, uint32_t bar, int col0, int row0, int rank) {   // boxes {64, 128}
+#pragma unroll
+  for (int b = 0; b < HD / 128; ++b) tma_load_2d_pair(dst + b * kChanBlock, m, bar, col0 + rank * (HD / 2) + 64 * b, row0);
 }
 
+// barriers set up in both blocks before anything remote touches them; TMEM allocated
+__device__ __forceinline__ uint32_t setup_end(int warp, uint32_t* tmem_slot) {
+  if (warp == 1) tmem_alloc_pair<512>(tmem_slot);
+  tc_fence_before();
+  __syncthreads();
+  __syncwarp();
+  cluster_sync();
+  tc_fence_after();
+  return *tmem_slot;
+}
 __device__ __forceinline__ void teardown(volatile int* abort_flag, int warp, uint32_t tmem_base) {
   tc_fence_before();
   __syncthreads();
@@ -134,100 +172,111 @@ __device__ __forceinline__ void teardown(volatile int* abort_flag, int warp, uin
     while (globaltimer_ns() - t0 < 200000ull) __nanosleep(1000);
     __syncthreads();
   }
+  __syncwarp();
+  cluster_sync();   // the leader's MMAs read the other block's memory, its arrivals go to the leader: nobody leaves first
   if (warp == 1) {
     tc_fence_after();
-    tmem_dealloc<512>(tmem_base);
+    tmem_dealloc_pair<512>(tmem_base);
+  }
+}
+
+// 32 accumulator columns of a row, times f, as bf16
+__device__ __forceinline__ void store_row32(__nv_bfloat16* dst, const uint32_t (&o)[32], float f) {
+#pragma unroll
+  for (int u = 0; u < 4; ++u) {
+    uint4 pk;
+    pk.x = pack_bf16x2(__uint_as_float(o[u * 8 + 0]) * f, __uint_as_float(o[u * 8 + 1]) * f);
+    pk.y = pack_bf16x2(__uint_as_float(o[u * 8 + 2]) * f, __uint_as_float(o[u * 8 + 3]) * f);
+    pk.z = pack_bf16x2(__uint_as_float(o[u * 8 + 4]) * f, __uint_as_float(o[u * 8 + 5]) * f);
+    pk.w = pack_bf16x2(__uint_as_float(o[u * 8 + 6]) * f, __uint_as_float(o[u * 8 + 7]) * f);
+    *reinterpret_cast<uint4*>(dst + u * 8) = pk;
   }
 }
 
 // ------------------------------------------------------------------------------------------------ forward
 struct FwdSmem {
   static constexpr int offQ = 0;
-  static constexpr int offK = kBigTile;                 // 2 stages
-  static constexpr int offV = offK + 2 * kSmallTile;    // 2 stages
-  static constexpr int offBar = offV + 2 * kSmallTile;  // 196608
+  static constexpr int offK = kBigTile;                // 2 stages, by rows
+  static constexpr int offV = offK + 2 * kHalfTile;    // 2 stages, by channels
+  static constexpr int offBar = offV + 2 * kHalfTile;  // 196608
   static constexpr int kSlack = 1024;
   static constexpr int kTotal = offBar + 256 + kSlack;
 };
+constexpr int kFwdThreads = 192;   // TMA, MMA, 4 compute warps with a row per thread
 
+// TMEM: score buffers at 0 and 128 (P(j) over the first 64 columns of its scores), output accumulator at 256.
+// Per step of 128 keys the tensor core needs about 2100 cycles (16 x 64 for the scores, 8 x 128 for the product) and a compute warp 1024 for
+// its exponentials; the scores of step j + 1 are issued before the product of step j, so it has work while the softmax runs.
 template <bool SEL>
-__global__ void __launch_bounds__(THREADS, 1)
+__global__ void __launch_bounds__(kFwdThreads, 1)
 attn256_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                    const __grid_constant__ CUtensorMap tmV, Params p) {
   using L = FwdSmem;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = align_smem<L::kSlack>(smem_raw);
-  if (smem == nullptr) { if (threadIdx.x == 0) atomicCAS(p.status, 0, kErrTimeoutOther); return; }
+  if (smem == nullptr) { if (threadIdx.x == 0) atomicCAS(p.status, 0, kErrTimeoutOther); return; }   // the same in both blocks
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + L::offBar);
-  uint64_t* q_full = bars;        // 1
+  uint64_t* q_full = bars;        // 1      (leader's: q_full, k_full, v_full, p_full)
   uint64_t* k_full = bars + 1;    // 2
   uint64_t* k_empty = bars + 3;   // 2
   uint64_t* v_full = bars + 5;    // 2
   uint64_t* v_empty = bars + 7;   // 2
   uint64_t* s_full = bars + 9;    // 2: S(j) is in score buffer j & 1
-  uint64_t* p_full = bars + 11;   // 2 (4 warps): P(j) is in score buffer j & 1
+  uint64_t* p_full = bars + 11;   // 2 (4 warps of each block): P(j) is in score buffer j & 1
   uint64_t* pv_done = bars + 13;  // 1: O holds the contributions of tiles 0..j
   uint64_t* o_done = bars + 14;   // 1
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 15);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const TileInfo ti = find_tile(p.cu, p.n_docs, blockIdx.x / p.Hq, BR);
-  if (!ti.valid) return;  // uniform for the whole CTA
-  const int hq = blockIdx.x % p.Hq;
-  const int hkv = hq / (p.Hq / p.Hkv);
-  const int kv_end = p.causal ? min(ti.doc_len, ti.q0 + BR) : ti.doc_len;
-  const int J = (kv_end + BC - 1) / BC;
-  constexpr int S_COL = 0, O_COL = 128;   // score buffers at 0 and 64, output accumulator at 128..383
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, rank = (int)cluster_rank();
+  const QueryTile t = query_tile(p, rank);
+  const TileInfo ti = t.ti;
+  if (!ti.valid) return;  // uniform for the pair
+  const int hq = t.hq, hkv = hq / (p.Hq / p.Hkv), J = t.steps;
+  constexpr int S_COL = 0, O_COL = 256;
 
   if (threadIdx.x == 0) {
     mbar_init(q_full, 1);
     for (int i = 0; i < 2; ++i) {
       mbar_init(&k_full[i], 1); mbar_init(&k_empty[i], 1); mbar_init(&v_full[i], 1); mbar_init(&v_empty[i], 1);
-      mbar_init(&s_full[i], 1); mbar_init(&p_full[i], 4);
+      mbar_init(&s_full[i], 1); mbar_init(&p_full[i], 8);
     }
     mbar_init(pv_done, 1); mbar_init(o_done, 1);
     *abort_flag = 0;
     fence_mbar_init();
     tma_prefetch_desc(&tmQ); tma_prefetch_desc(&tmK); tma_prefetch_desc(&tmV);
   }
-  if (warp == 1) tmem_alloc<512>(tmem_slot);
-  tc_fence_before();
-  __syncthreads();
-  tc_fence_after();
-  const uint32_t tmem_base = *tmem_slot;
+  const uint32_t tmem_base = setup_end(warp, tmem_slot);
 
   if (warp == 0) {
     if (lane == 0) {
-      mbar_expect_tx(q_full, kBigTile);
-      load_big(smem + L::offQ, &tmQ, q_full, hq * HD, ti.doc_start + ti.q0);
+      if (rank == 0) mbar_expect_tx(q_full, 2 * kBigTile);
+      load_big(smem + L::offQ, &tmQ, cluster_addr(q_full, 0), hq * HD, ti.doc_start + ti.q0);
       for (int j = 0; j < J; ++j) {
         const int s = j & 1;
         const uint32_t ph = ((j >> 1) & 1) ^ 1;
         const int krow = ti.doc_start + j * BC;
         if (!mbar_wait(&k_empty[s], ph, abort_flag, p.status, kErrTimeoutEmpty)) break;
-        mbar_expect_tx(&k_full[s], kSmallTile);
-        load_small(smem + L::offK + s * kSmallTile, &tmK, &k_full[s], hkv * HD, krow);
+        if (rank == 0) mbar_expect_tx(&k_full[s], 2 * kHalfTile);
+        load_rows(smem + L::offK + s * kHalfTile, &tmK, cluster_addr(&k_full[s], 0), hkv * HD, krow, rank);
         if (!mbar_wait(&v_empty[s], ph, abort_flag, p.status, kErrTimeoutEmpty)) break;
-        mbar_expect_tx(&v_full[s], kSmallTile);
-        load_small(smem + L::offV + s * kSmallTile, &tmV, &v_full[s], hkv * HD, krow);
+        if (rank == 0) mbar_expect_tx(&v_full[s], 2 * kHalfTile);
+        load_chans(smem + L::offV + s * kHalfTile, &tmV, cluster_addr(&v_full[s], 0), hkv * HD, krow, rank);
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      constexpr uint32_t idesc_s = make_idesc_bf16(BR, BC, false, false);
-      constexpr uint32_t idesc_pv = make_idesc_bf16(BR, HD, false, true);
+    if (lane == 0 && rank == 0) {
       const SmemDesc dQ = make_desc(smem_u32(smem + L::offQ), 16, 1024);
       const SmemDesc dK0 = make_desc(smem_u32(smem + L::offK), 16, 1024);
-      const SmemDesc dV0 = make_desc(smem_u32(smem + L::offV), kSmallBlock, 1024);
+      const SmemDesc dV0 = make_desc(smem_u32(smem + L::offV), kChanBlock, 1024);
       bool ok = mbar_wait(q_full, 0, abort_flag, p.status, kErrTimeoutFull);
       auto issue_S = [&](int j) -> bool {
         const int b = j & 1;
         if (!mbar_wait(&k_full[b], (j >> 1) & 1, abort_flag, p.status, kErrTimeoutFull)) return false;
         tc_fence_after();
-        issue_scores(tmem_base + S_COL + b * BC, dQ, desc_off(dK0, b * kSmallTile), idesc_s);
-        umma_commit(&s_full[b]);
-        umma_commit(&k_empty[b]);
+        issue_scores(tmem_base + S_COL + b * BC, dQ, desc_off(dK0, b * kHalfTile));
+        umma_commit_pair(&s_full[b]);
+        umma_commit_pair(&k_empty[b]);
         return true;
       };
       if (ok && J > 0) ok = issue_S(0);
@@ -238,11 +287,12 @@ attn256_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
         if (!mbar_wait(&v_full[b], (j >> 1) & 1, abort_flag, p.status, kErrTimeoutFull)) { ok = false; break; }
         if (!mbar_wait(&p_full[b], (j >> 1) & 1, abort_flag, p.status, kErrTimeoutOther)) { ok = false; break; }
         tc_fence_after();
-        issue_accumulate(tmem_base + O_COL, tmem_base + S_COL + b * BC, desc_off(dV0, b * kSmallTile), idesc_pv, (uint32_t)j);
-        umma_commit(&v_empty[b]);
-        umma_commit(pv_done);
+        const uint32_t a = tmem_base + S_COL + b * BC;
+        issue_accumulate(tmem_base + O_COL, a, a + 32, desc_off(dV0, b * kHalfTile), (uint32_t)j);
+        umma_commit_pair(&v_empty[b]);
+        umma_commit_pair(pv_done);
       }
-      if (ok) umma_commit(o_done);
+      if (ok) umma_commit_pair(o_done);
     }
   } else {
     const int q = warp & 3;                // TMEM lane quarter this warp may access
@@ -250,31 +300,29 @@ attn256_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
     const int qi = ti.q0 + r;              // query index local to the document
     const uint32_t lane_addr = (uint32_t)(q * 32) << 16;
     const uint32_t o_addr = tmem_base + O_COL + lane_addr;
+    const uint32_t p_bar0 = cluster_addr(&p_full[0], 0), p_bar1 = cluster_addr(&p_full[1], 0);
     const bool sel_doc = SEL && ti.doc_len > p.sel_topk;
     float m_used = SEL ? -INFINITY : 0.f, l = 0.f;   // SEL: a row may have no key in its first tiles
-    // a step's selection words are loaded during the step before
-    auto selection = [&](int j) { return sel_doc && qi < ti.doc_len ? __ldg(p.sel + (size_t)j * p.T + ti.doc_start + qi) : make_uint2(0u, 0u); };
-    uint2 kept_next = J > 0 ? selection(0) : make_uint2(0u, 0u);
+    // a step's selection words are loaded during the step before; words behind the causal keys of a query do not exist
+    auto selection = [&](int kt) { return sel_doc && qi < ti.doc_len && kt * 64 <= qi ? __ldg(p.sel + (size_t)kt * p.T + ti.doc_start + qi) : make_uint2(0u, 0u); };
+    uint2 next_lo = selection(0), next_hi = selection(1);
     bool ok = true;
     for (int j = 0; j < J && ok; ++j) {
       const int b = j & 1;
       const uint32_t s_addr = tmem_base + S_COL + b * BC + lane_addr;
-      const uint2 kept = kept_next;
-      if (j + 1 < J) kept_next = selection(j + 1);
+      const uint32_t kept[4] = {next_lo.x, next_lo.y, next_hi.x, next_hi.y};
+      if (SEL && j + 1 < J) { next_lo = selection(2 * j + 2); next_hi = selection(2 * j + 3); }
       if (!mbar_wait(&s_full[b], (j >> 1) & 1, abort_flag, p.status, kErrTimeoutTmemFull)) { ok = false; break; }
       tc_fence_after();
       uint32_t s[BC];
-      tmem_ld_32x32(s_addr, *reinterpret_cast<uint32_t(*)[32]>(&s[0]));
-      tmem_ld_32x32(s_addr + 32, *reinterpret_cast<uint32_t(*)[32]>(&s[32]));
+#pragma unroll
+      for (int c = 0; c < BC / 32; ++c) tmem_ld_32x32(s_addr + c * 32, *reinterpret_cast<uint32_t(*)[32]>(&s[c * 32]));
       tmem_ld_wait();
       const int kv0 = j * BC;
       const bool need_mask = (kv0 + BC > ti.doc_len) || (p.causal && kv0 + BC - 1 > ti.q0);
       if (sel_doc) {   // causality and the document's end are in the bits
 #pragma unroll
-        for (int i = 0; i < 32; ++i) {
-          if (!((kept.x >> i) & 1u)) s[i] = 0xff800000u;
-          if (!((kept.y >> i) & 1u)) s[32 + i] = 0xff800000u;
-        }
+        for (int i = 0; i < BC; ++i) if (!((kept[i >> 5] >> (i & 31)) & 1u)) s[i] = 0xff800000u;
       } else if (need_mask) {
         const int limit = (p.causal ? min(ti.doc_len - 1, qi) : ti.doc_len - 1) - kv0;  // last visible column of this tile
 #pragma unroll
@@ -323,12 +371,12 @@ attn256_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
           sum1 += e1;
           pk[i] = pack_bf16x2(e0, e1);
         }
-        tmem_st_32x16(s_addr + c * 16, pk);   // P(j) over the first 32 columns of its score buffer
+        tmem_st_32x16(s_addr + c * 16, pk);   // P(j) over the first 64 columns of its score buffer
       }
       tmem_st_wait();
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(&p_full[b]);
+      if (lane == 0) mbar_arrive_cluster(b ? p_bar1 : p_bar0);
       l += sum0 + sum1;
     }
     if (ok && J > 0 && mbar_wait(o_done, 0, abort_flag, p.status, kErrTimeoutTmemFull)) {
@@ -341,17 +389,7 @@ attn256_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
         uint32_t o[32];
         tmem_ld_32x32(o_addr + c * 32, o);
         tmem_ld_wait();
-        if (qi < ti.doc_len) {
-#pragma unroll
-          for (int u = 0; u < 4; ++u) {
-            uint4 pk;
-            pk.x = pack_bf16x2(__uint_as_float(o[u * 8 + 0]) * inv, __uint_as_float(o[u * 8 + 1]) * inv);
-            pk.y = pack_bf16x2(__uint_as_float(o[u * 8 + 2]) * inv, __uint_as_float(o[u * 8 + 3]) * inv);
-            pk.z = pack_bf16x2(__uint_as_float(o[u * 8 + 4]) * inv, __uint_as_float(o[u * 8 + 5]) * inv);
-            pk.w = pack_bf16x2(__uint_as_float(o[u * 8 + 6]) * inv, __uint_as_float(o[u * 8 + 7]) * inv);
-            *reinterpret_cast<uint4*>(dst + c * 32 + u * 8) = pk;
-          }
-        }
+        if (qi < ti.doc_len) store_row32(dst + c * 32, o, inv);
       }
       if (qi < ti.doc_len) p.LSE[(size_t)hq * p.T + tok] = l > 0.f ? (m_used + log2f(l)) * kLn2 : -INFINITY;
     }
@@ -360,490 +398,501 @@ attn256_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
 }
 
 // ------------------------------------------------------------------------------------------------ backward
-// Shared memory of both backward kernels: two stationary [128 x 256] tiles, a two-stage ring of [64 x 256] tiles for the
-// streamed operand that is needed until the end of a step, one buffer for the one that is free after the step's first half.
+// Shared memory of the dQ and dK kernels: two stationary [128 x 256] tiles and three half tiles, one buffer each.  Each is free one
+// product before its next load is needed, a thousand cycles or more.
 struct BwdSmem {
-  static constexpr int offA = 0;                        // dq: Q_i      | dk/dv: K_j
-  static constexpr int offB = kBigTile;                 // dq: dO_i     | dk/dv: V_j (dK pass only)
-  static constexpr int offC = 2 * kBigTile;             // 2 stages: dq K_j | dk/dv Q_i
-  static constexpr int offD = offC + 2 * kSmallTile;    // 1 stage:  dq V_j | dk/dv dO_i
-  static constexpr int offStat = offD + kSmallTile;     // dk/dv: per compute warp -lse2[64], -delta[64]
-  static constexpr int offBar = offStat + 4 * 128 * 4;
+  static constexpr int offA = 0;                       // dQ: Q_i               | dK: K_j
+  static constexpr int offB = kBigTile;                // dQ: dO_i              | dK: V_j
+  static constexpr int offS = 2 * kBigTile;            // dQ: K_j by rows       | dK: Q_i by rows        (scores)
+  static constexpr int offG = offS + kHalfTile;        // dQ: K_j by channels   | dK: Q_i by channels    (accumulation)
+  static constexpr int offD = offG + kHalfTile;        // dQ: V_j by rows       | dK: dO_i by rows       (dP)
+  static constexpr int offStat = offD + kHalfTile;     // dK: 2 stages of -lse2[128], -delta[128]
+  static constexpr int offBar = offStat + 2 * 2 * BC * 4;
   static constexpr int kSlack = 512;
-  static constexpr int kTotal = offBar + 256 + kSlack;  // 232192 <= 232448
+  static constexpr int kTotal = offBar + 256 + kSlack;
 };
+static_assert(BwdSmem::kTotal <= 232448, "shared memory");
 
 constexpr int kPartPitch = HD + 4;   // floats per row of a block's part of dK / dV in shared memory (conflict-free 16-byte stores)
 static_assert(BR * kPartPitch * 4 <= BwdSmem::offStat, "a part lies over the tiles");
 
-// dQ: one CTA per 128-query tile and query head, streaming 64-key tiles.
-// TMEM: S[2] at 0 / 64, dP[2] at 128 / 192, dQ at 256.  Tensor-core order: dQ(j), S(j+1), dP(j+1).  With the scores first, dQ(j) waited
-// for the load of K_(j+1), which waits for dQ(j-1): a memory latency in every step (16384 tokens in 5 documents, 16 heads: 1970 -> 1530 us).
+constexpr int kBwdThreads = 320;   // TMA, MMA, 8 compute warps: half of a row's 128 columns per thread
+
+// dQ: a block owns a 128-query tile of one query head, the pair streams 128-key tiles.
+// TMEM: two buffers of 128 columns that take turns, dQ at 256.  Step j: S(j) in one, dP(j) in the other, dS(j) over S(j).
+// Tensor-core order: S(j + 1) (into the buffer of dP(j), once it is in registers), dQ(j), dP(j + 1) (over S(j) and dS(j)): the exponentials
+// of step j + 1 run under dQ(j) and dP(j + 1), what stays exposed is the first half of dS(j).
 template <bool SEL>
-__global__ void __launch_bounds__(THREADS, 1)
-attn256_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
+__global__ void __launch_bounds__(kBwdThreads, 1)
+attn256_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmK2,
                       const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmdO, Params p) {
   using L = BwdSmem;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = align_smem<L::kSlack>(smem_raw);
   if (smem == nullptr) { if (threadIdx.x == 0) atomicCAS(p.status, 0, kErrTimeoutOther); return; }
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + L::offBar);
-  uint64_t* qdo_full = bars;       // 1
-  uint64_t* acc_done = bars + 1;   // 1
-  uint64_t* k_full = bars + 2;     // 2
-  uint64_t* k_empty = bars + 4;    // 2
-  uint64_t* v_full = bars + 6;     // 1
-  uint64_t* v_empty = bars + 7;    // 1
-  uint64_t* s_full = bars + 8;     // 2
-  uint64_t* dp_full = bars + 10;   // 2
-  uint64_t* ds_full = bars + 12;   // 2 (4 warps)
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 14);
+  uint64_t* qdo_full = bars;       // leader's: qdo_full, ks_full, kg_full, v_full, dp_read, ds_full
+  uint64_t* acc_done = bars + 1;
+  uint64_t* ks_full = bars + 2;
+  uint64_t* ks_empty = bars + 3;
+  uint64_t* kg_full = bars + 4;
+  uint64_t* kg_empty = bars + 5;
+  uint64_t* v_full = bars + 6;
+  uint64_t* v_empty = bars + 7;
+  uint64_t* s_full = bars + 8;
+  uint64_t* dp_full = bars + 9;
+  uint64_t* dp_read = bars + 10;   // 8 warps of each block: dP(j) is in registers
+  uint64_t* ds_full = bars + 11;   // 8 warps of each block: dS(j) is in TMEM
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 12);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const TileInfo ti = find_tile(p.cu, p.n_docs, blockIdx.x / p.Hq, BR);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, rank = (int)cluster_rank();
+  const QueryTile t = query_tile(p, rank);
+  const TileInfo ti = t.ti;
   if (!ti.valid) return;
-  const int hq = blockIdx.x % p.Hq;
-  const int hkv = hq / (p.Hq / p.Hkv);
-  const int kv_end = p.causal ? min(ti.doc_len, ti.q0 + BR) : ti.doc_len;
-  const int J = (kv_end + BC - 1) / BC;
-  constexpr int S_COL = 0, DP_COL = 128, DQ_COL = 256;
+  const int hq = t.hq, hkv = hq / (p.Hq / p.Hkv), J = t.steps;
+  constexpr int DQ_COL = 256;
 
   if (threadIdx.x == 0) {
-    mbar_init(qdo_full, 1); mbar_init(acc_done, 1); mbar_init(v_full, 1); mbar_init(v_empty, 1);
-    for (int i = 0; i < 2; ++i) {
-      mbar_init(&k_full[i], 1); mbar_init(&k_empty[i], 1); mbar_init(&s_full[i], 1); mbar_init(&dp_full[i], 1);
-      mbar_init(&ds_full[i], 4);
-    }
+    for (int i = 0; i < 12; ++i) mbar_init(&bars[i], i >= 10 ? 16 : 1);   // dp_read, ds_full: 16
     *abort_flag = 0;
     fence_mbar_init();
   }
-  if (warp == 1) tmem_alloc<512>(tmem_slot);
-  tc_fence_before();
-  __syncthreads();
-  tc_fence_after();
-  const uint32_t tmem_base = *tmem_slot;
+  const uint32_t tmem_base = setup_end(warp, tmem_slot);
 
   if (warp == 0) {
     if (lane == 0) {
       const int qrow = ti.doc_start + ti.q0;
-      mbar_expect_tx(qdo_full, 2 * kBigTile);
-      load_big(smem + L::offA, &tmQ, qdo_full, hq * HD, qrow);
-      load_big(smem + L::offB, &tmdO, qdo_full, hq * HD, qrow);
+      const uint32_t bar_s = cluster_addr(ks_full, 0), bar_g = cluster_addr(kg_full, 0), bar_v = cluster_addr(v_full, 0), bar_q = cluster_addr(qdo_full, 0);
+      if (rank == 0) mbar_expect_tx(qdo_full, 4 * kBigTile);
+      load_big(smem + L::offA, &tmQ, bar_q, hq * HD, qrow);
+      load_big(smem + L::offB, &tmdO, bar_q, hq * HD, qrow);
       for (int j = 0; j < J; ++j) {
-        const int s = j & 1;
         const int krow = ti.doc_start + j * BC;
-        if (!mbar_wait(&k_empty[s], ((j >> 1) & 1) ^ 1, abort_flag, p.status, kErrTimeoutEmpty)) break;
-        mbar_expect_tx(&k_full[s], kSmallTile);
-        load_small(smem + L::offC + s * kSmallTile, &tmK, &k_full[s], hkv * HD, krow);
-        if (!mbar_wait(v_empty, (j & 1) ^ 1, abort_flag, p.status, kErrTimeoutEmpty)) break;
-        mbar_expect_tx(v_full, kSmallTile);
-        load_small(smem + L::offD, &tmV, v_full, hkv * HD, krow);
+        const uint32_t ph = (j & 1) ^ 1;
+        if (!mbar_wait(ks_empty, ph, abort_flag, p.status, kErrTimeoutEmpty)) break;
+        if (rank == 0) mbar_expect_tx(ks_full, 2 * kHalfTile);
+        load_rows(smem + L::offS, &tmK, bar_s, hkv * HD, krow, rank);
+        if (!mbar_wait(v_empty, ph, abort_flag, p.status, kErrTimeoutEmpty)) break;
+        if (rank == 0) mbar_expect_tx(v_full, 2 * kHalfTile);
+        load_rows(smem + L::offD, &tmV, bar_v, hkv * HD, krow, rank);
+        if (!mbar_wait(kg_empty, ph, abort_flag, p.status, kErrTimeoutEmpty)) break;
+        if (rank == 0) mbar_expect_tx(kg_full, 2 * kHalfTile);
+        load_chans(smem + L::offG, &tmK2, bar_g, hkv * HD, krow, rank);
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      constexpr uint32_t idesc_s = make_idesc_bf16(BR, BC, false, false);
-      constexpr uint32_t idesc_g = make_idesc_bf16(BR, HD, false, true);
+    if (lane == 0 && rank == 0) {
       const SmemDesc dQ = make_desc(smem_u32(smem + L::offA), 16, 1024), dO = make_desc(smem_u32(smem + L::offB), 16, 1024);
-      const SmemDesc dKk = make_desc(smem_u32(smem + L::offC), 16, 1024);            // K tile, K-major view (scores)
-      const SmemDesc dKm = make_desc(smem_u32(smem + L::offC), kSmallBlock, 1024);   // K tile, MN-major view (dQ += dS K)
-      const SmemDesc dVk = make_desc(smem_u32(smem + L::offD), 16, 1024);
+      const SmemDesc dKs = make_desc(smem_u32(smem + L::offS), 16, 1024), dKg = make_desc(smem_u32(smem + L::offG), kChanBlock, 1024);
+      const SmemDesc dVs = make_desc(smem_u32(smem + L::offD), 16, 1024);
       bool ok = mbar_wait(qdo_full, 0, abort_flag, p.status, kErrTimeoutFull);
-      auto issue_step = [&](int j) -> bool {   // S(j) and dP(j) into the buffers of parity j & 1
-        const int b = j & 1;
-        if (!mbar_wait(&k_full[b], (j >> 1) & 1, abort_flag, p.status, kErrTimeoutFull)) return false;
+      auto issue_S = [&](int j) -> bool {
+        if (!mbar_wait(ks_full, j & 1, abort_flag, p.status, kErrTimeoutFull)) return false;
         tc_fence_after();
-        issue_scores(tmem_base + S_COL + b * BC, dQ, desc_off(dKk, b * kSmallTile), idesc_s);
-        umma_commit(&s_full[b]);
-        if (!mbar_wait(v_full, j & 1, abort_flag, p.status, kErrTimeoutFull)) return false;
-        tc_fence_after();
-        issue_scores(tmem_base + DP_COL + b * BC, dO, dVk, idesc_s);
-        umma_commit(&dp_full[b]);
-        umma_commit(v_empty);              // V_j was last read by dP(j)
+        issue_scores(tmem_base + (j & 1) * BC, dQ, dKs);
+        umma_commit_pair(s_full);
+        umma_commit_pair(ks_empty);
         return true;
       };
-      if (ok && J > 0) ok = issue_step(0);
-      for (int j = 0; j < J && ok; ++j) {
-        const int b = j & 1;
-        if (!mbar_wait(&ds_full[b], (j >> 1) & 1, abort_flag, p.status, kErrTimeoutOther)) { ok = false; break; }
+      auto issue_dP = [&](int j) -> bool {
+        if (!mbar_wait(v_full, j & 1, abort_flag, p.status, kErrTimeoutFull)) return false;
         tc_fence_after();
-        issue_accumulate(tmem_base + DQ_COL, tmem_base + DP_COL + b * BC, desc_off(dKm, b * kSmallTile), idesc_g, (uint32_t)j);
-        umma_commit(&k_empty[b]);          // K_j was last read by dQ(j)
-        // the buffers of parity (j + 1) & 1 held S(j - 1) (in registers of the compute warps since ds_full(j - 1)) and
-        // dS(j - 1) (read by dQ(j - 1), issued earlier by this thread)
-        if (j + 1 < J && !issue_step(j + 1)) { ok = false; break; }
+        issue_scores(tmem_base + ((j & 1) ^ 1) * BC, dO, dVs);
+        umma_commit_pair(dp_full);
+        umma_commit_pair(v_empty);
+        return true;
+      };
+      if (ok) ok = issue_S(0) && issue_dP(0);
+      for (int j = 0; j < J && ok; ++j) {
+        if (j + 1 < J) {
+          if (!mbar_wait(dp_read, j & 1, abort_flag, p.status, kErrTimeoutOther)) { ok = false; break; }
+          if (!issue_S(j + 1)) { ok = false; break; }
+        }
+        if (!mbar_wait(kg_full, j & 1, abort_flag, p.status, kErrTimeoutFull)) { ok = false; break; }
+        if (!mbar_wait(ds_full, j & 1, abort_flag, p.status, kErrTimeoutOther)) { ok = false; break; }
+        tc_fence_after();
+        const uint32_t a = tmem_base + (j & 1) * BC;
+        issue_accumulate(tmem_base + DQ_COL, a, a + BC / 2, dKg, (uint32_t)j);
+        umma_commit_pair(kg_empty);
+        if (j + 1 < J && !issue_dP(j + 1)) { ok = false; break; }   // over dS(j), which dQ(j), issued before, reads
       }
-      if (ok) umma_commit(acc_done);
+      if (ok) umma_commit_pair(acc_done);
     }
   } else {
-    const int q = warp & 3;
+    const int q = warp & 3, half = (warp - 2) >> 2;
     const int r = q * 32 + lane;
     const int qi = ti.q0 + r;
     const bool q_ok = qi < ti.doc_len;
     const uint32_t lane_addr = (uint32_t)(q * 32) << 16;
+    const uint32_t bar_read = cluster_addr(dp_read, 0), bar_ds = cluster_addr(ds_full, 0);
     const size_t sidx = (size_t)hq * p.T + ti.doc_start + (q_ok ? qi : 0);
     const float neg_lse2 = q_ok ? -p.LSE[sidx] * kLog2e : -INFINITY;   // rows beyond the document: P = 0
     const float neg_delta = q_ok ? -p.delta[sidx] : 0.f;
     const bool sel_doc = SEL && ti.doc_len > p.sel_topk;
-    // a step's selection words are loaded during the step before
-    auto selection = [&](int j) { return sel_doc && qi < ti.doc_len ? __ldg(p.sel + (size_t)j * p.T + ti.doc_start + qi) : make_uint2(0u, 0u); };
-    uint2 kept_next = J > 0 ? selection(0) : make_uint2(0u, 0u);
+    // a step's selection words are loaded during the step before; words behind the causal keys of a query do not exist
+    auto selection = [&](int kt) { return sel_doc && q_ok && kt * 64 <= qi ? __ldg(p.sel + (size_t)kt * p.T + ti.doc_start + qi) : make_uint2(0u, 0u); };
+    uint2 kept_next = selection(half);
     bool ok = true;
     for (int j = 0; j < J && ok; ++j) {
-      const int b = j & 1;
-      const uint32_t s_addr = tmem_base + S_COL + b * BC + lane_addr, dp_addr = tmem_base + DP_COL + b * BC + lane_addr;
+      const uint32_t s_addr = tmem_base + (j & 1) * BC + half * (BC / 2) + lane_addr, dp_addr = tmem_base + ((j & 1) ^ 1) * BC + half * (BC / 2) + lane_addr;
       const uint2 kept = kept_next;
-      if (j + 1 < J) kept_next = selection(j + 1);
-      if (!mbar_wait(&s_full[b], (j >> 1) & 1, abort_flag, p.status, kErrTimeoutTmemFull)) { ok = false; break; }
+      if (SEL && j + 1 < J) kept_next = selection(2 * j + 2 + half);
+      if (!mbar_wait(s_full, j & 1, abort_flag, p.status, kErrTimeoutTmemFull)) { ok = false; break; }
       tc_fence_after();
-      uint32_t s[BC];
-      tmem_ld_32x32(s_addr, *reinterpret_cast<uint32_t(*)[32]>(&s[0]));
-      tmem_ld_32x32(s_addr + 32, *reinterpret_cast<uint32_t(*)[32]>(&s[32]));
-      tmem_ld_wait();
-      const int kv0 = j * BC;
-      const int limit = (p.causal ? min(ti.doc_len - 1, qi) : ti.doc_len - 1) - kv0;   // last visible column
-      float pr[BC];
+      // visible columns of this thread's half as bits; an interior tile has them all
+      uint32_t seen[2] = {0xffffffffu, 0xffffffffu};
       if (sel_doc) {
-#pragma unroll
-        for (int i = 0; i < BC; ++i) {
-          const float x = fmaf(__uint_as_float(s[i]), p.scale_log2, neg_lse2);
-          pr[i] = (((i < 32 ? kept.x : kept.y) >> (i & 31)) & 1u) ? ex2_approx(x) : 0.f;
-        }
+        seen[0] = kept.x; seen[1] = kept.y;
       } else {
+        const int left = (p.causal ? min(ti.doc_len - 1, qi) : ti.doc_len - 1) - (j * BC + half * (BC / 2)) + 1;
 #pragma unroll
-        for (int i = 0; i < BC; ++i) {
-          const float x = fmaf(__uint_as_float(s[i]), p.scale_log2, neg_lse2);
-          pr[i] = i > limit ? 0.f : ex2_approx(x);
+        for (int c = 0; c < 2; ++c) seen[c] = left >= c * 32 + 32 ? 0xffffffffu : left > c * 32 ? (1u << (left - c * 32)) - 1u : 0u;
+      }
+      float pr[BC / 2];
+#pragma unroll
+      for (int c = 0; c < 2; ++c) {
+        uint32_t s[32];
+        tmem_ld_32x32(s_addr + c * 32, s);
+        tmem_ld_wait();
+        if (__all_sync(0xffffffffu, seen[c] == 0xffffffffu)) {
+#pragma unroll
+          for (int i = 0; i < 32; ++i) pr[c * 32 + i] = ex2_approx(fmaf(__uint_as_float(s[i]), p.scale_log2, neg_lse2));
+        } else {
+#pragma unroll
+          for (int i = 0; i < 32; ++i) {
+            const float x = fmaf(__uint_as_float(s[i]), p.scale_log2, neg_lse2);
+            pr[c * 32 + i] = ex2_approx((seen[c] >> i) & 1u ? x : -INFINITY);   // 2^-inf = 0
+          }
         }
       }
-      if (!mbar_wait(&dp_full[b], (j >> 1) & 1, abort_flag, p.status, kErrTimeoutTmemFull)) { ok = false; break; }
+      if (!mbar_wait(dp_full, j & 1, abort_flag, p.status, kErrTimeoutTmemFull)) { ok = false; break; }
       tc_fence_after();
+      uint32_t dr[BC / 2];
+      tmem_ld_32x32(dp_addr, *reinterpret_cast<uint32_t(*)[32]>(&dr[0]));
+      tmem_ld_32x32(dp_addr + 32, *reinterpret_cast<uint32_t(*)[32]>(&dr[32]));
+      tmem_ld_wait();
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive_cluster(bar_read);
 #pragma unroll
-      for (int c = 0; c < BC / 32; ++c) {
-        uint32_t dr[32];
-        tmem_ld_32x32(dp_addr + c * 32, dr);
-        tmem_ld_wait();
+      for (int c = 0; c < 2; ++c) {
         uint32_t pk[16];
 #pragma unroll
         for (int u = 0; u < 16; ++u) {
-          const float d0 = pr[c * 32 + 2 * u] * (__uint_as_float(dr[2 * u]) + neg_delta);
-          const float d1 = pr[c * 32 + 2 * u + 1] * (__uint_as_float(dr[2 * u + 1]) + neg_delta);
+          const float d0 = pr[c * 32 + 2 * u] * (__uint_as_float(dr[c * 32 + 2 * u]) + neg_delta);
+          const float d1 = pr[c * 32 + 2 * u + 1] * (__uint_as_float(dr[c * 32 + 2 * u + 1]) + neg_delta);
           pk[u] = pack_bf16x2(d0, d1);
         }
-        tmem_st_32x16(dp_addr + c * 16, pk);   // dS(j), packed, over the first 32 columns of the dP buffer
+        tmem_st_32x16(s_addr + c * 16, pk);   // dS(j), packed, over the first 32 of this thread's own 64 score columns
       }
       tmem_st_wait();
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(&ds_full[b]);
+      if (lane == 0) mbar_arrive_cluster(bar_ds);
     }
     if (ok && mbar_wait(acc_done, 0, abort_flag, p.status, kErrTimeoutTmemFull)) {
       tc_fence_after();
-      if (J > 0) {
-        __nv_bfloat16* dst = p.dQ + ((size_t)(ti.doc_start + qi) * p.Hq + hq) * HD;
+      __nv_bfloat16* dst = p.dQ + ((size_t)(ti.doc_start + qi) * p.Hq + hq) * HD;
 #pragma unroll 1
-        for (int c = 0; c < HD / 32; ++c) {
-          uint32_t o[32];
-          tmem_ld_32x32(tmem_base + DQ_COL + lane_addr + c * 32, o);
-          tmem_ld_wait();
-          if (q_ok) {
-#pragma unroll
-            for (int u = 0; u < 4; ++u) {
-              uint4 pk;
-              pk.x = pack_bf16x2(__uint_as_float(o[u * 8 + 0]) * p.scale, __uint_as_float(o[u * 8 + 1]) * p.scale);
-              pk.y = pack_bf16x2(__uint_as_float(o[u * 8 + 2]) * p.scale, __uint_as_float(o[u * 8 + 3]) * p.scale);
-              pk.z = pack_bf16x2(__uint_as_float(o[u * 8 + 4]) * p.scale, __uint_as_float(o[u * 8 + 5]) * p.scale);
-              pk.w = pack_bf16x2(__uint_as_float(o[u * 8 + 6]) * p.scale, __uint_as_float(o[u * 8 + 7]) * p.scale);
-              *reinterpret_cast<uint4*>(dst + c * 32 + u * 8) = pk;
-            }
-          }
-        }
+      for (int c = half * 4; c < half * 4 + 4; ++c) {
+        uint32_t o[32];
+        tmem_ld_32x32(tmem_base + DQ_COL + lane_addr + c * 32, o);
+        tmem_ld_wait();
+        if (q_ok) store_row32(dst + c * 32, o, p.scale);
       }
     }
   }
   teardown(abort_flag, warp, tmem_base);
 }
 
-// dK (DV = false) or dV (DV = true): one CTA per 128-key tile and kv head; rows = keys; loops over the 64-query tiles that
-// see the key tile and over the query heads of the GQA group.
-// TMEM: S^T[2] at 0 / 64, dP^T[2] at 128 / 192 (dK pass), accumulator at 256.
-//   dV pass: S^T(it+1), dV(it) += P^T(it) dO_it         dK pass: dK(it) += dS^T(it) Q_it, S^T(it+1), dP^T(it+1)
-// Bound by the chain of a step (scores, softmax, product) and not by the tensor core; what must stay off it are the loads: dO has two
-// buffers in the dV pass, and the order of the dK pass lets Q_(it+2) load during a whole step.
-// 16384 tokens in 5 documents, 16 / 4 heads, with the order of the tiles: dV 2624 -> 960 us, dK 2348 -> 1470 us.
-template <bool DV, bool SEL>
-__global__ void __launch_bounds__(THREADS, 1)
-attn256_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
-                       const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmdO, Params p) {
-  using L = BwdSmem;
-  extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = align_smem<L::kSlack>(smem_raw);
-  if (smem == nullptr) { if (threadIdx.x == 0) atomicCAS(p.status, 0, kErrTimeoutOther); return; }
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + L::offBar);
-  uint64_t* kv_full = bars;        // 1
-  uint64_t* acc_done = bars + 1;   // 1
-  uint64_t* q_full = bars + 2;     // 2
-  uint64_t* q_empty = bars + 4;    // 2
-  uint64_t* do_full = bars + 6;    // 2 (dK pass: 1)
-  uint64_t* do_empty = bars + 8;   // 2 (dK pass: 1)
-  uint64_t* s_full = bars + 10;    // 2
-  uint64_t* dp_full = bars + 12;   // 2
-  uint64_t* a_full = bars + 14;    // 2 (4 warps): the A operand of the accumulation (P^T or dS^T) of parity it & 1 is in TMEM
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 16);
-  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-  float* stat = reinterpret_cast<float*>(smem + L::offStat);
+// Sum of a cluster's parts of a [128 x 256] accumulator and its store.  Every block of the cluster gets here, also after an abort.
+// Its own part is in shared memory; the blocks that hold the same keys sum in order of their rank and store an equal share of the rows each.
+__device__ __forceinline__ void store_parts(uint8_t* smem, const Params& p, volatile int* abort_flag, int rank, __nv_bfloat16* base, float f,
+                                            const TileInfo& ti, int k0, int hkv) {
+  __syncwarp();
+  cluster_sync();
+  if (!*abort_flag) {
+    const int rows = BR / p.parts, row0 = (rank >> 1) * rows;
+    const uint32_t at = smem_u32(smem);
+    for (int i = threadIdx.x; i < rows * (HD / 4); i += blockDim.x) {
+      const int row = row0 + i / (HD / 4), col = i % (HD / 4) * 4;
+      float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+      for (int s = 0; s < p.parts; ++s) {
+        const float4 x = ld_cluster_f4(at + (uint32_t)(row * kPartPitch + col) * 4, 2 * s + (rank & 1));
+        v.x += x.x; v.y += x.y; v.z += x.z; v.w += x.w;
+      }
+      if (k0 + row < ti.doc_len)
+        *reinterpret_cast<uint2*>(base + ((size_t)(ti.doc_start + k0 + row) * p.Hkv + hkv) * HD + col) =
+            make_uint2(pack_bf16x2(v.x * f, v.y * f), pack_bf16x2(v.z * f, v.w * f));
+    }
+  }
+  __syncwarp();
+  cluster_sync();        // nobody leaves while its part is being read
+}
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int part = blockIdx.x % p.parts, hkv = blockIdx.x / p.parts % p.Hkv;   // a cluster: the parts of one tile
-  const TileInfo ti = find_tile<true>(p.cu, p.n_docs, blockIdx.x / p.parts / p.Hkv, BR);
-  if (!ti.valid) return;
-  const int group = p.Hq / p.Hkv / p.parts;          // query heads of this block
-  const int hq0 = hkv * (p.Hq / p.Hkv) + part * group;
-  const int k0 = ti.q0;   // first key row of the tile (local to the document)
-  const int n_qtiles = (ti.doc_len + BC - 1) / BC;
-  const int i_first = p.causal ? k0 / BC : 0;
-  const int n_iter = (n_qtiles - i_first) * group;
-  constexpr int S_COL = 0, DP_COL = 128, ACC_COL = 256;
-  // dV pass: dO has a second buffer where the dK pass keeps V
-  auto do_stage = [](int it) { return DV ? it & 1 : 0; };
-  auto do_phase = [](int it) { return (uint32_t)(DV ? (it >> 1) & 1 : it & 1); };
+constexpr int kDkvThreads = 352;   // as kBwdThreads, and a warp for the queries' statistics
+
+// dV pass: K by rows of the pair, Q by rows and dO by channels in two stages each.
+struct DvSmem {
+  static constexpr int offK = 0;
+  static constexpr int offQ = kBigTile;
+  static constexpr int offO = offQ + 2 * kHalfTile;
+  static constexpr int offStat = offO + 2 * kHalfTile;   // 2 stages of -lse2[128], -delta[128]
+  static constexpr int offBar = offStat + 2 * 2 * BC * 4;
+  static constexpr int kSlack = 1024;
+  static constexpr int kTotal = offBar + 256 + kSlack;
+};
+
+// dK (DV = false) or dV (DV = true): a block owns a 128-key tile of one kv head; rows = keys; the pair loops over the 128-query tiles
+// that see its 256 keys and over the query heads of the GQA group.
+//   dV pass: S^T(it+1), dV(it) += P^T(it) dO_it, two score buffers as in forward        dK pass: the order and buffers of the dQ kernel
+// One warp fetches the queries' statistics (columns here) a step ahead.
+template <bool DV, bool SEL>
+__global__ void __launch_bounds__(kDkvThreads, 1)
+attn256_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmQ2, const __grid_constant__ CUtensorMap tmK,
+                       const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmdO, Params p) {
+  constexpr int offStat = DV ? DvSmem::offStat : BwdSmem::offStat, offBar = DV ? DvSmem::offBar : BwdSmem::offBar;
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = align_smem<DV ? DvSmem::kSlack : BwdSmem::kSlack>(smem_raw);
+  if (smem == nullptr) { if (threadIdx.x == 0) atomicCAS(p.status, 0, kErrTimeoutOther); return; }
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + offBar);
+  uint64_t* kv_full = bars;          // leader's: kv_full, q_full, g_full, do_full, dp_read, a_full
+  uint64_t* acc_done = bars + 1;
+  uint64_t* q_full = bars + 2;       // 2 (dK pass: 1)
+  uint64_t* q_empty = bars + 4;      // 2 (dK pass: 1)
+  uint64_t* do_full = bars + 6;      // 2 (dK pass: 1)
+  uint64_t* do_empty = bars + 8;     // 2 (dK pass: 1)
+  uint64_t* g_full = bars + 10;      // dK pass: Q by channels
+  uint64_t* g_empty = bars + 11;
+  uint64_t* s_full = bars + 12;      // 2 (dK pass: 1)
+  uint64_t* dp_full = bars + 14;
+  uint64_t* dp_read = bars + 15;     // 8 warps of each block: dP^T(it) is in registers
+  uint64_t* a_full = bars + 16;      // 2 (dK pass: 1), 8 warps of each block: the A operand of the accumulation (P^T or dS^T) is in TMEM
+  uint64_t* stat_full = bars + 18;   // 2
+  uint64_t* stat_empty = bars + 20;  // 2 (8 warps)
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 22);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+  float* stat = reinterpret_cast<float*>(smem + offStat);
+
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, rank = (int)cluster_rank();
+  const int me = rank & 1, leader = rank & ~1;                           // place in the pair; the cluster holds `parts` pairs
+  const uint16_t both = (uint16_t)(3u << leader);
+  const int item = blockIdx.x / (2 * p.parts), hkv = item % p.Hkv;
+  const TileInfo ti = find_tile<true>(p.cu, p.n_docs, item / p.Hkv, 2 * BR);
+  if (!ti.valid) return;                             // uniform for the cluster
+  const int group = p.Hq / p.Hkv / p.parts;          // query heads of this pair
+  const int hq0 = hkv * (p.Hq / p.Hkv) + (rank >> 1) * group;
+  const int k0 = ti.q0 + me * BR;                    // first key row of the tile (local to the document), maybe beyond its end
+  const int i_first = p.causal ? ti.q0 / BC : 0;
+  const int n_iter = ((ti.doc_len + BC - 1) / BC - i_first) * group;
+  constexpr int ACC_COL = 256;
 
   if (threadIdx.x == 0) {
-    mbar_init(kv_full, 1); mbar_init(acc_done, 1);
-    for (int i = 0; i < 2; ++i) {
-      mbar_init(&q_full[i], 1); mbar_init(&q_empty[i], 1); mbar_init(&do_full[i], 1); mbar_init(&do_empty[i], 1); mbar_init(&s_full[i], 1); mbar_init(&dp_full[i], 1);
-      mbar_init(&a_full[i], 4);
-    }
+    for (int i = 0; i < 22; ++i) mbar_init(&bars[i], i >= 20 ? 8 : i >= 15 && i <= 17 ? 16 : 1);   // stat_empty: 8; dp_read, a_full: 16
     *abort_flag = 0;
     fence_mbar_init();
   }
-  if (warp == 1) tmem_alloc<512>(tmem_slot);
-  tc_fence_before();
-  __syncthreads();
-  tc_fence_after();
-  const uint32_t tmem_base = *tmem_slot;
+  const uint32_t tmem_base = setup_end(warp, tmem_slot);
+  // step `it` works on query tile i_first + it / group of head hq0 + it % group; a ring of two stages (dV pass) or one (dK pass)
+  auto stage_of = [](int it) { return DV ? it & 1 : 0; };
+  auto phase_of = [](int it) { return (uint32_t)(DV ? (it >> 1) & 1 : it & 1); };
 
   if (warp == 0) {
     if (lane == 0) {
       const int krow = ti.doc_start + k0;
-      mbar_expect_tx(kv_full, DV ? kBigTile : 2 * kBigTile);
-      load_big(smem + L::offA, &tmK, kv_full, hkv * HD, krow);
-      if (!DV) load_big(smem + L::offB, &tmV, kv_full, hkv * HD, krow);
-      auto load_q = [&](int it) -> bool {
-        const int s = it & 1;
-        if (!mbar_wait(&q_empty[s], ((it >> 1) & 1) ^ 1, abort_flag, p.status, kErrTimeoutEmpty)) return false;
-        mbar_expect_tx(&q_full[s], kSmallTile);
-        load_small(smem + L::offC + s * kSmallTile, &tmQ, &q_full[s], (hq0 + it % group) * HD, ti.doc_start + (i_first + it / group) * BC);
-        return true;
-      };
-      bool ok = !DV || load_q(0);
-      for (int it = 0; it < n_iter && ok; ++it) {
-        // dV pass: Q is needed for the scores only and runs a step ahead of dO
-        if (DV ? it + 1 < n_iter && !load_q(it + 1) : !load_q(it)) break;
-        const int ds = do_stage(it);
-        if (!mbar_wait(&do_empty[ds], do_phase(it) ^ 1, abort_flag, p.status, kErrTimeoutEmpty)) break;
-        mbar_expect_tx(&do_full[ds], kSmallTile);
-        load_small(smem + (ds ? L::offB : L::offD), &tmdO, &do_full[ds], (hq0 + it % group) * HD, ti.doc_start + (i_first + it / group) * BC);
+      const uint32_t bar_kv = cluster_addr(kv_full, leader);
+      if (me == 0) mbar_expect_tx(kv_full, (DV ? 2 : 4) * kBigTile);
+      load_big(smem + (DV ? DvSmem::offK : BwdSmem::offA), &tmK, bar_kv, hkv * HD, krow);
+      if (!DV) load_big(smem + BwdSmem::offB, &tmV, bar_kv, hkv * HD, krow);
+      for (int it = 0; it < n_iter; ++it) {
+        const int s = stage_of(it), col = (hq0 + it % group) * HD, row = ti.doc_start + (i_first + it / group) * BC;
+        const uint32_t ph = phase_of(it) ^ 1;
+        if (!mbar_wait(&q_empty[s], ph, abort_flag, p.status, kErrTimeoutEmpty)) break;
+        if (me == 0) mbar_expect_tx(&q_full[s], 2 * kHalfTile);
+        load_rows(smem + (DV ? DvSmem::offQ + s * kHalfTile : BwdSmem::offS), &tmQ, cluster_addr(&q_full[s], leader), col, row, me);
+        if (!mbar_wait(&do_empty[s], ph, abort_flag, p.status, kErrTimeoutEmpty)) break;
+        if (me == 0) mbar_expect_tx(&do_full[s], 2 * kHalfTile);
+        if (DV) load_chans(smem + DvSmem::offO + s * kHalfTile, &tmdO, cluster_addr(&do_full[s], leader), col, row, me);
+        else load_rows(smem + BwdSmem::offD, &tmdO, cluster_addr(&do_full[s], leader), col, row, me);
+        if (!DV) {
+          if (!mbar_wait(g_empty, ph, abort_flag, p.status, kErrTimeoutEmpty)) break;
+          if (me == 0) mbar_expect_tx(g_full, 2 * kHalfTile);
+          load_chans(smem + BwdSmem::offG, &tmQ2, cluster_addr(g_full, leader), col, row, me);
+        }
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      constexpr uint32_t idesc_s = make_idesc_bf16(BR, BC, false, false);   // [128 keys] x [64 queries], contraction over channels
-      constexpr uint32_t idesc_g = make_idesc_bf16(BR, HD, false, true);     // [128 keys] x [256], contraction over 64 queries
-      const SmemDesc dK = make_desc(smem_u32(smem + L::offA), 16, 1024), dV = make_desc(smem_u32(smem + L::offB), 16, 1024);
-      const SmemDesc dQk = make_desc(smem_u32(smem + L::offC), 16, 1024), dQm = make_desc(smem_u32(smem + L::offC), kSmallBlock, 1024);
-      const SmemDesc dOk = make_desc(smem_u32(smem + L::offD), 16, 1024), dOm = make_desc(smem_u32(smem + L::offD), kSmallBlock, 1024),
-                     dOm2 = make_desc(smem_u32(smem + L::offB), kSmallBlock, 1024);
+    if (lane == 0 && me == 0) {
+      const SmemDesc dK = make_desc(smem_u32(smem + (DV ? DvSmem::offK : BwdSmem::offA)), 16, 1024), dV = make_desc(smem_u32(smem + BwdSmem::offB), 16, 1024);
+      const SmemDesc dQs = make_desc(smem_u32(smem + (DV ? DvSmem::offQ : BwdSmem::offS)), 16, 1024), dQg = make_desc(smem_u32(smem + BwdSmem::offG), kChanBlock, 1024);
+      const SmemDesc dOs = make_desc(smem_u32(smem + BwdSmem::offD), 16, 1024), dOg = make_desc(smem_u32(smem + DvSmem::offO), kChanBlock, 1024);
       bool ok = mbar_wait(kv_full, 0, abort_flag, p.status, kErrTimeoutFull);
-      auto issue_step = [&](int it) -> bool {   // S^T(it) (and dP^T(it)) into the buffers of parity it & 1
-        const int b = it & 1;
-        if (!mbar_wait(&q_full[b], (it >> 1) & 1, abort_flag, p.status, kErrTimeoutFull)) return false;
+      auto issue_S = [&](int it) -> bool {
+        const int s = stage_of(it);
+        if (!mbar_wait(&q_full[s], phase_of(it), abort_flag, p.status, kErrTimeoutFull)) return false;
         tc_fence_after();
-        issue_scores(tmem_base + S_COL + b * BC, dK, desc_off(dQk, b * kSmallTile), idesc_s);
-        umma_commit(&s_full[b]);
-        if (!DV) {
-          if (!mbar_wait(&do_full[0], do_phase(it), abort_flag, p.status, kErrTimeoutFull)) return false;
-          tc_fence_after();
-          issue_scores(tmem_base + DP_COL + b * BC, dV, dOk, idesc_s);
-          umma_commit(&dp_full[b]);
-          umma_commit(&do_empty[0]);       // dO_it was last read by dP^T(it)
-        } else {
-          umma_commit(&q_empty[b]);        // the dV pass needs Q_it only for the scores
-        }
+        issue_scores(tmem_base + (it & 1) * BC, dK, desc_off(dQs, s * kHalfTile));
+        umma_commit_pair(&s_full[s], both);
+        umma_commit_pair(&q_empty[s], both);
         return true;
       };
-      if (ok && n_iter > 0) ok = issue_step(0);
-      for (int it = 0; it < n_iter && ok; ++it) {
-        const int b = it & 1;
-        // dV pass: the next scores before this step's product.  dK pass: after it, as in the dQ kernel
-        if (DV && it + 1 < n_iter && !issue_step(it + 1)) { ok = false; break; }
-        if (!mbar_wait(&a_full[b], (it >> 1) & 1, abort_flag, p.status, kErrTimeoutOther)) { ok = false; break; }
+      auto issue_dP = [&](int it) -> bool {
+        if (!mbar_wait(do_full, it & 1, abort_flag, p.status, kErrTimeoutFull)) return false;
         tc_fence_after();
-        if (DV) {
-          if (!mbar_wait(&do_full[b], do_phase(it), abort_flag, p.status, kErrTimeoutFull)) { ok = false; break; }
-          tc_fence_after();
-          issue_accumulate(tmem_base + ACC_COL, tmem_base + S_COL + b * BC, b ? dOm2 : dOm, idesc_g, (uint32_t)it);
-          umma_commit(&do_empty[b]);       // dO_it was last read by dV(it)
-        } else {
-          issue_accumulate(tmem_base + ACC_COL, tmem_base + DP_COL + b * BC, desc_off(dQm, b * kSmallTile), idesc_g, (uint32_t)it);
-          umma_commit(&q_empty[b]);        // Q_it was last read by dK(it)
-          if (it + 1 < n_iter && !issue_step(it + 1)) { ok = false; break; }
+        issue_scores(tmem_base + ((it & 1) ^ 1) * BC, dV, dOs);
+        umma_commit_pair(dp_full, both);
+        umma_commit_pair(do_empty, both);
+        return true;
+      };
+      if (ok) ok = issue_S(0) && (DV || issue_dP(0));
+      for (int it = 0; it < n_iter && ok; ++it) {
+        const int s = stage_of(it);
+        if (it + 1 < n_iter) {
+          if (!DV && !mbar_wait(dp_read, it & 1, abort_flag, p.status, kErrTimeoutOther)) { ok = false; break; }
+          if (!issue_S(it + 1)) { ok = false; break; }
         }
+        if (!mbar_wait(DV ? &do_full[s] : g_full, phase_of(it), abort_flag, p.status, kErrTimeoutFull)) { ok = false; break; }
+        if (!mbar_wait(&a_full[s], phase_of(it), abort_flag, p.status, kErrTimeoutOther)) { ok = false; break; }
+        tc_fence_after();
+        const uint32_t a = tmem_base + (it & 1) * BC;
+        issue_accumulate(tmem_base + ACC_COL, a, a + BC / 2, DV ? desc_off(dOg, s * kHalfTile) : dQg, (uint32_t)it);
+        umma_commit_pair(DV ? &do_empty[s] : g_empty, both);
+        if (!DV && it + 1 < n_iter && !issue_dP(it + 1)) { ok = false; break; }   // over dS(it), which dK(it), issued before, reads
       }
-      if (ok) umma_commit(acc_done);
+      if (ok) umma_commit_pair(acc_done, both);
+    }
+  } else if (warp == 10) {
+    // ------------------------------------------------------------ the queries' statistics
+    for (int it = 0; it < n_iter; ++it) {
+      const int s = it & 1, q0 = (i_first + it / group) * BC;
+      const size_t base = (size_t)(hq0 + it % group) * p.T + ti.doc_start;
+      float lse[4], delta[4];
+#pragma unroll
+      for (int h = 0; h < 4; ++h) {
+        const int qq = q0 + h * 32 + lane;
+        const bool qok = qq < ti.doc_len;
+        lse[h] = qok ? -p.LSE[base + qq] * kLog2e : -INFINITY;   // exp2(-inf) = 0 for queries beyond the document
+        if (!DV) delta[h] = qok ? -p.delta[base + qq] : 0.f;
+      }
+      if (!mbar_wait(&stat_empty[s], ((it >> 1) & 1) ^ 1, abort_flag, p.status, kErrTimeoutOther)) break;
+      float* dst = stat + s * 2 * BC;
+#pragma unroll
+      for (int h = 0; h < 4; ++h) {
+        dst[h * 32 + lane] = lse[h];
+        if (!DV) dst[BC + h * 32 + lane] = delta[h];
+      }
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&stat_full[s]);
     }
   } else {
-    const int cw = warp - 2;
-    const int q = warp & 3;
+    const int q = warp & 3, half = (warp - 2) >> 2;
     const int r = q * 32 + lane;           // key row of the tile owned by this thread
     const int kvi = k0 + r;                // key index local to the document
     const bool key_ok = kvi < ti.doc_len;
     const uint32_t lane_addr = (uint32_t)(q * 32) << 16;
-    float* wstat = stat + cw * 128;        // this warp's copy of the step's per-query statistics
+    const uint32_t bar_read = cluster_addr(dp_read, leader), bar_a0 = cluster_addr(&a_full[0], leader), bar_a1 = cluster_addr(&a_full[1], leader);
     const bool sel_doc = SEL && ti.doc_len > p.sel_topk;
-    // this warp's 32 keys are one half of a selection word: 32-bit word [key tile][query].{x, y}
-    const uint32_t* sel_row = SEL ? reinterpret_cast<const uint32_t*>(p.sel + (size_t)((k0 >> 6) + (q >> 1)) * p.T + ti.doc_start) + (q & 1) : nullptr;
-    uint32_t kept[2] = {0u, 0u};           // bit c of kept[h]: query 32 h + c of the step keeps this thread's key
-    // statistics and selection words are loaded a step ahead, while the step before is worked on
-    float next_lse[2], next_delta[2];
-    uint32_t next_sel[2] = {0u, 0u};
-    auto fetch = [&](int it) {
-      const int q0 = (i_first + it / group) * BC, hq = hq0 + it % group;
+    // this warp's 32 keys are one half of a selection word: 32-bit word [key tile][query].{x, y}; queries before the key tile have none
+    const int kt = (k0 >> 6) + (q >> 1);
+    const uint32_t* sel_row = SEL ? reinterpret_cast<const uint32_t*>(p.sel + (size_t)kt * p.T + ti.doc_start) + (q & 1) : nullptr;
+    uint32_t kept[2] = {0u, 0u};           // bit c of kept[h]: query 64 half + 32 h + c of the step keeps this thread's key
+    uint32_t next_sel[2] = {0u, 0u};       // loaded a step ahead, while the step before is worked on
+    auto fetch = [&](int it) {             // the selection is the same for every query head: read and transposed once per query tile
+      if (!sel_doc || it % group != 0) return;
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
-        const int qq = q0 + h * 32 + lane;
-        const bool qok = qq < ti.doc_len;
-        const size_t idx = (size_t)hq * p.T + ti.doc_start + (qok ? qq : 0);
-        next_lse[h] = qok ? -p.LSE[idx] * kLog2e : -INFINITY;   // exp2(-inf) = 0 for queries beyond the document
-        if (!DV) next_delta[h] = qok ? -p.delta[idx] : 0.f;
-        // the selection is the same for every query head: read and transposed once per query tile
-        if (sel_doc && it % group == 0) next_sel[h] = qok ? __ldg(sel_row + 2 * (size_t)qq) : 0u;
+        const int qq = (i_first + it / group) * BC + half * 64 + h * 32 + lane;
+        next_sel[h] = qq < ti.doc_len && kt * 64 <= qq ? __ldg(sel_row + 2 * (size_t)qq) : 0u;
       }
     };
-    if (n_iter > 0) fetch(0);
+    fetch(0);
     bool ok = true;
     for (int it = 0; it < n_iter && ok; ++it) {
-      const int b = it & 1;
-      const int i = i_first + it / group;
-      const int q0 = i * BC;               // first query (column) of the step, local to the document
-      __syncwarp();                        // every lane is done with the previous step's statistics
-#pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        wstat[h * 32 + lane] = next_lse[h];
-        if (!DV) wstat[64 + h * 32 + lane] = next_delta[h];
-        if (sel_doc && it % group == 0) kept[h] = warp_transpose_bits(next_sel[h], lane);
-      }
-      __syncwarp();
+      const int s = stage_of(it);
+      const int q0 = (i_first + it / group) * BC + half * (BC / 2);   // first query (column) of this thread's half
+      if (sel_doc && it % group == 0) { kept[0] = warp_transpose_bits(next_sel[0], lane); kept[1] = warp_transpose_bits(next_sel[1], lane); }
       if (it + 1 < n_iter) fetch(it + 1);
-      const uint32_t s_addr = tmem_base + S_COL + b * BC + lane_addr, dp_addr = tmem_base + DP_COL + b * BC + lane_addr;
-      if (!mbar_wait(&s_full[b], (it >> 1) & 1, abort_flag, p.status, kErrTimeoutTmemFull)) { ok = false; break; }
+      const uint32_t s_addr = tmem_base + (it & 1) * BC + half * (BC / 2) + lane_addr, dp_addr = tmem_base + ((it & 1) ^ 1) * BC + half * (BC / 2) + lane_addr;
+      if (!mbar_wait(&stat_full[it & 1], (it >> 1) & 1, abort_flag, p.status, kErrTimeoutOther)) { ok = false; break; }
+      const float* lse2 = stat + (it & 1) * 2 * BC + half * (BC / 2);
+      if (!mbar_wait(&s_full[s], phase_of(it), abort_flag, p.status, kErrTimeoutTmemFull)) { ok = false; break; }
       tc_fence_after();
       // column c (query q0 + c) is visible to this key iff the key exists and (causal) kvi <= q0 + c
       const int cmin = !key_ok ? (1 << 30) : (p.causal ? kvi - q0 : -(1 << 30));
-      float pr[BC];
+      float pr[BC / 2];
 #pragma unroll
-      for (int c = 0; c < BC / 32; ++c) {
+      for (int c = 0; c < 2; ++c) {
         uint32_t sr[32];
         tmem_ld_32x32(s_addr + c * 32, sr);
         tmem_ld_wait();
 #pragma unroll
-        for (int u = 0; u < 32; ++u) {
-          const float x = fmaf(__uint_as_float(sr[u]), p.scale_log2, wstat[c * 32 + u]);
-          const bool hidden = sel_doc ? !((kept[c] >> u) & 1u) : (c * 32 + u < cmin);
-          pr[c * 32 + u] = hidden ? 0.f : ex2_approx(x);
+        for (int u = 0; u < 32; ++u) pr[c * 32 + u] = fmaf(__uint_as_float(sr[u]), p.scale_log2, lse2[c * 32 + u]);
+        const int first = cmin - c * 32;   // visible columns as bits; an interior tile has them all
+        const uint32_t seen = sel_doc ? kept[c] : first <= 0 ? 0xffffffffu : first < 32 ? 0xffffffffu << first : 0u;
+        if (!__all_sync(0xffffffffu, seen == 0xffffffffu)) {
+#pragma unroll
+          for (int u = 0; u < 32; ++u) if (!((seen >> u) & 1u)) pr[c * 32 + u] = -INFINITY;   // 2^-inf = 0
         }
-        if (DV) {
+#pragma unroll
+        for (int u = 0; u < 32; ++u) pr[c * 32 + u] = ex2_approx(pr[c * 32 + u]);
+        if constexpr (DV) {
           uint32_t pk[16];
 #pragma unroll
           for (int u = 0; u < 16; ++u) pk[u] = pack_bf16x2(pr[c * 32 + 2 * u], pr[c * 32 + 2 * u + 1]);
-          tmem_st_32x16(s_addr + c * 16, pk);   // P^T(it), packed, over the first 32 columns of the score buffer
+          tmem_st_32x16(s_addr + c * 16, pk);   // P^T(it), packed, over the first 32 of this thread's own 64 score columns
         }
       }
-      if (!DV) {
-        if (!mbar_wait(&dp_full[b], (it >> 1) & 1, abort_flag, p.status, kErrTimeoutTmemFull)) { ok = false; break; }
+      if constexpr (!DV) {
+        if (!mbar_wait(dp_full, it & 1, abort_flag, p.status, kErrTimeoutTmemFull)) { ok = false; break; }
         tc_fence_after();
 #pragma unroll
-        for (int c = 0; c < BC / 32; ++c) {
-          uint32_t dr[32];
+        for (int c = 0; c < 2; ++c) {
+          uint32_t dr[32], pk[16];
           tmem_ld_32x32(dp_addr + c * 32, dr);
           tmem_ld_wait();
-          uint32_t pk[16];
+          if (c == 1) {
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive_cluster(bar_read);
+          }
 #pragma unroll
           for (int u = 0; u < 16; ++u) {
-            const float d0 = pr[c * 32 + 2 * u] * (__uint_as_float(dr[2 * u]) + wstat[64 + c * 32 + 2 * u]);
-            const float d1 = pr[c * 32 + 2 * u + 1] * (__uint_as_float(dr[2 * u + 1]) + wstat[64 + c * 32 + 2 * u + 1]);
+            const float d0 = pr[c * 32 + 2 * u] * (__uint_as_float(dr[2 * u]) + lse2[BC + c * 32 + 2 * u]);
+            const float d1 = pr[c * 32 + 2 * u + 1] * (__uint_as_float(dr[2 * u + 1]) + lse2[BC + c * 32 + 2 * u + 1]);
             pk[u] = pack_bf16x2(d0, d1);
           }
-          tmem_st_32x16(dp_addr + c * 16, pk);  // dS^T(it), packed, over the first 32 columns of the dP^T buffer
+          tmem_st_32x16(s_addr + c * 16, pk);   // dS^T(it), packed, over the first 32 of this thread's own 64 score columns
         }
       }
       tmem_st_wait();
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(&a_full[b]);
+      if (lane == 0) {
+        mbar_arrive(&stat_empty[it & 1]);
+        mbar_arrive_cluster(s ? bar_a1 : bar_a0);
+      }
     }
     if (ok && mbar_wait(acc_done, 0, abort_flag, p.status, kErrTimeoutTmemFull)) {
       tc_fence_after();
-      if (p.parts > 1) {
-        // every MMA has completed and every load has been consumed: the tiles' shared memory takes this part of the sum
-        float* mine = reinterpret_cast<float*>(smem) + r * kPartPitch;
+      // parts: every MMA has completed and every load has been consumed, the tiles' shared memory takes this part of the sum
+      float* mine = reinterpret_cast<float*>(smem) + r * kPartPitch;
+      __nv_bfloat16* dst = (DV ? p.dV : p.dK) + ((size_t)(ti.doc_start + kvi) * p.Hkv + hkv) * HD;
 #pragma unroll 1
-        for (int c = 0; c < HD / 32; ++c) {
-          uint32_t o[32];
-          tmem_ld_32x32(tmem_base + ACC_COL + lane_addr + c * 32, o);
-          tmem_ld_wait();
+      for (int c = half * 4; c < half * 4 + 4; ++c) {
+        uint32_t o[32];
+        tmem_ld_32x32(tmem_base + ACC_COL + lane_addr + c * 32, o);
+        tmem_ld_wait();
+        if (p.parts > 1) {
 #pragma unroll
           for (int u = 0; u < 32; u += 4) *reinterpret_cast<uint4*>(mine + c * 32 + u) = make_uint4(o[u], o[u + 1], o[u + 2], o[u + 3]);
-        }
-      } else if (n_iter > 0) {
-        __nv_bfloat16* base = DV ? p.dV : p.dK;
-        const float f = DV ? 1.f : p.scale;
-        __nv_bfloat16* dst = base + ((size_t)(ti.doc_start + kvi) * p.Hkv + hkv) * HD;
-#pragma unroll 1
-        for (int c = 0; c < HD / 32; ++c) {
-          uint32_t o[32];
-          tmem_ld_32x32(tmem_base + ACC_COL + lane_addr + c * 32, o);
-          tmem_ld_wait();
-          if (key_ok) {
-#pragma unroll
-            for (int u = 0; u < 4; ++u) {
-              uint4 pk;
-              pk.x = pack_bf16x2(__uint_as_float(o[u * 8 + 0]) * f, __uint_as_float(o[u * 8 + 1]) * f);
-              pk.y = pack_bf16x2(__uint_as_float(o[u * 8 + 2]) * f, __uint_as_float(o[u * 8 + 3]) * f);
-              pk.z = pack_bf16x2(__uint_as_float(o[u * 8 + 4]) * f, __uint_as_float(o[u * 8 + 5]) * f);
-              pk.w = pack_bf16x2(__uint_as_float(o[u * 8 + 6]) * f, __uint_as_float(o[u * 8 + 7]) * f);
-              *reinterpret_cast<uint4*>(dst + c * 32 + u * 8) = pk;
-            }
-          }
+        } else if (key_ok) {
+          store_row32(dst + c * 32, o, DV ? 1.f : p.scale);
         }
       }
     }
   }
-  if (p.parts > 1) {
-    __syncwarp();
-    cluster_sync();        // every block of the cluster gets here, also after an abort
-    if (!*abort_flag) {
-      // the parts are summed in order of their rank; block `part` stores its share of the rows
-      const int rows = BR / p.parts, row0 = part * rows;
-      const float f = DV ? 1.f : p.scale;
-      __nv_bfloat16* base = DV ? p.dV : p.dK;
-      const uint32_t at = smem_u32(smem);
-      for (int i = threadIdx.x; i < rows * (HD / 4); i += THREADS) {
-        const int row = row0 + i / (HD / 4), col = i % (HD / 4) * 4;
-        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-        for (int s = 0; s < p.parts; ++s) {
-          const float4 x = ld_cluster_f4(at + (uint32_t)(row * kPartPitch + col) * 4, s);
-          v.x += x.x; v.y += x.y; v.z += x.z; v.w += x.w;
-        }
-        if (k0 + row < ti.doc_len)
-          *reinterpret_cast<uint2*>(base + ((size_t)(ti.doc_start + k0 + row) * p.Hkv + hkv) * HD + col) =
-              make_uint2(pack_bf16x2(v.x * f, v.y * f), pack_bf16x2(v.z * f, v.w * f));
-      }
-    }
-    __syncwarp();
-    cluster_sync();        // nobody leaves while its part is being read
-  }
+  if (p.parts > 1) store_parts(smem, p, abort_flag, rank, DV ? p.dV : p.dK, DV ? 1.f : p.scale, ti, k0, hkv);
   teardown(abort_flag, warp, tmem_base);
 }
 
@@ -871,9 +920,21 @@ __global__ void attn256_delta_kernel(const __nv_bfloat16* __restrict__ dO, const
 int make_map(CUtensorMap* m, const void* base, int T, int cols, long ld, int box_rows) {
   return vlmt_make_tmap_2d_bf16(m, base, (uint64_t)cols, (uint64_t)T, (uint64_t)ld * 2, 64, (uint32_t)box_rows);
 }
-template <typename K>
-int set_smem(K kern, int bytes) {
-  return (int)cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+template <typename K, typename... A>
+int launch(K kern, unsigned clusters, int cluster, int threads, int smem, cudaStream_t st, A&&... args) {
+  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  if (e != cudaSuccess) return (int)e;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(clusters * cluster); cfg.blockDim = dim3(threads); cfg.dynamicSmemBytes = smem; cfg.stream = st;
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.x = cluster; attr.val.clusterDim.y = 1; attr.val.clusterDim.z = 1;
+  cfg.attrs = &attr; cfg.numAttrs = 1;
+  return (int)cudaLaunchKernelEx(&cfg, kern, args...);
+}
+// clusters of a forward or dQ launch: query tiles (an upper bound) times heads
+unsigned query_pairs(const Params& p) {
+  return p.pair_heads ? (unsigned)(p.T / BR + p.n_docs + 1) * (p.Hq / 2) : (unsigned)(p.T / (2 * BR) + p.n_docs + 1) * p.Hq;
 }
 }  // namespace
 
@@ -884,17 +945,13 @@ extern "C" int vlmt_attn256_fwd(const void* q, const void* k, const void* v, voi
   CUtensorMap tq, tk, tv;
   int r;
   if ((r = make_map(&tq, q, T, Hq * HD, ldq, BR))) return 1000 + r;
-  if ((r = make_map(&tk, k, T, Hkv * HD, ldk, BC))) return 2000 + r;
+  if ((r = make_map(&tk, k, T, Hkv * HD, ldk, BC / 2))) return 2000 + r;
   if ((r = make_map(&tv, v, T, Hkv * HD, ldv, BC))) return 3000 + r;
   Params p{};
   p.O = reinterpret_cast<__nv_bfloat16*>(o); p.LSE = lse; p.cu = cu; p.n_docs = n_docs; p.T = T; p.Hq = Hq; p.Hkv = Hkv;
   p.scale = scale; p.scale_log2 = scale * kLog2e; p.causal = causal; p.status = status;
-  p.sel = reinterpret_cast<const uint2*>(sel); p.sel_topk = sel_topk;
-  auto kern = sel ? attn256_fwd_kernel<true> : attn256_fwd_kernel<false>;
-  if ((r = set_smem(kern, FwdSmem::kTotal))) return r;
-  const unsigned grid = (unsigned)(T / BR + n_docs + 1) * Hq;
-  kern<<<grid, THREADS, FwdSmem::kTotal, st>>>(tq, tk, tv, p);
-  return (int)cudaGetLastError();
+  p.sel = reinterpret_cast<const uint2*>(sel); p.sel_topk = sel_topk; p.pair_heads = Hq / Hkv % 2 == 0;
+  return launch(sel ? attn256_fwd_kernel<true> : attn256_fwd_kernel<false>, query_pairs(p), 2, kFwdThreads, FwdSmem::kTotal, st, tq, tk, tv, p);
 }
 
 extern "C" int vlmt_attn256_bwd(const void* dout, const void* q, const void* k, const void* v, const void* o, const float* lse, float* delta,
@@ -903,39 +960,35 @@ extern "C" int vlmt_attn256_bwd(const void* dout, const void* q, const void* k, 
   if (T <= 0 || n_docs <= 0) return 0;
   attn256_delta_kernel<<<(T * Hq * 32 + 255) / 256, 256, 0, st>>>(reinterpret_cast<const __nv_bfloat16*>(dout),
                                                                   reinterpret_cast<const __nv_bfloat16*>(o), delta, T, Hq);
-  CUtensorMap q_big, q_small, k_big, k_small, v_big, v_small, do_big, do_small;
+  CUtensorMap q128, q64, k128, k64, v128, v64, do128, do64;   // by the rows of a box: stationary tiles and channel halves 128, row halves 64
   int r;
   const long ldq = (long)Hq * HD, ldk = (long)Hkv * HD;
-  if ((r = make_map(&q_big, q, T, Hq * HD, ldq, BR)) || (r = make_map(&q_small, q, T, Hq * HD, ldq, BC))) return 1000 + r;
-  if ((r = make_map(&k_big, k, T, Hkv * HD, ldk, BR)) || (r = make_map(&k_small, k, T, Hkv * HD, ldk, BC))) return 2000 + r;
-  if ((r = make_map(&v_big, v, T, Hkv * HD, ldk, BR)) || (r = make_map(&v_small, v, T, Hkv * HD, ldk, BC))) return 3000 + r;
-  if ((r = make_map(&do_big, dout, T, Hq * HD, ldq, BR)) || (r = make_map(&do_small, dout, T, Hq * HD, ldq, BC))) return 4000 + r;
+  if ((r = make_map(&q128, q, T, Hq * HD, ldq, BC)) || (r = make_map(&q64, q, T, Hq * HD, ldq, BC / 2))) return 1000 + r;
+  if ((r = make_map(&k128, k, T, Hkv * HD, ldk, BC)) || (r = make_map(&k64, k, T, Hkv * HD, ldk, BC / 2))) return 2000 + r;
+  if ((r = make_map(&v128, v, T, Hkv * HD, ldk, BC)) || (r = make_map(&v64, v, T, Hkv * HD, ldk, BC / 2))) return 3000 + r;
+  if ((r = make_map(&do128, dout, T, Hq * HD, ldq, BC)) || (r = make_map(&do64, dout, T, Hq * HD, ldq, BC / 2))) return 4000 + r;
   Params p{};
   p.dQ = reinterpret_cast<__nv_bfloat16*>(dq); p.dK = reinterpret_cast<__nv_bfloat16*>(dk); p.dV = reinterpret_cast<__nv_bfloat16*>(dv);
   p.LSE = const_cast<float*>(lse); p.delta = delta; p.cu = cu; p.n_docs = n_docs; p.T = T; p.Hq = Hq; p.Hkv = Hkv;
   p.scale = scale; p.scale_log2 = scale * kLog2e; p.causal = causal; p.status = status;
-  p.sel = reinterpret_cast<const uint2*>(sel); p.sel_topk = sel_topk;
-  auto k_dv = sel ? attn256_bwd_dkv_kernel<true, true> : attn256_bwd_dkv_kernel<true, false>;
-  auto k_dk = sel ? attn256_bwd_dkv_kernel<false, true> : attn256_bwd_dkv_kernel<false, false>;
-  auto k_dq = sel ? attn256_bwd_dq_kernel<true> : attn256_bwd_dq_kernel<false>;
-  if ((r = set_smem(k_dv, BwdSmem::kTotal)) || (r = set_smem(k_dk, BwdSmem::kTotal)) || (r = set_smem(k_dq, BwdSmem::kTotal))) return r;
-  const unsigned tiles = (unsigned)(T / BR + n_docs + 1);
-  // Key tiles times key heads are few and of very different length (a key tile meets every later query of its document, with every
-  // query head of its group): the heads of a group are split over a cluster of up to 4 blocks until about 5 blocks per SM are there.
-  // Sparse attention forward and backward with 1 / 2 / 4 parts: 12301 tokens, 2 key heads 3956 / 3196 / 3106 us, 3000 tokens 871 / 544 / 374;
-  // dense, 16384 tokens, 4 key heads, dK + dV 2.50 to 2.97 / 2.41 / 2.81 ms.
+  p.sel = reinterpret_cast<const uint2*>(sel); p.sel_topk = sel_topk; p.pair_heads = Hq / Hkv % 2 == 0;
+  // Pairs of key tiles times key heads are few and of very different length (a key tile meets every later query of its document, with
+  // every query head of its group): the heads of a group are split over a cluster of up to 4 pairs until about 1.5 pairs per pair of SMs
+  // are there, over 4 only where documents are long enough to leave a pair some steps.  dV + dK with 1 / 2 / 4 parts, us: 16384 tokens in 5
+  // documents, 16 / 4 heads 1713 / 1811 / 1811; 8192 in 1 1028 / 1093 / 1268; 5000 in 9 270 / 201 / 278; 3000 in 3 246 / 143 / 174; 1500 in 1
+  // 214 / 114 / 90; sparse, 16 / 2 heads, 12301 in 4 1328 / 982 / 1015; 3000 in 1 741 / 403 / 224.
   int dev = 0, sms = 148;
   if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  const int max_parts = T >= 1280l * n_docs ? 4 : 2;
   p.parts = 1;
-  while (p.parts < 4 && Hq / Hkv % (2 * p.parts) == 0 && (long)(T / BR + 1) * Hkv * p.parts < 5l * sms) p.parts *= 2;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(tiles * Hkv * p.parts); cfg.blockDim = dim3(THREADS); cfg.dynamicSmemBytes = BwdSmem::kTotal; cfg.stream = st;
-  cudaLaunchAttribute attr;
-  attr.id = cudaLaunchAttributeClusterDimension;
-  attr.val.clusterDim.x = p.parts; attr.val.clusterDim.y = 1; attr.val.clusterDim.z = 1;
-  cfg.attrs = &attr; cfg.numAttrs = p.parts > 1 ? 1 : 0;
-  if ((r = (int)cudaLaunchKernelEx(&cfg, k_dv, q_small, k_big, v_big, do_small, p))) return r;
-  if ((r = (int)cudaLaunchKernelEx(&cfg, k_dk, q_small, k_big, v_big, do_small, p))) return r;
-  k_dq<<<tiles * Hq, THREADS, BwdSmem::kTotal, st>>>(q_big, k_small, v_small, do_big, p);
-  return (int)cudaGetLastError();
+  while (p.parts < max_parts && Hq / Hkv % (2 * p.parts) == 0 && 4l * (T / (2 * BR) + 1) * Hkv * p.parts < 3l * sms) p.parts *= 2;
+  const unsigned clusters = (unsigned)(T / (2 * BR) + n_docs + 1) * Hkv;
+  if ((r = launch(sel ? attn256_bwd_dkv_kernel<true, true> : attn256_bwd_dkv_kernel<true, false>, clusters, 2 * p.parts, kDkvThreads, DvSmem::kTotal, st,
+                  q64, q128, k128, v128, do128, p)))
+    return r;
+  if ((r = launch(sel ? attn256_bwd_dkv_kernel<false, true> : attn256_bwd_dkv_kernel<false, false>, clusters, 2 * p.parts, kDkvThreads, BwdSmem::kTotal, st,
+                  q64, q128, k128, v128, do64, p)))
+    return r;
+  return launch(sel ? attn256_bwd_dq_kernel<true> : attn256_bwd_dq_kernel<false>, query_pairs(p), 2, kBwdThreads, BwdSmem::kTotal, st, q128, k64, k128, v64,
+                do128, p);
 }

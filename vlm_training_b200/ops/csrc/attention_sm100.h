@@ -11,7 +11,7 @@ extern "C" {
 // fused projection are read in place; d a multiple of 8 up to 128, or 256.  o [T,Hq,d] contiguous; lse [Hq,T] (natural log).
 // cu: int32 [n_docs+1] device pointer.  The kernels work on 64- or 128-wide tiles: TMA zero-fills the channels between d
 // and the tile width, the contractions over the head dim stop at the next multiple of 16 and the output-side products are
-// only that wide.  d = 256: the single-tile kernels of attention256_sm100.cu (heads contiguous).
+// only that wide.  d = 256: the kernels of attention256_sm100.cu (heads contiguous).
 int vlmt_attn_fwd(const void* q, const void* k, const void* v, void* o, float* lse, const int* cu, int n_docs, int T, int Hq, int Hkv,
                   int d, long ldq, long hsq, long ldk, long hsk, long ldv, long hsv, float scale, int causal, int* status, cudaStream_t st);
 // dout, o, dq, dk, dv contiguous; delta is fp32 scratch [Hq,T]

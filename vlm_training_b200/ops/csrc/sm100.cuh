@@ -292,9 +292,11 @@ __device__ __forceinline__ float4 ld_cluster_f4(uint32_t addr, uint32_t rank) {
                : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr), "r"(rank) : "memory");
   return v;
 }
-// arrive on a barrier of another block of the cluster (address from cluster_addr)
+// Arrive on a barrier of another block of the cluster (address from cluster_addr).  What such an arrival announces is tensor memory that
+// was read or written, ordered by the tcgen05 fences on both sides; a release at cluster scope would wait for every outstanding access
+// of the thread to memory as well (about 1900 cycles in every step of the attention kernels).
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar_addr) {
-  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar_addr) : "memory");
+  asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(bar_addr) : "memory");
 }
 template <int kCols>
 __device__ __forceinline__ void tmem_alloc_pair(uint32_t* smem_result) {
@@ -312,10 +314,11 @@ __device__ __forceinline__ void tma_load_2d_pair(void* smem_dst, const CUtensorM
       ::"r"(smem_u32(smem_dst)), "l"(reinterpret_cast<uint64_t>(map)), "r"(bar_addr), "r"(x), "r"(y)
       : "memory");
 }
-// arrive on the barrier at this offset in both blocks once every MMA issued so far by this thread has completed
-__device__ __forceinline__ void umma_commit_pair(uint64_t* bar) {
+// arrive on the barrier at this offset in both blocks once every MMA issued so far by this thread has completed; `blocks`: bit mask
+// of the pair's ranks in its cluster
+__device__ __forceinline__ void umma_commit_pair(uint64_t* bar, uint16_t blocks = 3) {
   asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
-               ::"r"(smem_u32(bar)), "h"((uint16_t)3) : "memory");
+               ::"r"(smem_u32(bar)), "h"(blocks) : "memory");
 }
 template <int ACC, bool FP8 = false>
 __device__ __forceinline__ void umma_ss_pair(uint32_t tmem_d, SmemDesc a, SmemDesc b, uint32_t idesc, uint32_t flag = 0) {
@@ -329,6 +332,14 @@ __device__ __forceinline__ void umma_ss_pair(uint32_t tmem_d, SmemDesc a, SmemDe
                  "tcgen05.mma.cta_group::2.kind::f16 [%0], da, db, %5, p;\n\t}"
                  ::"r"(tmem_d), "r"(a.lo), "r"(a.hi), "r"(b.lo), "r"(b.hi), "r"(idesc), "r"(on) : "memory");
   }
+}
+// A operand from tensor memory: each block's own 128 rows
+template <int ACC>
+__device__ __forceinline__ void umma_ts_pair(uint32_t tmem_d, uint32_t tmem_a, SmemDesc b, uint32_t idesc, uint32_t flag = 0) {
+  const uint32_t on = ACC == 2 ? flag : (uint32_t)ACC;
+  asm volatile("{\n\t.reg .pred p;\n\t.reg .b64 db;\n\tsetp.ne.b32 p, %5, 0;\n\tmov.b64 db, {%2, %3};\n\t"
+               "tcgen05.mma.cta_group::2.kind::f16 [%0], [%1], db, %4, p;\n\t}"
+               ::"r"(tmem_d), "r"(tmem_a), "r"(b.lo), "r"(b.hi), "r"(idesc), "r"(on) : "memory");
 }
 
 }  // namespace sm100

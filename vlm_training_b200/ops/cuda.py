@@ -425,7 +425,7 @@ def _pad_heads(t, d_to):
 
 def attention_varlen(q, k, v, cu_seqlens, max_seqlen, causal=True, scale=None):
     """Varlen attention over packed rows.  Head sizes that are a multiple of 8 up to 128 run as they are (the kernels' tiles
-    are 64 or 128 wide and TMA zero-fills the rest), 256 on the single-tile kernels; sizes in between are zero-padded."""
+    are 64 or 128 wide and TMA zero-fills the rest), 256 on the CTA-pair kernels; sizes in between are zero-padded."""
     D = q.shape[-1]
     scale = scale if scale is not None else 1.0 / math.sqrt(D)
     if q.dtype != torch.bfloat16:
