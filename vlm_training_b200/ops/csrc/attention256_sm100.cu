@@ -328,56 +328,62 @@ attn256_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
 #pragma unroll
         for (int i = 0; i < BC; ++i) if (i > limit) s[i] = 0xff800000u;  // -inf
       }
-      float mx0 = -INFINITY, mx1 = -INFINITY;
+      // The running maximum moves per 64 keys and the row sum is formed per 64 keys, whatever the width of a step: the probabilities keep
+      // the bits that they have under 64-row tiles, and with them FP8 linears behind this kernel the scales of their tensors.
+      const float m_old = m_used;
 #pragma unroll
-      for (int i = 0; i < BC; i += 4) {
-        mx0 = fmax3(mx0, __uint_as_float(s[i]), __uint_as_float(s[i + 1]));
-        mx1 = fmax3(mx1, __uint_as_float(s[i + 2]), __uint_as_float(s[i + 3]));
+      for (int h = 0; h < 2; ++h) {
+        float mx0 = -INFINITY, mx1 = -INFINITY;
+#pragma unroll
+        for (int i = h * 64; i < h * 64 + 64; i += 4) {
+          mx0 = fmax3(mx0, __uint_as_float(s[i]), __uint_as_float(s[i + 1]));
+          mx1 = fmax3(mx1, __uint_as_float(s[i + 2]), __uint_as_float(s[i + 3]));
+        }
+        const float mx = fmaxf(mx0, mx1) * p.scale_log2;   // the scale is positive: it commutes with max
+        if (j == 0 && h == 0) m_used = (!SEL && mx == -INFINITY) ? 0.f : mx;
+        else if (mx > m_used + kRescaleThreshold) m_used = mx;
       }
-      const float mx = fmaxf(mx0, mx1) * p.scale_log2;   // the scale is positive: it commutes with max
-      if (j == 0) {
-        m_used = (!SEL && mx == -INFINITY) ? 0.f : mx;
-      } else {
-        const bool grow = mx > m_used + kRescaleThreshold;
-        if (__any_sync(0xffffffffu, grow)) {
-          // O must hold every earlier tile and the tensor core must not touch it: P(j - 1) V has completed, P(j) V is not
-          // issued before this warp publishes P(j)
-          if (!mbar_wait(pv_done, (j - 1) & 1, abort_flag, p.status, kErrTimeoutTmemFull)) { ok = false; break; }
-          tc_fence_after();
-          const float alpha = grow ? ex2_approx(m_used - mx) : 1.f;
-          if (grow) m_used = mx;
-          l *= alpha;
+      const bool grow = j > 0 && m_used != m_old;
+      if (__any_sync(0xffffffffu, grow)) {
+        // O must hold every earlier tile and the tensor core must not touch it: P(j - 1) V has completed, P(j) V is not
+        // issued before this warp publishes P(j)
+        if (!mbar_wait(pv_done, (j - 1) & 1, abort_flag, p.status, kErrTimeoutTmemFull)) { ok = false; break; }
+        tc_fence_after();
+        const float alpha = grow ? ex2_approx(m_old - m_used) : 1.f;
+        l *= alpha;
 #pragma unroll 1
-          for (int c = 0; c < HD / 32; ++c) {
-            uint32_t o[32];
-            tmem_ld_32x32(o_addr + c * 32, o);
-            tmem_ld_wait();
+        for (int c = 0; c < HD / 32; ++c) {
+          uint32_t o[32];
+          tmem_ld_32x32(o_addr + c * 32, o);
+          tmem_ld_wait();
 #pragma unroll
-            for (int i = 0; i < 32; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
-            tmem_st_32x32(o_addr + c * 32, o);
-          }
+          for (int i = 0; i < 32; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
+          tmem_st_32x32(o_addr + c * 32, o);
         }
       }
       const float neg_m = (SEL && m_used == -INFINITY) ? 0.f : -m_used;
-      float sum0 = 0.f, sum1 = 0.f;
 #pragma unroll
-      for (int c = 0; c < BC / 32; ++c) {
-        uint32_t pk[16];
+      for (int h = 0; h < 2; ++h) {
+        float sum0 = 0.f, sum1 = 0.f;
 #pragma unroll
-        for (int i = 0; i < 16; ++i) {
-          const float e0 = ex2_approx(fmaf(__uint_as_float(s[c * 32 + 2 * i]), p.scale_log2, neg_m));
-          const float e1 = ex2_approx(fmaf(__uint_as_float(s[c * 32 + 2 * i + 1]), p.scale_log2, neg_m));
-          sum0 += e0;
-          sum1 += e1;
-          pk[i] = pack_bf16x2(e0, e1);
+        for (int c = 2 * h; c < 2 * h + 2; ++c) {
+          uint32_t pk[16];
+#pragma unroll
+          for (int i = 0; i < 16; ++i) {
+            const float e0 = ex2_approx(fmaf(__uint_as_float(s[c * 32 + 2 * i]), p.scale_log2, neg_m));
+            const float e1 = ex2_approx(fmaf(__uint_as_float(s[c * 32 + 2 * i + 1]), p.scale_log2, neg_m));
+            sum0 += e0;
+            sum1 += e1;
+            pk[i] = pack_bf16x2(e0, e1);
+          }
+          tmem_st_32x16(s_addr + c * 16, pk);   // P(j) over the first 64 columns of its score buffer
         }
-        tmem_st_32x16(s_addr + c * 16, pk);   // P(j) over the first 64 columns of its score buffer
+        l += sum0 + sum1;
       }
       tmem_st_wait();
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive_cluster(b ? p_bar1 : p_bar0);
-      l += sum0 + sum1;
     }
     if (ok && J > 0 && mbar_wait(o_done, 0, abort_flag, p.status, kErrTimeoutTmemFull)) {
       tc_fence_after();
