@@ -29,6 +29,7 @@
 #include "attention_sm100.h"
 #include "sm100.cuh"
 
+#include "pdl.cuh"
 #include <cuda_bf16.h>
 #include <math.h>
 
@@ -211,6 +212,7 @@ template <bool SEL>
 __global__ void __launch_bounds__(kFwdThreads, 1)
 attn256_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                    const __grid_constant__ CUtensorMap tmV, Params p) {
+  pdl_wait();
   using L = FwdSmem;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = align_smem<L::kSlack>(smem_raw);
@@ -263,6 +265,7 @@ attn256_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
         if (rank == 0) mbar_expect_tx(&v_full[s], 2 * kHalfTile);
         load_chans(smem + L::offV + s * kHalfTile, &tmV, cluster_addr(&v_full[s], 0), hkv * HD, krow, rank);
       }
+      pdl_trigger();   // the last loads are on their way
     }
   } else if (warp == 1) {
     if (lane == 0 && rank == 0) {
@@ -432,6 +435,7 @@ template <bool SEL>
 __global__ void __launch_bounds__(kBwdThreads, 1)
 attn256_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmK2,
                       const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmdO, Params p) {
+  pdl_wait();
   using L = BwdSmem;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = align_smem<L::kSlack>(smem_raw);
@@ -486,6 +490,7 @@ attn256_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
         if (rank == 0) mbar_expect_tx(kg_full, 2 * kHalfTile);
         load_chans(smem + L::offG, &tmK2, bar_g, hkv * HD, krow, rank);
       }
+      pdl_trigger();   // the last loads are on their way
     }
   } else if (warp == 1) {
     if (lane == 0 && rank == 0) {
@@ -658,6 +663,7 @@ template <bool DV, bool SEL>
 __global__ void __launch_bounds__(kDkvThreads, 1)
 attn256_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmQ2, const __grid_constant__ CUtensorMap tmK,
                        const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmdO, Params p) {
+  pdl_wait();
   constexpr int offStat = DV ? DvSmem::offStat : BwdSmem::offStat, offBar = DV ? DvSmem::offBar : BwdSmem::offBar;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = align_smem<DV ? DvSmem::kSlack : BwdSmem::kSlack>(smem_raw);
@@ -727,6 +733,7 @@ attn256_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
           load_chans(smem + BwdSmem::offG, &tmQ2, cluster_addr(g_full, leader), col, row, me);
         }
       }
+      pdl_trigger();   // the last loads are on their way
     }
   } else if (warp == 1) {
     if (lane == 0 && me == 0) {
@@ -905,6 +912,7 @@ attn256_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
 // delta[h, t] = sum_d dO[t,h,d] * O[t,h,d]
 __global__ void attn256_delta_kernel(const __nv_bfloat16* __restrict__ dO, const __nv_bfloat16* __restrict__ O, float* __restrict__ delta,
                                      int T, int H) {
+  pdl_begin();
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (warp >= T * H) return;
   const int t = warp / H, h = warp - t * H;
@@ -930,13 +938,7 @@ template <typename K, typename... A>
 int launch(K kern, unsigned clusters, int cluster, int threads, int smem, cudaStream_t st, A&&... args) {
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (e != cudaSuccess) return (int)e;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(clusters * cluster); cfg.blockDim = dim3(threads); cfg.dynamicSmemBytes = smem; cfg.stream = st;
-  cudaLaunchAttribute attr;
-  attr.id = cudaLaunchAttributeClusterDimension;
-  attr.val.clusterDim.x = cluster; attr.val.clusterDim.y = 1; attr.val.clusterDim.z = 1;
-  cfg.attrs = &attr; cfg.numAttrs = 1;
-  return (int)cudaLaunchKernelEx(&cfg, kern, args...);
+  return launch_pdl(kern, dim3(clusters * cluster), dim3(threads), (size_t)smem, st, cluster, args...);
 }
 // clusters of a forward or dQ launch: query tiles (an upper bound) times heads
 unsigned query_pairs(const Params& p) {
@@ -964,7 +966,7 @@ extern "C" int vlmt_attn256_bwd(const void* dout, const void* q, const void* k, 
                                 void* dq, void* dk, void* dv, const int* cu, int n_docs, int T, int Hq, int Hkv, float scale, int causal,
                                 const void* sel, int sel_topk, int* status, cudaStream_t st) {
   if (T <= 0 || n_docs <= 0) return 0;
-  attn256_delta_kernel<<<(T * Hq * 32 + 255) / 256, 256, 0, st>>>(reinterpret_cast<const __nv_bfloat16*>(dout),
+  launch_pdl(attn256_delta_kernel, dim3((T * Hq * 32 + 255) / 256), dim3(256), 0, st, 1, reinterpret_cast<const __nv_bfloat16*>(dout),
                                                                   reinterpret_cast<const __nv_bfloat16*>(o), delta, T, Hq);
   CUtensorMap q128, q64, k128, k64, v128, v64, do128, do64;   // by the rows of a box: stationary tiles and channel halves 128, row halves 64
   int r;

@@ -27,6 +27,7 @@
 #include "attention_sm100.h"
 #include "sm100.cuh"
 
+#include "pdl.cuh"
 #include <cuda_bf16.h>
 #include <math.h>
 
@@ -101,6 +102,7 @@ template <int D>
 __global__ void __launch_bounds__(ATT_THREADS, 1)
 attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                 const __grid_constant__ CUtensorMap tmV, FwdParams p) {
+  pdl_wait();
   using L = FwdSmem<D>;
   constexpr int DB = D / 64;  // 64-column blocks along the head dim
   extern __shared__ uint8_t smem_raw[];
@@ -171,6 +173,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
 #pragma unroll
         for (int b = 0; b < DB; ++b) tma_load_3d(smem + L::offV + s * L::kKV + b * 16384, &tmV, &v_full[s], 64 * b, hkv, krow);
       }
+      pdl_trigger();   // the last loads are on their way
     }
   } else if (warp == 1) {
     if (lane == 0) {
@@ -351,6 +354,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
 // Channels 32 apart are added in one lane and the butterfly runs from distance 16 down to 1, the order of a warp per head.
 __global__ void __launch_bounds__(256) attn_delta_kernel(const __nv_bfloat16* __restrict__ dO, const __nv_bfloat16* __restrict__ O,
                                                          float* __restrict__ delta, int T, int H, int D, int vec) {
+  pdl_begin();
   const long item = (blockIdx.x * (long)blockDim.x + threadIdx.x) >> 3;
   const int l = threadIdx.x & 7;
   const bool there = item < (long)T * H;   // every lane takes part in the shuffles
@@ -454,6 +458,7 @@ template <int D>
 __global__ void __launch_bounds__(64 + 32 * NCW, 1)
 attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                      const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmdO, BwdParams p) {
+  pdl_wait();
   using L = BwdSmem<D>;
   constexpr int DB = D / 64;
   extern __shared__ uint8_t smem_raw[];
@@ -525,6 +530,7 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
         for (int b = 0; b < DB; ++b) tma_load_3d(smem + L::offD + ds * L::kTile + b * 16384, &tmdO, &do_full[ds], 64 * b, hq, qrow);
         if (++qs == 3) { qs = 0; qph ^= 1; }
       }
+      pdl_trigger();   // the last loads are on their way
     }
   } else if (warp == 1) {
     if (lane == 0) {
@@ -740,6 +746,7 @@ template <int D>
 __global__ void __launch_bounds__(64 + 32 * NCW, 1)
 attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                    const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmdO, BwdParams p) {
+  pdl_wait();
   using L = BwdSmem<D>;
   constexpr int DB = D / 64;
   extern __shared__ uint8_t smem_raw[];
@@ -809,6 +816,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
         for (int b = 0; b < DB; ++b) tma_load_3d(smem + L::offD + vs * L::kTile + b * 16384, &tmV, &v_full[vs], 64 * b, hkv, krow);
         if (++ks == 3) { ks = 0; kph ^= 1; }
       }
+      pdl_trigger();   // the last loads are on their way
     }
   } else if (warp == 1) {
     if (lane == 0) {
@@ -1026,10 +1034,10 @@ extern "C" int vlmt_attn_fwd(const void* q, const void* k, const void* v, void* 
   const unsigned grid = (unsigned)(T / (2 * BM) + n_docs + 1) * Hq;
   if (D == 128) {
     if ((r = set_smem(attn_fwd_kernel<128>, FwdSmem<128>::kTotal))) return r;
-    attn_fwd_kernel<128><<<grid, ATT_THREADS, FwdSmem<128>::kTotal, st>>>(tq, tk, tv, p);
+    launch_pdl(attn_fwd_kernel<128>, dim3(grid), dim3(ATT_THREADS), FwdSmem<128>::kTotal, st, 1, tq, tk, tv, p);
   } else {
     if ((r = set_smem(attn_fwd_kernel<64>, FwdSmem<64>::kTotal))) return r;
-    attn_fwd_kernel<64><<<grid, ATT_THREADS, FwdSmem<64>::kTotal, st>>>(tq, tk, tv, p);
+    launch_pdl(attn_fwd_kernel<64>, dim3(grid), dim3(ATT_THREADS), FwdSmem<64>::kTotal, st, 1, tq, tk, tv, p);
   }
   return (int)cudaGetLastError();
 }
@@ -1046,7 +1054,7 @@ extern "C" int vlmt_attn_bwd(const void* dout, const void* q, const void* k, con
   const int D = d <= 64 ? 64 : 128;
   {
     const int vec = ((reinterpret_cast<uintptr_t>(dout) | reinterpret_cast<uintptr_t>(o)) & 7) == 0;
-    attn_delta_kernel<<<(unsigned)(((long)T * Hq + 31) / 32), 256, 0, st>>>(reinterpret_cast<const __nv_bfloat16*>(dout),
+    launch_pdl(attn_delta_kernel, dim3((unsigned)(((long)T * Hq + 31) / 32)), dim3(256), 0, st, 1, reinterpret_cast<const __nv_bfloat16*>(dout),
                                                                             reinterpret_cast<const __nv_bfloat16*>(o), delta, T, Hq, d, vec);
   }
   CUtensorMap tq, tk, tv, tdo;
@@ -1074,8 +1082,8 @@ extern "C" int vlmt_attn_bwd(const void* dout, const void* q, const void* k, con
     int rr;
     if ((rr = set_smem(attn_bwd_dkdv_kernel<Dh>, BwdSmem<Dh>::kTotal))) return rr;
     if ((rr = set_smem(attn_bwd_dq_kernel<Dh>, BwdSmem<Dh>::kTotal))) return rr;
-    attn_bwd_dkdv_kernel<Dh><<<grid_kv, 64 + 32 * NCW, BwdSmem<Dh>::kTotal, st>>>(tq, tk, tv, tdo, p);
-    attn_bwd_dq_kernel<Dh><<<grid_q, 64 + 32 * NCW, BwdSmem<Dh>::kTotal, st>>>(tq, tk, tv, tdo, p);
+    launch_pdl(attn_bwd_dkdv_kernel<Dh>, dim3(grid_kv), dim3(64 + 32 * NCW), BwdSmem<Dh>::kTotal, st, 1, tq, tk, tv, tdo, p);
+    launch_pdl(attn_bwd_dq_kernel<Dh>, dim3(grid_q), dim3(64 + 32 * NCW), BwdSmem<Dh>::kTotal, st, 1, tq, tk, tv, tdo, p);
     return 0;
   };
   if (D == 128) r = launch(std::integral_constant<int, 128>{});

@@ -16,6 +16,7 @@
 #include "gemm_sm100.h"
 #include "sm100.cuh"
 
+#include "pdl.cuh"
 #include <cuda_bf16.h>
 
 namespace {
@@ -35,6 +36,7 @@ struct ScoreParams {
 
 __global__ void __launch_bounds__(128, 1)
 dsa_index_scores_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK, ScoreParams p) {
+  pdl_begin();
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   constexpr int kQ = 4 * 16384, kK = 16384;         // [128 x 256] and [128 x 64] bf16 tiles
@@ -196,6 +198,7 @@ struct TopkParams {
 // positions, which is as far as the attention kernels read.
 template <bool BITS>
 __global__ void __launch_bounds__(TOPK_THREADS) dsa_topk_kernel(TopkParams p) {
+  pdl_begin();
   extern __shared__ uint32_t keys[];            // n keys, then the histogram (2048 bins) and scratch
   const int b = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int n = p.q_pos0 + b + 1;               // causal keys of this query
@@ -277,7 +280,7 @@ extern "C" int vlmt_dsa_index_scores(const void* iq, const void* ik, const float
   const int smem = 4 * 16384 + 16384 + 64 + 1024;
   if (cudaFuncSetAttribute(dsa_index_scores_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return -4;
   dim3 grid((B + 127) / 128, (n_keys + 127) / 128);
-  dsa_index_scores_kernel<<<grid, 128, smem, st>>>(tq, tk, p);
+  launch_pdl(dsa_index_scores_kernel, dim3(grid), dim3(128), smem, st, 1, tq, tk, p);
   return cudaGetLastError() == cudaSuccess ? 0 : -5;
 }
 
@@ -289,7 +292,7 @@ int launch_topk(const TopkParams& p, cudaStream_t st) {
   const int smem = (((n_max + 3) & ~3) + 2048 + 4 + 16) * 4;
   if (smem > 227 * 1024) return -3;
   if (cudaFuncSetAttribute(dsa_topk_kernel<BITS>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return -4;
-  dsa_topk_kernel<BITS><<<p.B, TOPK_THREADS, smem, st>>>(p);
+  launch_pdl(dsa_topk_kernel<BITS>, dim3(p.B), dim3(TOPK_THREADS), smem, st, 1, p);
   return cudaGetLastError() == cudaSuccess ? 0 : -5;
 }
 }  // namespace

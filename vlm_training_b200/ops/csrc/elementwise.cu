@@ -9,6 +9,7 @@
 #include "elementwise.h"
 #include "no_alloc_entry.h"
 
+#include "pdl.cuh"
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -330,6 +331,7 @@ template <typename WT, int VPT>
 __global__ void __launch_bounds__(kRT) rmsnorm_fwd_tile_kernel(const bf16* __restrict__ x, const bf16* __restrict__ res,
                                                               const WT* __restrict__ w, bf16* __restrict__ y, bf16* __restrict__ r_out,
                                                               float* __restrict__ rstd, int rows, int D, float eps, int offset) {
+  pdl_begin();
   constexpr int RR = TileRows<VPT>::value;
   extern __shared__ uint4 ring[];
   __shared__ float sm[2 * kRR * 8];
@@ -419,6 +421,7 @@ __global__ void __launch_bounds__(kRT) rmsnorm_bwd_tile_kernel(const bf16* __res
                                                               const WT* __restrict__ w, const float* __restrict__ rstd,
                                                               const bf16* __restrict__ dres, bf16* __restrict__ dx,
                                                               float* __restrict__ dw_partial, int rows, int D, int offset) {
+  pdl_begin();
   constexpr int RR = TileRows<VPT>::value;
   extern __shared__ uint4 ring[];
   __shared__ float sm[2 * kRR * 8];
@@ -521,6 +524,7 @@ __global__ void __launch_bounds__(kRT) layernorm_fwd_tile_kernel(const bf16* __r
                                                                 const bf16* __restrict__ b, bf16* __restrict__ y,
                                                                 float* __restrict__ mean, float* __restrict__ rstd, int rows, int D,
                                                                 float eps) {
+  pdl_begin();
   constexpr int RR = TileRows<VPT>::value;
   extern __shared__ uint4 ring[];
   __shared__ float sm[2 * kRR * 8];
@@ -609,6 +613,7 @@ __global__ void __launch_bounds__(kRT) layernorm_bwd_tile_kernel(const bf16* __r
                                                                 const float* __restrict__ rstd, bf16* __restrict__ dx,
                                                                 float* __restrict__ dw_partial, float* __restrict__ db_partial, int rows,
                                                                 int D) {
+  pdl_begin();
   constexpr int RR = TileRows<VPT>::value;
   extern __shared__ uint4 ring[];
   __shared__ float sm[2 * 2 * kRR * 8];
@@ -720,6 +725,7 @@ __global__ void __launch_bounds__(kLnWarpsFwd * 32) layernorm_fwd_warp_kernel(co
                                                                              const bf16* __restrict__ b, bf16* __restrict__ y,
                                                                              float* __restrict__ mean, float* __restrict__ rstd, int rows,
                                                                              int D, float eps) {
+  pdl_begin();
   extern __shared__ uint4 dyn[];
   float* sw = reinterpret_cast<float*>(dyn);        // weights and bias as floats, [D] each
   float* sb = sw + D;
@@ -797,6 +803,7 @@ __global__ void __launch_bounds__(kLnWarpsFwd * 32) layernorm_fwd_warp_kernel(co
 // y = x * rstd * w * z * sigmoid(z), rows of D (<= 256), one warp per row
 __global__ void rmsnorm_gated_fwd_kernel(const bf16* __restrict__ x, const bf16* __restrict__ z, const bf16* __restrict__ w,
                                          bf16* __restrict__ y, float* __restrict__ rstd, int rows, int D, float eps) {
+  pdl_begin();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   for (int row = blockIdx.x * kWarpsPerBlock + warp; row < rows; row += gridDim.x * kWarpsPerBlock) {
     float ss = 0.f;
@@ -813,6 +820,7 @@ __global__ void rmsnorm_gated_fwd_kernel(const bf16* __restrict__ x, const bf16*
 __global__ void rmsnorm_gated_bwd_kernel(const bf16* __restrict__ dy, const bf16* __restrict__ x, const bf16* __restrict__ z,
                                          const bf16* __restrict__ w, const float* __restrict__ rstd, bf16* __restrict__ dx,
                                          bf16* __restrict__ dz, float* __restrict__ dw_partial, int rows, int D) {
+  pdl_begin();
   extern __shared__ float sm_dw[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int nwarps = blockDim.x >> 5;
@@ -849,6 +857,7 @@ for (int wi = 0; wi < nwarps; ++wi) s += sm_dw[(size_t)wi * D + i];
 
 // ----------------------------------------------------------------------------------- SwiGLU
 __global__ void swiglu_fwd_kernel(const bf16* __restrict__ gu, bf16* __restrict__ out, long rows, int I) {
+  pdl_begin();
   const long nvec = rows * (I >> 3);
   const int vper = I >> 3;
   for (long v = blockIdx.x * (long)blockDim.x + threadIdx.x; v < nvec; v += (long)gridDim.x * blockDim.x) {
@@ -868,6 +877,7 @@ __global__ void swiglu_fwd_kernel(const bf16* __restrict__ gu, bf16* __restrict_
 // each group of 8 is read before it is written, so the activation costs no memory of its own at the peak of the backward pass.
 __global__ void swiglu_bwd_kernel(const bf16* dout, const bf16* __restrict__ gu, bf16* __restrict__ dgu, bf16* out,
                                   long rows, int I) {
+  pdl_begin();
   const long nvec = rows * (I >> 3);
   const int vper = I >> 3;
   for (long v = blockIdx.x * (long)blockDim.x + threadIdx.x; v < nvec; v += (long)gridDim.x * blockDim.x) {
@@ -895,6 +905,7 @@ __global__ void swiglu_bwd_kernel(const bf16* dout, const bf16* __restrict__ gu,
 
 // ----------------------------------------------------------------------------------- x * sigmoid(gate)
 __global__ void sigmoid_mul_fwd_kernel(const bf16* __restrict__ x, const bf16* __restrict__ gate, bf16* __restrict__ out, long n8) {
+  pdl_begin();
   for (long v = blockIdx.x * (long)blockDim.x + threadIdx.x; v < n8; v += (long)gridDim.x * blockDim.x) {
     float a[8], g[8];
     unpack8(reinterpret_cast<const uint4*>(x)[v], a);
@@ -906,6 +917,7 @@ __global__ void sigmoid_mul_fwd_kernel(const bf16* __restrict__ x, const bf16* _
 }
 __global__ void sigmoid_mul_bwd_kernel(const bf16* __restrict__ dout, const bf16* __restrict__ x, const bf16* __restrict__ gate,
                                        bf16* __restrict__ dx, bf16* __restrict__ dgate, long n8) {
+  pdl_begin();
   for (long v = blockIdx.x * (long)blockDim.x + threadIdx.x; v < n8; v += (long)gridDim.x * blockDim.x) {
     float a[8], g[8], d[8], o1[8], o2[8];
     unpack8(reinterpret_cast<const uint4*>(x)[v], a);
@@ -943,6 +955,7 @@ __device__ __forceinline__ float gelu_grad_f(float x, int tanh_approx) {
 // four vectors per thread and iteration, all loads first: one 16-byte load in flight per thread leaves a streaming kernel
 // at less than half of the memory bandwidth
 __global__ void gelu_fwd_kernel(const bf16* __restrict__ x, bf16* __restrict__ y, long n8, int tanh_approx) {
+  pdl_begin();
   constexpr int U = 4;
   const long stride = (long)gridDim.x * blockDim.x;
   long v = blockIdx.x * (long)blockDim.x + threadIdx.x;
@@ -970,6 +983,7 @@ __global__ void gelu_fwd_kernel(const bf16* __restrict__ x, bf16* __restrict__ y
 // `y` (may be null, may be `dy`): gelu(x) again, as above for swiglu
 __global__ void gelu_bwd_kernel(const bf16* dy, const bf16* __restrict__ x, bf16* __restrict__ dx, bf16* y, long n8,
                                 int tanh_approx) {
+  pdl_begin();
   constexpr int U = 4;
   const long stride = (long)gridDim.x * blockDim.x;
   long v = blockIdx.x * (long)blockDim.x + threadIdx.x;
@@ -1071,6 +1085,7 @@ __global__ void qkv_norm_rope_fwd_kernel(const bf16* __restrict__ qkv, const bf1
                                          bf16* __restrict__ k, bf16* __restrict__ v, bf16* __restrict__ gate,
                                          float* __restrict__ rstd, int T, int n_q, int n_kv, int R, float eps, int offset,
                                          int gated, int has_norm) {
+  pdl_begin();
   constexpr int D = E * 32;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int slots = n_q + 2 * n_kv;
@@ -1160,6 +1175,7 @@ __global__ void qkv_norm_rope_bwd_kernel(const bf16* __restrict__ dq, const bf16
                                          const bf16* __restrict__ kw, const float* __restrict__ cosv, const float* __restrict__ sinv,
                                          const float* __restrict__ rstd, bf16* __restrict__ dqkv, float* __restrict__ dw_partial,
                                          int T, int n_q, int n_kv, int R, int offset, int gated, int has_norm) {
+  pdl_begin();
   constexpr int D = E * 32;
   __shared__ float sm_dw[kWarpsPerBlock][2][D];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -1276,6 +1292,7 @@ qkv_norm_rope128_fwd_kernel(const bf16* __restrict__ qkv, const bf16* __restrict
                             const float* __restrict__ cosv, const float* __restrict__ sinv, bf16* __restrict__ q, bf16* __restrict__ k,
                             bf16* __restrict__ v, bf16* __restrict__ gate, float* __restrict__ rstd, int T, int n_q, int n_kv, float eps,
                             int offset, int gated, int has_norm) {
+  pdl_begin();
   constexpr int D = 128;
   const int warp = threadIdx.x >> 5, l = threadIdx.x & 15, which = (threadIdx.x >> 4) & 1;
   const int slots = n_q + 2 * n_kv, qstride = gated ? 2 * D : D, W = n_q * qstride + 2 * n_kv * D;
@@ -1354,6 +1371,7 @@ qkv_norm_rope128_bwd_kernel(const bf16* __restrict__ dq, const bf16* __restrict_
                             const bf16* __restrict__ qkv, const bf16* __restrict__ qw, const bf16* __restrict__ kw,
                             const float* __restrict__ cosv, const float* __restrict__ sinv, const float* __restrict__ rstd,
                             bf16* __restrict__ dqkv, float* __restrict__ dw_partial, int T, int n_q, int n_kv, int offset, int gated) {
+  pdl_begin();
   constexpr int D = 128;
   __shared__ float sm_dw[kWarpsPerBlock * 2][2][D];
   const int warp = threadIdx.x >> 5, l = threadIdx.x & 15, which = (threadIdx.x >> 4) & 1;
@@ -1467,6 +1485,7 @@ template <typename IdxT>
 __global__ void rope_generic_vec4_kernel(const bf16* __restrict__ x, long ss, long hs, const float* __restrict__ cosv,
                                          const float* __restrict__ sinv, bf16* __restrict__ out, long oss, long ohs, int S, int H, int D,
                                          int transpose) {
+  pdl_begin();
   const int half = D >> 1;
   const IdxT hq = (IdxT)(half >> 2), nh = (IdxT)H;
   const IdxT total = (IdxT)S * nh * hq;
@@ -1520,6 +1539,7 @@ __global__ void rope_generic_kernel(const bf16* __restrict__ x, long ss, long hs
 __global__ void gdn_gates_fwd_kernel(const bf16* __restrict__ a, const bf16* __restrict__ b, long row_stride,
                                      const float* __restrict__ A_log, const float* __restrict__ dt_bias, float* __restrict__ g,
                                      bf16* __restrict__ beta, long T, int H) {
+  pdl_begin();
   const long n = T * H;
   for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x) {
     const long t = i / H;
@@ -1536,6 +1556,7 @@ __global__ void gdn_gates_bwd_kernel(const float* __restrict__ dg, const bf16* _
                                      const bf16* __restrict__ b, long row_stride, const float* __restrict__ A_log,
                                      const float* __restrict__ dt_bias, bf16* __restrict__ da, bf16* __restrict__ db,
                                      long out_stride, float* __restrict__ partial, long T, int H) {
+  pdl_begin();
   extern __shared__ float sm[];  // [2][H]
   for (int i = threadIdx.x; i < 2 * H; i += blockDim.x) sm[i] = 0.f;
   __syncthreads();
@@ -1566,6 +1587,7 @@ __global__ void gdn_gates_bwd_kernel(const float* __restrict__ dg, const bf16* _
 template <int K>
 __global__ void __launch_bounds__(128, 4) conv1d_silu_fwd_kernel(const bf16* __restrict__ x, long xs, const bf16* __restrict__ w, const int* __restrict__ seq_idx,
                                        bf16* __restrict__ y, long ys, int T, int C, int rows_per_thread) {
+  pdl_begin();
   static_assert(K == 4, "window code below is written for K = 4");
   const int c = (blockIdx.x * blockDim.x + threadIdx.x) * 8;
   if (c >= C) return;
@@ -1635,6 +1657,7 @@ template <int K>
 __global__ void __launch_bounds__(128, 4) conv1d_silu_bwd_kernel(const bf16* __restrict__ dy, long dys, const bf16* __restrict__ x, long xs,
                                        const bf16* __restrict__ w, const int* __restrict__ seq_idx, bf16* __restrict__ dx, long dxs,
                                        float* __restrict__ dw_partial, int T, int C, int t_per_block) {
+  pdl_begin();
   static_assert(K == 4, "window code below is written for K = 4");
   constexpr int V = 4, U = 4;
   const int c = (blockIdx.x * blockDim.x + threadIdx.x) * V;
@@ -1742,6 +1765,7 @@ __global__ void __launch_bounds__(128, 4) conv1d_silu_bwd_kernel(const bf16* __r
 // out[index[i], :] (=|+=) src[i, :]   (index rows are unique)
 __global__ void rows_update_kernel(bf16* __restrict__ out, const long* __restrict__ index, const bf16* __restrict__ src, long n_rows,
                                    int D, int add) {
+  pdl_begin();
   const int vper = D >> 3;
   const long total = n_rows * vper;
   for (long v = blockIdx.x * (long)blockDim.x + threadIdx.x; v < total; v += (long)gridDim.x * blockDim.x) {
@@ -1763,6 +1787,7 @@ __global__ void rows_update_kernel(bf16* __restrict__ out, const long* __restric
 // dst[i, :] = src[index[i], :]
 __global__ void rows_gather_kernel(bf16* __restrict__ dst, const long* __restrict__ index, const bf16* __restrict__ src, long n_rows,
                                    int D) {
+  pdl_begin();
   const int vper = D >> 3;
   const long total = n_rows * vper;
   for (long v = blockIdx.x * (long)blockDim.x + threadIdx.x; v < total; v += (long)gridDim.x * blockDim.x) {
@@ -1838,7 +1863,7 @@ void vlmt_rmsnorm_fwd(const void* x, const void* res, const void* w, int w_fp32,
   const int vpt = tile_vpt(D);
   if (vpt) {
 #define RF(WT, V) do { const size_t sb = ring_bytes(D, TileRows<V>::value, res ? 2 : 1); auto kf = rmsnorm_fwd_tile_kernel<WT, V>; allow_smem(kf, sb); \
-    kf<<<tile_grid(kf, rows, tile_threads(D, vpt), TileRows<V>::value, sb), tile_threads(D, vpt), sb, st>>>(BF(x), BF(res), (const WT*)w, BFM(y), BFM(r_out), rstd, rows, D, eps, offset); } while (0)
+    launch_pdl(kf, dim3(tile_grid(kf, rows, tile_threads(D, vpt), TileRows<V>::value, sb)), dim3(tile_threads(D, vpt)), sb, st, 1, BF(x), BF(res), (const WT*)w, BFM(y), BFM(r_out), rstd, rows, D, eps, offset); } while (0)
     if (w_fp32) TILE_DISPATCH(vpt, RF(float, 1), RF(float, 2), RF(float, 4));
     else TILE_DISPATCH(vpt, RF(bf16, 1), RF(bf16, 2), RF(bf16, 4));
 #undef RF
@@ -1858,7 +1883,7 @@ int vlmt_rmsnorm_bwd(const void* dy, const void* x, const void* w, int w_fp32, c
   const int vpt = tile_vpt(D);
   if (vpt) {
 #define RB(WT, V) do { const size_t sb = ring_bytes(D, TileRows<V>::value, dres ? 3 : 2); auto kb = rmsnorm_bwd_tile_kernel<WT, V>; allow_smem(kb, sb); \
-    kb<<<grid, tile_threads(D, vpt), sb, st>>>(BF(dy), BF(x), (const WT*)w, rstd, BF(dres), BFM(dx), dw_partial, rows, D, offset); } while (0)
+    launch_pdl(kb, dim3(grid), dim3(tile_threads(D, vpt)), sb, st, 1, BF(dy), BF(x), (const WT*)w, rstd, BF(dres), BFM(dx), dw_partial, rows, D, offset); } while (0)
     if (w_fp32) TILE_DISPATCH(vpt, RB(float, 1), RB(float, 2), RB(float, 4));
     else TILE_DISPATCH(vpt, RB(bf16, 1), RB(bf16, 2), RB(bf16, 4));
 #undef RB
@@ -1887,7 +1912,7 @@ void vlmt_layernorm_fwd(const void* x, const void* w, const void* b, void* y, fl
   if (vl) {
     const size_t sb = 2 * (size_t)D * sizeof(float) + (size_t)kLnWarpsFwd * kLnPipeFwd * (D >> 3) * sizeof(uint4);
 #define LW(V) do { auto kf = layernorm_fwd_warp_kernel<V>; allow_smem(kf, sb); \
-    kf<<<tile_grid(kf, rows, kLnWarpsFwd * 32, kLnWarpsFwd, sb), kLnWarpsFwd * 32, sb, st>>>(BF(x), BF(w), BF(b), BFM(y), mean, rstd, rows, D, eps); } while (0)
+    launch_pdl(kf, dim3(tile_grid(kf, rows, kLnWarpsFwd * 32, kLnWarpsFwd, sb)), dim3(kLnWarpsFwd * 32), sb, st, 1, BF(x), BF(w), BF(b), BFM(y), mean, rstd, rows, D, eps); } while (0)
     if (vl == 4) LW(4); else LW(5);
 #undef LW
     return;
@@ -1895,7 +1920,7 @@ void vlmt_layernorm_fwd(const void* x, const void* w, const void* b, void* y, fl
   const int vpt = tile_vpt(D);
   if (vpt) {
 #define LF(V) do { const size_t sb = ring_bytes(D, TileRows<V>::value, 1); auto kf = layernorm_fwd_tile_kernel<V>; allow_smem(kf, sb); \
-    kf<<<tile_grid(kf, rows, tile_threads(D, vpt), TileRows<V>::value, sb), tile_threads(D, vpt), sb, st>>>(BF(x), BF(w), BF(b), BFM(y), mean, rstd, rows, D, eps); } while (0)
+    launch_pdl(kf, dim3(tile_grid(kf, rows, tile_threads(D, vpt), TileRows<V>::value, sb)), dim3(tile_threads(D, vpt)), sb, st, 1, BF(x), BF(w), BF(b), BFM(y), mean, rstd, rows, D, eps); } while (0)
     TILE_DISPATCH(vpt, LF(1), LF(2), LF(4));
 #undef LF
     return;
@@ -1908,7 +1933,7 @@ int vlmt_layernorm_bwd(const void* dy, const void* x, const void* w, const float
   const int vpt = tile_vpt(D);
   if (vpt) {
 #define LB(V) do { const size_t sb = ring_bytes(D, TileRows<V>::value, 2); auto kb = layernorm_bwd_tile_kernel<V>; allow_smem(kb, sb); \
-    kb<<<grid, tile_threads(D, vpt), sb, st>>>(BF(dy), BF(x), BF(w), mean, rstd, BFM(dx), dw_partial, db_partial, rows, D); } while (0)
+    launch_pdl(kb, dim3(grid), dim3(tile_threads(D, vpt)), sb, st, 1, BF(dy), BF(x), BF(w), mean, rstd, BFM(dx), dw_partial, db_partial, rows, D); } while (0)
     TILE_DISPATCH(vpt, LB(1), LB(2), LB(4));
 #undef LB
     return grid;
@@ -1922,33 +1947,33 @@ int vlmt_layernorm_bwd(const void* dy, const void* x, const void* w, const float
 }
 
 void vlmt_rmsnorm_gated_fwd(const void* x, const void* z, const void* w, void* y, float* rstd, int rows, int D, float eps, cudaStream_t st) {
-  rmsnorm_gated_fwd_kernel<<<grid_for(rows, kWarpsPerBlock, 148 * 16), kThreads, 0, st>>>(BF(x), BF(z), BF(w), BFM(y), rstd, rows, D, eps);
+  launch_pdl(rmsnorm_gated_fwd_kernel, dim3(grid_for(rows, kWarpsPerBlock, 148 * 16)), dim3(kThreads), 0, st, 1, BF(x), BF(z), BF(w), BFM(y), rstd, rows, D, eps);
 }
 int vlmt_rmsnorm_gated_bwd(const void* dy, const void* x, const void* z, const void* w, const float* rstd, void* dx, void* dz,
                            float* dw_partial, int rows, int D, cudaStream_t st) {
   const int grid = vlmt_norm_blocks(rows);
-  rmsnorm_gated_bwd_kernel<<<grid, kThreads, (size_t)kWarpsPerBlock * D * sizeof(float), st>>>(BF(dy), BF(x), BF(z), BF(w), rstd, BFM(dx),
+  launch_pdl(rmsnorm_gated_bwd_kernel, dim3(grid), dim3(kThreads), (size_t)kWarpsPerBlock * D * sizeof(float), st, 1, BF(dy), BF(x), BF(z), BF(w), rstd, BFM(dx),
                                                                                             BFM(dz), dw_partial, rows, D);
   return grid;
 }
 
 void vlmt_swiglu_fwd(const void* gu, void* out, long rows, int I, cudaStream_t st) {
-  swiglu_fwd_kernel<<<grid_for(rows * (I >> 3), 256, 148 * 16), 256, 0, st>>>(BF(gu), BFM(out), rows, I);
+  launch_pdl(swiglu_fwd_kernel, dim3(grid_for(rows * (I >> 3), 256, 148 * 16)), dim3(256), 0, st, 1, BF(gu), BFM(out), rows, I);
 }
 void vlmt_swiglu_bwd(const void* dout, const void* gu, void* dgu, void* out, long rows, int I, cudaStream_t st) {
-  swiglu_bwd_kernel<<<grid_for(rows * (I >> 3), 256, 148 * 16), 256, 0, st>>>(BF(dout), BF(gu), BFM(dgu), BFM(out), rows, I);
+  launch_pdl(swiglu_bwd_kernel, dim3(grid_for(rows * (I >> 3), 256, 148 * 16)), dim3(256), 0, st, 1, BF(dout), BF(gu), BFM(dgu), BFM(out), rows, I);
 }
 void vlmt_sigmoid_mul_fwd(const void* x, const void* gate, void* out, long n, cudaStream_t st) {
-  sigmoid_mul_fwd_kernel<<<grid_for(n >> 3, 256, 148 * 16), 256, 0, st>>>(BF(x), BF(gate), BFM(out), n >> 3);
+  launch_pdl(sigmoid_mul_fwd_kernel, dim3(grid_for(n >> 3, 256, 148 * 16)), dim3(256), 0, st, 1, BF(x), BF(gate), BFM(out), n >> 3);
 }
 void vlmt_sigmoid_mul_bwd(const void* dout, const void* x, const void* gate, void* dx, void* dgate, long n, cudaStream_t st) {
-  sigmoid_mul_bwd_kernel<<<grid_for(n >> 3, 256, 148 * 16), 256, 0, st>>>(BF(dout), BF(x), BF(gate), BFM(dx), BFM(dgate), n >> 3);
+  launch_pdl(sigmoid_mul_bwd_kernel, dim3(grid_for(n >> 3, 256, 148 * 16)), dim3(256), 0, st, 1, BF(dout), BF(x), BF(gate), BFM(dx), BFM(dgate), n >> 3);
 }
 void vlmt_gelu_fwd(const void* x, void* y, long n, int tanh_approx, cudaStream_t st) {
-  gelu_fwd_kernel<<<grid_for(n >> 3, 256, 148 * 16), 256, 0, st>>>(BF(x), BFM(y), n >> 3, tanh_approx);
+  launch_pdl(gelu_fwd_kernel, dim3(grid_for(n >> 3, 256, 148 * 16)), dim3(256), 0, st, 1, BF(x), BFM(y), n >> 3, tanh_approx);
 }
 void vlmt_gelu_bwd(const void* dy, const void* x, void* dx, void* y, long n, int tanh_approx, cudaStream_t st) {
-  gelu_bwd_kernel<<<grid_for(n >> 3, 256, 148 * 16), 256, 0, st>>>(BF(dy), BF(x), BFM(dx), BFM(y), n >> 3, tanh_approx);
+  launch_pdl(gelu_bwd_kernel, dim3(grid_for(n >> 3, 256, 148 * 16)), dim3(256), 0, st, 1, BF(dy), BF(x), BFM(dx), BFM(y), n >> 3, tanh_approx);
 }
 
 static bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
@@ -1962,12 +1987,12 @@ int vlmt_qkv_norm_rope_fwd(const void* qkv, const void* qw, const void* kw, cons
   if (D % 32 || R > D || (R / 2) % E || (((R / 2) / E) & ((R / 2) / E - 1)) || (R / 2) / E >= 32) return -1;
   const int grid = vlmt_qkv_blocks((long)T * ((n_q + 2 * n_kv + kQkvGroup - 1) / kQkvGroup));  // one warp per token and group of heads
   if (D == 128 && R == 128 && aligned16(cosv) && aligned16(sinv)) {   // the presets' head; other sizes and partial rotary: general form
-    qkv_norm_rope128_fwd_kernel<<<grid, kThreads, 0, st>>>(BF(qkv), BF(qw), BF(kw), cosv, sinv, BFM(q), BFM(k), BFM(v), BFM(gate), rstd, T,
+    launch_pdl(qkv_norm_rope128_fwd_kernel, dim3(grid), dim3(kThreads), 0, st, 1, BF(qkv), BF(qw), BF(kw), cosv, sinv, BFM(q), BFM(k), BFM(v), BFM(gate), rstd, T,
                                                            n_q, n_kv, eps, offset, gated, has_norm);
     return 0;
   }
 #define LAUNCH(E_)                                                                                                              \
-  qkv_norm_rope_fwd_kernel<E_><<<grid, kThreads, 0, st>>>(BF(qkv), BF(qw), BF(kw), cosv, sinv, BFM(q), BFM(k), BFM(v), BFM(gate), \
+  launch_pdl(qkv_norm_rope_fwd_kernel<E_>, dim3(grid), dim3(kThreads), 0, st, 1, BF(qkv), BF(qw), BF(kw), cosv, sinv, BFM(q), BFM(k), BFM(v), BFM(gate), \
                                                           rstd, T, n_q, n_kv, R, eps, offset, gated, has_norm)
   switch (E) {
     case 1: LAUNCH(1); break;
@@ -1985,12 +2010,12 @@ int vlmt_qkv_norm_rope_bwd(const void* dq, const void* dk, const void* dv, const
   const int E = D / 32;
   const int grid = vlmt_qkv_blocks((long)T * (n_q + 2 * n_kv));
   if (D == 128 && R == 128 && has_norm && aligned16(cosv) && aligned16(sinv)) {
-    qkv_norm_rope128_bwd_kernel<<<grid, kThreads, 0, st>>>(BF(dq), BF(dk), BF(dv), BF(dgate), BF(qkv), BF(qw), BF(kw), cosv, sinv, rstd,
+    launch_pdl(qkv_norm_rope128_bwd_kernel, dim3(grid), dim3(kThreads), 0, st, 1, BF(dq), BF(dk), BF(dv), BF(dgate), BF(qkv), BF(qw), BF(kw), cosv, sinv, rstd,
                                                            BFM(dqkv), dw_partial, T, n_q, n_kv, offset, gated);
     return grid;
   }
 #define LAUNCH(E_)                                                                                                               \
-  qkv_norm_rope_bwd_kernel<E_><<<grid, kThreads, 0, st>>>(BF(dq), BF(dk), BF(dv), BF(dgate), BF(qkv), BF(qw), BF(kw), cosv, sinv, \
+  launch_pdl(qkv_norm_rope_bwd_kernel<E_>, dim3(grid), dim3(kThreads), 0, st, 1, BF(dq), BF(dk), BF(dv), BF(dgate), BF(qkv), BF(qw), BF(kw), cosv, sinv, \
                                                           rstd, BFM(dqkv), dw_partial, T, n_q, n_kv, R, offset, gated, has_norm)
   switch (E) {
     case 1: LAUNCH(1); break;
@@ -2012,9 +2037,9 @@ void vlmt_rope_generic(const void* x, long ss, long hs, const float* cosv, const
     const long items = (long)S * H * (half / 4);
     const int grid = grid_for(items, 256, 148 * 16);
     if (items + (long)grid * 256 < (1l << 32))   // the loop's last increment must not wrap
-      rope_generic_vec4_kernel<unsigned><<<grid, 256, 0, st>>>(BF(x), ss, hs, cosv, sinv, BFM(out), oss, ohs, S, H, D, transpose);
+      launch_pdl(rope_generic_vec4_kernel<unsigned>, dim3(grid), dim3(256), 0, st, 1, BF(x), ss, hs, cosv, sinv, BFM(out), oss, ohs, S, H, D, transpose);
     else
-      rope_generic_vec4_kernel<long><<<grid, 256, 0, st>>>(BF(x), ss, hs, cosv, sinv, BFM(out), oss, ohs, S, H, D, transpose);
+      launch_pdl(rope_generic_vec4_kernel<long>, dim3(grid), dim3(256), 0, st, 1, BF(x), ss, hs, cosv, sinv, BFM(out), oss, ohs, S, H, D, transpose);
     return;
   }
   rope_generic_kernel<<<grid_for((long)S * H * (D / 2), 256, 148 * 16), 256, 0, st>>>(BF(x), ss, hs, cosv, sinv, BFM(out), oss, ohs, S, H, D,
@@ -2023,12 +2048,12 @@ void vlmt_rope_generic(const void* x, long ss, long hs, const float* cosv, const
 
 void vlmt_gdn_gates_fwd(const void* a, const void* b, long row_stride, const float* A_log, const float* dt_bias, float* g, void* beta,
                         long T, int H, cudaStream_t st) {
-  gdn_gates_fwd_kernel<<<grid_for(T * H, 256, 148 * 8), 256, 0, st>>>(BF(a), BF(b), row_stride, A_log, dt_bias, g, BFM(beta), T, H);
+  launch_pdl(gdn_gates_fwd_kernel, dim3(grid_for(T * H, 256, 148 * 8)), dim3(256), 0, st, 1, BF(a), BF(b), row_stride, A_log, dt_bias, g, BFM(beta), T, H);
 }
 int vlmt_gdn_gates_bwd(const float* dg, const void* dbeta, const void* a, const void* b, long row_stride, const float* A_log,
                        const float* dt_bias, void* da, void* db, long out_stride, float* partial, long T, int H, cudaStream_t st) {
   const int grid = grid_for(T * H, 256, 148 * 2);
-  gdn_gates_bwd_kernel<<<grid, 256, 2 * H * sizeof(float), st>>>(dg, BF(dbeta), BF(a), BF(b), row_stride, A_log, dt_bias, BFM(da), BFM(db),
+  launch_pdl(gdn_gates_bwd_kernel, dim3(grid), dim3(256), 2 * H * sizeof(float), st, 1, dg, BF(dbeta), BF(a), BF(b), row_stride, A_log, dt_bias, BFM(da), BFM(db),
                                                                out_stride, partial, T, H);
   return grid;
 }
@@ -2037,7 +2062,7 @@ int vlmt_conv1d_silu_fwd(const void* x, long xs, const void* w, const int* seq_i
   if (K != 4 || (C & 7)) return -1;
   const int rows = 64;
   dim3 grid(((C >> 3) + 127) / 128, (T + rows - 1) / rows);
-  conv1d_silu_fwd_kernel<4><<<grid, 128, 0, st>>>(BF(x), xs, BF(w), seq_idx, BFM(y), ys, T, C, rows);
+  launch_pdl(conv1d_silu_fwd_kernel<4>, dim3(grid), dim3(128), 0, st, 1, BF(x), xs, BF(w), seq_idx, BFM(y), ys, T, C, rows);
   return 0;
 }
 int vlmt_conv1d_bwd_slabs(int T) { return (T + kConvSlab - 1) / kConvSlab; }
@@ -2045,17 +2070,17 @@ int vlmt_conv1d_silu_bwd(const void* dy, long dys, const void* x, long xs, const
                          float* dw_partial, int T, int C, int K, cudaStream_t st) {
   if (K != 4 || (C & 3)) return -1;
   dim3 grid(((C >> 2) + 127) / 128, vlmt_conv1d_bwd_slabs(T));
-  conv1d_silu_bwd_kernel<4><<<grid, 128, 0, st>>>(BF(dy), dys, BF(x), xs, BF(w), seq_idx, BFM(dx), dxs, dw_partial, T, C, kConvSlab);
+  launch_pdl(conv1d_silu_bwd_kernel<4>, dim3(grid), dim3(128), 0, st, 1, BF(dy), dys, BF(x), xs, BF(w), seq_idx, BFM(dx), dxs, dw_partial, T, C, kConvSlab);
   return 0;
 }
 
 void vlmt_rows_update(void* out, const long* index, const void* src, long n_rows, int D, int add, cudaStream_t st) {
   if (n_rows == 0) return;
-  rows_update_kernel<<<grid_for(n_rows * (D >> 3), 256, 148 * 16), 256, 0, st>>>(BFM(out), index, BF(src), n_rows, D, add);
+  launch_pdl(rows_update_kernel, dim3(grid_for(n_rows * (D >> 3), 256, 148 * 16)), dim3(256), 0, st, 1, BFM(out), index, BF(src), n_rows, D, add);
 }
 void vlmt_rows_gather(void* dst, const long* index, const void* src, long n_rows, int D, cudaStream_t st) {
   if (n_rows == 0) return;
-  rows_gather_kernel<<<grid_for(n_rows * (D >> 3), 256, 148 * 16), 256, 0, st>>>(BFM(dst), index, BF(src), n_rows, D);
+  launch_pdl(rows_gather_kernel, dim3(grid_for(n_rows * (D >> 3), 256, 148 * 16)), dim3(256), 0, st, 1, BFM(dst), index, BF(src), n_rows, D);
 }
 
 }  // extern "C"

@@ -12,6 +12,7 @@
 //   The scale s = rec_a[1] * rec_b[1] is read from device memory, so quantisation and GEMM queue without a host sync.
 #include "sm100.cuh"
 
+#include "pdl.cuh"
 #include <cuda_fp8.h>
 #include <stdlib.h>
 
@@ -28,6 +29,7 @@ using namespace sm100;
 // twelve scans of an 8B layer on 8192 tokens took 325 us, now 285 us).
 __global__ void __launch_bounds__(256) amax_kernel(const __nv_bfloat16* __restrict__ x, long ld, long rows, long vec_per_row,
                                                    float* __restrict__ rec) {
+  pdl_begin();
   constexpr int U = 4;
   const long nvec = rows * vec_per_row, stride = (long)gridDim.x * blockDim.x;
   __nv_bfloat162 m2 = __floats2bfloat162_rn(0.f, 0.f);
@@ -76,6 +78,7 @@ template <int FMT>
 __global__ void __launch_bounds__(256) cast_kernel(const __nv_bfloat16* __restrict__ x, long ld, long rows, long cols,
                                                    float* __restrict__ rec, uint8_t* __restrict__ out_rm, long ld_rm,
                                                    uint8_t* __restrict__ out_t, long ld_t) {
+  pdl_begin();
   __shared__ __align__(16) uint8_t tile[CT_ROWS * CT_PITCH];
   constexpr float kMax = FMT == FP8_E4M3 ? 448.f : 57344.f;
   const float amax = fmaxf(rec[0], 1e-12f);
@@ -327,7 +330,7 @@ extern "C" int vlmt_fp8_amax(const void* x, long ld, long rows, long cols, float
   const long nvec = rows * (cols / 8);
   if (ld == cols) { cols *= rows; rows = 1; }
   const int grid = (int)((nvec + 255) / 256 < 1184 ? (nvec + 255) / 256 : 1184);   // 8 blocks per SM
-  amax_kernel<<<grid, 256, 0, stream>>>(reinterpret_cast<const __nv_bfloat16*>(x), ld, rows, cols / 8, rec);
+  launch_pdl(amax_kernel, dim3(grid), dim3(256), 0, stream, 1, reinterpret_cast<const __nv_bfloat16*>(x), ld, rows, cols / 8, rec);
   return (int)cudaGetLastError();
 }
 
@@ -342,8 +345,8 @@ extern "C" int vlmt_fp8_cast(const void* x, long ld, long rows, long cols, float
   auto* xp = reinterpret_cast<const __nv_bfloat16*>(x);
   auto* rm = reinterpret_cast<uint8_t*>(out_rm);
   auto* tp = reinterpret_cast<uint8_t*>(out_t);
-  if (format == FP8_E4M3) cast_kernel<FP8_E4M3><<<grid, 256, 0, stream>>>(xp, ld, rows, cols, rec, rm, ld_rm, tp, ld_t);
-  else if (format == FP8_E5M2) cast_kernel<FP8_E5M2><<<grid, 256, 0, stream>>>(xp, ld, rows, cols, rec, rm, ld_rm, tp, ld_t);
+  if (format == FP8_E4M3) launch_pdl(cast_kernel<FP8_E4M3>, dim3(grid), dim3(256), 0, stream, 1, xp, ld, rows, cols, rec, rm, ld_rm, tp, ld_t);
+  else if (format == FP8_E5M2) launch_pdl(cast_kernel<FP8_E5M2>, dim3(grid), dim3(256), 0, stream, 1, xp, ld, rows, cols, rec, rm, ld_rm, tp, ld_t);
   else return -6;
   return (int)cudaGetLastError();
 }

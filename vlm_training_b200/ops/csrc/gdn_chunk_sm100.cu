@@ -21,6 +21,7 @@
 #include "gemm_sm100.h"
 #include "sm100.cuh"
 
+#include "pdl.cuh"
 #include <cuda_bf16.h>
 
 namespace {
@@ -161,6 +162,7 @@ struct PrepSmem {
 __global__ void __launch_bounds__(THREADS, 2)
 gdn_prepare_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                        const __grid_constant__ CUtensorMap tmV, PrepParams p) {
+  pdl_begin();
   using L = PrepSmem;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -365,6 +367,7 @@ struct OutSmem {
 __global__ void __launch_bounds__(THREADS, 2)
 gdn_output_fwd_kernel(const __grid_constant__ CUtensorMap tmQg, const __grid_constant__ CUtensorMap tmP,
                       const __grid_constant__ CUtensorMap tmS, const __grid_constant__ CUtensorMap tmVn, OutParams p) {
+  pdl_begin();
   using L = OutSmem;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -436,6 +439,7 @@ __global__ void __launch_bounds__(THREADS, 2)
 gdn_output_bwd_kernel(const __grid_constant__ CUtensorMap tmDo, const __grid_constant__ CUtensorMap tmQg,
                       const __grid_constant__ CUtensorMap tmP, const __grid_constant__ CUtensorMap tmS,
                       const __grid_constant__ CUtensorMap tmVn, OutBwdParams p) {
+  pdl_begin();
   using L = OutBwdSmem;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -578,6 +582,7 @@ gdn_prepare_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
                        const __grid_constant__ CUtensorMap tmDu, const __grid_constant__ CUtensorMap tmDqg,
                        const __grid_constant__ CUtensorMap tmDp, const __grid_constant__ CUtensorMap tmPp,
                        const __grid_constant__ CUtensorMap tmTm, PrepBwdParams p) {
+  pdl_begin();
   using L = PrepBwdSmem;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -952,7 +957,7 @@ extern "C" int vlmt_gdn_prepare_fwd(const void* q, const void* k, const void* v,
   p.P = (__nv_bfloat16*)P; p.Tm = (__nv_bfloat16*)Tm; p.gc = gc; p.decay = decay;
   p.scale = scale; p.eps = eps; p.H = H; p.N = N; p.status = status;
   if ((r = set_smem(gdn_prepare_fwd_kernel, PrepSmem::kTotal))) return r;
-  gdn_prepare_fwd_kernel<<<dim3(N, H), THREADS, PrepSmem::kTotal, st>>>(tq, tk, tv, p);
+  launch_pdl(gdn_prepare_fwd_kernel, dim3(dim3(N, H)), dim3(THREADS), PrepSmem::kTotal, st, 1, tq, tk, tv, p);
   return (int)cudaGetLastError();
 }
 
@@ -969,7 +974,7 @@ extern "C" int vlmt_gdn_output_fwd(const void* qg, const void* P, const void* st
   OutParams p;
   p.chunks = reinterpret_cast<const int2*>(chunks); p.o = (__nv_bfloat16*)o; p.H = H; p.N = N; p.status = status;
   if ((r = set_smem(gdn_output_fwd_kernel, OutSmem::kTotal))) return r;
-  gdn_output_fwd_kernel<<<dim3(N, H), THREADS, OutSmem::kTotal, st>>>(tqg, tp, ts, tvn, p);
+  launch_pdl(gdn_output_fwd_kernel, dim3(dim3(N, H)), dim3(THREADS), OutSmem::kTotal, st, 1, tqg, tp, ts, tvn, p);
   return (int)cudaGetLastError();
 }
 
@@ -990,7 +995,7 @@ extern "C" int vlmt_gdn_output_bwd(const void* dout, long ld_do, const void* qg,
   p.dqg = (__nv_bfloat16*)dqg; p.dvn = (__nv_bfloat16*)dvn; p.dP = (__nv_bfloat16*)dP; p.dS = (__nv_bfloat16*)dS;
   p.H = H; p.N = N; p.status = status;
   if ((r = set_smem(gdn_output_bwd_kernel, OutBwdSmem::kTotal))) return r;
-  gdn_output_bwd_kernel<<<dim3(N, H), THREADS, OutBwdSmem::kTotal, st>>>(tdo, tqg, tp, ts, tvn, p);
+  launch_pdl(gdn_output_bwd_kernel, dim3(dim3(N, H)), dim3(THREADS), OutBwdSmem::kTotal, st, 1, tdo, tqg, tp, ts, tvn, p);
   return (int)cudaGetLastError();
 }
 
@@ -1018,6 +1023,6 @@ extern "C" int vlmt_gdn_prepare_bwd(const void* q, const void* k, const void* v,
   p.dq = (__nv_bfloat16*)dq; p.dk = (__nv_bfloat16*)dk; p.dv = (__nv_bfloat16*)dv; p.dg = dg; p.dbeta = dbeta;
   p.scale = scale; p.eps = eps; p.H = H; p.N = N; p.status = status;
   if ((r = set_smem(gdn_prepare_bwd_kernel, PrepBwdSmem::kTotal))) return r;
-  gdn_prepare_bwd_kernel<<<dim3(N, H), THREADS, PrepBwdSmem::kTotal, st>>>(tq, tk, tv, ts, tg, tvn, tdu, tdqg, tdp, tpp, ttm, p);
+  launch_pdl(gdn_prepare_bwd_kernel, dim3(dim3(N, H)), dim3(THREADS), PrepBwdSmem::kTotal, st, 1, tq, tk, tv, ts, tg, tvn, tdu, tdqg, tdp, tpp, ttm, p);
   return (int)cudaGetLastError();
 }

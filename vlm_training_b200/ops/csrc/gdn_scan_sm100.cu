@@ -26,6 +26,7 @@
 #include "gemm_sm100.h"
 #include "sm100.cuh"
 
+#include "pdl.cuh"
 #include <cuda_bf16.h>
 
 namespace {
@@ -56,6 +57,7 @@ template <bool REVERSE>
 __global__ void __launch_bounds__(THREADS, 2)
 gdn_scan_kernel(const __grid_constant__ CUtensorMap tmX1, const __grid_constant__ CUtensorMap tmX2,
                 const __grid_constant__ CUtensorMap tmE, Params p) {
+  pdl_begin();
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + offBar);
@@ -286,7 +288,7 @@ int launch(const CUtensorMap& t1, const CUtensorMap& t2, const CUtensorMap& te, 
     attr_set = true;
   }
   dim3 grid(n_docs, p.H);
-  gdn_scan_kernel<REVERSE><<<grid, THREADS, kSmem, stream>>>(t1, t2, te, p);
+  launch_pdl(gdn_scan_kernel<REVERSE>, dim3(grid), dim3(THREADS), kSmem, stream, 1, t1, t2, te, p);
   return cudaGetLastError() == cudaSuccess ? 0 : -11;
 }
 }  // namespace

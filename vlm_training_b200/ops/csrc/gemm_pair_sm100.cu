@@ -13,6 +13,7 @@
 // The leader (even rank) issues every MMA; both blocks' loads complete on the leader's "full" barrier; commits arrive on both
 // blocks' "empty" and "accumulator full" barriers; both epilogues arrive on the leader's "accumulator free" barrier.
 #include "gemm_epilogue.cuh"
+#include "pdl.cuh"
 #include "gemm_pair_sm100.h"
 #include "sm100.cuh"
 
@@ -82,6 +83,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
   cluster_sync();   // both blocks' barriers are initialised before anything remote touches them
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  pdl_wait();
 
   auto k_range = [&](int item, int& tile, int& kb_lo, int& kb_hi) {
     tile = item; kb_lo = 0; kb_hi = num_kb;
@@ -123,6 +125,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
           if (++stage == STAGES) { stage = 0; phase ^= 1; }
         }
       }
+      pdl_trigger();
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer (leader only)
@@ -202,7 +205,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
       __syncwarp();
       if (lane == 0) mbar_arrive_cluster(cluster_addr(&tmem_empty[acc], 0));
     }
-    if (lane == 0) tma_store_wait<0>();
+    if (lane == 0) tma_store_wait_read<0>();
   }
   // ---------------------------------------------------------------- teardown
   tc_fence_before();
@@ -229,7 +232,7 @@ int launch(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& td, 
   cudaLaunchAttribute attr;
   attr.id = cudaLaunchAttributeClusterDimension;
   attr.val.clusterDim.x = 2; attr.val.clusterDim.y = 1; attr.val.clusterDim.z = 1;
-  cfg.blockDim = dim3(NUM_THREADS); cfg.dynamicSmemBytes = kSmem; cfg.stream = st;
+  cfg.blockDim = dim3(NUM_THREADS); cfg.dynamicSmemBytes = kSmem;
   cfg.attrs = &attr; cfg.numAttrs = 1;
   std::call_once(once, [&] {
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem) != cudaSuccess) return;
@@ -239,8 +242,7 @@ int launch(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& td, 
   });
   if (max_pairs <= 0) return -50;
   const int items = ((p.M + 2 * BM - 1) / (2 * BM)) * ((p.N + BN - 1) / BN) * p.k_splits;
-  cfg.gridDim = dim3(2 * (items < max_pairs ? items : max_pairs));
-  return (int)cudaLaunchKernelEx(&cfg, kern, ta, tb, td, p);
+  return launch_pdl(kern, dim3(2 * (items < max_pairs ? items : max_pairs)), dim3(NUM_THREADS), kSmem, st, 2, ta, tb, td, p);
 }
 }  // namespace
 

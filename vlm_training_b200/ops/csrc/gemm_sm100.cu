@@ -24,6 +24,7 @@
 // loads the first tile of that peer's rows from the LOCAL gathered buffer, so remote rows cross NVLink once and the
 // transfer hides behind the own rows' tiles.
 #include "gemm_epilogue.cuh"
+#include "pdl.cuh"
 #include "sm100.cuh"
 
 #include <stdlib.h>
@@ -212,13 +213,6 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int tiles_n = (p.N + BN - 1) / BN;
-  const int tiles_m = p.grp_mode == 1 ? p.grp_prefix[p.grp_count] : (p.M + BM - 1) / BM;
-  const int tiles_per_group = tiles_m * tiles_n;                       // grp_mode 2: one [M, N] output per group
-  const int num_tiles = p.grp_mode == 2 ? tiles_per_group * p.grp_count : tiles_per_group;
-  const int num_kb = (p.K + BK - 1) / BK;
-  const int num_items = num_tiles * p.k_splits;
-  const int m_limit = p.grp_mode == 1 ? tiles_m * BM : p.M;           // rows that exist
   constexpr int TMEM_COLS = 2 * BN;  // 256 or 512: a power of two >= 32
 
   if (threadIdx.x == 0) {
@@ -230,6 +224,20 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
     tma_prefetch_desc(&tmap_b);
     if (AG) tma_prefetch_desc(&tmap_a2);
   }
+  if (warp == 1) tmem_alloc<TMEM_COLS>(tmem_slot);
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem_base = *tmem_slot;
+  pdl_wait();
+
+  const int tiles_n = (p.N + BN - 1) / BN;
+  const int tiles_m = p.grp_mode == 1 ? p.grp_prefix[p.grp_count] : (p.M + BM - 1) / BM;
+  const int tiles_per_group = tiles_m * tiles_n;                       // grp_mode 2: one [M, N] output per group
+  const int num_tiles = p.grp_mode == 2 ? tiles_per_group * p.grp_count : tiles_per_group;
+  const int num_kb = (p.K + BK - 1) / BK;
+  const int num_items = num_tiles * p.k_splits;
+  const int m_limit = p.grp_mode == 1 ? tiles_m * BM : p.M;           // rows that exist
   // AG: M tiles are visited starting with this rank's own block, so the peers' rows are needed as late as possible
   const int ag_rot = (AG && p.ag_world > 0) ? p.ag_rank * (p.ag_rows / BM) : 0;
   // weight gather: N tiles are visited starting with the first tile of this rank's own part of the weight
@@ -241,11 +249,6 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
   }
   // the MMA thread and the epilogue depend on a producer that may be waiting for a peer: their own bound covers that wait
   const unsigned long long wait_ns = AG ? kWaitLimitNs + g_gemm_flag_wait_ns : kWaitLimitNs;
-  if (warp == 1) tmem_alloc<TMEM_COLS>(tmem_slot);
-  tc_fence_before();
-  __syncthreads();
-  tc_fence_after();
-  const uint32_t tmem_base = *tmem_slot;
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer
@@ -346,6 +349,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
           if (++stage == STAGES) { stage = 0; phase ^= 1; }
         }
       }
+      if (!AG) pdl_trigger();   // this block's last loads are on their way; AG waits for peers
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer
@@ -604,7 +608,10 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
     cluster_sync();   // nobody leaves while its part is being read
   }
   // ---------------------------------------------------------------- teardown
-  if (warp >= 2 && warp < 6 && lane == 0 && p.tma_store && p.cluster <= 1) tma_store_wait<0>();
+  if (warp >= 2 && warp < 6 && lane == 0 && p.tma_store && p.cluster <= 1) {
+    // the stores have read their staging buffers; that they have landed is the end of the kernel's business, but for a peer's memory
+    if (p.rs_world > 0) tma_store_wait<0>(); else tma_store_wait_read<0>();
+  }
   tc_fence_before();
   __syncthreads();
   if (*abort_flag) {
@@ -836,18 +843,9 @@ int launch_variant(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorM
     configured = true;
   }
   const int tiles = ((p.M + BM - 1) / BM) * ((p.N + BN - 1) / BN) * (p.grp_mode == 2 ? p.grp_count : 1) * p.k_splits;
-  if (!AG && p.cluster > 1) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(tiles); cfg.blockDim = dim3(NUM_THREADS); cfg.dynamicSmemBytes = L::kTotal; cfg.stream = stream;
-    cudaLaunchAttribute attr;
-    attr.id = cudaLaunchAttributeClusterDimension;
-    attr.val.clusterDim.x = p.cluster; attr.val.clusterDim.y = 1; attr.val.clusterDim.z = 1;
-    cfg.attrs = &attr; cfg.numAttrs = 1;
-    return (int)cudaLaunchKernelEx(&cfg, kern, ta, tb, td, ta2, rsm, p);
-  }
+  if (!AG && p.cluster > 1) return launch_pdl(kern, dim3(tiles), dim3(NUM_THREADS), L::kTotal, stream, p.cluster, ta, tb, td, ta2, rsm, p);
   const int grid = tiles < num_sms ? tiles : num_sms;   // grp_mode 1: p.M is the row capacity, an upper bound
-  kern<<<grid, AG ? NUM_THREADS + AG_PUSH_THREADS : NUM_THREADS, L::kTotal, stream>>>(ta, tb, td, ta2, rsm, p);
-  return (int)cudaGetLastError();
+  return launch_pdl(kern, dim3(grid), dim3(AG ? NUM_THREADS + AG_PUSH_THREADS : NUM_THREADS), L::kTotal, stream, 1, ta, tb, td, ta2, rsm, p);
 }
 
 int gemm_launch(const void* A, const void* B, void* D, float* Dacc32, const void* bias, int M, int N, int K, int lda, int ldb, int ldd,

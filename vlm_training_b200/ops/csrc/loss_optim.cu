@@ -2,6 +2,7 @@
 // AdamW update on flat fp32 master weights with a bf16 parameter write-back.
 #include "loss_optim.h"
 
+#include "pdl.cuh"
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -31,6 +32,7 @@ template <bool GRAD>
 __global__ void __launch_bounds__(CE_THREADS)
 ce_fwd_bwd_kernel(bf16* __restrict__ logits, long ld, const long* __restrict__ targets, float* __restrict__ loss, float grad_scale,
                   int V, long ignore_index) {
+  pdl_begin();
   __shared__ float s_m[CE_THREADS / 32], s_s[CE_THREADS / 32];
   __shared__ float s_max, s_lse;
   const long row = blockIdx.x;
@@ -236,6 +238,7 @@ adamw_bucket_kernel(bf16* __restrict__ grad, float* __restrict__ master, MT* __r
 // out[c] = sum_r x[r, c]  (bf16 in, fp32 accumulate): one thread per column pair inside a row slab, partials per slab
 __global__ void __launch_bounds__(256) colsum_kernel(const bf16* __restrict__ x, long ld, int rows, int cols, float* __restrict__ partial,
                                                       int rows_per_slab) {
+  pdl_begin();
   // block = 8 warps on the same 256 columns (lane <-> 8 columns, one 16-byte load per row); warp w takes rows w, w + 8, ...
   // of the slab, eight loads in flight; the warps' sums meet in shared memory
   __shared__ float red[8][256];
@@ -296,6 +299,7 @@ __device__ __forceinline__ void put_sum(void* out, int mode, long c, float t) {
 
 // out[c] = sum of the slabs' partial sums
 __global__ void colsum_finish_kernel(const float* __restrict__ partial, int slabs, int cols, void* __restrict__ out, int mode) {
+  pdl_begin();
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= cols) return;
   float t = 0.f;
@@ -307,6 +311,7 @@ __global__ void colsum_finish_kernel(const float* __restrict__ partial, int slab
 // A block owns 16 columns; its 256 threads are 16 row lanes x 16 columns, lane j adds rows j, j + 16, ... and the 16 lane
 // sums are added in lane order, so the result does not depend on timing.  blockIdx.y: which of up to two sums of a launch.
 __global__ void __launch_bounds__(256) sum_rows_kernel(const __grid_constant__ VlmtRowSums a, int rows, int cols) {
+  pdl_begin();
   const float* __restrict__ partial = a.partial[blockIdx.y];
   const long ld = a.ld;
   __shared__ float sm[16][17];
@@ -360,7 +365,7 @@ void vlmt_ce_fwd_bwd(void* logits, long ld, const long* targets, float* loss, fl
                      int want_grad, cudaStream_t st) {
   if (rows <= 0) return;
   auto kern = want_grad ? ce_fwd_bwd_kernel<true> : ce_fwd_bwd_kernel<false>;
-  kern<<<rows, CE_THREADS, 0, st>>>(reinterpret_cast<bf16*>(logits), ld, targets, loss, grad_scale, V, ignore_index);
+  launch_pdl(kern, dim3(rows), dim3(CE_THREADS), 0, st, 1, reinterpret_cast<bf16*>(logits), ld, targets, loss, grad_scale, V, ignore_index);
 }
 void vlmt_adamw(void* grad, int grad_fp32, float* master, void* m, void* v, int state_bf16, void* param, long n, float lr, float b1,
                 float b2, float eps, float wd, float bc1, float bc2, float grad_scale, int zero_grad, cudaStream_t st) {
@@ -421,14 +426,14 @@ void vlmt_colsum(const void* x, long ld, int rows, int cols, float* partial, voi
   const int slabs = rows > 0 ? vlmt_colsum_slabs(rows) : 0;
   if (slabs > 0) {
     dim3 grid((cols + 255) / 256, slabs);
-    colsum_kernel<<<grid, 256, 0, st>>>(reinterpret_cast<const bf16*>(x), ld, rows, cols, partial, 256);
+    launch_pdl(colsum_kernel, dim3(grid), dim3(256), 0, st, 1, reinterpret_cast<const bf16*>(x), ld, rows, cols, partial, 256);
   }
-  colsum_finish_kernel<<<(cols + 255) / 256, 256, 0, st>>>(partial, slabs, cols, out, mode);
+  launch_pdl(colsum_finish_kernel, dim3((cols + 255) / 256), dim3(256), 0, st, 1, partial, slabs, cols, out, mode);
 }
 // out[c] = sum over `rows` partial rows (the per-block weight-gradient sums of the norm kernels)
 void vlmt_sum_rows(const VlmtRowSums* a, int sums, int rows, int cols, cudaStream_t st) {
   if (cols <= 0 || sums <= 0) return;
-  sum_rows_kernel<<<dim3((cols + 15) / 16, sums), 256, 0, st>>>(*a, rows, cols);
+  launch_pdl(sum_rows_kernel, dim3(dim3((cols + 15) / 16, sums)), dim3(256), 0, st, 1, *a, rows, cols);
 }
 void vlmt_sumsq(const void* x, int fp32, long n, float* out, cudaStream_t st) {
   if (n <= 0) return;

@@ -14,6 +14,7 @@
 // the owner stores the expert output back into the source rank's per-slot buffer (kernels at the end of this file).
 #include "moe_kernels.h"
 
+#include "pdl.cuh"
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -41,6 +42,7 @@ __device__ __forceinline__ float warp_sum(float v) {
 template <typename LT>
 __global__ void moe_route_fwd_kernel(const LT* __restrict__ logits, int T, int E, int k, int renorm, float* __restrict__ weights,
                                      int* __restrict__ experts, int* __restrict__ counts) {
+  pdl_begin();
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (warp >= T) return;
   const LT* row = logits + (size_t)warp * E;
@@ -98,6 +100,7 @@ __global__ void moe_route_fwd_kernel(const LT* __restrict__ logits, int T, int E
 template <typename LT>
 __global__ void moe_route_bwd_kernel(const LT* __restrict__ logits, const int* __restrict__ experts, const float* __restrict__ weights,
                                      const float* __restrict__ dweights, int T, int E, int k, int renorm, LT* __restrict__ dlogits) {
+  pdl_begin();
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (warp >= T) return;
   const LT* row = logits + (size_t)warp * E;
@@ -153,6 +156,7 @@ __global__ void moe_route_bwd_kernel(const LT* __restrict__ logits, const int* _
 // ---------------------------------------------------------------------------------------------------- plan
 // Pass 1: per-block histogram of the experts of its chunk of slots -> hist[block][E]
 __global__ void moe_plan_hist_kernel(const int* __restrict__ experts, long n_slots, int E, int* __restrict__ hist) {
+  pdl_begin();
   extern __shared__ int sh[];
   for (int e = threadIdx.x; e < E; e += blockDim.x) sh[e] = 0;
   __syncthreads();
@@ -165,6 +169,7 @@ __global__ void moe_plan_hist_kernel(const int* __restrict__ experts, long n_slo
 // Pass 2 (one block): hist[b][e] becomes the exclusive prefix over blocks; counts[e] the total; prefix[e] the first tile of
 // expert e; prefix[E] the number of tiles in use.
 __global__ void moe_plan_scan_kernel(int* __restrict__ hist, int n_blocks, int E, int* __restrict__ counts, int* __restrict__ prefix) {
+  pdl_begin();
   extern __shared__ int tiles[];
   for (int e = threadIdx.x; e < E; e += blockDim.x) {
     int run = 0;
@@ -191,6 +196,7 @@ __global__ void moe_plan_scan_kernel(int* __restrict__ hist, int n_blocks, int E
 __global__ void moe_plan_place_kernel(const int* __restrict__ experts, long n_slots, int E, const int* __restrict__ hist,
                                       const int* __restrict__ prefix, const int* __restrict__ row_base, long cap_rows,
                                       int* __restrict__ dest, int* __restrict__ slot_of_row) {
+  pdl_begin();
   extern __shared__ int cursor[];
   for (int e = threadIdx.x; e < E; e += blockDim.x)
     cursor[e] = (row_base ? row_base[e] : prefix[e] * TILE) + hist[(size_t)blockIdx.x * E + e];
@@ -224,6 +230,7 @@ __global__ void moe_plan_place_kernel(const int* __restrict__ experts, long n_sl
 // scale: optional per-slot factor (the routing weight in the backward of combine).  One warp per row, 16-byte vectors.
 __global__ void moe_rows_from_tokens_kernel(const bf16* __restrict__ src, const int* __restrict__ slot_of_row, const int* __restrict__ prefix,
                                             int E, int k, int H, const float* __restrict__ scale, bf16* __restrict__ rows, long cap_rows) {
+  pdl_begin();
   const long row = ((long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   const long used = (long)prefix[E] * TILE;
@@ -258,6 +265,7 @@ __global__ void moe_rows_from_tokens_kernel(const bf16* __restrict__ src, const 
 __global__ void moe_tokens_from_rows_kernel(const bf16* __restrict__ rows, const int* __restrict__ dest, const float* __restrict__ w,
                                             int T, int k, int H, bf16* __restrict__ out, const bf16* __restrict__ g,
                                             float* __restrict__ dw) {
+  pdl_begin();
   const int t = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (t >= T) return;
   const int nvec = H >> 3;
@@ -428,8 +436,8 @@ int vlmt_moe_route_fwd(const void* logits, int logits_fp32, int T, int E, int k,
   if (E > 32 * MAX_E_PER_LANE || k > 32 || k > E) return -1;
   if (T <= 0) return 0;
   const int blocks = (T + 7) / 8;
-  if (logits_fp32) moe_route_fwd_kernel<float><<<blocks, 256, 0, st>>>((const float*)logits, T, E, k, renorm, weights, experts, counts);
-  else moe_route_fwd_kernel<bf16><<<blocks, 256, 0, st>>>((const bf16*)logits, T, E, k, renorm, weights, experts, counts);
+  if (logits_fp32) launch_pdl(moe_route_fwd_kernel<float>, dim3(blocks), dim3(256), 0, st, 1, (const float*)logits, T, E, k, renorm, weights, experts, counts);
+  else launch_pdl(moe_route_fwd_kernel<bf16>, dim3(blocks), dim3(256), 0, st, 1, (const bf16*)logits, T, E, k, renorm, weights, experts, counts);
   return (int)cudaGetLastError();
 }
 int vlmt_moe_route_bwd(const void* logits, int logits_fp32, const int* experts, const float* weights, const float* dweights, int T, int E,
@@ -438,9 +446,9 @@ int vlmt_moe_route_bwd(const void* logits, int logits_fp32, const int* experts, 
   if (T <= 0) return 0;
   const int blocks = (T + 7) / 8;
   if (logits_fp32)
-    moe_route_bwd_kernel<float><<<blocks, 256, 0, st>>>((const float*)logits, experts, weights, dweights, T, E, k, renorm, (float*)dlogits);
+    launch_pdl(moe_route_bwd_kernel<float>, dim3(blocks), dim3(256), 0, st, 1, (const float*)logits, experts, weights, dweights, T, E, k, renorm, (float*)dlogits);
   else
-    moe_route_bwd_kernel<bf16><<<blocks, 256, 0, st>>>((const bf16*)logits, experts, weights, dweights, T, E, k, renorm, (bf16*)dlogits);
+    launch_pdl(moe_route_bwd_kernel<bf16>, dim3(blocks), dim3(256), 0, st, 1, (const bf16*)logits, experts, weights, dweights, T, E, k, renorm, (bf16*)dlogits);
   return (int)cudaGetLastError();
 }
 int vlmt_moe_plan_blocks(long n_slots) { return (int)((n_slots + PLAN_CHUNK - 1) / PLAN_CHUNK); }
@@ -448,8 +456,8 @@ int vlmt_moe_plan_blocks(long n_slots) { return (int)((n_slots + PLAN_CHUNK - 1)
 int vlmt_moe_plan_count(const int* experts, long n_slots, int E, int* hist, int* counts, int* prefix, cudaStream_t st) {
   if (E > 4096) return -1;
   const int nb = vlmt_moe_plan_blocks(n_slots);
-  if (nb > 0) moe_plan_hist_kernel<<<nb, PLAN_THREADS, E * sizeof(int), st>>>(experts, n_slots, E, hist);
-  moe_plan_scan_kernel<<<1, 256, E * sizeof(int), st>>>(hist, nb, E, counts, prefix);
+  if (nb > 0) launch_pdl(moe_plan_hist_kernel, dim3(nb), dim3(PLAN_THREADS), E * sizeof(int), st, 1, experts, n_slots, E, hist);
+  launch_pdl(moe_plan_scan_kernel, dim3(1), dim3(256), E * sizeof(int), st, 1, hist, nb, E, counts, prefix);
   return (int)cudaGetLastError();
 }
 // stage 2: dest [n_slots]; slot_of_row [cap_rows] (optional; set to -1 first); row_base (optional) replaces prefix * 128
@@ -462,7 +470,7 @@ int vlmt_moe_plan_place(const int* experts, long n_slots, int E, const int* hist
   }
   const int nb = vlmt_moe_plan_blocks(n_slots);
   if (nb > 0)
-    moe_plan_place_kernel<<<nb, PLAN_THREADS, E * sizeof(int), st>>>(experts, n_slots, E, hist, prefix, row_base, cap_rows, dest, slot_of_row);
+    launch_pdl(moe_plan_place_kernel, dim3(nb), dim3(PLAN_THREADS), E * sizeof(int), st, 1, experts, n_slots, E, hist, prefix, row_base, cap_rows, dest, slot_of_row);
   return (int)cudaGetLastError();
 }
 int vlmt_moe_plan(const int* experts, long n_slots, int E, int* hist, int* counts, int* prefix, int* dest, int* slot_of_row, long cap_rows,
@@ -476,14 +484,14 @@ int vlmt_moe_rows_from_tokens(const void* src, const int* slot_of_row, const int
   if (H & 7) return -1;
   if (cap_rows <= 0) return 0;
   const long blocks = (cap_rows + 7) / 8;
-  moe_rows_from_tokens_kernel<<<(unsigned)blocks, 256, 0, st>>>((const bf16*)src, slot_of_row, prefix, E, k, H, scale, (bf16*)rows, cap_rows);
+  launch_pdl(moe_rows_from_tokens_kernel, dim3((unsigned)blocks), dim3(256), 0, st, 1, (const bf16*)src, slot_of_row, prefix, E, k, H, scale, (bf16*)rows, cap_rows);
   return (int)cudaGetLastError();
 }
 int vlmt_moe_tokens_from_rows(const void* rows, const int* dest, const float* w, int T, int k, int H, void* out, const void* g, float* dw,
                               cudaStream_t st) {
   if (H & 7) return -1;
   if (T <= 0) return 0;
-  moe_tokens_from_rows_kernel<<<(T + 7) / 8, 256, 0, st>>>((const bf16*)rows, dest, w, T, k, H, (bf16*)out, (const bf16*)g, dw);
+  launch_pdl(moe_tokens_from_rows_kernel, dim3((T + 7) / 8), dim3(256), 0, st, 1, (const bf16*)rows, dest, w, T, k, H, (bf16*)out, (const bf16*)g, dw);
   return (int)cudaGetLastError();
 }
 

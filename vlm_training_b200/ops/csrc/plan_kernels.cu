@@ -3,12 +3,14 @@
 // by launches and host work.
 #include "plan_kernels.h"
 
+#include "pdl.cuh"
 #include <cuda_bf16.h>
 #include <stdint.h>
 
 namespace {
 __global__ void rope_tables_kernel(const long* __restrict__ pos, int axes, const float* __restrict__ inv_freq, int n, int sec1, int sec2, long T,
                                    float* __restrict__ cosv, float* __restrict__ sinv) {
+  pdl_begin();
   const long i = blockIdx.x * (long)blockDim.x + threadIdx.x;
   if (i >= T * n) return;
   const long t = i / n;
@@ -42,6 +44,7 @@ __device__ __forceinline__ Cell cell_of(int i, int count, int side, double step)
 
 __global__ void vision_plan_kernel(const int* __restrict__ images, int n_img, const float2* __restrict__ trig, int coords, int nf, int side, int merge, long N,
                                    float* __restrict__ cosv, float* __restrict__ sinv, long* __restrict__ pe_index, float* __restrict__ pe_weight) {
+  pdl_begin();
   // a warp per patch: lanes share its angles
   const long n = (blockIdx.x * (long)blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
@@ -86,6 +89,7 @@ __device__ __forceinline__ uint4 pack8(const float (&f)[8]) {
 __global__ void __launch_bounds__(256) pos_embed_fwd_kernel(const uint4* __restrict__ x, const uint4* __restrict__ table,
                                                             const long* __restrict__ pe_index, const float* __restrict__ pe_weight,
                                                             uint4* __restrict__ out, long N, int dv) {
+  pdl_begin();
   const long i = blockIdx.x * (long)blockDim.x + threadIdx.x;
   if (i >= N * dv) return;
   const long n = i / dv;
@@ -114,6 +118,7 @@ __global__ void __launch_bounds__(256) pos_embed_fwd_kernel(const uint4* __restr
 // within one cell of it), so the gradient is a gather in fixed order: no sort, no atomics, every dy row read by four cells.
 __global__ void __launch_bounds__(256) pos_embed_bwd_kernel(const uint4* __restrict__ dy, const int* __restrict__ images, int n_img, int side,
                                                             int merge, long N, uint4* __restrict__ dtable, int accumulate, int dv) {
+  pdl_begin();
   const int cr = blockIdx.x / side, cc = blockIdx.x % side;
   for (int v = threadIdx.x; v < dv; v += blockDim.x) {
     float a[8];
@@ -163,22 +168,22 @@ extern "C" {
 void vlmt_rope_tables(const long* pos, int axes, const float* inv_freq, int n, int sec1, int sec2, long T, float* cosv, float* sinv,
                       cudaStream_t st) {
   if (T <= 0 || n <= 0) return;
-  rope_tables_kernel<<<(unsigned)((T * n + 255) / 256), 256, 0, st>>>(pos, axes, inv_freq, n, sec1, sec2, T, cosv, sinv);
+  launch_pdl(rope_tables_kernel, dim3((unsigned)((T * n + 255) / 256)), dim3(256), 0, st, 1, pos, axes, inv_freq, n, sec1, sec2, T, cosv, sinv);
 }
 void vlmt_vision_plan(const int* images, int n_img, const float* trig, int coords, int nf, int side, int merge, long N, float* cosv,
                       float* sinv, long* pe_index, float* pe_weight, cudaStream_t st) {
   if (N <= 0) return;
-  vision_plan_kernel<<<(unsigned)((N * 32 + 255) / 256), 256, 0, st>>>(images, n_img, (const float2*)trig, coords, nf, side, merge, N, cosv, sinv, pe_index, pe_weight);
+  launch_pdl(vision_plan_kernel, dim3((unsigned)((N * 32 + 255) / 256)), dim3(256), 0, st, 1, images, n_img, (const float2*)trig, coords, nf, side, merge, N, cosv, sinv, pe_index, pe_weight);
 }
 void vlmt_pos_embed_fwd(const void* x, const void* table, const long* pe_index, const float* pe_weight, void* out, long N, int D,
                         cudaStream_t st) {
   if (N <= 0) return;
-  pos_embed_fwd_kernel<<<(unsigned)((N * (D / 8) + 255) / 256), 256, 0, st>>>((const uint4*)x, (const uint4*)table, pe_index, pe_weight, (uint4*)out,
+  launch_pdl(pos_embed_fwd_kernel, dim3((unsigned)((N * (D / 8) + 255) / 256)), dim3(256), 0, st, 1, (const uint4*)x, (const uint4*)table, pe_index, pe_weight, (uint4*)out,
                                                                               N, D / 8);
 }
 void vlmt_pos_embed_bwd(const void* dy, const int* images, int n_img, int side, int merge, long N, void* dtable, int accumulate, int D,
                         cudaStream_t st) {
   const int dv = D / 8, threads = dv >= 256 ? 256 : (dv + 31) / 32 * 32;
-  pos_embed_bwd_kernel<<<side * side, threads, 0, st>>>((const uint4*)dy, images, n_img, side, merge, N, (uint4*)dtable, accumulate, dv);
+  launch_pdl(pos_embed_bwd_kernel, dim3(side * side), dim3(threads), 0, st, 1, (const uint4*)dy, images, n_img, side, merge, N, (uint4*)dtable, accumulate, dv);
 }
 }
