@@ -75,6 +75,17 @@ def test_gemm_cta_pairs(M, N, K, layout):
     cu.check_status()
 
 
+# CTA pairs with between half a wave and one wave of tiles, where K would else be split; raster groups of 16 pairs, the last one short
+@pytest.mark.parametrize("M,N,K", [(300, 6144, 520), (1000, 2600, 72), (4360, 8200, 2056)])
+def test_gemm_cta_pairs_raster_and_single_wave(M, N, K):
+    from vlm_training_b200.ops import cuda as cu
+
+    a, b, bias = _rand(M, K, scale=0.5), _rand(N, K, scale=0.5), _rand(N)
+    want = a.float() @ b.float().t() + bias.float()
+    torch.testing.assert_close(cu._gemm(a, b, bias=bias).float(), want, atol=1e-2, rtol=8e-3)   # one bf16 rounding (2^-8 of the value)
+    cu.check_status()
+
+
 # the first case keeps d(logits) for backward (T <= 2 H), the second forms the gradients chunk by chunk (T > 2 H, V large)
 @pytest.mark.parametrize("T,H,V,chunk", [(700, 512, 5000, 256), (1030, 256, 151936, 512)])
 def test_linear_cross_entropy_both_gradient_forms_and_evaluation(T, H, V, chunk):

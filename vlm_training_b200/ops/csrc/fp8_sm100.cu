@@ -203,7 +203,7 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
         const int kb_lo = p.k_splits > 1 ? ks * p.kb_per_split : 0;
         const int kb_hi = p.k_splits > 1 ? min(num_kb, kb_lo + p.kb_per_split) : num_kb;
         int tm, tn;
-        tile_coords<GROUP_M>(tile, tiles_m, tiles_n, tm, tn);
+        tile_coords(GROUP_M, tile, tiles_m, tiles_n, tm, tn);
         const int m0 = tm * BM, n0 = tn * BN;
         for (int kb = kb_lo; kb < kb_hi; ++kb) {
           if (!mbar_wait(&empty_bar[stage], phase ^ 1, abort_flag, p.status, kErrTimeoutEmpty)) { ok = false; break; }
@@ -261,7 +261,7 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
     for (int item = blockIdx.x; item < num_items && ok; item += gridDim.x, ++it) {
       const int tile = item % num_tiles;
       int tm, tn;
-      tile_coords<GROUP_M>(tile, tiles_m, tiles_n, tm, tn);
+      tile_coords(GROUP_M, tile, tiles_m, tiles_n, tm, tn);
       const int acc = it & 1;
       const uint32_t acc_phase = (it >> 1) & 1;
       if (!mbar_wait(&tmem_full[acc], acc_phase, abort_flag, p.status, kErrTimeoutTmemFull)) { ok = false; break; }

@@ -5,13 +5,12 @@
 #include "sm100.cuh"
 
 namespace sm100 {
-// Tiles in groups of GROUP_M rows of tiles, columns inside a group: the group's rows of A and the B panel they meet share L2.
-template <int GROUP_M>
-__device__ __forceinline__ void tile_coords(int tile, int tiles_m, int tiles_n, int& tm, int& tn) {
-  const int per_group = GROUP_M * tiles_n;
+// Tiles in groups of `group_m` rows of tiles, columns inside a group: the group's rows of A and the B panel they meet share L2.
+__device__ __forceinline__ void tile_coords(int group_m, int tile, int tiles_m, int tiles_n, int& tm, int& tn) {
+  const int per_group = group_m * tiles_n;
   const int g = tile / per_group;
-  const int first_m = g * GROUP_M;
-  const int gsz = min(GROUP_M, tiles_m - first_m);
+  const int first_m = g * group_m;
+  const int gsz = min(group_m, tiles_m - first_m);
   const int r = tile - g * per_group;
   tm = first_m + r % gsz;
   tn = r / gsz;

@@ -26,7 +26,12 @@ using namespace sm100;
 
 constexpr int BM = 128, BN = 256, BK = 64, UMMA_K = 16, STAGES = 6;   // BK, UMMA_K in bf16 elements; FP8: twice as many of a byte each
 constexpr int NUM_THREADS = 192;
-constexpr int GROUP_M = 8;   // pairs of M tiles per raster group: 2048 rows of A and the B panel they meet share L2
+
+// Pairs of M tiles per raster group: their rows of A and the B panel they meet share L2.  Every group reads all of B, so where B does not
+// stay in L2 (32 MB and more) and 4096 rows of A do (K up to 4096 bf16 values) a group is 16 pairs, else 8.  PFLOP/s with 8 / 16, under the power limit:
+// 8192 x 24576 x 4096 1.33 / 1.40, 8192 x 12288 x 4096 1.33 / 1.38, 8192 x 6144 x 4096 1.28 / 1.31; 8192 x 4096 x 12288 1.27 / 1.25,
+// weight gradient 24576 x 4096 x 8192 1.25 / 1.24, 28672 x 1152 x 4304 1.12 / 1.08.
+int raster_group(long n_bytes, long k_bytes) { return n_bytes >= (32l << 20) && 4096 * k_bytes <= (36l << 20) ? 16 : 8; }
 
 constexpr int kABytes = BM * BK * 2, kBBytes = (BN / 2) * BK * 2, kStageBytes = kABytes + kBBytes;
 constexpr int kOutOffset = STAGES * kStageBytes;       // epilogue staging: 4 warps x 2 buffers x [32 rows][128 B]
@@ -36,6 +41,7 @@ static_assert(kSmem <= 232448, "shared memory");
 
 struct Params {
   int M, N, K;
+  int group_m;
   const __nv_bfloat16* bias;
   const float* alpha;
   int epilogue, accumulate;
@@ -103,7 +109,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
       for (int item = pair; item < num_items && ok; item += pairs) {
         int tile, kb_lo, kb_hi, tm, tn;
         k_range(item, tile, kb_lo, kb_hi);
-        tile_coords<GROUP_M>(tile, tiles_m, tiles_n, tm, tn);
+        tile_coords(p.group_m, tile, tiles_m, tiles_n, tm, tn);
         const int m0 = (tm * 2 + (int)rank) * BM, n0 = tn * BN + (int)rank * (BN / 2);
         for (int kb = kb_lo; kb < kb_hi; ++kb) {
           if (!mbar_wait(&empty_bar[stage], phase ^ 1, abort_flag, p.status, kErrTimeoutEmpty)) { ok = false; break; }
@@ -169,7 +175,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
     for (int item = pair; item < num_items; item += pairs, ++it) {
       const int tile = p.k_splits > 1 ? item % num_tiles : item;
       int tm, tn;
-      tile_coords<GROUP_M>(tile, tiles_m, tiles_n, tm, tn);
+      tile_coords(p.group_m, tile, tiles_m, tiles_n, tm, tn);
       const int acc = it & 1;
       if (!mbar_wait(&tmem_full[acc], (it >> 1) & 1, abort_flag, p.status, kErrTimeoutTmemFull)) break;
       tc_fence_after();
@@ -266,6 +272,7 @@ extern "C" int vlmt_gemm_pair(const void* A, const void* B, void* D, const void*
   Params p = {};
   p.M = M; p.N = N; p.K = K; p.bias = reinterpret_cast<const __nv_bfloat16*>(bias); p.alpha = alpha; p.epilogue = epilogue;
   p.accumulate = accumulate; p.k_splits = k_splits; p.kb_per_split = kb_per_split; p.status = status;
+  p.group_m = raster_group(2l * N * K, 2l * K);
   if (a_mn_major) return b_mn_major ? launch<true, true>(ta, tb, td, p, stream) : launch<true, false>(ta, tb, td, p, stream);
   return b_mn_major ? launch<false, true>(ta, tb, td, p, stream) : launch<false, false>(ta, tb, td, p, stream);
 }
@@ -281,5 +288,6 @@ extern "C" int vlmt_gemm_pair_fp8(const void* A, const void* B, void* D, int M, 
   Params p = {};
   p.M = M; p.N = N; p.K = K; p.rec_a = rec_a; p.rec_b = rec_b; p.idesc = idesc;
   p.accumulate = accumulate; p.k_splits = k_splits; p.kb_per_split = kb_per_split; p.status = status;
+  p.group_m = raster_group((long)N * K, K);
   return launch<false, false, true>(ta, tb, td, p, stream);
 }

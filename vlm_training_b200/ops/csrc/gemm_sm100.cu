@@ -266,11 +266,11 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
         }
         if (p.grp_mode == 2) {
           const int g = tile / tiles_per_group;
-          tile_coords<GROUP_M>(tile - g * tiles_per_group, tiles_m, tiles_n, tm, tn);
+          tile_coords(GROUP_M, tile - g * tiles_per_group, tiles_m, tiles_n, tm, tn);
           kb_lo = p.grp_prefix[g] * (BM / BK);
           kb_hi = p.grp_prefix[g + 1] * (BM / BK);
         } else {
-          tile_coords<GROUP_M>(tile, tiles_m, tiles_n, tm, tn);
+          tile_coords(GROUP_M, tile, tiles_m, tiles_n, tm, tn);
           if (p.grp_mode == 1) b_row = group_of_tile(p.grp_prefix, p.grp_count, tm) * p.grp_b_rows;
         }
         if (AG) { tm += ag_rot; if (tm >= tiles_m) tm -= tiles_m; tn += wg_rot; if (tn >= tiles_n) tn -= tiles_n; }
@@ -471,11 +471,11 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
       bool empty_group = false;   // grp_mode 2: no rows for this group, the accumulator was never written -> zeros
       if (p.grp_mode == 2) {
         const int g = tile / tiles_per_group;
-        tile_coords<GROUP_M>(tile - g * tiles_per_group, tiles_m, tiles_n, tm, tn);
+        tile_coords(GROUP_M, tile - g * tiles_per_group, tiles_m, tiles_n, tm, tn);
         d_row0 = g * p.M;
         empty_group = p.grp_prefix[g + 1] == p.grp_prefix[g];
       } else {
-        tile_coords<GROUP_M>(tile, tiles_m, tiles_n, tm, tn);
+        tile_coords(GROUP_M, tile, tiles_m, tiles_n, tm, tn);
       }
       if (AG) { tm += ag_rot; if (tm >= tiles_m) tm -= tiles_m; tn += wg_rot; if (tn >= tiles_n) tn -= tiles_n; }
       const int acc = it & 1;
@@ -600,7 +600,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
   if (p.cluster > 1) {
     // one item per block; every thread of the cluster passes both barriers, also after an abort
     int tm, tn;
-    tile_coords<GROUP_M>(blockIdx.x / p.cluster, tiles_m, tiles_n, tm, tn);
+    tile_coords(GROUP_M, blockIdx.x / p.cluster, tiles_m, tiles_n, tm, tn);
     __syncwarp();
     cluster_sync();
     if (!*abort_flag) store_cluster_sum<BN>(smem, p, tm * BM, tn * BN, blockIdx.x % p.cluster, p.alpha != nullptr ? __ldg(p.alpha) : 1.f);
@@ -929,8 +929,16 @@ int gemm_launch(const void* A, const void* B, void* D, float* Dacc32, const void
   }
   // large bf16 outputs go to CTA pairs: at least one wave of 256 x 256 tiles, so the coarser tiles leave no SM idle.  With one row of
   // 128-row tiles half of every pair would have no rows (37 x 24576 x 4096 63.5 us in pairs, 53.3 us without, 1200 x 24576 x 4096 164 and 193).
-  if (plain && M > BM && p.tma_store && p.cluster <= 1 && vlmt_gemm_pair_enabled() &&
-      (long)((M + 255) / 256) * ((N + 255) / 256) * p.k_splits >= num_sms / 2)
+  // More than half a wave of them also beats narrower tiles and K split over clusters, which are bound by their loads (128 + 128 rows of
+  // operands for half the product): 451 x 6144 x 4096 (48 tiles) 29.8 -> 25.4 us, 700 x 4096 x 12288 (48) 77 -> 65, 1000 x 4096 x 4608 (64)
+  // 32.0 -> 28.2, 2500 x 1152 x 4304 (50) 31.6 -> 25.6; below that the idle SMs weigh more (451 x 4096 x 12288, 32 tiles, 51 -> 60).
+  const long pair_tiles = (long)((M + 255) / 256) * ((N + 255) / 256);
+  const bool one_wave = (p.cluster > 1 || p.k_splits == 1) && pair_tiles * 2 <= num_sms && pair_tiles * 37 >= num_sms * 10;
+  if (plain && M > BM && p.tma_store && vlmt_gemm_pair_enabled() && one_wave) {
+    p.cluster = p.k_splits = 1;
+    p.kb_per_split = (K + BK - 1) / BK;
+  }
+  if (plain && M > BM && p.tma_store && p.cluster <= 1 && vlmt_gemm_pair_enabled() && (one_wave || pair_tiles * p.k_splits >= num_sms / 2))
     return vlmt_gemm_pair(A, B, D, bias, M, N, K, lda, ldb, ldd, a_mn_major, b_mn_major, epilogue, accumulate, x.alpha, p.k_splits, p.kb_per_split,
                           status, stream);
   p.ag_world = 0; p.ag_rank = 0; p.ag_rows = 0; p.ag_epoch = 0;
