@@ -75,6 +75,16 @@ def test_gemm_cta_pairs(M, N, K, layout):
     cu.check_status()
 
 
+# two CTA pairs of a cluster share a tile and its K: rows and columns off the tile edges, an odd number of K blocks, every layout, added to D
+@pytest.mark.parametrize("M,N,K,layout", [(451, 4104, 4160, "fwd"), (520, 2056, 2056, "dgrad"), (392, 3200, 8200, "wgrad")])
+def test_gemm_cta_pairs_split_over_k(M, N, K, layout):
+    test_gemm_cta_pairs(M, N, K, layout)
+    from vlm_training_b200.ops import cuda as cu
+
+    a, b = _rand(M, K, scale=0.5), _rand(N, K, scale=0.5)
+    assert torch.equal(cu._gemm(a, b), cu._gemm(a, b))   # the parts are summed in rank order
+
+
 # CTA pairs with between half a wave and one wave of tiles, where K would else be split; raster groups of 16 pairs, the last one short
 @pytest.mark.parametrize("M,N,K", [(300, 6144, 520), (1000, 2600, 72), (4360, 8200, 2056)])
 def test_gemm_cta_pairs_raster_and_single_wave(M, N, K):

@@ -42,6 +42,9 @@ static_assert(kSmem <= 232448, "shared memory");
 struct Params {
   int M, N, K;
   int group_m;
+  int parts;                    // pairs of a cluster that share one tile: each computes a part of K, then all sum the parts and store
+  __nv_bfloat16* D;             // parts > 1
+  int ldd;
   const __nv_bfloat16* bias;
   const float* alpha;
   int epilogue, accumulate;
@@ -51,6 +54,50 @@ struct Params {
   uint32_t idesc;               // FP8: carries the two formats
   int* status;
 };
+
+constexpr int kPartPitch = BN + 4;   // floats per row of a block's part in shared memory (conflict-free 16-byte stores)
+static_assert(BM * kPartPitch * 4 <= kOutOffset, "a part lies over the operand stages");
+
+// Sum of the parts of this block's 128 rows and the epilogue, four columns at a time; the blocks of the cluster that hold the same rows
+// (every second one) take an equal share each and sum in order of their rank.
+__device__ __forceinline__ void store_parts(const uint8_t* smem, const Params& p, int m0, int n0, int rank, float alpha) {
+  constexpr int GROUPS = BN / 4, U = 8;   // U groups per thread and round: their remote loads are in flight together
+  const int rows = min(BM, p.M - m0), step = p.parts * NUM_THREADS;
+  const uint32_t base = smem_u32(smem);
+  for (int i0 = (rank >> 1) * NUM_THREADS + threadIdx.x; i0 < rows * GROUPS; i0 += U * step) {
+    float v[U][4];
+#pragma unroll
+    for (int u = 0; u < U; ++u) v[u][0] = v[u][1] = v[u][2] = v[u][3] = 0.f;
+    for (int s = 0; s < p.parts; ++s) {
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const int i = min(i0 + u * step, rows * GROUPS - 1);
+        const float4 f = ld_cluster_f4(base + (uint32_t)((i / GROUPS) * kPartPitch + (i % GROUPS) * 4) * 4, 2 * s + (rank & 1));
+        v[u][0] += f.x; v[u][1] += f.y; v[u][2] += f.z; v[u][3] += f.w;
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int i = i0 + u * step, col = n0 + (i % GROUPS) * 4;
+      if (i >= rows * GROUPS || col >= p.N) continue;
+      __nv_bfloat16* dst = p.D + (size_t)(m0 + i / GROUPS) * p.ldd + col;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        float x = v[u][j] * alpha;
+        if (p.bias != nullptr && col + j < p.N) x += __bfloat162float(p.bias[col + j]);
+        if (p.epilogue == GEMM_EPI_GELU_TANH) x = gelu_tanh_f(x);
+        else if (p.epilogue == GEMM_EPI_GELU_ERF) x = gelu_erf_f(x);
+        v[u][j] = p.accumulate && col + j < p.N ? x + __bfloat162float(dst[j]) : x;
+      }
+      if (col + 4 <= p.N) {   // rows of D start on 16 bytes
+        *reinterpret_cast<uint2*>(dst) = make_uint2(pack_bf16x2(v[u][0], v[u][1]), pack_bf16x2(v[u][2], v[u][3]));
+      } else {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) if (col + j < p.N) dst[j] = __float2bfloat16(v[u][j]);
+      }
+    }
+  }
+}
 
 template <bool A_MN, bool B_MN, bool FP8>
 __global__ void __launch_bounds__(NUM_THREADS, 1)
@@ -66,9 +113,10 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const uint32_t rank = cluster_rank();
+  const uint32_t rank = cluster_rank() & 1, lead = cluster_rank() & ~1u;   // place in the pair; its leader's rank in the cluster
   const bool leader = rank == 0;
-  const int pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
+  const uint16_t both = (uint16_t)(3u << lead);
+  const int pair = blockIdx.x / (2 * p.parts), pairs = gridDim.x / (2 * p.parts);   // parts > 1: one tile per cluster
   const int tiles_m = (p.M + 2 * BM - 1) / (2 * BM), tiles_n = (p.N + BN - 1) / BN;
   const int num_tiles = tiles_m * tiles_n, num_items = num_tiles * p.k_splits;
   constexpr int kStageK = FP8 ? 2 * BK : BK;
@@ -93,6 +141,10 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
 
   auto k_range = [&](int item, int& tile, int& kb_lo, int& kb_hi) {
     tile = item; kb_lo = 0; kb_hi = num_kb;
+    if (p.parts > 1) {
+      kb_lo = (int)(lead >> 1) * p.kb_per_split;
+      kb_hi = min(num_kb, kb_lo + p.kb_per_split);
+    }
     if (p.k_splits > 1) {
       const int ks = item / num_tiles;
       tile = item - ks * num_tiles;
@@ -115,7 +167,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
           if (!mbar_wait(&empty_bar[stage], phase ^ 1, abort_flag, p.status, kErrTimeoutEmpty)) { ok = false; break; }
           uint8_t* sa = smem + stage * kStageBytes;
           uint8_t* sb = sa + kABytes;
-          const uint32_t bar = cluster_addr(&full_bar[stage], 0);
+          const uint32_t bar = cluster_addr(&full_bar[stage], lead);
           if (leader) mbar_expect_tx(&full_bar[stage], 2 * kStageBytes);
           const int k0 = kb * kStageK;   // a multiple of 128 bytes
           if (!A_MN) tma_load_2d_pair(sa, &tmap_a, bar, k0, m0);                     // box {64 k, 128 m}
@@ -159,10 +211,10 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
             if (k == 0) umma_ss_pair<2, FP8>(d_tmem, ad, bd, idesc, (uint32_t)(kb - kb_lo));
             else umma_ss_pair<1, FP8>(d_tmem, ad, bd, idesc);
           }
-          umma_commit_pair(&empty_bar[stage]);
+          umma_commit_pair(&empty_bar[stage], both);
           if (++stage == STAGES) { stage = 0; phase ^= 1; }
         }
-        if (ok) umma_commit_pair(&tmem_full[acc]);
+        if (ok) umma_commit_pair(&tmem_full[acc], both);
       }
     }
   } else {
@@ -181,6 +233,19 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
       tc_fence_after();
       const int row0 = (tm * 2 + (int)rank) * BM + q * 32, n0 = tn * BN;
       const uint32_t taddr = tmem_base + acc * BN + ((uint32_t)(q * 32) << 16);
+      if (p.parts > 1) {
+        // the operand stages are free: every MMA of the pair's only item has completed
+        float* part = reinterpret_cast<float*>(smem) + (q * 32 + lane) * kPartPitch;
+#pragma unroll 1
+        for (int c = 0; c < BN / 32; ++c) {
+          uint32_t r[32];
+          tmem_ld_32x32(taddr + c * 32, r);
+          tmem_ld_wait();
+#pragma unroll
+          for (int i = 0; i < 32; i += 4) *reinterpret_cast<uint4*>(part + c * 32 + i) = make_uint4(r[i], r[i + 1], r[i + 2], r[i + 3]);
+        }
+        break;
+      }
 #pragma unroll 1
       for (int c = 0; c < BN / 64; ++c) {
         const int col0 = n0 + c * 64;
@@ -209,9 +274,18 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
       }
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive_cluster(cluster_addr(&tmem_empty[acc], 0));
+      if (lane == 0) mbar_arrive_cluster(cluster_addr(&tmem_empty[acc], lead));
     }
     if (lane == 0) tma_store_wait_read<0>();
+  }
+  if (p.parts > 1) {   // every block of the cluster passes both barriers, also after an abort
+    int tm, tn;
+    tile_coords(p.group_m, pair, tiles_m, tiles_n, tm, tn);
+    __syncwarp();
+    cluster_sync();
+    if (!*abort_flag) store_parts(smem, p, (tm * 2 + (int)rank) * BM, tn * BN, (int)(lead + rank), p.alpha != nullptr ? __ldg(p.alpha) : 1.f);
+    __syncwarp();
+    cluster_sync();    // nobody leaves while its part is being read
   }
   // ---------------------------------------------------------------- teardown
   tc_fence_before();
@@ -247,6 +321,10 @@ int launch(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& td, 
     if (cudaOccupancyMaxActiveClusters(&n, kern, &cfg) == cudaSuccess) max_pairs = n;
   });
   if (max_pairs <= 0) return -50;
+  if (p.parts > 1) {
+    const int tiles = ((p.M + 2 * BM - 1) / (2 * BM)) * ((p.N + BN - 1) / BN);
+    return launch_pdl(kern, dim3(2 * p.parts * tiles), dim3(NUM_THREADS), kSmem, st, 2 * p.parts, ta, tb, td, p);
+  }
   const int items = ((p.M + 2 * BM - 1) / (2 * BM)) * ((p.N + BN - 1) / BN) * p.k_splits;
   return launch_pdl(kern, dim3(2 * (items < max_pairs ? items : max_pairs)), dim3(NUM_THREADS), kSmem, st, 2, ta, tb, td, p);
 }
@@ -257,9 +335,30 @@ extern "C" int vlmt_gemm_pair_enabled() {
   return on;
 }
 
+// Clusters of two pairs that the GPU holds at once (0: not known).  All variants have the same footprint.
+extern "C" int vlmt_gemm_pair_clusters() {
+  static int cap = 0;
+  static std::once_flag once;
+  std::call_once(once, [] {
+    auto kern = gemm_pair_kernel<false, false, false>;
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = 4; attr.val.clusterDim.y = 1; attr.val.clusterDim.z = 1;
+    cfg.gridDim = dim3(4); cfg.blockDim = dim3(NUM_THREADS); cfg.dynamicSmemBytes = kSmem;
+    cfg.attrs = &attr; cfg.numAttrs = 1;
+    int n = 0;
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem) == cudaSuccess &&
+        cudaOccupancyMaxActiveClusters(&n, kern, &cfg) == cudaSuccess)
+      cap = n;
+    (void)cudaGetLastError();
+  });
+  return cap;
+}
+
 extern "C" int vlmt_gemm_pair(const void* A, const void* B, void* D, const void* bias, int M, int N, int K, int lda, int ldb, int ldd,
                               int a_mn_major, int b_mn_major, int epilogue, int accumulate, const float* alpha, int k_splits, int kb_per_split,
-                              int* status, cudaStream_t stream) {
+                              int parts, int* status, cudaStream_t stream) {
   CUtensorMap ta, tb, td;
   int r;
   if (!a_mn_major) r = vlmt_make_tmap_2d_bf16(&ta, A, (uint64_t)K, (uint64_t)M, (uint64_t)lda * 2, 64, 128);
@@ -273,6 +372,7 @@ extern "C" int vlmt_gemm_pair(const void* A, const void* B, void* D, const void*
   p.M = M; p.N = N; p.K = K; p.bias = reinterpret_cast<const __nv_bfloat16*>(bias); p.alpha = alpha; p.epilogue = epilogue;
   p.accumulate = accumulate; p.k_splits = k_splits; p.kb_per_split = kb_per_split; p.status = status;
   p.group_m = raster_group(2l * N * K, 2l * K);
+  p.parts = parts; p.D = reinterpret_cast<__nv_bfloat16*>(D); p.ldd = ldd;
   if (a_mn_major) return b_mn_major ? launch<true, true>(ta, tb, td, p, stream) : launch<true, false>(ta, tb, td, p, stream);
   return b_mn_major ? launch<false, true>(ta, tb, td, p, stream) : launch<false, false>(ta, tb, td, p, stream);
 }
@@ -289,5 +389,6 @@ extern "C" int vlmt_gemm_pair_fp8(const void* A, const void* B, void* D, int M, 
   p.M = M; p.N = N; p.K = K; p.rec_a = rec_a; p.rec_b = rec_b; p.idesc = idesc;
   p.accumulate = accumulate; p.k_splits = k_splits; p.kb_per_split = kb_per_split; p.status = status;
   p.group_m = raster_group((long)N * K, K);
+  p.parts = 1;
   return launch<false, false, true>(ta, tb, td, p, stream);
 }

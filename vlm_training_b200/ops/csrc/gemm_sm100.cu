@@ -938,9 +938,20 @@ int gemm_launch(const void* A, const void* B, void* D, float* Dacc32, const void
     p.cluster = p.k_splits = 1;
     p.kb_per_split = (K + BK - 1) / BK;
   }
-  if (plain && M > BM && p.tma_store && p.cluster <= 1 && vlmt_gemm_pair_enabled() && (one_wave || pair_tiles * p.k_splits >= num_sms / 2))
+  // Fewer tiles of a long K (16 blocks of 64 and more for each part): two pairs of a cluster share a tile while all clusters fit the GPU at
+  // once and keep two thirds of it busy.  451 x 4096 x 12288 (32 tiles) 51.4 -> 44.1 us, 300 x 4096 x 12288 50.1 -> 43.3, 451 x 4096 x 4096 25.0 -> 23.0,
+  // 200 x 6144 x 4096 (24) 26.2 -> 23.0; with fewer tiles, or four pairs to one, the exchange costs more (200 x 4096 x 12288, 16 tiles, 35.6 -> 41.2).
+  int parts = 1;
+  const int k_half = ((K + BK - 1) / BK + 1) / 2;
+  if (plain && M > BM && p.tma_store && vlmt_gemm_pair_enabled() && split_k_enabled() && !one_wave && (p.cluster > 1 || p.k_splits == 1) &&
+      k_half >= 16 && pair_tiles * 37 >= num_sms * 6 && pair_tiles <= vlmt_gemm_pair_clusters()) {
+    parts = 2;
+    p.cluster = p.k_splits = 1;
+    p.kb_per_split = k_half;
+  }
+  if (plain && M > BM && p.tma_store && p.cluster <= 1 && vlmt_gemm_pair_enabled() && (one_wave || parts > 1 || pair_tiles * p.k_splits >= num_sms / 2))
     return vlmt_gemm_pair(A, B, D, bias, M, N, K, lda, ldb, ldd, a_mn_major, b_mn_major, epilogue, accumulate, x.alpha, p.k_splits, p.kb_per_split,
-                          status, stream);
+                          parts, status, stream);
   p.ag_world = 0; p.ag_rank = 0; p.ag_rows = 0; p.ag_epoch = 0;
   p.ag_src = nullptr; p.ag_flags = nullptr; p.ag_counter = nullptr;
   p.wg_world = 0; p.wg_rank = 0; p.wg_epoch = 0; p.wg_shard = 0; p.wg_lo = 0; p.wg_dst = nullptr; p.wg_flags = nullptr; p.wg_counters = nullptr;
