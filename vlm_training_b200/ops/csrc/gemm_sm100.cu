@@ -349,7 +349,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
           if (++stage == STAGES) { stage = 0; phase ^= 1; }
         }
       }
-      if (!AG) pdl_trigger();   // this block's last loads are on their way; AG waits for peers
+      // this block's last loads are on their way; AG waits for peers, and beside grouped products the optimizer's updates want the SMs
+      if (!AG && p.grp_mode == 0) pdl_trigger();
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer

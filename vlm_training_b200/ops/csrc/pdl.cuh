@@ -15,10 +15,11 @@
 
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-// first statement of a kernel that needs nothing set up before
+// First statement of a kernel that needs nothing set up before.  Small grids let the next kernel in at once, they are over in a few
+// microseconds; larger ones when their blocks exit, for the reason above (256 experts, 16384 tokens 6.59 -> 6.68 ms with all of them).
 __device__ __forceinline__ void pdl_begin() {
   pdl_wait();
-  pdl_trigger();
+  if (gridDim.x * gridDim.y * gridDim.z <= 296) pdl_trigger();
 }
 
 template <typename... P, typename... A>
