@@ -6,7 +6,7 @@ host copy of the boundaries (no device read), the scores in query blocks of 1024
 Head size 256 and documents up to ``_DENSE_TIMES x topk`` tokens: the selection becomes one bit per query and causal key, and the
 dense kernels of ``csrc/attention256_sm100.cu`` compute every tile up to the diagonal with the bits as a mask, one launch per pass
 for the whole row (:class:`_MaskedAttention`).  That does more arithmetic than the selection needs, but as full 128-row tiles on the
-tensor cores: 12301 tokens in documents of 1303 to 5015, 16 heads, forward and backward 32.9 -> 3.1 ms.
+tensor cores: 12301 tokens in documents of 1303 to 5015, 16 heads, forward and backward 32.9 -> 2.4 ms.
 
 Longer documents and other head sizes go block by block:
 
@@ -32,7 +32,7 @@ from . import cuda as cu
 _QBLOCK = 1024
 # Forward + backward with 16 heads, the masked dense form costs 0.10 to 0.15 ns per query and CAUSAL key, the gathered form 1.7 to 2.3 ns per
 # query and SELECTED key (topk 512: 4.09 and 8.70 ms at 16 times topk, 14.75 and 19.01 ms at 32 times; topk 2048: 54.6 and 119.7 ms at
-# 16 times): they meet near 40 times topk.  The limit is lower because the mask is one bit per query and causal key, kept for backward, and
+# 16 times): they meet near 40 times topk (figures of 64-row key tiles; on CTA pairs the dense form takes three quarters of that).  The limit is lower because the mask is one bit per query and causal key, kept for backward, and
 # grows with the square of the document, the gathered form's lists with its length (16 times 2048: 134 MB and 268 MB, 40 times: 840 and 671).
 _DENSE_TIMES = 16
 
