@@ -1,0 +1,15 @@
+"""Which form of a kernel a call takes: pure functions of its sizes, no GPU needed."""
+import pytest
+
+
+# 24 to 37 tiles of 256 x 256: CTA pairs share a tile's K only where it would be split in two anyway.  Whole, it is faster in narrow tiles
+# (454 x 4096 x 2048 14.8 us against 18.4, added to D 14.6 against 28.9), and so are four parts of it (381 x 3072 x 3072).
+@pytest.mark.parametrize("M,N,K,parts", [(454, 4096, 2048, 1), (507, 4088, 3072, 1), (251, 8184, 2560, 1), (381, 3072, 3072, 1), (1275, 1280, 2048, 1),
+                                         (451, 4096, 4096, 2), (451, 4096, 12288, 2), (200, 6144, 4096, 2), (300, 4096, 12288, 2), (200, 4096, 12288, 1)])
+@pytest.mark.parametrize("parts_of_d", [False, True])
+def test_pairs_share_the_k_of_a_tile_only_where_it_would_be_split(M, N, K, parts, parts_of_d):
+    from vlm_training_b200.ops import cuda as cu
+
+    bn, cluster, k_splits, pairs, got = cu._C.gemm_form(M, N, K, parts_of_d)
+    assert got == parts and pairs == (parts == 2)
+    assert cu._C.gemm_form(M, N, K, parts_of_d, pair_clusters=0)[4] == 1   # a GPU that cannot hold such clusters

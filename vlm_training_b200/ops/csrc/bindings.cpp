@@ -7,6 +7,7 @@
 
 #include "elementwise.h"
 #include "gdn_scan_sm100.h"
+#include "gemm_pair_sm100.h"
 #include "gemm_sm100.h"
 #include "loss_optim.h"
 #include "torch_ops.h"
@@ -548,6 +549,15 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("gemm_rs_push", &gemm_rs_push);
   m.def("gemm_ag", &gemm_ag);
   m.def("gemm_wgather", &gemm_wgather);
+  // (tile width, blocks of a cluster that share a tile's K, parts of K added to D, CTA pairs, pairs that share a tile's K); the defaults
+  // are a B200's: SMs, clusters of 2, 4 and 8 blocks and of two pairs that it holds at once
+  m.def("gemm_form", [](int M, int N, int K, bool parts_of_d, int sms, std::array<int, 3> capacity, int pair_clusters) {
+    int f[5];
+    vlmt_gemm_form(M, N, K, parts_of_d, sms, capacity.data(), pair_clusters, f);
+    return std::make_tuple(f[0], f[1], f[2], f[3] != 0, f[4]);
+  }, py::arg("M"), py::arg("N"), py::arg("K"), py::arg("parts_of_d") = false, py::arg("sms") = 148,
+        py::arg("capacity") = std::array<int, 3>{74, 33, 14}, py::arg("pair_clusters") = 33);
+  m.def("gemm_pair_clusters", &vlmt_gemm_pair_clusters);
   m.def("gemm_set_flag_wait_ms", [](int64_t ms) {
     int r = vlmt_gemm_set_flag_wait_ms((long)ms);
     TORCH_CHECK(r == 0, "vlmt_gemm_set_flag_wait_ms failed with code ", r);

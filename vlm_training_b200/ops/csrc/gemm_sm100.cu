@@ -832,6 +832,57 @@ SplitPlan plan_gemm(int M, int N, int K, int num_sms, const int* capacity) {
   return best;
 }
 
+// The form of a GEMM: tile width, blocks of a cluster that share a tile's K, parts of K that are added to D one by one, or CTA pairs (256 x 256
+// tiles) and the pairs of a cluster that share a tile's K.  `plain`: no collective, no groups; `pairs_fit`: an output that pairs can write;
+// `parts_of_d`: a product that may be added to D in parts.
+struct GemmForm { int bn, cluster, k_splits, kb_per; bool pairs; int parts; };
+
+GemmForm gemm_form(int M, int N, int K, bool plain, bool pairs_fit, bool parts_of_d, int num_sms, const int* capacity, int pair_clusters) {
+  const int num_kb = (K + BK - 1) / BK;
+  SplitPlan plan{N > 128 ? 256 : 128, 1, num_kb};
+  if (plain && split_k_enabled()) plan = plan_gemm(M, N, K, num_sms, capacity);
+  GemmForm p{plan.bn, plan.splits, plan.splits, plan.kb_per, false, 1};
+  if (plan.splits == 1 && parts_of_d && split_k_enabled()) {
+    // few output tiles and a long K: cut K so that the work items fill whole waves of SMs (at least 1024 of K per part)
+    const long tiles = (long)((M + BM - 1) / BM) * ((N + plan.bn - 1) / plan.bn);
+    auto wave_eff = [&](long items) { return (double)items / (double)(((items + num_sms - 1) / num_sms) * num_sms); };
+    int best = 1;
+    double best_eff = wave_eff(tiles);
+    for (int sp : {2, 3, 4, 6, 8}) {
+      if (num_kb / sp < 16) break;
+      const double e = wave_eff(tiles * sp);
+      if (e > best_eff + 0.04) { best = sp; best_eff = e; }
+    }
+    if (best > 1) {
+      p.kb_per = (num_kb + best - 1) / best;
+      p.k_splits = (num_kb + p.kb_per - 1) / p.kb_per;
+    }
+  }
+  if (!pairs_fit || M <= BM || !vlmt_gemm_pair_enabled()) return p;
+  // large bf16 outputs go to CTA pairs: at least one wave of 256 x 256 tiles, so the coarser tiles leave no SM idle.  With one row of
+  // 128-row tiles half of every pair would have no rows (37 x 24576 x 4096 63.5 us in pairs, 53.3 us without, 1200 x 24576 x 4096 164 and 193).
+  // More than half a wave of them also beats narrower tiles and K split over clusters, which are bound by their loads (128 + 128 rows of
+  // operands for half the product): 451 x 6144 x 4096 (48 tiles) 29.8 -> 25.4 us, 700 x 4096 x 12288 (48) 77 -> 65, 1000 x 4096 x 4608 (64)
+  // 32.0 -> 28.2, 2500 x 1152 x 4304 (50) 31.6 -> 25.6; below that the idle SMs weigh more (451 x 4096 x 12288, 32 tiles, 51 -> 60).
+  const long pair_tiles = (long)((M + 255) / 256) * ((N + 255) / 256);
+  const bool one_wave = (p.cluster > 1 || p.k_splits == 1) && pair_tiles * 2 <= num_sms && pair_tiles * 37 >= num_sms * 10;
+  if (one_wave) {
+    p.cluster = p.k_splits = 1;
+    p.kb_per = num_kb;
+  }
+  // Fewer tiles (24 to 33 on 148 SMs) of a K from 3840, where K would be split in two: two pairs of a cluster share a tile while all clusters fit
+  // the GPU at once.  451 x 4096 x 12288 (32 tiles) 51.4 -> 44.1 us, 300 x 4096 x 12288 50.1 -> 43.3, 451 x 4096 x 4096 25.0 -> 23.0, 200 x 6144 x 4096 (24)
+  // 26.2 -> 23.0; with fewer tiles, or four pairs to one, the exchange costs more (200 x 4096 x 12288, 16 tiles, 35.6 -> 41.2), and so it does where
+  // K stays whole (454 x 4096 x 2048 14.8 -> 18.4, added to D 14.6 -> 28.9) or is shorter (381 x 3072 x 3072 0.85, added to D 0.76).
+  if (split_k_enabled() && !one_wave && p.cluster == 2 && num_kb >= 60 && pair_tiles * 37 >= num_sms * 6 && pair_tiles <= pair_clusters) {
+    p.parts = 2;
+    p.cluster = p.k_splits = 1;
+    p.kb_per = (num_kb + 1) / 2;
+  }
+  p.pairs = p.cluster <= 1 && (one_wave || p.parts > 1 || pair_tiles * p.k_splits >= num_sms / 2);
+  return p;
+}
+
 template <int BN, bool A_MN, bool B_MN, bool AG>
 int launch_variant(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& td, const CUtensorMap& ta2, const RsMaps& rsm,
                    const Params& p, int num_sms, cudaStream_t stream) {
@@ -861,9 +912,6 @@ int gemm_launch(const void* A, const void* B, void* D, float* Dacc32, const void
   else r = vlmt_make_tmap_2d_bf16(&ta, A, (uint64_t)M, (uint64_t)K, (uint64_t)lda * 2, 64, 64);
   if (r) return 1000 + r;
   const bool plain = x.grp_mode == 0 && x.rs_world == 0 && x.ag_world == 0 && x.wg_world == 0;
-  SplitPlan plan{N > 128 ? 256 : 128, 1, (K + BK - 1) / BK};
-  if (plain && split_k_enabled()) plan = plan_gemm(M, N, K, num_sms, cluster_capacity());
-  const bool bn256 = plan.bn == 256;
   const uint64_t b_groups = x.grp_mode == 1 ? (uint64_t)x.grp_count : 1;   // grouped forward / dgrad: one B per group, stacked along the rows
   if (!b_mn_major) r = vlmt_make_tmap_2d_bf16(&tb, B, (uint64_t)K, (uint64_t)N * b_groups, (uint64_t)ldb * 2, 64, 128);
   else r = vlmt_make_tmap_2d_bf16(&tb, B, (uint64_t)N, (uint64_t)K * b_groups, (uint64_t)ldb * 2, 64, 64);
@@ -909,50 +957,14 @@ int gemm_launch(const void* A, const void* B, void* D, float* Dacc32, const void
   p.Dacc32 = Dacc32;
   p.alpha = x.alpha;
   p.epilogue = epilogue; p.accumulate = accumulate; p.status = status;
-  p.k_splits = p.cluster = plan.splits; p.kb_per_split = plan.kb_per;
-  if (plan.splits == 1 && accumulate && !x.one_sum && p.tma_store && x.grp_mode == 0 && x.rs_world == 0 && x.ag_world == 0 && bias == nullptr && epilogue == GEMM_EPI_NONE &&
-      Dacc32 == nullptr && split_k_enabled()) {
-    // few output tiles and a long K: cut K so that the work items fill whole waves of SMs (at least 1024 of K per part)
-    const long tiles = (long)((M + BM - 1) / BM) * ((N + (bn256 ? 256 : 128) - 1) / (bn256 ? 256 : 128));
-    const int num_kb = (K + BK - 1) / BK;
-    auto wave_eff = [&](long items) { return (double)items / (double)(((items + num_sms - 1) / num_sms) * num_sms); };
-    int best = 1;
-    double best_eff = wave_eff(tiles);
-    for (int sp : {2, 3, 4, 6, 8}) {
-      if (num_kb / sp < 16) break;
-      const double e = wave_eff(tiles * sp);
-      if (e > best_eff + 0.04) { best = sp; best_eff = e; }
-    }
-    if (best > 1) {
-      p.kb_per_split = (num_kb + best - 1) / best;
-      p.k_splits = (num_kb + p.kb_per_split - 1) / p.kb_per_split;
-    }
-  }
-  // large bf16 outputs go to CTA pairs: at least one wave of 256 x 256 tiles, so the coarser tiles leave no SM idle.  With one row of
-  // 128-row tiles half of every pair would have no rows (37 x 24576 x 4096 63.5 us in pairs, 53.3 us without, 1200 x 24576 x 4096 164 and 193).
-  // More than half a wave of them also beats narrower tiles and K split over clusters, which are bound by their loads (128 + 128 rows of
-  // operands for half the product): 451 x 6144 x 4096 (48 tiles) 29.8 -> 25.4 us, 700 x 4096 x 12288 (48) 77 -> 65, 1000 x 4096 x 4608 (64)
-  // 32.0 -> 28.2, 2500 x 1152 x 4304 (50) 31.6 -> 25.6; below that the idle SMs weigh more (451 x 4096 x 12288, 32 tiles, 51 -> 60).
-  const long pair_tiles = (long)((M + 255) / 256) * ((N + 255) / 256);
-  const bool one_wave = (p.cluster > 1 || p.k_splits == 1) && pair_tiles * 2 <= num_sms && pair_tiles * 37 >= num_sms * 10;
-  if (plain && M > BM && p.tma_store && vlmt_gemm_pair_enabled() && one_wave) {
-    p.cluster = p.k_splits = 1;
-    p.kb_per_split = (K + BK - 1) / BK;
-  }
-  // Fewer tiles of a long K (16 blocks of 64 and more for each part): two pairs of a cluster share a tile while all clusters fit the GPU at
-  // once and keep two thirds of it busy.  451 x 4096 x 12288 (32 tiles) 51.4 -> 44.1 us, 300 x 4096 x 12288 50.1 -> 43.3, 451 x 4096 x 4096 25.0 -> 23.0,
-  // 200 x 6144 x 4096 (24) 26.2 -> 23.0; with fewer tiles, or four pairs to one, the exchange costs more (200 x 4096 x 12288, 16 tiles, 35.6 -> 41.2).
-  int parts = 1;
-  const int k_half = ((K + BK - 1) / BK + 1) / 2;
-  if (plain && M > BM && p.tma_store && vlmt_gemm_pair_enabled() && split_k_enabled() && !one_wave && (p.cluster > 1 || p.k_splits == 1) &&
-      k_half >= 16 && pair_tiles * 37 >= num_sms * 6 && pair_tiles <= vlmt_gemm_pair_clusters()) {
-    parts = 2;
-    p.cluster = p.k_splits = 1;
-    p.kb_per_split = k_half;
-  }
-  if (plain && M > BM && p.tma_store && p.cluster <= 1 && vlmt_gemm_pair_enabled() && (one_wave || parts > 1 || pair_tiles * p.k_splits >= num_sms / 2))
+  const bool parts_of_d = accumulate && !x.one_sum && p.tma_store && x.grp_mode == 0 && x.rs_world == 0 && x.ag_world == 0 && bias == nullptr &&
+                          epilogue == GEMM_EPI_NONE && Dacc32 == nullptr;
+  const GemmForm form = gemm_form(M, N, K, plain, plain && p.tma_store, parts_of_d, num_sms, cluster_capacity(), vlmt_gemm_pair_clusters());
+  const bool bn256 = form.bn == 256;
+  p.cluster = form.cluster; p.k_splits = form.k_splits; p.kb_per_split = form.kb_per;
+  if (form.pairs)
     return vlmt_gemm_pair(A, B, D, bias, M, N, K, lda, ldb, ldd, a_mn_major, b_mn_major, epilogue, accumulate, x.alpha, p.k_splits, p.kb_per_split,
-                          parts, status, stream);
+                          form.parts, status, stream);
   p.ag_world = 0; p.ag_rank = 0; p.ag_rows = 0; p.ag_epoch = 0;
   p.ag_src = nullptr; p.ag_flags = nullptr; p.ag_counter = nullptr;
   p.wg_world = 0; p.wg_rank = 0; p.wg_epoch = 0; p.wg_shard = 0; p.wg_lo = 0; p.wg_dst = nullptr; p.wg_flags = nullptr; p.wg_counters = nullptr;
@@ -1052,6 +1064,12 @@ extern "C" int vlmt_gemm_bf16_ag(const void* src, void* A_full, const void* B, v
   x.ag_src = src; x.ag_dst = gathered; x.ag_flag_dst = flag_dst; x.ag_flags = flags; x.ag_counter = counter;
   return gemm_launch(A_full, B, D, nullptr, nullptr, world * rows, N, K, K, ldb, ldd, 0, b_mn_major, GEMM_EPI_NONE, 0, x, status, num_sms,
                      stream);
+}
+
+extern "C" void vlmt_gemm_form(int M, int N, int K, int parts_of_d, int num_sms, const int* capacity, int pair_clusters, int* out) {
+  const int cap[9] = {0, 0, capacity[0], 0, capacity[1], 0, 0, 0, capacity[2]};
+  const GemmForm f = gemm_form(M, N, K, true, true, parts_of_d != 0, num_sms, cap, pair_clusters);
+  out[0] = f.bn; out[1] = f.cluster; out[2] = f.k_splits; out[3] = f.pairs; out[4] = f.parts;
 }
 
 extern "C" int vlmt_gemm_set_flag_wait_ms(long ms) {

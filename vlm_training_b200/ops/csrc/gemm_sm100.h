@@ -42,6 +42,9 @@ int vlmt_gemm_bf16_wgather(const void* X, void* D, const void* bias, int M, int 
 int vlmt_gemm_bf16_ag(const void* src, void* A_full, const void* B, void* D, void* const* gathered, void* const* flag_dst,
                       const int* flags, unsigned* counter, int epoch, int world, int rank, int rows, int N, int K, int ldb, int ldd,
                       int b_mn_major, int* status, int num_sms, cudaStream_t stream);
+// The form of a plain bf16 GEMM: out = tile width, blocks of a cluster that share a tile's K, parts of K added to D, CTA pairs or not, pairs that
+// share a tile's K.  capacity: clusters of 2, 4 and 8 blocks, pair_clusters: clusters of two pairs that the GPU holds at once.
+void vlmt_gemm_form(int M, int N, int K, int parts_of_d, int num_sms, const int* capacity, int pair_clusters, int* out);
 // bound of the in-GEMM wait for a peer's flag on the current device, in milliseconds (default 20 000)
 int vlmt_gemm_set_flag_wait_ms(long ms);
 // 2-D bf16 tensor map with 128-byte swizzle; `out_map` points at 128 bytes (CUtensorMap).
