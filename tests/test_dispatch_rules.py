@@ -13,3 +13,13 @@ def test_pairs_share_the_k_of_a_tile_only_where_it_would_be_split(M, N, K, parts
     bn, cluster, k_splits, pairs, got = cu._C.gemm_form(M, N, K, parts_of_d)
     assert got == parts and pairs == (parts == 2)
     assert cu._C.gemm_form(M, N, K, parts_of_d, pair_clusters=0)[4] == 1   # a GPU that cannot hold such clusters
+
+
+# Up to half as many 256 x 256 tiles as SMs: pairs where 128 x 128 tiles do not fit one wave and K is not tiny, and where those would be split in two
+@pytest.mark.parametrize("M,N,K,pairs", [(1961, 1152, 3456, False), (1661, 1408, 1152, False), (893, 2432, 12288, False), (381, 6144, 8192, False),
+                                         (1019, 4088, 256, False), (2043, 2040, 72, False), (451, 6144, 4096, True), (700, 4096, 12288, True),
+                                         (2500, 1152, 4304, True), (1000, 4096, 512, True), (381, 6144, 4304, True)])
+def test_a_wave_of_pairs_only_where_it_is_the_faster_one(M, N, K, pairs):
+    from vlm_training_b200.ops import cuda as cu
+
+    assert cu._C.gemm_form(M, N, K)[3] == pairs

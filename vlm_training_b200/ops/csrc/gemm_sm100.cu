@@ -861,11 +861,14 @@ GemmForm gemm_form(int M, int N, int K, bool plain, bool pairs_fit, bool parts_o
   if (!pairs_fit || M <= BM || !vlmt_gemm_pair_enabled()) return p;
   // large bf16 outputs go to CTA pairs: at least one wave of 256 x 256 tiles, so the coarser tiles leave no SM idle.  With one row of
   // 128-row tiles half of every pair would have no rows (37 x 24576 x 4096 63.5 us in pairs, 53.3 us without, 1200 x 24576 x 4096 164 and 193).
-  // More than half a wave of them also beats narrower tiles and K split over clusters, which are bound by their loads (128 + 128 rows of
-  // operands for half the product): 451 x 6144 x 4096 (48 tiles) 29.8 -> 25.4 us, 700 x 4096 x 12288 (48) 77 -> 65, 1000 x 4096 x 4608 (64)
-  // 32.0 -> 28.2, 2500 x 1152 x 4304 (50) 31.6 -> 25.6; below that the idle SMs weigh more (451 x 4096 x 12288, 32 tiles, 51 -> 60).
-  const long pair_tiles = (long)((M + 255) / 256) * ((N + 255) / 256);
-  const bool one_wave = (p.cluster > 1 || p.k_splits == 1) && pair_tiles * 2 <= num_sms && pair_tiles * 37 >= num_sms * 10;
+  // One wave of pairs or less also beats narrower tiles and K split over clusters, which are bound by their loads (128 + 128 rows of
+  // operands for half the product), where 128 x 128 tiles no longer fit one wave: 451 x 6144 x 4096 29.8 -> 25.4 us, 700 x 4096 x 12288 77 -> 65,
+  // 1000 x 4096 x 4608 32.0 -> 28.2, 2500 x 1152 x 4304 31.6 -> 25.6, from 152 such tiles on 1.02 to 1.28 times for K from 512 (at 256 0.96); up to 147
+  // they are the faster ones (1661 x 1408 x 1152, 143 tiles, 0.87).  Where those would be split in two, pairs win from 40 tiles and up to a K of
+  // 4608 (381 x 6144 x 4304, 48 tiles, 29.8 -> 27.7; x 8192 42.1 -> 46.2).
+  const long pair_tiles = (long)((M + 255) / 256) * ((N + 255) / 256), narrow_tiles = (long)((M + 127) / 128) * ((N + 127) / 128);
+  const bool one_wave = (p.cluster > 1 || p.k_splits == 1) && pair_tiles * 2 <= num_sms &&
+                        (narrow_tiles > num_sms ? num_kb >= 8 : p.cluster == 2 && pair_tiles * 37 >= num_sms * 10 && num_kb <= 72);
   if (one_wave) {
     p.cluster = p.k_splits = 1;
     p.kb_per = num_kb;
