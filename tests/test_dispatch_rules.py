@@ -23,3 +23,24 @@ def test_a_wave_of_pairs_only_where_it_is_the_faster_one(M, N, K, pairs):
     from vlm_training_b200.ops import cuda as cu
 
     assert cu._C.gemm_form(M, N, K)[3] == pairs
+
+
+# Heads of 256: rows of short documents on single blocks, whose blocks all have keys; long ones, and all with a selection, on pairs
+@pytest.mark.parametrize("lens,Hq,Hkv,forward,backward", [([64], 16, 4, False, False), ([128] * 64, 16, 4, False, False), ([64] * 32, 16, 2, False, False),
+                                                          ([128] * 64, 4, 4, False, False), ([150] * 4, 16, 2, False, False), ([900], 16, 2, True, True),
+                                                          ([8192], 16, 4, True, True), ([700] * 11, 16, 4, True, True), ([16384], 4, 4, True, True)])
+def test_heads_of_256_take_pairs_where_documents_are_long(lens, Hq, Hkv, forward, backward):
+    from vlm_training_b200.ops import cuda as cu
+
+    row = sum(lens), len(lens), max(lens), Hq, Hkv, True
+    assert cu._C.attn256_plan(*row, False)[:2] == (forward, backward)
+    assert cu._C.attn256_plan(*row, True)[:2] == (True, True)
+
+
+# The parts of a key tile's query heads: as many as fill the GPU and no more; they divide the group
+@pytest.mark.parametrize("lens,Hq,Hkv,parts", [([900], 16, 2, 4), ([900], 6, 2, 1), ([300], 12, 2, 2), ([128] * 64, 16, 2, 1), ([64] * 32, 16, 4, 1),
+                                               ([8192], 16, 4, 1), ([16384], 16, 2, 1), ([1500], 16, 4, 4)])
+def test_parts_of_a_key_tile_of_256_wide_heads(lens, Hq, Hkv, parts):
+    from vlm_training_b200.ops import cuda as cu
+
+    assert cu._C.attn256_plan(sum(lens), len(lens), max(lens), Hq, Hkv, True, False)[2] == parts

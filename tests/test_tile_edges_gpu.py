@@ -348,6 +348,27 @@ def test_attention_256_shared_key_tiles(lens, Hq, Hkv, causal):
     for a, b, n in ((q, qr, "dq"), (k, kr, "dk"), (v, vr, "dv")):   # sums over up to Hq / Hkv heads of bf16 products
         _close(a.grad, b.grad, 0.05 * max(1.0, (Hq / Hkv) ** 0.5 / 2), 3e-2, n)
 
+
+# heads of 256 on single blocks (rows of short documents): a key to a tile and a bit, key tiles shared by 4 blocks and by none, an odd group, no
+# causal mask, more documents than a warp has lanes and twice that
+@pytest.mark.parametrize("lens,Hq,Hkv,causal", [([1, 63, 64, 65, 127, 128, 129], 16, 2, True), ([65, 129], 8, 2, False), ([40] * 40, 4, 4, True),
+                                                ([3] * 70, 5, 1, False), ([128] * 33, 2, 1, True), ([100], 8, 1, True)])
+def test_attention_256_short_documents(lens, Hq, Hkv, causal):
+    from vlm_training_b200.ops import cuda as cu
+
+    assert cu._C.attn256_plan(sum(lens), len(lens), max(lens), Hq, Hkv, causal, False)[:2] == (False, False)
+    test_attention_256_shared_key_tiles(lens, Hq, Hkv, causal)
+
+
+# a block looks for its document 32 at a time: on pairs too, with documents that have no rows
+@pytest.mark.parametrize("lens,Hq,Hkv", [([200 + 40 * i for i in range(34)], 2, 1), ([50, 0, 90, 0, 0, 700], 4, 2), ([0, 0, 0, 1500], 2, 2)])
+def test_attention_256_pairs_find_their_document(lens, Hq, Hkv):
+    from vlm_training_b200.ops import cuda as cu
+
+    assert all(cu._C.attn256_plan(sum(lens), len(lens), max(lens), Hq, Hkv, True, False)[:2])
+    test_attention_256_shared_key_tiles(lens, Hq, Hkv, True)
+
+
 # heads of 256 on CTA pairs: key tiles shared by 4 pairs and by none; an odd number of heads per key head, whose pairs take neighbouring
 # query tiles, with the second one missing, of one row, and full
 @pytest.mark.parametrize("lens,Hq,Hkv,causal", [([1300], 8, 2, True), ([2600], 20, 10, True), ([127, 257, 256], 5, 1, True), ([129, 128], 3, 3, False)])

@@ -6,7 +6,8 @@
 // loads 128 of them, all rows), so a tile that both kinds of product need comes in twice, by halves.
 // A single block has room for streamed tiles of 64 rows only, whose score products (N = 64) keep the tensor core busy for 70 cycles
 // and use 32 of them.  Against that form, us: 8192 tokens in one document, 16 / 4 heads, forward 540 -> 378, dV 641 -> 368, dK 982 -> 660,
-// dQ 827 -> 580; 12301 tokens in 4 documents with 2048 keys kept, 16 / 2 heads, 445 -> 344, 650 -> 366, 863 -> 617, 653 -> 482.  The
+// dQ 827 -> 580; 12301 tokens in 4 documents with 2048 keys kept, 16 / 2 heads, 445 -> 344, 650 -> 366, 863 -> 617, 653 -> 482.  Rows of
+// short documents leave half of a pair without work and stay in that form (attention256_single_sm100.cu; plan_backward below).  The
 // forward step takes 2410 cycles of which the tensor core needs 2048, the dQ step 4140 of 3072 (it waits for the first half of dS).
 //
 //   forward   block = (128 queries, query head).  S(j) = Q K_j^T, online softmax with lazy rescale of the [128 x 256] fp32 output
@@ -26,61 +27,14 @@
 // Roles per block: warp 0 issues TMA loads (both blocks' loads of a tile complete on the barrier of the even one, the leader), one
 // thread of the leader's warp 1 issues every MMA, the compute warps own the rows of their block.  Every wait is bounded
 // (sm100::mbar_wait).  No atomics: results are bit-reproducible.
-#include "attention_sm100.h"
-#include "sm100.cuh"
-
-#include "pdl.cuh"
-#include <cuda_bf16.h>
-#include <math.h>
+#include "attention256.cuh"
 
 namespace {
-using namespace sm100;
+using namespace attn256;
 
-constexpr int HD = 256;            // head size
-constexpr int BR = 128;            // rows of a block's stationary tile
 constexpr int BC = 128;            // rows of a streamed tile
-constexpr float kLog2e = 1.4426950408889634f;
-constexpr float kLn2 = 0.6931471805599453f;
-constexpr float kRescaleThreshold = 8.f;
-constexpr int kBigTile = BR * HD * 2;          // 65536: a stationary tile, 4 blocks of [128 rows x 64 channels]
 constexpr int kHalfTile = BC * HD;             // 32768: half a streamed tile, by rows (4 blocks of [64 rows x 64 channels]) or by channels (2 of [128 x 64])
-constexpr int kBigBlock = BR * 128, kRowBlock = BC / 2 * 128, kChanBlock = BC * 128;   // bytes of one 64-channel block
-
-struct TileInfo {
-  int doc_start, doc_len, q0;
-  bool valid;
-};
-// Tiles of a document, the longest-running first: under the causal mask its last queries, its first keys.  Grids run over (tile, head)
-// with the heads fastest, so the short blocks of all heads are left for the end.
-template <bool KEYS = false>
-__device__ __forceinline__ TileInfo find_tile(const int* __restrict__ cu, int n_docs, int tile, int block_rows) {
-  TileInfo ti;
-  ti.valid = false;
-  ti.doc_start = ti.doc_len = ti.q0 = 0;
-  int acc = 0;
-  for (int d = 0; d < n_docs; ++d) {
-    const int s = cu[d], e = cu[d + 1];
-    const int nb = (e - s + block_rows - 1) / block_rows;
-    if (tile < acc + nb) {
-      ti.doc_start = s;
-      ti.doc_len = e - s;
-      ti.q0 = (KEYS ? tile - acc : nb - 1 - (tile - acc)) * block_rows;
-      ti.valid = true;
-      return ti;
-    }
-    acc += nb;
-  }
-  return ti;
-}
-
-template <int kSlack>
-__device__ __forceinline__ uint8_t* align_smem(uint8_t* raw) {
-  uint8_t* a = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(raw) + 1023) & ~uintptr_t(1023));
-  return (a - raw) <= kSlack ? a : nullptr;
-}
-
-// k-step kk (16 channels) of a K-major [rows x 256] tile stored as 64-channel blocks of `block_bytes`
-__device__ __forceinline__ uint32_t kmajor_off(int kk, int block_bytes) { return (kk >> 2) * block_bytes + (kk & 3) * 32; }
+constexpr int kRowBlock = BC / 2 * 128, kChanBlock = BC * 128;   // bytes of one 64-channel block
 
 // D[256 x 128] = A[256 x 256] (K-major, both blocks' stationary tiles) x B[128 x 256]^T (K-major, a streamed tile by rows): 16 MMAs
 __device__ __forceinline__ void issue_scores(uint32_t dst, SmemDesc a_big, SmemDesc b_rows) {
@@ -101,21 +55,6 @@ __device__ __forceinline__ void issue_accumulate(uint32_t dst, uint32_t a_lo, ui
     if (kk == 0) umma_ts_pair<2>(dst, a, b, idesc, acc); else umma_ts_pair<1>(dst, a, b, idesc);
   }
 }
-
-struct Params {
-  __nv_bfloat16 *O, *dQ, *dK, *dV;
-  float* LSE;            // [Hq, T], natural log (written by forward, read by backward)
-  const float* delta;    // [Hq, T]
-  const int* cu;
-  int n_docs, T, Hq, Hkv;
-  float scale, scale_log2;
-  int causal;
-  int* status;
-  const uint2* sel;      // SEL: [key tiles of 64][T] 64-bit words, word [kt][t] = keys 64 kt .. 64 kt + 63 of t's document kept by query t
-  int sel_topk;          // SEL: documents up to this length keep every causal key and have no words
-  int pair_heads;        // forward, dQ: the blocks of a pair are two query heads of one kv head; else two neighbouring query tiles
-  int parts;             // dK / dV: pairs (a cluster) that share two key tiles, each with an equal part of the group's query heads
-};
 
 // The pair of a forward or dQ block: its query tile, its query head, and the steps that both blocks take.
 struct QueryTile { TileInfo ti; int hq, steps; };
@@ -178,19 +117,6 @@ __device__ __forceinline__ void teardown(volatile int* abort_flag, int warp, uin
   if (warp == 1) {
     tc_fence_after();
     tmem_dealloc_pair<512>(tmem_base);
-  }
-}
-
-// 32 accumulator columns of a row, times f, as bf16
-__device__ __forceinline__ void store_row32(__nv_bfloat16* dst, const uint32_t (&o)[32], float f) {
-#pragma unroll
-  for (int u = 0; u < 4; ++u) {
-    uint4 pk;
-    pk.x = pack_bf16x2(__uint_as_float(o[u * 8 + 0]) * f, __uint_as_float(o[u * 8 + 1]) * f);
-    pk.y = pack_bf16x2(__uint_as_float(o[u * 8 + 2]) * f, __uint_as_float(o[u * 8 + 3]) * f);
-    pk.z = pack_bf16x2(__uint_as_float(o[u * 8 + 4]) * f, __uint_as_float(o[u * 8 + 5]) * f);
-    pk.w = pack_bf16x2(__uint_as_float(o[u * 8 + 6]) * f, __uint_as_float(o[u * 8 + 7]) * f);
-    *reinterpret_cast<uint4*>(dst + u * 8) = pk;
   }
 }
 
@@ -422,7 +348,6 @@ struct BwdSmem {
 };
 static_assert(BwdSmem::kTotal <= 232448, "shared memory");
 
-constexpr int kPartPitch = HD + 4;   // floats per row of a block's part of dK / dV in shared memory (conflict-free 16-byte stores)
 static_assert(BR * kPartPitch * 4 <= BwdSmem::offStat, "a part lies over the tiles");
 
 constexpr int kBwdThreads = 320;   // TMA, MMA, 8 compute warps: half of a row's 128 columns per thread
@@ -931,43 +856,111 @@ __global__ void attn256_delta_kernel(const __nv_bfloat16* __restrict__ dO, const
   if (lane == 0) delta[(size_t)h * T + t] = acc;
 }
 
-int make_map(CUtensorMap* m, const void* base, int T, int cols, long ld, int box_rows) {
-  return vlmt_make_tmap_2d_bf16(m, base, (uint64_t)cols, (uint64_t)T, (uint64_t)ld * 2, 64, (uint32_t)box_rows);
-}
-template <typename K, typename... A>
-int launch(K kern, unsigned clusters, int cluster, int threads, int smem, cudaStream_t st, A&&... args) {
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-  if (e != cudaSuccess) return (int)e;
-  return launch_pdl(kern, dim3(clusters * cluster), dim3(threads), (size_t)smem, st, cluster, args...);
-}
 // clusters of a forward or dQ launch: query tiles (an upper bound) times heads
 unsigned query_pairs(const Params& p) {
   return p.pair_heads ? (unsigned)(p.T / BR + p.n_docs + 1) * (p.Hq / 2) : (unsigned)(p.T / (2 * BR) + p.n_docs + 1) * p.Hq;
 }
+
+// Which form a row takes, and into how many parts the query heads of a key tile are split, below an average of 1280 tokens per document: the
+// cheapest by a rough time in us of its launches, from what the host knows of the row.  A pair that holds 256 keys, or two query tiles, idles
+// beside a short document, and a block pays for its set-up whatever it then does.  Fitted to 236 rows of 64 to 16384 tokens in 1 to 256 documents,
+// 16 / 4, 16 / 2, 6 / 2 and 4 / 4 heads: on average within 1 % of the best form, forward and backward.  us, pairs with one rule for all rows -> this
+// choice: 8192 tokens in 64 documents, 16 / 4 heads, forward 84 -> 70, backward 256 -> 198; 16 / 2 heads, backward 275 -> 180; 4 / 4 heads
+// 37 -> 17 and 134 -> 71; 64 in one, 16 / 2 heads, 8.1 -> 5.6 and 43 -> 29; 900 in one, backward 162 -> 105.
+struct Row {
+  int T, n_docs, longest, causal, sms;
+  double tiles(int rows) const { return n_docs * fmax(1.0, (double)T / n_docs / rows + 0.5); }   // of all documents
+  // items of `fixed` + `per_step` x their steps over `slots`: tiles of `rows` rows against tiles of `cols`, `heads` of them in each step
+  double us(double items, double slots, int rows, int cols, double heads, double fixed, double per_step) const {
+    const double n = fmax(1.0, (double)T / n_docs / cols + 0.5), across = (double)rows / cols, waves = items / slots;
+    const double mean = fixed + per_step * heads * (causal && n > across ? fmax(1.0, 0.5 * (n + across)) : n);
+    return fmax(fixed + per_step * heads * ((longest + cols - 1) / cols), waves > 1.0 ? mean * (waves > 3.0 ? waves : ceil(waves)) : 0.0);
+  }
+};
+Row row_of(int T, int n_docs, int longest, int causal) {
+  const int mean = (T + n_docs - 1) / n_docs;
+  Row r{T, n_docs, longest < mean ? mean : longest < T ? longest : T, causal, 148};
+  int dev = 0;
+  if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&r.sms, cudaDevAttrMultiProcessorCount, dev);
+  return r;
+}
+bool long_documents(const Row& r) { return r.T >= 1280l * r.n_docs; }
+// forward or dQ on pairs / on single blocks
+double query_us(const Row& r, int Hq, int Hkv, bool pairs, double fixed, double per_step) {
+  if (!pairs) return r.us(r.tiles(BR) * Hq, r.sms, BR, BC / 2, 1, fixed, per_step);
+  const int rows = Hq / Hkv % 2 == 0 ? BR : 2 * BR;
+  return r.us(r.tiles(rows) * (rows == BR ? Hq / 2 : Hq), r.sms / 2, rows, BC, 1, fixed, per_step);
+}
+bool forward_on_pairs(const Row& r, int Hq, int Hkv, bool selected) {
+  return selected || long_documents(r) || query_us(r, Hq, Hkv, true, 8.8, 1.4) <= query_us(r, Hq, Hkv, false, 6.2, 1.15);
+}
+struct BackwardPlan { bool pairs; int parts; };
+BackwardPlan plan_backward(const Row& r, int Hq, int Hkv, bool selected) {
+  const int group = Hq / Hkv;
+  BackwardPlan best{true, 1};
+  if (selected || long_documents(r)) {
+    // Pairs of key tiles times key heads are few and of very different length (a key tile meets every later query of its document, with
+    // every query head of its group): the heads of a group are split over a cluster of up to 4 pairs until about 1.5 pairs per pair of SMs
+    // are there, over 4 only where documents are long enough to leave a pair some steps.  dV + dK with 1 / 2 / 4 parts, us: 16384 tokens in 5
+    // documents, 16 / 4 heads 1713 / 1811 / 1811; 8192 in 1 1028 / 1093 / 1268; 1500 in 1 214 / 114 / 90; sparse, 16 / 2 heads, 12301 in 4
+    // 1328 / 982 / 1015; 3000 in 1 741 / 403 / 224.
+    const int max_parts = long_documents(r) ? 4 : 2;
+    while (best.parts < max_parts && group % (2 * best.parts) == 0 && 4l * (r.T / (2 * BR) + 1) * Hkv * best.parts < 3l * r.sms) best.parts *= 2;
+    return best;
+  }
+  double best_us = 1e30;
+  for (int single = 0; single < 2; ++single) {
+    const int rows = single ? BR : 2 * BR;
+    const double dq = single ? query_us(r, Hq, Hkv, false, 8.8, 2.8) : query_us(r, Hq, Hkv, true, 14.0, 2.1);
+    for (int p = 1; p <= 4 && group % p == 0; p *= 2) {
+      // blocks or clusters that the GPU holds at once: clusters of 4 and 8 blocks do not take all of its SMs
+      const double slots = r.sms / 148.0 * (single ? (p == 1 ? 148 : p == 2 ? 74 : 36) : (p == 1 ? 74 : p == 2 ? 42 : 13));
+      const double us = dq + r.us(r.tiles(rows) * Hkv, slots, rows, single ? BC / 2 : BC, (double)group / p,
+                                  (single ? 8.2 : 12.2) + (p > 1 ? 7.7 : 0.0), single ? 2.9 : 3.8);
+      if (us < 0.97 * best_us) { best_us = us; best = {!single, p}; }
+    }
+  }
+  return best;
+}
 }  // namespace
 
+extern "C" void vlmt_attn256_plan(int T, int n_docs, int longest, int Hq, int Hkv, int causal, int selected, int* out) {
+  const Row row = row_of(T, n_docs, longest, causal);
+  const BackwardPlan plan = plan_backward(row, Hq, Hkv, selected != 0);
+  out[0] = forward_on_pairs(row, Hq, Hkv, selected != 0); out[1] = plan.pairs; out[2] = plan.parts;
+}
+
 extern "C" int vlmt_attn256_fwd(const void* q, const void* k, const void* v, void* o, float* lse, const int* cu, int n_docs, int T, int Hq,
-                                int Hkv, long ldq, long ldk, long ldv, float scale, int causal, const void* sel, int sel_topk, int* status,
-                                cudaStream_t st) {
+                                int Hkv, long ldq, long ldk, long ldv, float scale, int causal, int longest, const void* sel, int sel_topk,
+                                int* status, cudaStream_t st) {
   if (T <= 0 || n_docs <= 0) return 0;
+  Params p{};
+  p.O = reinterpret_cast<__nv_bfloat16*>(o); p.LSE = lse; p.cu = cu; p.n_docs = n_docs; p.T = T; p.Hq = Hq; p.Hkv = Hkv;
+  p.scale = scale; p.scale_log2 = scale * kLog2e; p.causal = causal; p.status = status;
+  p.sel = reinterpret_cast<const uint2*>(sel); p.sel_topk = sel_topk; p.pair_heads = Hq / Hkv % 2 == 0;
+  if (!forward_on_pairs(row_of(T, n_docs, longest, causal), Hq, Hkv, sel != nullptr)) return single_fwd(q, k, v, ldq, ldk, ldv, p, st);
   CUtensorMap tq, tk, tv;
   int r;
   if ((r = make_map(&tq, q, T, Hq * HD, ldq, BR))) return 1000 + r;
   if ((r = make_map(&tk, k, T, Hkv * HD, ldk, BC / 2))) return 2000 + r;
   if ((r = make_map(&tv, v, T, Hkv * HD, ldv, BC))) return 3000 + r;
-  Params p{};
-  p.O = reinterpret_cast<__nv_bfloat16*>(o); p.LSE = lse; p.cu = cu; p.n_docs = n_docs; p.T = T; p.Hq = Hq; p.Hkv = Hkv;
-  p.scale = scale; p.scale_log2 = scale * kLog2e; p.causal = causal; p.status = status;
-  p.sel = reinterpret_cast<const uint2*>(sel); p.sel_topk = sel_topk; p.pair_heads = Hq / Hkv % 2 == 0;
   return launch(sel ? attn256_fwd_kernel<true> : attn256_fwd_kernel<false>, query_pairs(p), 2, kFwdThreads, FwdSmem::kTotal, st, tq, tk, tv, p);
 }
 
 extern "C" int vlmt_attn256_bwd(const void* dout, const void* q, const void* k, const void* v, const void* o, const float* lse, float* delta,
                                 void* dq, void* dk, void* dv, const int* cu, int n_docs, int T, int Hq, int Hkv, float scale, int causal,
-                                const void* sel, int sel_topk, int* status, cudaStream_t st) {
+                                int longest, const void* sel, int sel_topk, int* status, cudaStream_t st) {
   if (T <= 0 || n_docs <= 0) return 0;
   launch_pdl(attn256_delta_kernel, dim3((T * Hq * 32 + 255) / 256), dim3(256), 0, st, 1, reinterpret_cast<const __nv_bfloat16*>(dout),
                                                                   reinterpret_cast<const __nv_bfloat16*>(o), delta, T, Hq);
+  Params p{};
+  p.dQ = reinterpret_cast<__nv_bfloat16*>(dq); p.dK = reinterpret_cast<__nv_bfloat16*>(dk); p.dV = reinterpret_cast<__nv_bfloat16*>(dv);
+  p.LSE = const_cast<float*>(lse); p.delta = delta; p.cu = cu; p.n_docs = n_docs; p.T = T; p.Hq = Hq; p.Hkv = Hkv;
+  p.scale = scale; p.scale_log2 = scale * kLog2e; p.causal = causal; p.status = status;
+  p.sel = reinterpret_cast<const uint2*>(sel); p.sel_topk = sel_topk; p.pair_heads = Hq / Hkv % 2 == 0;
+  const BackwardPlan plan = plan_backward(row_of(T, n_docs, longest, causal), Hq, Hkv, sel != nullptr);
+  p.parts = plan.parts;
+  if (!plan.pairs) return single_bwd(dout, q, k, v, p, st);
   CUtensorMap q128, q64, k128, k64, v128, v64, do128, do64;   // by the rows of a box: stationary tiles and channel halves 128, row halves 64
   int r;
   const long ldq = (long)Hq * HD, ldk = (long)Hkv * HD;
@@ -975,21 +968,6 @@ extern "C" int vlmt_attn256_bwd(const void* dout, const void* q, const void* k, 
   if ((r = make_map(&k128, k, T, Hkv * HD, ldk, BC)) || (r = make_map(&k64, k, T, Hkv * HD, ldk, BC / 2))) return 2000 + r;
   if ((r = make_map(&v128, v, T, Hkv * HD, ldk, BC)) || (r = make_map(&v64, v, T, Hkv * HD, ldk, BC / 2))) return 3000 + r;
   if ((r = make_map(&do128, dout, T, Hq * HD, ldq, BC)) || (r = make_map(&do64, dout, T, Hq * HD, ldq, BC / 2))) return 4000 + r;
-  Params p{};
-  p.dQ = reinterpret_cast<__nv_bfloat16*>(dq); p.dK = reinterpret_cast<__nv_bfloat16*>(dk); p.dV = reinterpret_cast<__nv_bfloat16*>(dv);
-  p.LSE = const_cast<float*>(lse); p.delta = delta; p.cu = cu; p.n_docs = n_docs; p.T = T; p.Hq = Hq; p.Hkv = Hkv;
-  p.scale = scale; p.scale_log2 = scale * kLog2e; p.causal = causal; p.status = status;
-  p.sel = reinterpret_cast<const uint2*>(sel); p.sel_topk = sel_topk; p.pair_heads = Hq / Hkv % 2 == 0;
-  // Pairs of key tiles times key heads are few and of very different length (a key tile meets every later query of its document, with
-  // every query head of its group): the heads of a group are split over a cluster of up to 4 pairs until about 1.5 pairs per pair of SMs
-  // are there, over 4 only where documents are long enough to leave a pair some steps.  dV + dK with 1 / 2 / 4 parts, us: 16384 tokens in 5
-  // documents, 16 / 4 heads 1713 / 1811 / 1811; 8192 in 1 1028 / 1093 / 1268; 5000 in 9 270 / 201 / 278; 3000 in 3 246 / 143 / 174; 1500 in 1
-  // 214 / 114 / 90; sparse, 16 / 2 heads, 12301 in 4 1328 / 982 / 1015; 3000 in 1 741 / 403 / 224.
-  int dev = 0, sms = 148;
-  if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  const int max_parts = T >= 1280l * n_docs ? 4 : 2;
-  p.parts = 1;
-  while (p.parts < max_parts && Hq / Hkv % (2 * p.parts) == 0 && 4l * (T / (2 * BR) + 1) * Hkv * p.parts < 3l * sms) p.parts *= 2;
   const unsigned clusters = (unsigned)(T / (2 * BR) + n_docs + 1) * Hkv;
   if ((r = launch(sel ? attn256_bwd_dkv_kernel<true, true> : attn256_bwd_dkv_kernel<true, false>, clusters, 2 * p.parts, kDkvThreads, DvSmem::kTotal, st,
                   q64, q128, k128, v128, do128, p)))

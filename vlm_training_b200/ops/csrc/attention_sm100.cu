@@ -1012,12 +1012,12 @@ int set_smem(K kern, int bytes) {
 }  // namespace
 
 extern "C" int vlmt_attn_fwd(const void* q, const void* k, const void* v, void* o, float* lse, const int* cu, int n_docs, int T, int Hq,
-                             int Hkv, int d, long ldq, long hsq, long ldk, long hsk, long ldv, long hsv, float scale, int causal, int* status,
-                             cudaStream_t st) {
+                             int Hkv, int d, long ldq, long hsq, long ldk, long hsk, long ldv, long hsv, float scale, int causal, int longest,
+                             int* status, cudaStream_t st) {
   if (T <= 0 || n_docs <= 0) return 0;
   if (d == 256) {
     if (hsq != 256 || hsk != 256 || hsv != 256) return -11;
-    return vlmt_attn256_fwd(q, k, v, o, lse, cu, n_docs, T, Hq, Hkv, ldq, ldk, ldv, scale, causal, nullptr, 0, status, st);
+    return vlmt_attn256_fwd(q, k, v, o, lse, cu, n_docs, T, Hq, Hkv, ldq, ldk, ldv, scale, causal, longest, nullptr, 0, status, st);
   }
   if (d <= 0 || d > 128 || (d & 7)) return -10;
   const int D = d <= 64 ? 64 : 128;   // tile width; TMA zero-fills the channels between d and D
@@ -1044,11 +1044,11 @@ extern "C" int vlmt_attn_fwd(const void* q, const void* k, const void* v, void* 
 
 extern "C" int vlmt_attn_bwd(const void* dout, const void* q, const void* k, const void* v, const void* o, const float* lse, float* delta,
                              void* dq, void* dk, void* dv, const int* cu, int n_docs, int T, int Hq, int Hkv, int d, long ldq, long hsq,
-                             long ldk, long hsk, long ldv, long hsv, float scale, int causal, int* status, cudaStream_t st) {
+                             long ldk, long hsk, long ldv, long hsv, float scale, int causal, int longest, int* status, cudaStream_t st) {
   if (T <= 0 || n_docs <= 0) return 0;
   if (d == 256) {
     if (hsq != 256 || hsk != 256 || hsv != 256 || ldq != (long)Hq * 256 || ldk != (long)Hkv * 256 || ldv != (long)Hkv * 256) return -11;
-    return vlmt_attn256_bwd(dout, q, k, v, o, lse, delta, dq, dk, dv, cu, n_docs, T, Hq, Hkv, scale, causal, nullptr, 0, status, st);
+    return vlmt_attn256_bwd(dout, q, k, v, o, lse, delta, dq, dk, dv, cu, n_docs, T, Hq, Hkv, scale, causal, longest, nullptr, 0, status, st);
   }
   if (d <= 0 || d > 128 || (d & 7)) return -10;
   const int D = d <= 64 ? 64 : 128;

@@ -30,9 +30,8 @@ std::vector<Tensor> vlmt::attn_fwd(const Tensor& q, const Tensor& k, const Tenso
   Tensor st = vlmt_status_tensor();
   int r = vlmt_attn_fwd(q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), lse.data_ptr<float>(), cu.data_ptr<int>(),
                         (int)cu.numel() - 1, T, Hq, Hkv, D, q.stride(0), q.stride(1), k.stride(0), k.stride(1), v.stride(0), v.stride(1),
-                        (float)scale, causal, st.data_ptr<int>(), at::cuda::getCurrentCUDAStream().stream());
+                        (float)scale, causal, (int)max_seqlen, st.data_ptr<int>(), at::cuda::getCurrentCUDAStream().stream());
   TORCH_CHECK(r == 0, "vlmt_attn_fwd failed with code ", r, " (head_dim ", D, ")");
-  (void)max_seqlen;
   return {o, lse};
 }
 
@@ -48,9 +47,8 @@ std::vector<Tensor> vlmt::attn_bwd(const Tensor& dout, const Tensor& q, const Te
   int r = vlmt_attn_bwd(dout.data_ptr(), q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), lse.data_ptr<float>(),
                         delta.data_ptr<float>(), dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), cu.data_ptr<int>(), (int)cu.numel() - 1, T, Hq,
                         Hkv, D, q.stride(0), q.stride(1), k.stride(0), k.stride(1), v.stride(0), v.stride(1), (float)scale, causal,
-                        st.data_ptr<int>(), at::cuda::getCurrentCUDAStream().stream());
+                        (int)max_seqlen, st.data_ptr<int>(), at::cuda::getCurrentCUDAStream().stream());
   TORCH_CHECK(r == 0, "vlmt_attn_bwd failed with code ", r);
-  (void)max_seqlen;
   return {dq, dk, dv};
 }
 
@@ -181,7 +179,7 @@ static std::vector<Tensor> attn_selected_fwd(const Tensor& q, const Tensor& k, c
   const int T = q.size(0), Hq = q.size(1), Hkv = k.size(1);
   Tensor o = torch::empty_like(q), lse = torch::empty({Hq, T}, q.options().dtype(torch::kFloat)), st = vlmt_status_tensor();
   int r = vlmt_attn256_fwd(q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), lse.data_ptr<float>(), cu.data_ptr<int>(), (int)cu.numel() - 1,
-                           T, Hq, Hkv, Hq * 256L, Hkv * 256L, Hkv * 256L, (float)scale, 1, bits.data_ptr(), (int)topk, st.data_ptr<int>(),
+                           T, Hq, Hkv, Hq * 256L, Hkv * 256L, Hkv * 256L, (float)scale, 1, 0, bits.data_ptr(), (int)topk, st.data_ptr<int>(),
                            at::cuda::getCurrentCUDAStream().stream());
   TORCH_CHECK(r == 0, "vlmt_attn256_fwd failed with code ", r);
   return {o, lse};
@@ -195,13 +193,19 @@ static std::vector<Tensor> attn_selected_bwd(const Tensor& dout, const Tensor& q
   Tensor dq = torch::empty_like(q), dk = torch::empty_like(k), dv = torch::empty_like(v);
   Tensor delta = torch::empty({Hq, T}, q.options().dtype(torch::kFloat)), st = vlmt_status_tensor();
   int r = vlmt_attn256_bwd(dout.data_ptr(), q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), lse.data_ptr<float>(), delta.data_ptr<float>(),
-                           dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), cu.data_ptr<int>(), (int)cu.numel() - 1, T, Hq, Hkv, (float)scale, 1,
+                           dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), cu.data_ptr<int>(), (int)cu.numel() - 1, T, Hq, Hkv, (float)scale, 1, 0,
                            bits.data_ptr(), (int)topk, st.data_ptr<int>(), at::cuda::getCurrentCUDAStream().stream());
   TORCH_CHECK(r == 0, "vlmt_attn256_bwd failed with code ", r);
   return {dq, dk, dv};
 }
 
 void bind_attention(pybind11::module_& m) {
+  // (forward on CTA pairs, backward on CTA pairs, parts of a key tile's query heads) for a row of heads of 256
+  m.def("attn256_plan", [](int T, int n_docs, int longest, int Hq, int Hkv, bool causal, bool selected) {
+    int plan[3];
+    vlmt_attn256_plan(T, n_docs, longest, Hq, Hkv, causal, selected, plan);
+    return std::make_tuple(plan[0] != 0, plan[1] != 0, plan[2]);
+  });
   m.def("dsa_select_bits", &dsa_select_bits);
   m.def("attn_selected_fwd", &attn_selected_fwd);
   m.def("attn_selected_bwd", &attn_selected_bwd);
