@@ -44,3 +44,23 @@ def test_parts_of_a_key_tile_of_256_wide_heads(lens, Hq, Hkv, parts):
     from vlm_training_b200.ops import cuda as cu
 
     assert cu._C.attn256_plan(sum(lens), len(lens), max(lens), Hq, Hkv, True, False)[2] == parts
+
+
+def test_tensor_memory_is_allocated_before_the_next_kernel_may_start():
+    """The GEMMs allocate tensor memory before they wait for their predecessor.  A predecessor that let them in before it had its own
+    columns could wait for them for ever, on an SM that they share."""
+    import pathlib
+    import re
+
+    import vlm_training_b200.ops as ops
+
+    allocating = set()
+    for path in sorted((pathlib.Path(ops.__file__).parent / "csrc").glob("*.cu")):
+        src = re.sub(r"__launch_bounds__\([^)]*\)", "", re.sub(r"//[^\n]*", "", path.read_text()))
+        for m in re.finditer(r"__global__[^;{]*?(\w+)\s*\([^{;]*\)\s*\{", src):
+            body = src[m.end():src.index("\n}", m.end())]
+            at = max(body.find(s) for s in ("tmem_alloc", "cta_setup<", "setup_end("))   # the last two: functions that allocate
+            if at >= 0:
+                allocating.add(m.group(1))
+                assert "pdl_begin" not in body and "pdl_trigger" not in body[:at], m.group(1)
+    assert {"gemm_kernel", "gemm_pair_kernel", "gdn_scan_kernel", "gdn_prepare_fwd_kernel", "dsa_index_scores_kernel", "attn256_fwd_kernel"} <= allocating

@@ -36,7 +36,7 @@ struct ScoreParams {
 
 __global__ void __launch_bounds__(128, 1)
 dsa_index_scores_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK, ScoreParams p) {
-  pdl_begin();
+  pdl_wait();
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   constexpr int kQ = 4 * 16384, kK = 16384;         // [128 x 256] and [128 x 64] bf16 tiles
@@ -65,6 +65,7 @@ dsa_index_scores_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
 #pragma unroll
     for (int h = 0; h < HI; ++h) tma_load_2d(smem + h * 16384, &tmQ, bar_tma, h * DI, p.q_tok0 + tq * 128);
     tma_load_2d(smem + kQ, &tmK, bar_tma, 0, p.k_tok0 + tk * 128);
+    pdl_trigger_small();
   }
   bool ok = mbar_wait(bar_tma, 0, abort_flag, p.status, kErrTimeoutFull);
   ok = __syncthreads_and(ok);

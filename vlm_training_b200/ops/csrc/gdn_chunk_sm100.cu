@@ -162,7 +162,7 @@ struct PrepSmem {
 __global__ void __launch_bounds__(THREADS, 2)
 gdn_prepare_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                        const __grid_constant__ CUtensorMap tmV, PrepParams p) {
-  pdl_begin();
+  pdl_wait();
   using L = PrepSmem;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -191,6 +191,7 @@ gdn_prepare_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
       tma_load_2d(smem + L::offQ + b * kBlk, &tmQ, ctl.bar_tma, h * D + 64 * b, tok0);
       tma_load_2d(smem + L::offV + b * kBlk, &tmV, ctl.bar_tma, h * D + 64 * b, tok0);
     }
+    pdl_trigger_small();
   }
   if (cb == 0) {
     sg[r] = valid ? p.g[(size_t)(tok0 + r) * p.H + h] : 0.f;
@@ -367,7 +368,7 @@ struct OutSmem {
 __global__ void __launch_bounds__(THREADS, 2)
 gdn_output_fwd_kernel(const __grid_constant__ CUtensorMap tmQg, const __grid_constant__ CUtensorMap tmP,
                       const __grid_constant__ CUtensorMap tmS, const __grid_constant__ CUtensorMap tmVn, OutParams p) {
-  pdl_begin();
+  pdl_wait();
   using L = OutSmem;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -387,6 +388,7 @@ gdn_output_fwd_kernel(const __grid_constant__ CUtensorMap tmQg, const __grid_con
       tma_load_2d(smem + L::offS + b * kSBlk, &tmS, ctl.bar_tma, 64 * b, tile * 128);
     }
     tma_load_2d(smem + L::offP, &tmP, ctl.bar_tma, 0, tile * 64);
+    pdl_trigger_small();
   }
   bool ok = mbar_wait(ctl.bar_tma, 0, ctl.abort_flag, p.status, kErrTimeoutFull);
   ok = __syncthreads_and(ok);
@@ -439,7 +441,7 @@ __global__ void __launch_bounds__(THREADS, 2)
 gdn_output_bwd_kernel(const __grid_constant__ CUtensorMap tmDo, const __grid_constant__ CUtensorMap tmQg,
                       const __grid_constant__ CUtensorMap tmP, const __grid_constant__ CUtensorMap tmS,
                       const __grid_constant__ CUtensorMap tmVn, OutBwdParams p) {
-  pdl_begin();
+  pdl_wait();
   using L = OutBwdSmem;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -461,6 +463,7 @@ gdn_output_bwd_kernel(const __grid_constant__ CUtensorMap tmDo, const __grid_con
       tma_load_2d(smem + L::offS + b * kSBlk, &tmS, ctl.bar_tma, 64 * b, tile * 128);
     }
     tma_load_2d(smem + L::offP, &tmP, ctl.bar_tma, 0, tile * 64);
+    pdl_trigger_small();
   }
   bool ok = mbar_wait(ctl.bar_tma, 0, ctl.abort_flag, p.status, kErrTimeoutFull);
   ok = __syncthreads_and(ok);
@@ -582,7 +585,7 @@ gdn_prepare_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
                        const __grid_constant__ CUtensorMap tmDu, const __grid_constant__ CUtensorMap tmDqg,
                        const __grid_constant__ CUtensorMap tmDp, const __grid_constant__ CUtensorMap tmPp,
                        const __grid_constant__ CUtensorMap tmTm, PrepBwdParams p) {
-  pdl_begin();
+  pdl_wait();
   using L = PrepBwdSmem;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -622,6 +625,7 @@ gdn_prepare_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
     tma_load_2d(smem + L::offDp, &tmDp, ctl.bar_tma, 0, tile * 64);
     tma_load_2d(smem + L::offPp, &tmPp, ctl.bar_tma, 0, tile * 64);
     tma_load_2d(smem + L::offTm, &tmTm, ctl.bar_tma, 0, tile * 64);
+    pdl_trigger_small();
   }
   if (cb == 0) {
     sb[r] = valid ? p.beta[(size_t)(tok0 + r) * p.H + h] : 0.f;

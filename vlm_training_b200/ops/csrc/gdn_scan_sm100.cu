@@ -57,7 +57,7 @@ template <bool REVERSE>
 __global__ void __launch_bounds__(THREADS, 2)
 gdn_scan_kernel(const __grid_constant__ CUtensorMap tmX1, const __grid_constant__ CUtensorMap tmX2,
                 const __grid_constant__ CUtensorMap tmE, Params p) {
-  pdl_begin();
+  pdl_wait();
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + offBar);
@@ -108,6 +108,7 @@ gdn_scan_kernel(const __grid_constant__ CUtensorMap tmX1, const __grid_constant_
           tma_load_2d(st + 2 * kTile + b * 8192, &tmE, &x_full[s], 64 * b, row);
         }
       }
+      pdl_trigger();   // the last loads are on their way: a few blocks scan for a millisecond where documents are long
     }
   } else if (warp == 1) {
     if (lane == 0) {

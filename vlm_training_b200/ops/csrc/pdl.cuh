@@ -4,6 +4,8 @@
 //     free): the call returns when the kernels before it have completed and their writes are visible, as without the attribute;
 //   * calls it on every path, also in blocks that have nothing to do: a grid that ends without waiting would no longer order what follows
 //     it behind what precedes it.
+//   * if it allocates tensor memory, calls pdl_trigger() behind the allocation: the GEMMs allocate before they wait, and a block of theirs
+//     on the same SM would hold the columns until this kernel ends, which would wait for them without a bound.
 // pdl_trigger() lets the next kernel of the stream be launched into free resources once every block has called it (or exited).  Blocks
 // that are launched ahead hold registers and thread slots while they wait, so long kernels call it near their end: at the start of the
 // GEMMs it kept the optimizer's updates, which run beside them on a stream of their own, off the SMs (256 experts, 8192 tokens 5.14 -> 5.31 ms).
@@ -15,11 +17,14 @@
 
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-// First statement of a kernel that needs nothing set up before.  Small grids let the next kernel in at once, they are over in a few
-// microseconds; larger ones when their blocks exit, for the reason above (256 experts, 16384 tokens 6.59 -> 6.68 ms with all of them).
+// Small grids let the next kernel in at once, larger ones when their blocks exit, for the reason above (256 experts, 16384 tokens 6.59 -> 6.68 ms
+// with all of them).
+__device__ __forceinline__ void pdl_trigger_small() { if (gridDim.x * gridDim.y * gridDim.z <= 296) pdl_trigger(); }
+// First statement of a kernel that needs nothing set up before and no tensor memory, and that is over in tens of microseconds where it has so
+// few blocks.
 __device__ __forceinline__ void pdl_begin() {
   pdl_wait();
-  if (gridDim.x * gridDim.y * gridDim.z <= 296) pdl_trigger();
+  pdl_trigger_small();
 }
 
 template <typename... P, typename... A>
