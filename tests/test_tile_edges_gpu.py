@@ -75,21 +75,34 @@ def test_gemm_cta_pairs(M, N, K, layout):
     cu.check_status()
 
 
-# two CTA pairs of a cluster share a tile and its K: rows and columns off the tile edges, an odd number of K blocks, every layout, added to D
-@pytest.mark.parametrize("M,N,K,layout", [(451, 4104, 4160, "fwd"), (520, 2056, 2056, "dgrad"), (392, 3200, 8200, "wgrad")])
+# two CTA pairs of a cluster share a tile and its K: rows and columns off the tile edges, an odd number of K blocks, every layout, added to D,
+# activations, and a last column off the groups of four
+@pytest.mark.parametrize("M,N,K,layout", [(451, 3592, 4168, "fwd"), (520, 2056, 4104, "dgrad"), (392, 3200, 8200, "wgrad")])
 def test_gemm_cta_pairs_split_over_k(M, N, K, layout):
-    test_gemm_cta_pairs(M, N, K, layout)
     from vlm_training_b200.ops import cuda as cu
 
+    assert cu._C.gemm_form(M, N, K, pair_clusters=cu._C.gemm_pair_clusters())[3:] == (True, 2)
+    test_gemm_cta_pairs(M, N, K, layout)
     a, b = _rand(M, K, scale=0.5), _rand(N, K, scale=0.5)
     assert torch.equal(cu._gemm(a, b), cu._gemm(a, b))   # the parts are summed in rank order
+    bias, n = _rand(N), N - 6
+    pre = (a.float() @ b.float().t() + bias.float()) / 16
+    for epilogue, approximate in ((1, "tanh"), (2, "none")):
+        got = cu._gemm(a, b / 16, bias=bias / 16, epilogue=epilogue)
+        torch.testing.assert_close(got.float(), torch.nn.functional.gelu(pre, approximate=approximate), atol=1e-2, rtol=8e-3)
+    out = torch.full((M, N), 7.0, device=DEV, dtype=torch.bfloat16)
+    cu._gemm(a, b[:n], bias=bias[:n], out=out[:, :n])
+    torch.testing.assert_close(out[:, :n].float(), pre[:, :n] * 16, atol=1e-2, rtol=8e-3)
+    assert bool((out[:, n:] == 7.0).all())   # columns behind the last one are not written
+    cu.check_status()
 
 
-# CTA pairs with between half a wave and one wave of tiles, where K would else be split; raster groups of 16 pairs, the last one short
-@pytest.mark.parametrize("M,N,K", [(300, 6144, 520), (1000, 2600, 72), (4360, 8200, 2056)])
-def test_gemm_cta_pairs_raster_and_single_wave(M, N, K):
+# CTA pairs with up to one wave of tiles, where K would else be split; raster groups of 16 pairs, the last one short
+@pytest.mark.parametrize("M,N,K,pairs", [(300, 6536, 520, True), (1000, 5000, 584, True), (1000, 2600, 72, False), (4360, 8200, 2056, True)])
+def test_gemm_cta_pairs_raster_and_single_wave(M, N, K, pairs):
     from vlm_training_b200.ops import cuda as cu
 
+    assert cu._C.gemm_form(M, N, K)[3] == pairs
     a, b, bias = _rand(M, K, scale=0.5), _rand(N, K, scale=0.5), _rand(N)
     want = a.float() @ b.float().t() + bias.float()
     torch.testing.assert_close(cu._gemm(a, b, bias=bias).float(), want, atol=1e-2, rtol=8e-3)   # one bf16 rounding (2^-8 of the value)
@@ -330,7 +343,7 @@ def test_fp8_amax(rows, cols, pad):
         assert float(cu._C.fp8_quantize(x, 0, True, False)[2][0]) == 7.0
 
 
-# heads of 256: key tiles shared by clusters of 1, 2 and 4 blocks, documents of one key, of one tile and a bit, no causal mask
+# heads of 256: key tiles shared by clusters of 1, 2 and 4 blocks or pairs, documents of one key, of one tile and a bit, no causal mask
 @pytest.mark.parametrize("lens,Hq,Hkv,causal", [([130, 1, 700], 16, 2, True), ([65, 129], 8, 2, False), ([64, 300], 6, 3, True), ([200], 3, 1, True)])
 def test_attention_256_shared_key_tiles(lens, Hq, Hkv, causal):
     from vlm_training_b200.ops import cuda as cu, reference as ref
@@ -369,11 +382,50 @@ def test_attention_256_pairs_find_their_document(lens, Hq, Hkv):
     test_attention_256_shared_key_tiles(lens, Hq, Hkv, True)
 
 
-# heads of 256 on CTA pairs: key tiles shared by 4 pairs and by none; an odd number of heads per key head, whose pairs take neighbouring
-# query tiles, with the second one missing, of one row, and full
-@pytest.mark.parametrize("lens,Hq,Hkv,causal", [([1300], 8, 2, True), ([2600], 20, 10, True), ([127, 257, 256], 5, 1, True), ([129, 128], 3, 3, False)])
-def test_attention_256_pairs(lens, Hq, Hkv, causal):
+# heads of 256 on CTA pairs: key tiles shared by 4 and 2 pairs and by none, groups of 2 and 4 heads; an odd number of heads per key head, whose pairs
+# take neighbouring query tiles, with the second one missing, of one row, and full
+@pytest.mark.parametrize("lens,Hq,Hkv,causal,parts", [([1300], 8, 2, True, 4), ([2600], 20, 10, True, 2), ([2816], 20, 10, True, 1), ([2816], 40, 10, True, 1),
+                                                      ([1152, 1409, 1536], 5, 1, True, 1), ([1409, 1280], 3, 3, False, 1)])
+def test_attention_256_pairs(lens, Hq, Hkv, causal, parts):
+    from vlm_training_b200.ops import cuda as cu
+
+    assert cu._C.attn256_plan(sum(lens), len(lens), max(lens), Hq, Hkv, causal, False) == (True, True, parts)
     test_attention_256_shared_key_tiles(lens, Hq, Hkv, causal)
+
+
+# the running maximum jumps by 17 powers of two in the second 64 keys of a step: in the first step, after several, in the last; without and with a
+# selection, whose bits are fetched once per group of heads, and with the group of heads split over pairs and whole
+@pytest.mark.parametrize("L,Hq,Hkv,topk,parts", [(1500, 4, 2, 0, 2), (1500, 8, 1, 64, 4), (2816, 20, 10, 96, 1)])
+def test_attention_256_maximum_jumps_within_a_step(L, Hq, Hkv, topk, parts):
+    from vlm_training_b200.ops import cuda as cu
+    from vlm_training_b200.ops.dsa_cuda import _MaskedAttention
+
+    assert cu._C.attn256_plan(L, 1, L, Hq, Hkv, True, topk > 0) == (True, True, parts)
+    q, k, v, g = _rand(L, Hq, 256), _rand(L, Hkv, 256), _rand(L, Hkv, 256), _rand(L, Hq, 256)
+    at = torch.arange(L, device=DEV)
+    q[..., 0] = 16.0   # channel 0 adds its key's value to every score (the scale is 1 / 16)
+    k[..., 0] = (12.0 * ((at >= 64).float() + (at >= 4 * 128 + 64) + (at >= L - L % 128 - 64)))[:, None].to(k.dtype)
+    keep = torch.ones(L, L, dtype=torch.bool, device=DEV).tril()
+    leaves, ref = [t.clone().requires_grad_() for t in (q, k, v)], [t.float().requires_grad_() for t in (q, k, v)]
+    if topk:
+        index = _rand(L, 4, 64), _rand(L, 64), _rand(L, 4).float()
+        bits = cu._C.dsa_select_bits(*index, [0, L], topk)
+        sel = cu._C.dsa_select(*index, 0, 0, 0, L, topk).long()
+        keep = torch.zeros(L, L + 1, dtype=torch.bool, device=DEV).scatter_(1, torch.where(sel < 0, L, sel), True)[:, :L]
+        o = _MaskedAttention.apply(*leaves, torch.tensor([0, L], dtype=torch.int32, device=DEV), bits, topk, 1 / 16)
+    else:
+        o = ops.attention_varlen(*leaves, torch.tensor([0, L], dtype=torch.int32, device=DEV), L, True, None)
+    o.backward(g)
+    att = torch.einsum("qhd,khd->hqk", ref[0], ref[1].repeat_interleave(Hq // Hkv, 1)) / 16
+    o_r = torch.einsum("hqk,khd->qhd", att.masked_fill(~keep, float("-inf")).softmax(-1), ref[2].repeat_interleave(Hq // Hkv, 1))
+    o_r.backward(g.float())
+    cu.check_status()
+    _close(o, o_r, 0.03, 2e-2, "out")
+    # few keys carry a row, so dS is of order 1: its bf16 rounding (2^-9) times keys and queries of order 4, for a key over hundreds of rows;
+    # channel 0 multiplies it by up to 36 and is left out
+    for a, b, n in zip(leaves, ref, ("dq", "dk", "dv")):
+        err, size = (a.grad.float() - b.grad)[..., 1:], b.grad[..., 1:]
+        assert float(err.norm() / size.norm()) < 6e-3, n   # bf16 P and dS, bf16 result: 2.3e-3 to 2.7e-3 on random rows
 
 
 def test_rope_tables_and_position_embedding_outside_the_kernels_forms():
