@@ -257,8 +257,10 @@ attn256_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
 #pragma unroll
         for (int i = 0; i < BC; ++i) if (i > limit) s[i] = 0xff800000u;  // -inf
       }
-      // The running maximum moves per 64 keys and the row sum is formed per 64 keys, whatever the width of a step: the probabilities keep
-      // the bits that they have under 64-row tiles, and with them FP8 linears behind this kernel the scales of their tensors.
+      // The running maximum moves per 64 keys and the row sum is formed per 64 keys, as with 64-row tiles: while no second half of a step raises
+      // the maximum by more than the threshold the probabilities have the bits that they have there, and with them FP8 linears behind this
+      // kernel the scales of their tensors.  Where one does, both halves are rounded under the new maximum; with 64-row tiles the first half is
+      // rounded under the old one and rescaled in fp32: as exact, other bits.
       const float m_old = m_used;
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
