@@ -21,8 +21,8 @@
 // SEL variants (sparse attention): every query of a document longer than `sel_topk` sees only the keys whose bit is set in
 // a selection bit mask (one bit per query and causal key, made by dsa_indexer_sm100.cu).  Every tile up to the diagonal is
 // still computed: gathering a query's 2048 key rows feeds the tensor core 8 query rows at a time and is bound by L2 gather
-// and scatter-add traffic (1.7 to 2.3 ns per query and key, forward + backward, 16 heads), a masked pair costs 0.10 to 0.15 ns, so
-// the dense form wins while documents are shorter than about 40 times the number of selected keys (the limit in use: ops/dsa_cuda.py).
+// and scatter-add traffic (1.7 to 2.3 ns per query and key, forward + backward, 16 heads), a masked pair costs 0.08 to 0.10 ns, so
+// the dense form wins while documents are shorter than about 55 times the number of selected keys (the limit in use: ops/dsa_cuda.py).
 //
 // Roles per block: warp 0 issues TMA loads (both blocks' loads of a tile complete on the barrier of the even one, the leader), one
 // thread of the leader's warp 1 issues every MMA, the compute warps own the rows of their block.  Every wait is bounded
@@ -954,7 +954,7 @@ extern "C" int vlmt_attn256_bwd(const void* dout, const void* q, const void* k, 
                                 int longest, const void* sel, int sel_topk, int* status, cudaStream_t st) {
   if (T <= 0 || n_docs <= 0) return 0;
   launch_pdl(attn256_delta_kernel, dim3((T * Hq * 32 + 255) / 256), dim3(256), 0, st, 1, reinterpret_cast<const __nv_bfloat16*>(dout),
-                                                                  reinterpret_cast<const __nv_bfloat16*>(o), delta, T, Hq);
+             reinterpret_cast<const __nv_bfloat16*>(o), delta, T, Hq);
   Params p{};
   p.dQ = reinterpret_cast<__nv_bfloat16*>(dq); p.dK = reinterpret_cast<__nv_bfloat16*>(dk); p.dV = reinterpret_cast<__nv_bfloat16*>(dv);
   p.LSE = const_cast<float*>(lse); p.delta = delta; p.cu = cu; p.n_docs = n_docs; p.T = T; p.Hq = Hq; p.Hkv = Hkv;

@@ -25,9 +25,9 @@
 // Building with -DVLMT_ATTN_TRACE records clock64 stamps of the MMA thread and of one compute warp of CTA (0,0) of
 // the dQ kernel and prints them after the third backward call (a timeline tool; no effect on regular builds).
 #include "attention_sm100.h"
+#include "pdl.cuh"
 #include "sm100.cuh"
 
-#include "pdl.cuh"
 #include <cuda_bf16.h>
 #include <math.h>
 
@@ -1055,7 +1055,7 @@ extern "C" int vlmt_attn_bwd(const void* dout, const void* q, const void* k, con
   {
     const int vec = ((reinterpret_cast<uintptr_t>(dout) | reinterpret_cast<uintptr_t>(o)) & 7) == 0;
     launch_pdl(attn_delta_kernel, dim3((unsigned)(((long)T * Hq + 31) / 32)), dim3(256), 0, st, 1, reinterpret_cast<const __nv_bfloat16*>(dout),
-                                                                            reinterpret_cast<const __nv_bfloat16*>(o), delta, T, Hq, d, vec);
+               reinterpret_cast<const __nv_bfloat16*>(o), delta, T, Hq, d, vec);
   }
   CUtensorMap tq, tk, tv, tdo;
   int r;

@@ -14,9 +14,9 @@
 //                             still needed.  Rows with n <= k keep every key.  Deterministic; unused slots are -1.
 #include "dsa_attention.h"
 #include "gemm_sm100.h"
+#include "pdl.cuh"
 #include "sm100.cuh"
 
-#include "pdl.cuh"
 #include <cuda_bf16.h>
 
 namespace {
@@ -281,7 +281,7 @@ extern "C" int vlmt_dsa_index_scores(const void* iq, const void* ik, const float
   const int smem = 4 * 16384 + 16384 + 64 + 1024;
   if (cudaFuncSetAttribute(dsa_index_scores_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return -4;
   dim3 grid((B + 127) / 128, (n_keys + 127) / 128);
-  launch_pdl(dsa_index_scores_kernel, dim3(grid), dim3(128), smem, st, 1, tq, tk, p);
+  launch_pdl(dsa_index_scores_kernel, grid, dim3(128), smem, st, 1, tq, tk, p);
   return cudaGetLastError() == cudaSuccess ? 0 : -5;
 }
 

@@ -8,8 +8,8 @@
 // bit-reproducible run to run.
 #include "elementwise.h"
 #include "no_alloc_entry.h"
-
 #include "pdl.cuh"
+
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -1953,7 +1953,7 @@ int vlmt_rmsnorm_gated_bwd(const void* dy, const void* x, const void* z, const v
                            float* dw_partial, int rows, int D, cudaStream_t st) {
   const int grid = vlmt_norm_blocks(rows);
   launch_pdl(rmsnorm_gated_bwd_kernel, dim3(grid), dim3(kThreads), (size_t)kWarpsPerBlock * D * sizeof(float), st, 1, BF(dy), BF(x), BF(z), BF(w), rstd, BFM(dx),
-                                                                                            BFM(dz), dw_partial, rows, D);
+             BFM(dz), dw_partial, rows, D);
   return grid;
 }
 
@@ -1988,12 +1988,12 @@ int vlmt_qkv_norm_rope_fwd(const void* qkv, const void* qw, const void* kw, cons
   const int grid = vlmt_qkv_blocks((long)T * ((n_q + 2 * n_kv + kQkvGroup - 1) / kQkvGroup));  // one warp per token and group of heads
   if (D == 128 && R == 128 && aligned16(cosv) && aligned16(sinv)) {   // the presets' head; other sizes and partial rotary: general form
     launch_pdl(qkv_norm_rope128_fwd_kernel, dim3(grid), dim3(kThreads), 0, st, 1, BF(qkv), BF(qw), BF(kw), cosv, sinv, BFM(q), BFM(k), BFM(v), BFM(gate), rstd, T,
-                                                           n_q, n_kv, eps, offset, gated, has_norm);
+               n_q, n_kv, eps, offset, gated, has_norm);
     return 0;
   }
 #define LAUNCH(E_)                                                                                                              \
   launch_pdl(qkv_norm_rope_fwd_kernel<E_>, dim3(grid), dim3(kThreads), 0, st, 1, BF(qkv), BF(qw), BF(kw), cosv, sinv, BFM(q), BFM(k), BFM(v), BFM(gate), \
-                                                          rstd, T, n_q, n_kv, R, eps, offset, gated, has_norm)
+             rstd, T, n_q, n_kv, R, eps, offset, gated, has_norm)
   switch (E) {
     case 1: LAUNCH(1); break;
     case 2: LAUNCH(2); break;
@@ -2011,12 +2011,12 @@ int vlmt_qkv_norm_rope_bwd(const void* dq, const void* dk, const void* dv, const
   const int grid = vlmt_qkv_blocks((long)T * (n_q + 2 * n_kv));
   if (D == 128 && R == 128 && has_norm && aligned16(cosv) && aligned16(sinv)) {
     launch_pdl(qkv_norm_rope128_bwd_kernel, dim3(grid), dim3(kThreads), 0, st, 1, BF(dq), BF(dk), BF(dv), BF(dgate), BF(qkv), BF(qw), BF(kw), cosv, sinv, rstd,
-                                                           BFM(dqkv), dw_partial, T, n_q, n_kv, offset, gated);
+               BFM(dqkv), dw_partial, T, n_q, n_kv, offset, gated);
     return grid;
   }
 #define LAUNCH(E_)                                                                                                               \
   launch_pdl(qkv_norm_rope_bwd_kernel<E_>, dim3(grid), dim3(kThreads), 0, st, 1, BF(dq), BF(dk), BF(dv), BF(dgate), BF(qkv), BF(qw), BF(kw), cosv, sinv, \
-                                                          rstd, BFM(dqkv), dw_partial, T, n_q, n_kv, R, offset, gated, has_norm)
+             rstd, BFM(dqkv), dw_partial, T, n_q, n_kv, R, offset, gated, has_norm)
   switch (E) {
     case 1: LAUNCH(1); break;
     case 2: LAUNCH(2); break;
@@ -2054,7 +2054,7 @@ int vlmt_gdn_gates_bwd(const float* dg, const void* dbeta, const void* a, const 
                        const float* dt_bias, void* da, void* db, long out_stride, float* partial, long T, int H, cudaStream_t st) {
   const int grid = grid_for(T * H, 256, 148 * 2);
   launch_pdl(gdn_gates_bwd_kernel, dim3(grid), dim3(256), 2 * H * sizeof(float), st, 1, dg, BF(dbeta), BF(a), BF(b), row_stride, A_log, dt_bias, BFM(da), BFM(db),
-                                                               out_stride, partial, T, H);
+             out_stride, partial, T, H);
   return grid;
 }
 
@@ -2062,7 +2062,7 @@ int vlmt_conv1d_silu_fwd(const void* x, long xs, const void* w, const int* seq_i
   if (K != 4 || (C & 7)) return -1;
   const int rows = 64;
   dim3 grid(((C >> 3) + 127) / 128, (T + rows - 1) / rows);
-  launch_pdl(conv1d_silu_fwd_kernel<4>, dim3(grid), dim3(128), 0, st, 1, BF(x), xs, BF(w), seq_idx, BFM(y), ys, T, C, rows);
+  launch_pdl(conv1d_silu_fwd_kernel<4>, grid, dim3(128), 0, st, 1, BF(x), xs, BF(w), seq_idx, BFM(y), ys, T, C, rows);
   return 0;
 }
 int vlmt_conv1d_bwd_slabs(int T) { return (T + kConvSlab - 1) / kConvSlab; }
@@ -2070,7 +2070,7 @@ int vlmt_conv1d_silu_bwd(const void* dy, long dys, const void* x, long xs, const
                          float* dw_partial, int T, int C, int K, cudaStream_t st) {
   if (K != 4 || (C & 3)) return -1;
   dim3 grid(((C >> 2) + 127) / 128, vlmt_conv1d_bwd_slabs(T));
-  launch_pdl(conv1d_silu_bwd_kernel<4>, dim3(grid), dim3(128), 0, st, 1, BF(dy), dys, BF(x), xs, BF(w), seq_idx, BFM(dx), dxs, dw_partial, T, C, kConvSlab);
+  launch_pdl(conv1d_silu_bwd_kernel<4>, grid, dim3(128), 0, st, 1, BF(dy), dys, BF(x), xs, BF(w), seq_idx, BFM(dx), dxs, dw_partial, T, C, kConvSlab);
   return 0;
 }
 

@@ -10,9 +10,9 @@
 //       warp 1      allocates TMEM (two 256-column accumulators), one lane issues the MMAs
 //       warps 2..5  epilogue: tcgen05.ld, scale, bf16, swizzled staging, TMA store or TMA reduce-add
 //   The scale s = rec_a[1] * rec_b[1] is read from device memory, so quantisation and GEMM queue without a host sync.
+#include "pdl.cuh"
 #include "sm100.cuh"
 
-#include "pdl.cuh"
 #include <cuda_fp8.h>
 #include <stdlib.h>
 
@@ -345,8 +345,8 @@ extern "C" int vlmt_fp8_cast(const void* x, long ld, long rows, long cols, float
   auto* xp = reinterpret_cast<const __nv_bfloat16*>(x);
   auto* rm = reinterpret_cast<uint8_t*>(out_rm);
   auto* tp = reinterpret_cast<uint8_t*>(out_t);
-  if (format == FP8_E4M3) launch_pdl(cast_kernel<FP8_E4M3>, dim3(grid), dim3(256), 0, stream, 1, xp, ld, rows, cols, rec, rm, ld_rm, tp, ld_t);
-  else if (format == FP8_E5M2) launch_pdl(cast_kernel<FP8_E5M2>, dim3(grid), dim3(256), 0, stream, 1, xp, ld, rows, cols, rec, rm, ld_rm, tp, ld_t);
+  if (format == FP8_E4M3) launch_pdl(cast_kernel<FP8_E4M3>, grid, dim3(256), 0, stream, 1, xp, ld, rows, cols, rec, rm, ld_rm, tp, ld_t);
+  else if (format == FP8_E5M2) launch_pdl(cast_kernel<FP8_E5M2>, grid, dim3(256), 0, stream, 1, xp, ld, rows, cols, rec, rm, ld_rm, tp, ld_t);
   else return -6;
   return (int)cudaGetLastError();
 }

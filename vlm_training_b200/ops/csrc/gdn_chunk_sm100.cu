@@ -19,9 +19,9 @@
 // Every wait is bounded; a wait that runs out sets the status word and the CTA leaves through the common teardown.
 #include "gdn_chunk_sm100.h"
 #include "gemm_sm100.h"
+#include "pdl.cuh"
 #include "sm100.cuh"
 
-#include "pdl.cuh"
 #include <cuda_bf16.h>
 
 namespace {
@@ -961,7 +961,7 @@ extern "C" int vlmt_gdn_prepare_fwd(const void* q, const void* k, const void* v,
   p.P = (__nv_bfloat16*)P; p.Tm = (__nv_bfloat16*)Tm; p.gc = gc; p.decay = decay;
   p.scale = scale; p.eps = eps; p.H = H; p.N = N; p.status = status;
   if ((r = set_smem(gdn_prepare_fwd_kernel, PrepSmem::kTotal))) return r;
-  launch_pdl(gdn_prepare_fwd_kernel, dim3(dim3(N, H)), dim3(THREADS), PrepSmem::kTotal, st, 1, tq, tk, tv, p);
+  launch_pdl(gdn_prepare_fwd_kernel, dim3(N, H), dim3(THREADS), PrepSmem::kTotal, st, 1, tq, tk, tv, p);
   return (int)cudaGetLastError();
 }
 
@@ -978,7 +978,7 @@ extern "C" int vlmt_gdn_output_fwd(const void* qg, const void* P, const void* st
   OutParams p;
   p.chunks = reinterpret_cast<const int2*>(chunks); p.o = (__nv_bfloat16*)o; p.H = H; p.N = N; p.status = status;
   if ((r = set_smem(gdn_output_fwd_kernel, OutSmem::kTotal))) return r;
-  launch_pdl(gdn_output_fwd_kernel, dim3(dim3(N, H)), dim3(THREADS), OutSmem::kTotal, st, 1, tqg, tp, ts, tvn, p);
+  launch_pdl(gdn_output_fwd_kernel, dim3(N, H), dim3(THREADS), OutSmem::kTotal, st, 1, tqg, tp, ts, tvn, p);
   return (int)cudaGetLastError();
 }
 
@@ -999,7 +999,7 @@ extern "C" int vlmt_gdn_output_bwd(const void* dout, long ld_do, const void* qg,
   p.dqg = (__nv_bfloat16*)dqg; p.dvn = (__nv_bfloat16*)dvn; p.dP = (__nv_bfloat16*)dP; p.dS = (__nv_bfloat16*)dS;
   p.H = H; p.N = N; p.status = status;
   if ((r = set_smem(gdn_output_bwd_kernel, OutBwdSmem::kTotal))) return r;
-  launch_pdl(gdn_output_bwd_kernel, dim3(dim3(N, H)), dim3(THREADS), OutBwdSmem::kTotal, st, 1, tdo, tqg, tp, ts, tvn, p);
+  launch_pdl(gdn_output_bwd_kernel, dim3(N, H), dim3(THREADS), OutBwdSmem::kTotal, st, 1, tdo, tqg, tp, ts, tvn, p);
   return (int)cudaGetLastError();
 }
 
@@ -1027,6 +1027,6 @@ extern "C" int vlmt_gdn_prepare_bwd(const void* q, const void* k, const void* v,
   p.dq = (__nv_bfloat16*)dq; p.dk = (__nv_bfloat16*)dk; p.dv = (__nv_bfloat16*)dv; p.dg = dg; p.dbeta = dbeta;
   p.scale = scale; p.eps = eps; p.H = H; p.N = N; p.status = status;
   if ((r = set_smem(gdn_prepare_bwd_kernel, PrepBwdSmem::kTotal))) return r;
-  launch_pdl(gdn_prepare_bwd_kernel, dim3(dim3(N, H)), dim3(THREADS), PrepBwdSmem::kTotal, st, 1, tq, tk, tv, ts, tg, tvn, tdu, tdqg, tdp, tpp, ttm, p);
+  launch_pdl(gdn_prepare_bwd_kernel, dim3(N, H), dim3(THREADS), PrepBwdSmem::kTotal, st, 1, tq, tk, tv, ts, tg, tvn, tdu, tdqg, tdp, tpp, ttm, p);
   return (int)cudaGetLastError();
 }

@@ -24,9 +24,9 @@
 // CTA leaves through the common teardown (TMEM freed).
 #include "gdn_scan_sm100.h"
 #include "gemm_sm100.h"
+#include "pdl.cuh"
 #include "sm100.cuh"
 
-#include "pdl.cuh"
 #include <cuda_bf16.h>
 
 namespace {
@@ -289,7 +289,7 @@ int launch(const CUtensorMap& t1, const CUtensorMap& t2, const CUtensorMap& te, 
     attr_set = true;
   }
   dim3 grid(n_docs, p.H);
-  launch_pdl(gdn_scan_kernel<REVERSE>, dim3(grid), dim3(THREADS), kSmem, stream, 1, t1, t2, te, p);
+  launch_pdl(gdn_scan_kernel<REVERSE>, grid, dim3(THREADS), kSmem, stream, 1, t1, t2, te, p);
   return cudaGetLastError() == cudaSuccess ? 0 : -11;
 }
 }  // namespace

@@ -13,8 +13,8 @@
 // The leader (even rank) issues every MMA; both blocks' loads complete on the leader's "full" barrier; commits arrive on both
 // blocks' "empty" and "accumulator full" barriers; both epilogues arrive on the leader's "accumulator free" barrier.
 #include "gemm_epilogue.cuh"
-#include "pdl.cuh"
 #include "gemm_pair_sm100.h"
+#include "pdl.cuh"
 #include "sm100.cuh"
 
 #include <cuda_runtime.h>
@@ -28,9 +28,10 @@ constexpr int BM = 128, BN = 256, BK = 64, UMMA_K = 16, STAGES = 6;   // BK, UMM
 constexpr int NUM_THREADS = 192;
 
 // Pairs of M tiles per raster group: their rows of A and the B panel they meet share L2.  Every group reads all of B, so where B does not
-// stay in L2 (32 MB and more) and 4096 rows of A do (K up to 4096 bf16 values) a group is 16 pairs, else 8.  PFLOP/s with 8 / 16, under the power limit:
+// stay in L2 (32 MB and more) and 4096 rows of A do (36 MB: K up to 4608 in bf16, 9216 in FP8) a group is 16 pairs, else 8.  PFLOP/s with 8 / 16, under the power limit:
 // 8192 x 24576 x 4096 1.33 / 1.40, 8192 x 12288 x 4096 1.33 / 1.38, 8192 x 6144 x 4096 1.28 / 1.31; 8192 x 4096 x 12288 1.27 / 1.25,
-// weight gradient 24576 x 4096 x 8192 1.25 / 1.24, 28672 x 1152 x 4304 1.12 / 1.08.
+// weight gradient 24576 x 4096 x 8192 1.25 / 1.24, 28672 x 1152 x 4304 1.12 / 1.08.  FP8 where it is 16: 8192 x 24576 x 4096 2.49 / 2.59,
+// 16384 x 24576 x 4096 2.44 / 2.53, 8192 x 12288 x 4096 2.41 / 2.50, 16384 x 9216 x 8192 2.49 / 2.55.
 int raster_group(long n_bytes, long k_bytes) { return n_bytes >= (32l << 20) && 4096 * k_bytes <= (36l << 20) ? 16 : 8; }
 
 constexpr int kABytes = BM * BK * 2, kBBytes = (BN / 2) * BK * 2, kStageBytes = kABytes + kBBytes;

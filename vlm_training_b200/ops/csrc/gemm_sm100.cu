@@ -780,7 +780,7 @@ bool split_k_enabled() {
 // of its load (45 bytes per cycle and SM when most SMs load) and MMA time, wave by wave and not below the wave's
 // share of the operands at the memory's rate (23 bytes per cycle and SM with all of them loading); a split adds the
 // exchange of the parts.  A split is a cluster of 2, 4 or 8 blocks with at least 4 k-blocks each, all clusters resident at once
-// (measured: 37 x 4096 x 12288 75.8 -> 23.4 us, 37 x 6144 x 4096 29.4 -> 16.5 us, 451 x 4096 x 12288 75.6 -> 52 us).
+// (measured: 37 x 4096 x 12288 75.8 -> 23.4 us, 37 x 6144 x 4096 29.4 -> 16.5 us).
 struct SplitPlan { int bn, splits, kb_per; };
 
 template <int BN, bool A_MN, bool B_MN, bool AG>

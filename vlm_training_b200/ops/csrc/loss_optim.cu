@@ -1,8 +1,8 @@
 // Cross-entropy over one chunk of logits (forward loss + in-place gradient) and the fused
 // AdamW update on flat fp32 master weights with a bf16 parameter write-back.
 #include "loss_optim.h"
-
 #include "pdl.cuh"
+
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -426,14 +426,14 @@ void vlmt_colsum(const void* x, long ld, int rows, int cols, float* partial, voi
   const int slabs = rows > 0 ? vlmt_colsum_slabs(rows) : 0;
   if (slabs > 0) {
     dim3 grid((cols + 255) / 256, slabs);
-    launch_pdl(colsum_kernel, dim3(grid), dim3(256), 0, st, 1, reinterpret_cast<const bf16*>(x), ld, rows, cols, partial, 256);
+    launch_pdl(colsum_kernel, grid, dim3(256), 0, st, 1, reinterpret_cast<const bf16*>(x), ld, rows, cols, partial, 256);
   }
   launch_pdl(colsum_finish_kernel, dim3((cols + 255) / 256), dim3(256), 0, st, 1, partial, slabs, cols, out, mode);
 }
 // out[c] = sum over `rows` partial rows (the per-block weight-gradient sums of the norm kernels)
 void vlmt_sum_rows(const VlmtRowSums* a, int sums, int rows, int cols, cudaStream_t st) {
   if (cols <= 0 || sums <= 0) return;
-  launch_pdl(sum_rows_kernel, dim3(dim3((cols + 15) / 16, sums)), dim3(256), 0, st, 1, *a, rows, cols);
+  launch_pdl(sum_rows_kernel, dim3((cols + 15) / 16, sums), dim3(256), 0, st, 1, *a, rows, cols);
 }
 void vlmt_sumsq(const void* x, int fp32, long n, float* out, cudaStream_t st) {
   if (n <= 0) return;

@@ -13,8 +13,8 @@
 // rank's per-expert counts), dispatch stores a slot's row straight into the memory of the rank that owns the expert, and
 // the owner stores the expert output back into the source rank's per-slot buffer (kernels at the end of this file).
 #include "moe_kernels.h"
-
 #include "pdl.cuh"
+
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>

@@ -2,8 +2,8 @@
 // the vision plan, 0.4 ms of numpy per call), and the calls that need them most, a chat turn and a small training step, are bound
 // by launches and host work.
 #include "plan_kernels.h"
-
 #include "pdl.cuh"
+
 #include <cuda_bf16.h>
 #include <stdint.h>
 
@@ -179,7 +179,7 @@ void vlmt_pos_embed_fwd(const void* x, const void* table, const long* pe_index, 
                         cudaStream_t st) {
   if (N <= 0) return;
   launch_pdl(pos_embed_fwd_kernel, dim3((unsigned)((N * (D / 8) + 255) / 256)), dim3(256), 0, st, 1, (const uint4*)x, (const uint4*)table, pe_index, pe_weight, (uint4*)out,
-                                                                              N, D / 8);
+             N, D / 8);
 }
 void vlmt_pos_embed_bwd(const void* dy, const int* images, int n_img, int side, int merge, long N, void* dtable, int accumulate, int D,
                         cudaStream_t st) {

@@ -30,10 +30,10 @@ import torch.utils.checkpoint as _ckpt
 from . import cuda as cu
 
 _QBLOCK = 1024
-# Forward + backward with 16 heads, the masked dense form costs 0.10 to 0.15 ns per query and CAUSAL key, the gathered form 1.7 to 2.3 ns per
-# query and SELECTED key (topk 512: 4.09 and 8.70 ms at 16 times topk, 14.75 and 19.01 ms at 32 times; topk 2048: 54.6 and 119.7 ms at
-# 16 times): they meet near 40 times topk (figures of 64-row key tiles; on CTA pairs the dense form takes three quarters of that).  The limit is lower because the mask is one bit per query and causal key, kept for backward, and
-# grows with the square of the document, the gathered form's lists with its length (16 times 2048: 134 MB and 268 MB, 40 times: 840 and 671).
+# Forward + backward with 16 heads, the masked dense form costs 0.08 to 0.10 ns per query and CAUSAL key, the gathered form 1.7 to 2.3 ns per
+# query and SELECTED key (topk 512: 2.70 and 8.65 ms at 16 times topk, 10.3 and 19.0 ms at 32 times; topk 2048: 42.2 and 119 ms at 16 times):
+# they meet near 55 times topk.  The limit is lower because the mask is one bit per query and causal key, kept for backward, and grows with
+# the square of the document, the gathered form's lists with its length (16 times 2048: 134 MB and 268 MB, 40 times: 840 and 671).
 _DENSE_TIMES = 16
 
 
