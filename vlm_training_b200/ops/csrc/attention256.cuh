@@ -103,6 +103,33 @@ __device__ __forceinline__ void store_row32(__nv_bfloat16* dst, const uint32_t (
   }
 }
 
+// Sum of a cluster's parts of a [128 x 256] accumulator and its store.  Every block of the cluster gets here, also after an abort.
+// Its own part is in shared memory; the blocks that hold the same keys sum in order of their rank and store an equal share of the rows each.
+// STRIDE: ranks from one part of the same keys to the next.
+template <int STRIDE>
+__device__ __forceinline__ void store_parts(uint8_t* smem, const Params& p, volatile int* abort_flag, int rank, __nv_bfloat16* base, float f,
+                                            const TileInfo& ti, int k0, int hkv) {
+  __syncwarp();
+  cluster_sync();
+  if (!*abort_flag) {
+    const int rows = BR / p.parts, row0 = rank / STRIDE * rows;
+    const uint32_t at = smem_u32(smem);
+    for (int i = threadIdx.x; i < rows * (HD / 4); i += blockDim.x) {
+      const int row = row0 + i / (HD / 4), col = i % (HD / 4) * 4;
+      float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+      for (int s = 0; s < p.parts; ++s) {
+        const float4 x = ld_cluster_f4(at + (uint32_t)(row * kPartPitch + col) * 4, STRIDE * s + rank % STRIDE);
+        v.x += x.x; v.y += x.y; v.z += x.z; v.w += x.w;
+      }
+      if (k0 + row < ti.doc_len)
+        *reinterpret_cast<uint2*>(base + ((size_t)(ti.doc_start + k0 + row) * p.Hkv + hkv) * HD + col) =
+            make_uint2(pack_bf16x2(v.x * f, v.y * f), pack_bf16x2(v.z * f, v.w * f));
+    }
+  }
+  __syncwarp();
+  cluster_sync();        // nobody leaves while its part is being read
+}
+
 inline int make_map(CUtensorMap* m, const void* base, int T, int cols, long ld, int box_rows) {
   return vlmt_make_tmap_2d_bf16(m, base, (uint64_t)cols, (uint64_t)T, (uint64_t)ld * 2, 64, (uint32_t)box_rows);
 }

@@ -675,30 +675,7 @@ attn256_single_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __g
       }
     }
   }
-  if (p.parts > 1) {
-    __syncwarp();
-    cluster_sync();        // every block of the cluster gets here, also after an abort
-    if (!*abort_flag) {
-      // the parts are summed in order of their rank; block `part` stores its share of the rows
-      const int rows = BR / p.parts, row0 = part * rows;
-      const float f = DV ? 1.f : p.scale;
-      __nv_bfloat16* base = DV ? p.dV : p.dK;
-      const uint32_t at = smem_u32(smem);
-      for (int i = threadIdx.x; i < rows * (HD / 4); i += THREADS) {
-        const int row = row0 + i / (HD / 4), col = i % (HD / 4) * 4;
-        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-        for (int s = 0; s < p.parts; ++s) {
-          const float4 x = ld_cluster_f4(at + (uint32_t)(row * kPartPitch + col) * 4, s);
-          v.x += x.x; v.y += x.y; v.z += x.z; v.w += x.w;
-        }
-        if (k0 + row < ti.doc_len)
-          *reinterpret_cast<uint2*>(base + ((size_t)(ti.doc_start + k0 + row) * p.Hkv + hkv) * HD + col) =
-              make_uint2(pack_bf16x2(v.x * f, v.y * f), pack_bf16x2(v.z * f, v.w * f));
-      }
-    }
-    __syncwarp();
-    cluster_sync();        // nobody leaves while its part is being read
-  }
+  if (p.parts > 1) store_parts<1>(smem, p, abort_flag, part, DV ? p.dV : p.dK, DV ? 1.f : p.scale, ti, k0, hkv);
   teardown(abort_flag, warp, tmem_base);
 }
 

@@ -544,31 +544,6 @@ attn256_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
   teardown(abort_flag, warp, tmem_base);
 }
 
-// Sum of a cluster's parts of a [128 x 256] accumulator and its store.  Every block of the cluster gets here, also after an abort.
-// Its own part is in shared memory; the blocks that hold the same keys sum in order of their rank and store an equal share of the rows each.
-__device__ __forceinline__ void store_parts(uint8_t* smem, const Params& p, volatile int* abort_flag, int rank, __nv_bfloat16* base, float f,
-                                            const TileInfo& ti, int k0, int hkv) {
-  __syncwarp();
-  cluster_sync();
-  if (!*abort_flag) {
-    const int rows = BR / p.parts, row0 = (rank >> 1) * rows;
-    const uint32_t at = smem_u32(smem);
-    for (int i = threadIdx.x; i < rows * (HD / 4); i += blockDim.x) {
-      const int row = row0 + i / (HD / 4), col = i % (HD / 4) * 4;
-      float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-      for (int s = 0; s < p.parts; ++s) {
-        const float4 x = ld_cluster_f4(at + (uint32_t)(row * kPartPitch + col) * 4, 2 * s + (rank & 1));
-        v.x += x.x; v.y += x.y; v.z += x.z; v.w += x.w;
-      }
-      if (k0 + row < ti.doc_len)
-        *reinterpret_cast<uint2*>(base + ((size_t)(ti.doc_start + k0 + row) * p.Hkv + hkv) * HD + col) =
-            make_uint2(pack_bf16x2(v.x * f, v.y * f), pack_bf16x2(v.z * f, v.w * f));
-    }
-  }
-  __syncwarp();
-  cluster_sync();        // nobody leaves while its part is being read
-}
-
 constexpr int kDkvThreads = 352;   // as kBwdThreads, and a warp for the queries' statistics
 
 // dV pass: K by rows of the pair, Q by rows and dO by channels in two stages each.
@@ -832,7 +807,7 @@ attn256_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
       }
     }
   }
-  if (p.parts > 1) store_parts(smem, p, abort_flag, rank, DV ? p.dV : p.dK, DV ? 1.f : p.scale, ti, k0, hkv);
+  if (p.parts > 1) store_parts<2>(smem, p, abort_flag, rank, DV ? p.dV : p.dK, DV ? 1.f : p.scale, ti, k0, hkv);
   teardown(abort_flag, warp, tmem_base);
 }
 
