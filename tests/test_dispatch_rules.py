@@ -25,6 +25,20 @@ def test_a_wave_of_pairs_only_where_it_is_the_faster_one(M, N, K, pairs):
     assert cu._C.gemm_form(M, N, K)[3] == pairs
 
 
+# At most 128 rows: the blocks that share a tile's K all have a part of it and fit a cluster; where one-block tiles are faster they are taken
+@pytest.mark.parametrize("M,N,K,splits", [(37, 6144, 4096, 3), (37, 4096, 4096, 4), (37, 24576, 4096, 1), (37, 10240, 4096, 3), (37, 18944, 4096, 2), (8, 1152, 4304, 8),
+                                          (64, 2048, 2048, 4), (64, 512, 512, 1), (8, 8, 64, 1), (64, 151936, 4096, 1), (65, 151936, 4096, 0),
+                                          (128, 18944, 4096, 0), (129, 4096, 4096, 0)])
+def test_blocks_that_share_a_tile_of_few_rows(M, N, K, splits):
+    from vlm_training_b200.ops import cuda as cu
+
+    assert cu._C.gemm_rows_splits(M, N, K) == splits
+    for n in range(8, 30000, 552):
+        for k in range(8, 13000, 488):
+            s, kb = cu._C.gemm_rows_splits(M, n, k), (k + 63) // 64
+            assert 0 <= s <= 8 and (s <= 1 or (s - 1) * ((kb + s - 1) // s) < kb)
+
+
 # Heads of 256: rows of short documents on single blocks, whose blocks all have keys; long ones, and all with a selection, on pairs
 @pytest.mark.parametrize("lens,Hq,Hkv,forward,backward", [([64], 16, 4, False, False), ([128] * 64, 16, 4, False, False), ([64] * 32, 16, 2, False, False),
                                                           ([128] * 64, 4, 4, False, False), ([150] * 4, 16, 2, False, False), ([900], 16, 2, True, True),

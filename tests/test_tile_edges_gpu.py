@@ -54,6 +54,31 @@ def test_gemm_split_over_k(M, N, K, layout):
     cu.check_status()
 
 
+# at most 128 rows: every width of the row tile at its edges, a feature tile that ends early, a short last block and part of K, activations, rows and
+# columns behind the last ones, an output whose rows start anywhere
+@pytest.mark.parametrize("M", [1, 16, 17, 48, 49, 64, 65, 96, 97, 128])
+@pytest.mark.parametrize("N,K,splits", [(24584, 72, 1), (9224, 520, None), (136, 1160, None), (4304, 1152, 4), (8, 2056, None)])
+def test_gemm_of_few_rows(M, N, K, splits):
+    from vlm_training_b200.ops import cuda as cu
+
+    assert cu._C.gemm_rows_splits(M, N, K) == splits or (splits is None and cu._C.gemm_rows_splits(M, N, K) > 0)
+    a, w, bias, alpha = _rand(M, K, scale=0.5), _rand(N, K, scale=0.5), _rand(N), torch.tensor(0.37, device=DEV)
+    want = 0.37 * (a.float() @ w.float().t()) + bias.float()
+    # fp32 accumulation of K products of size about 0.25, then one bf16 rounding (2^-8 of the value)
+    tol = dict(atol=2e-2 * (K / 4096) ** 0.5, rtol=8e-3)
+    got = [cu._gemm(a, w, bias=bias, alpha=alpha) for _ in range(2)]
+    torch.testing.assert_close(got[0].float(), want, **tol)
+    assert torch.equal(got[0], got[1])   # the parts are summed in rank order
+    for epilogue, approximate in ((1, "tanh"), (2, "none")):
+        got = cu._gemm(a, w, bias=bias, alpha=alpha, epilogue=epilogue)
+        torch.testing.assert_close(got.float(), torch.nn.functional.gelu(want, approximate=approximate), **tol)
+    out = torch.full((M + 1, N + 3), 7.0, device=DEV, dtype=torch.bfloat16)
+    cu._gemm(a, w, bias=bias, alpha=alpha, out=out[:M, 1:1 + N])
+    torch.testing.assert_close(out[:M, 1:1 + N].float(), want, **tol)
+    assert bool((out[M] == 7.0).all() and (out[:, 0] == 7.0).all() and (out[:, 1 + N:] == 7.0).all())
+    cu.check_status()
+
+
 # large outputs on CTA pairs (256 x 256 tiles): rows and columns off the tile edges, a pair whose second block has no rows, a K tail
 @pytest.mark.parametrize("M,N,K", [(2500, 2600, 520), (2304 + 100, 2304, 1096), (10000, 512, 72)])
 @pytest.mark.parametrize("layout", ["fwd", "dgrad", "wgrad"])

@@ -8,6 +8,7 @@
 #include "elementwise.h"
 #include "gdn_scan_sm100.h"
 #include "gemm_pair_sm100.h"
+#include "gemm_rows_sm100.h"
 #include "gemm_sm100.h"
 #include "loss_optim.h"
 #include "torch_ops.h"
@@ -558,6 +559,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   }, py::arg("M"), py::arg("N"), py::arg("K"), py::arg("parts_of_d") = false, py::arg("sms") = 148,
         py::arg("capacity") = std::array<int, 3>{74, 33, 14}, py::arg("pair_clusters") = 33);
   m.def("gemm_pair_clusters", &vlmt_gemm_pair_clusters);
+  m.def("gemm_rows_splits", &vlmt_gemm_rows_splits, py::arg("M"), py::arg("N"), py::arg("K"), py::arg("sms") = 148);
   m.def("gemm_set_flag_wait_ms", [](int64_t ms) {
     int r = vlmt_gemm_set_flag_wait_ms((long)ms);
     TORCH_CHECK(r == 0, "vlmt_gemm_set_flag_wait_ms failed with code ", r);

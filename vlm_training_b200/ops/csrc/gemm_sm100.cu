@@ -29,6 +29,7 @@
 
 #include <stdlib.h>
 #include "gemm_pair_sm100.h"
+#include "gemm_rows_sm100.h"
 #include "gemm_sm100.h"
 
 #include <cuda_runtime.h>
@@ -909,12 +910,17 @@ int gemm_launch(const void* A, const void* B, void* D, float* Dacc32, const void
   if (M <= 0 || N <= 0 || K <= 0) return 0;
   if ((lda & 7) || (ldb & 7)) return -2;  // TMA needs 16-byte row strides
   if ((reinterpret_cast<uintptr_t>(A) & 15) || (reinterpret_cast<uintptr_t>(B) & 15)) return -3;
+  const bool plain = x.grp_mode == 0 && x.rs_world == 0 && x.ag_world == 0 && x.wg_world == 0;
+  if (plain && M <= BM && !a_mn_major && !b_mn_major && !accumulate && Dacc32 == nullptr) {
+    const int splits = vlmt_gemm_rows_splits(M, N, K, num_sms);
+    if (splits > 0)
+      return vlmt_gemm_rows(A, B, D, bias, M, N, K, lda, ldb, ldd, epilogue, x.alpha, split_k_enabled() ? splits : 1, status, num_sms, stream);
+  }
   CUtensorMap ta, tb;
   int r;
   if (!a_mn_major) r = vlmt_make_tmap_2d_bf16(&ta, A, (uint64_t)K, (uint64_t)M, (uint64_t)lda * 2, 64, 128);
   else r = vlmt_make_tmap_2d_bf16(&ta, A, (uint64_t)M, (uint64_t)K, (uint64_t)lda * 2, 64, 64);
   if (r) return 1000 + r;
-  const bool plain = x.grp_mode == 0 && x.rs_world == 0 && x.ag_world == 0 && x.wg_world == 0;
   const uint64_t b_groups = x.grp_mode == 1 ? (uint64_t)x.grp_count : 1;   // grouped forward / dgrad: one B per group, stacked along the rows
   if (!b_mn_major) r = vlmt_make_tmap_2d_bf16(&tb, B, (uint64_t)K, (uint64_t)N * b_groups, (uint64_t)ldb * 2, 64, 128);
   else r = vlmt_make_tmap_2d_bf16(&tb, B, (uint64_t)N, (uint64_t)K * b_groups, (uint64_t)ldb * 2, 64, 64);

@@ -1,7 +1,7 @@
 // Programmatic dependent launch: a kernel launched through `launch_pdl` may start while the kernel before it in its stream drains, so
 // its launch latency and set-up (barriers, tensor memory, shared memory) are off the critical path.  Such a kernel
-//   * calls pdl_wait() in every thread before it touches global memory (reads, writes, prefetches of data; its own parameters are
-//     free): the call returns when the kernels before it have completed and their writes are visible, as without the attribute;
+//   * calls pdl_wait() in every thread before it touches global memory (reads and writes; its own parameters are free, and so are prefetches
+//     of data into L2, which is where the GPU's memory is coherent): the call returns when the kernels before it have completed and their writes are visible, as without the attribute;
 //   * calls it on every path, also in blocks that have nothing to do: a grid that ends without waiting would no longer order what follows
 //     it behind what precedes it.
 //   * if it allocates tensor memory, calls pdl_trigger() behind the allocation: the GEMMs allocate before they wait, and a block of theirs
