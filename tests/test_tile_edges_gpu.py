@@ -187,6 +187,40 @@ def test_adamw_bucket_matches_segment_launches(lens, state):
 
 
 # documents below, at and beyond the number of selected keys; ends on and off the 64- / 128-row tiles; one token; 1, 2 and 8 query heads per kv head
+# the selection where it can go wrong: integer scores, so the oracle's are the same to the last bit; a bin of equal steps between smallest and largest
+# score holds few keys ("spread"), a few hundred of them equal ("equal"), nearly all ("clustered": one far outlier), infinite scores, one value only
+@pytest.mark.parametrize("kind", ["spread", "equal", "clustered", "infinite", "constant"])
+@pytest.mark.parametrize("L,topk", [(1500, 64), (1301, 1000), (129, 128), (2500, 1)])
+def test_dsa_selection_of_integer_scores(kind, L, topk):
+    from vlm_training_b200.ops import cuda as cu
+
+    iq, ik, w = torch.randint(-3, 4, (L, 4, 64), device=DEV), torch.randint(-3, 4, (L, 64), device=DEV), torch.randint(-2, 3, (L, 4), device=DEV)
+    if kind == "equal":
+        ik[:, 2:] = 0
+    elif kind == "clustered":
+        ik[3], iq[..., 0], w[:] = 128, iq[..., 0].abs() + 200, 1
+    elif kind == "constant":
+        ik[:] = 0
+    iq, ik, w = iq.to(torch.bfloat16), ik.to(torch.bfloat16), w.float()
+    if kind == "infinite":
+        iq[..., 0], ik[7, 0], w[:] = 1.0, float("inf"), 1.0
+    scores = (torch.einsum("thd,sd->ths", iq.float(), ik.float()).relu() * w[..., None]).sum(1)
+    pos = torch.arange(L, device=DEV)
+    causal = pos[None, :] <= pos[:, None]
+    # the largest first, equal ones (-0 below 0, as the kernel orders them) in the order of their index
+    order = torch.where(causal, scores, float("-inf")).sort(dim=1, descending=True, stable=True).indices[:, :topk]
+    want = torch.zeros(L, L, dtype=torch.bool, device=DEV).scatter_(1, order, True) & causal
+    bits = cu._C.dsa_select_bits(iq, ik, w, [0, L], topk)
+    cu.check_status()
+    got = ((bits[: (L + 63) // 64].t()[:, pos // 64] >> (pos % 64)) & 1).bool() & (pos[None, :] <= (pos[:, None] | 127))
+    assert torch.equal(got.sum(1), want.sum(1)) and bool((got <= causal).all())
+    assert torch.equal(got & (scores != 0), want & (scores != 0))   # zeros carry a sign, which a different order of the sum may change
+    b0 = max(0, L - 1024)
+    rows = cu._C.dsa_select(iq, ik, w, b0, b0, 0, L - b0, min(topk, L)).long()
+    listed = torch.zeros(L - b0, L + 1, dtype=torch.bool, device=DEV).scatter_(1, torch.where(rows < 0, L, rows), True)[:, :L]
+    assert torch.equal(listed, got[b0:])
+
+
 @pytest.mark.parametrize("lens,topk,Hq,Hkv", [([700, 64, 1, 129, 300], 64, 16, 2), ([128, 1024, 257], 128, 8, 1), ([2100, 90], 512, 4, 4), ([1090], 1000, 4, 2)])
 def test_dsa_masked_dense_attention(lens, topk, Hq, Hkv):
     """Bit masks hold exactly the keys of the list form, and attention under them (forward, all gradients) matches the float32

@@ -119,7 +119,7 @@ static Tensor dsa_select(const Tensor& iq, const Tensor& ik, const Tensor& w, in
   Tensor sel = torch::empty({B, kk}, iq.options().dtype(torch::kInt));
   Tensor st = vlmt_status_tensor();
   auto stream = at::cuda::getCurrentCUDAStream().stream();
-  int r = vlmt_dsa_index_scores(iq.data_ptr(), ik.data_ptr(), w.data_ptr<float>(), T, (int)q_tok0, (int)q_pos0, (int)k_tok0, (int)B, n_keys,
+  int r = vlmt_dsa_index_scores(iq.data_ptr(), ik.data_ptr(), w.data_ptr<float>(), T, (int)q_tok0, (int)q_pos0, (int)k_tok0, (int)B,
                                 scores.data_ptr<float>(), ld, st.data_ptr<int>(), stream);
   TORCH_CHECK(r == 0, "vlmt_dsa_index_scores failed with code ", r);
   r = vlmt_dsa_topk(scores.data_ptr<float>(), (int)B, ld, (int)q_pos0, (int)kk, sel.data_ptr<int>(), stream);
@@ -128,7 +128,7 @@ static Tensor dsa_select(const Tensor& iq, const Tensor& ik, const Tensor& w, in
 }
 
 // Selection of every document longer than `topk` as bits: int64 [ceil(longest / 64), T] (attention256_sm100.cu).  `bounds`: the
-// documents' boundaries on the host.  Queries are scored in blocks of 1024, two launches each, through one score buffer.
+// documents' boundaries on the host.  Queries are scored in blocks of 1024, as many per launch as the score buffer holds.
 static Tensor dsa_select_bits(const Tensor& iq, const Tensor& ik, const Tensor& w, const std::vector<int64_t>& bounds, int64_t topk) {
   TORCH_CHECK(iq.is_cuda() && iq.scalar_type() == at::kBFloat16 && iq.is_contiguous() && iq.dim() == 3 && iq.size(1) == 4 && iq.size(2) == 64,
               "indexer queries must be contiguous bf16 [T, 4, 64]");
@@ -141,24 +141,20 @@ static Tensor dsa_select_bits(const Tensor& iq, const Tensor& ik, const Tensor& 
     TORCH_CHECK(bounds[i] >= 0 && bounds[i] <= bounds[i + 1] && bounds[i + 1] <= T, "document boundaries outside the row");
     longest = std::max(longest, bounds[i + 1] - bounds[i]);
   }
-  constexpr int64_t kBlock = 1024;
-  const int64_t ld_max = (longest + 3) & ~int64_t(3);
-  Tensor scores = torch::empty({kBlock * ld_max}, iq.options().dtype(torch::kFloat));
+  constexpr int64_t kBlock = 1024, kRoom = 16 << 20;   // 64 MB of scores at a time stay in L2
+  int64_t all = 0;
+  for (size_t i = 0; i + 1 < bounds.size(); ++i) {
+    const int64_t L = bounds[i + 1] - bounds[i];
+    if (L > topk) all += L * ((L + 3) & ~int64_t(3));
+  }
+  const int64_t room = std::min(all, std::max(kRoom, kBlock * ((longest + 3) & ~int64_t(3))));
+  Tensor scores = torch::empty({room}, iq.options().dtype(torch::kFloat));
   Tensor bits = torch::empty({(longest + 127) / 128 * 2, T}, iq.options().dtype(torch::kLong));
   Tensor st = vlmt_status_tensor();
-  auto stream = at::cuda::getCurrentCUDAStream().stream();
-  for (size_t i = 0; i + 1 < bounds.size(); ++i) {
-    const int64_t s = bounds[i], L = bounds[i + 1] - s;
-    if (L <= topk) continue;
-    for (int64_t b0 = 0; b0 < L; b0 += kBlock) {
-      const int B = (int)std::min(kBlock, L - b0), n_keys = (int)b0 + B, ld = (n_keys + 3) & ~3;
-      int r = vlmt_dsa_index_scores(iq.data_ptr(), ik.data_ptr(), w.data_ptr<float>(), (int)T, (int)(s + b0), (int)b0, (int)s, B, n_keys,
-                                    scores.data_ptr<float>(), ld, st.data_ptr<int>(), stream);
-      TORCH_CHECK(r == 0, "vlmt_dsa_index_scores failed with code ", r);
-      r = vlmt_dsa_topk_bits(scores.data_ptr<float>(), B, ld, (int)b0, (int)topk, bits.data_ptr(), (int)(s + b0), (int)T, stream);
-      TORCH_CHECK(r == 0, "vlmt_dsa_topk_bits failed with code ", r);
-    }
-  }
+  const std::vector<long> b(bounds.begin(), bounds.end());
+  int r = vlmt_dsa_select_bits(iq.data_ptr(), ik.data_ptr(), w.data_ptr<float>(), (int)T, b.data(), (int)b.size() - 1, (int)topk, (int)kBlock,
+                               scores.data_ptr<float>(), (long)room, bits.data_ptr(), st.data_ptr<int>(), at::cuda::getCurrentCUDAStream().stream());
+  TORCH_CHECK(r == 0, "vlmt_dsa_select_bits failed with code ", r);
   return bits;
 }
 

@@ -18,11 +18,13 @@ int vlmt_dsa_bwd_tc(const void* q, const void* k, const void* v, const int* sel,
 int vlmt_dsa_bwd(const void* q, const void* k, const void* v, const int* sel, const void* o, const float* lse, const void* d_o,
                  float* dq, float* dk, float* dv, int B, int Hkv, int rep, int D, int kk, float scale, cudaStream_t st);
 // lightning indexer (dsa_indexer_sm100.cu): scores of one query block and the per-query top-k selection
-int vlmt_dsa_index_scores(const void* iq, const void* ik, const float* w, int T, int q_tok0, int q_pos0, int k_tok0, int B, int n_keys,
-                          float* scores, int ld, int* status, cudaStream_t st);
+int vlmt_dsa_index_scores(const void* iq, const void* ik, const float* w, int T, int q_tok0, int q_pos0, int k_tok0, int B, float* scores, int ld,
+                          int* status, cudaStream_t st);
 int vlmt_dsa_topk(const float* scores, int B, int ld, int q_pos0, int kk, int* sel, cudaStream_t st);
-// the selection as a bit mask for the dense kernels (attention256_sm100.cu): [ceil(L / 64)][T] 64-bit words
-int vlmt_dsa_topk_bits(const float* scores, int B, int ld, int q_pos0, int kk, void* bits, int q_tok0, int T, cudaStream_t st);
+// both for the documents of a row that are longer than kk, the selection as a bit mask for the dense kernels (attention256_sm100.cu):
+// [ceil(L / 64)][T] 64-bit words; scores: `room` floats, at least `rows` x the longest document rounded up to 4
+int vlmt_dsa_select_bits(const void* iq, const void* ik, const float* w, int T, const long* bounds, int n_docs, int kk, int rows, float* scores,
+                         long room, void* bits, int* status, cudaStream_t st);
 #ifdef __cplusplus
 }
 #endif

@@ -140,7 +140,7 @@ def dsa_attention_cuda(q, k, v, idx_q, idx_k, idx_w, cu_seqlens, topk, scale=Non
     # the masked kernels take the row maximum before the scale and mask by -inf: a scale that is not positive goes to the gathered form
     if D == 256 and fused_select and longest <= _DENSE_TIMES * topk and scale > 0:
         bits = cu._C.dsa_select_bits(iq_c, ik_c, iw_c, bounds, int(topk))
-        cu._tick(2 * sum((b - a + _QBLOCK - 1) // _QBLOCK for a, b in zip(bounds[:-1], bounds[1:]) if b - a > topk))
+        cu._tick(2)
         o = _MaskedAttention.apply(q[:n], k[:n], v[:n], _device_bounds(cu_seqlens, bounds, q.device), bits[:, :n].contiguous() if n < T else bits, int(topk), float(scale))
         return o if n == T else torch.cat((o, q.new_zeros(T - n, Hq, D)), 0)
     # documents end where the packed row ends: tokens behind the last boundary are padding
