@@ -141,8 +141,11 @@ def dsa_attention_cuda(q, k, v, idx_q, idx_k, idx_w, cu_seqlens, topk, scale=Non
     if D == 256 and fused_select and longest <= _DENSE_TIMES * topk and scale > 0:
         bits = cu._C.dsa_select_bits(iq_c, ik_c, iw_c, bounds, int(topk))
         cu._tick(2)
-        o = _MaskedAttention.apply(q[:n], k[:n], v[:n], _device_bounds(cu_seqlens, bounds, q.device), bits[:, :n].contiguous() if n < T else bits, int(topk), float(scale))
-        return o if n == T else torch.cat((o, q.new_zeros(T - n, Hq, D)), 0)
+        on_device = _device_bounds(cu_seqlens, bounds, q.device)
+        if n == T:   # a slice of everything would still cost a zero fill and a copy per gradient
+            return _MaskedAttention.apply(q, k, v, on_device, bits, int(topk), float(scale))
+        o = _MaskedAttention.apply(q[:n], k[:n], v[:n], on_device, bits[:, :n].contiguous(), int(topk), float(scale))
+        return torch.cat((o, q.new_zeros(T - n, Hq, D)), 0)
     # documents end where the packed row ends: tokens behind the last boundary are padding
     outs = []
     for s, e in zip(bounds[:-1], bounds[1:]):
