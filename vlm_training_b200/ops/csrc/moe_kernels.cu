@@ -261,7 +261,10 @@ __global__ void moe_rows_from_tokens_kernel(const bf16* __restrict__ src, const 
 }
 
 // out[t, :] = sum_j (w ? w[t*k+j] : 1) * rows[dest[t*k+j], :]   (fp32 accumulation, slot order); optionally also
-// dw[t*k+j] = <g[t, :], rows[dest[t*k+j], :]>  (the routing-weight gradient, when g is given).  One warp per token.
+// dw[t*k+j] = <g[t, :], rows[dest[t*k+j], :]>  (the routing-weight gradient, when g is given).  One warp per token, U of its rows
+// in flight together: one row after the other left the memory idle (8192 tokens, 8 rows of 2048 each: 79 -> 57 us; dw, four pieces of a row and of g,
+// 81 -> 68).  With up to 4 rows per token the registers would cost more warps than that gains (2 rows of 1024: U = 8 13.2 us, U = 2 9.9, one after the other 9.6).
+template <int U>
 __global__ void moe_tokens_from_rows_kernel(const bf16* __restrict__ rows, const int* __restrict__ dest, const float* __restrict__ w,
                                             int T, int k, int H, bf16* __restrict__ out, const bf16* __restrict__ g,
                                             float* __restrict__ dw) {
@@ -269,19 +272,29 @@ __global__ void moe_tokens_from_rows_kernel(const bf16* __restrict__ rows, const
   const int t = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (t >= T) return;
   const int nvec = H >> 3;
-  for (int c0 = 0; c0 < nvec; c0 += 32) {
-    const int c = c0 + lane;
-    float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-    if (c < nvec && out != nullptr) {
-      for (int j = 0; j < k; ++j) {
-        const float wj = w ? w[(size_t)t * k + j] : 1.f;
-        const uint4 v = reinterpret_cast<const uint4*>(rows + (size_t)dest[(size_t)t * k + j] * H)[c];
-        const __nv_bfloat162* p = reinterpret_cast<const __nv_bfloat162*>(&v);
+  constexpr int P = 4;
+  if (out != nullptr) {
+    for (int c = lane; c < nvec; c += 32) {
+      float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+      for (int j0 = 0; j0 < k; j0 += U) {
+        uint4 v[U];
+        float wj[U];
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const float2 f = __bfloat1622float2(p[i]);
-          acc[2 * i] += wj * f.x;
-          acc[2 * i + 1] += wj * f.y;
+        for (int u = 0; u < U; ++u) {
+          if (j0 + u >= k) break;
+          v[u] = reinterpret_cast<const uint4*>(rows + (size_t)dest[(size_t)t * k + j0 + u] * H)[c];
+          wj[u] = w ? w[(size_t)t * k + j0 + u] : 1.f;
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+          if (j0 + u >= k) break;
+          const __nv_bfloat162* p = reinterpret_cast<const __nv_bfloat162*>(&v[u]);
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            const float2 f = __bfloat1622float2(p[i]);
+            acc[2 * i] += wj[u] * f.x;
+            acc[2 * i + 1] += wj[u] * f.y;
+          }
         }
       }
       uint4 o;
@@ -292,17 +305,28 @@ __global__ void moe_tokens_from_rows_kernel(const bf16* __restrict__ rows, const
     }
   }
   if (g != nullptr && dw != nullptr) {
+    const uint4* gt = reinterpret_cast<const uint4*>(g + (size_t)t * H);
     for (int j = 0; j < k; ++j) {
-      const bf16* r = rows + (size_t)dest[(size_t)t * k + j] * H;
+      const uint4* r = reinterpret_cast<const uint4*>(rows + (size_t)dest[(size_t)t * k + j] * H);
       float dot = 0.f;
-      for (int c = lane; c < nvec; c += 32) {
-        const uint4 a = reinterpret_cast<const uint4*>(g + (size_t)t * H)[c], b = reinterpret_cast<const uint4*>(r)[c];
-        const __nv_bfloat162* pa = reinterpret_cast<const __nv_bfloat162*>(&a);
-        const __nv_bfloat162* pb = reinterpret_cast<const __nv_bfloat162*>(&b);
+      for (int c0 = lane; c0 < nvec; c0 += 32 * P) {
+        uint4 a[P], b[P];
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const float2 fa = __bfloat1622float2(pa[i]), fb = __bfloat1622float2(pb[i]);
-          dot += fa.x * fb.x + fa.y * fb.y;
+        for (int u = 0; u < P; ++u) {
+          if (c0 + 32 * u >= nvec) break;
+          a[u] = gt[c0 + 32 * u];
+          b[u] = r[c0 + 32 * u];
+        }
+#pragma unroll
+        for (int u = 0; u < P; ++u) {
+          if (c0 + 32 * u >= nvec) break;
+          const __nv_bfloat162* pa = reinterpret_cast<const __nv_bfloat162*>(&a[u]);
+          const __nv_bfloat162* pb = reinterpret_cast<const __nv_bfloat162*>(&b[u]);
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            const float2 fa = __bfloat1622float2(pa[i]), fb = __bfloat1622float2(pb[i]);
+            dot += fa.x * fb.x + fa.y * fb.y;
+          }
         }
       }
       dot = warp_sum(dot);
@@ -491,7 +515,7 @@ int vlmt_moe_tokens_from_rows(const void* rows, const int* dest, const float* w,
                               cudaStream_t st) {
   if (H & 7) return -1;
   if (T <= 0) return 0;
-  launch_pdl(moe_tokens_from_rows_kernel, dim3((T + 7) / 8), dim3(256), 0, st, 1, (const bf16*)rows, dest, w, T, k, H, (bf16*)out, (const bf16*)g, dw);
+  launch_pdl(k > 4 && out != nullptr ? moe_tokens_from_rows_kernel<8> : moe_tokens_from_rows_kernel<2>, dim3((T + 7) / 8), dim3(256), 0, st, 1, (const bf16*)rows, dest, w, T, k, H, (bf16*)out, (const bf16*)g, dw);
   return (int)cudaGetLastError();
 }
 
