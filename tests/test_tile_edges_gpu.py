@@ -54,6 +54,17 @@ def test_gemm_split_over_k(M, N, K, layout):
     cu.check_status()
 
 
+# column sums: one cluster per 64 columns up to 2048 rows (a last block with fewer rows or none), slabs of 256 rows behind
+@pytest.mark.parametrize("rows", [1, 256, 257, 513, 1793, 2048, 2049])
+@pytest.mark.parametrize("cols", [8, 64, 72, 1160])
+def test_column_sums(rows, cols):
+    from vlm_training_b200.ops import cuda as cu
+
+    x = _rand(rows, cols + 8)[:, :cols]
+    # fp32 sums of up to 2049 values of size 1: a few roundings of 2^-24 of partial sums up to about 100
+    torch.testing.assert_close(cu._C.colsum(x).double(), x.double().sum(0), atol=1e-4, rtol=1e-6)
+
+
 # at most 128 rows: every width of the row tile at its edges, a feature tile that ends early, a short last block and part of K, activations, rows and
 # columns behind the last ones, an output whose rows start anywhere
 @pytest.mark.parametrize("M", [1, 16, 17, 48, 49, 64, 65, 96, 97, 128])

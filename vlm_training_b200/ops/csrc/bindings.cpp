@@ -513,8 +513,11 @@ void colsum_into(const Tensor& x, void* out, int mode) {
                   reinterpret_cast<uintptr_t>(x.data_ptr()) % 16 == 0, "colsum: bf16 [rows, cols], cols and row stride multiples of 8");
   c10::cuda::CUDAGuard guard(x.device());
   const int rows = x.size(0), cols = x.size(1);
-  Tensor partial = torch::empty({vlmt_colsum_slabs(rows), cols}, x.options().dtype(torch::kFloat));
-  vlmt_colsum(x.data_ptr(), x.stride(0), rows, cols, partial.data_ptr<float>(), out, mode, cur_stream());
+  const int slabs = vlmt_colsum_slabs(rows);
+  Tensor partial;
+  if (slabs > 0) partial = torch::empty({slabs, cols}, x.options().dtype(torch::kFloat));
+  const int r = vlmt_colsum(x.data_ptr(), x.stride(0), rows, cols, slabs > 0 ? partial.data_ptr<float>() : nullptr, out, mode, cur_stream());
+  TORCH_CHECK(r == 0, "vlmt_colsum failed with code ", r);
 }
 Tensor colsum(const Tensor& x) {
   Tensor out = torch::empty({x.size(1)}, x.options().dtype(torch::kFloat));
