@@ -221,7 +221,7 @@ Tensor sum_partials(const Tensor& partial) {
   return out;
 }
 std::vector<Tensor> rmsnorm_bwd_partial(const Tensor& dy, const Tensor& x, const Tensor& w, const Tensor& rstd, const c10::optional<Tensor>& dres,
-                                bool offset) {
+                                bool offset, Tensor* yn) {
   check_bf16(dy, "dy"); check_contig(dy, "dy"); check_contig(x, "x");
   c10::cuda::CUDAGuard guard(x.device());
   const int D = x.size(-1);
@@ -231,7 +231,8 @@ std::vector<Tensor> rmsnorm_bwd_partial(const Tensor& dy, const Tensor& x, const
   Tensor partial = torch::empty({blocks, D}, x.options().dtype(torch::kFloat));
   if (dres.has_value()) check_contig(*dres, "dres");
   vlmt_rmsnorm_bwd(dy.data_ptr(), x.data_ptr(), w.data_ptr(), w.scalar_type() == at::kFloat, rstd.data_ptr<float>(), optptr(dres),
-                   dx.data_ptr(), partial.data_ptr<float>(), rows, D, offset, cur_stream());
+                   dx.data_ptr(), yn != nullptr && vlmt_norm_rewrites(D) ? (*yn = dy).data_ptr() : nullptr, partial.data_ptr<float>(), rows, D, offset,
+                   cur_stream());
   return {dx, partial};
 }
 std::vector<Tensor> rmsnorm_bwd(const Tensor& dy, const Tensor& x, const Tensor& w, const Tensor& rstd, const c10::optional<Tensor>& dres,
@@ -251,7 +252,8 @@ std::vector<Tensor> layernorm_fwd(const Tensor& x, const Tensor& w, const c10::o
                      (float)eps, cur_stream());
   return {y, mean, rstd};
 }
-std::vector<Tensor> layernorm_bwd_partial(const Tensor& dy, const Tensor& x, const Tensor& w, const Tensor& mean, const Tensor& rstd) {
+std::vector<Tensor> layernorm_bwd_partial(const Tensor& dy, const Tensor& x, const Tensor& w, const Tensor& mean, const Tensor& rstd,
+                                          const c10::optional<Tensor>& b, Tensor* yn) {
   check_contig(dy, "dy"); check_contig(x, "x");
   c10::cuda::CUDAGuard guard(x.device());
   const int D = x.size(-1);
@@ -259,8 +261,8 @@ std::vector<Tensor> layernorm_bwd_partial(const Tensor& dy, const Tensor& x, con
   Tensor dx = torch::empty_like(x);
   const int blocks = vlmt_norm_blocks(rows);
   Tensor pw = torch::empty({blocks, D}, x.options().dtype(torch::kFloat)), pb = torch::empty_like(pw);
-  vlmt_layernorm_bwd(dy.data_ptr(), x.data_ptr(), w.data_ptr(), mean.data_ptr<float>(), rstd.data_ptr<float>(), dx.data_ptr(),
-                     pw.data_ptr<float>(), pb.data_ptr<float>(), rows, D, cur_stream());
+  vlmt_layernorm_bwd(dy.data_ptr(), x.data_ptr(), w.data_ptr(), optptr(b), mean.data_ptr<float>(), rstd.data_ptr<float>(), dx.data_ptr(),
+                     yn != nullptr && vlmt_norm_rewrites(D) ? (*yn = dy).data_ptr() : nullptr, pw.data_ptr<float>(), pb.data_ptr<float>(), rows, D, cur_stream());
   return {dx, pw, pb};
 }
 std::vector<Tensor> layernorm_bwd(const Tensor& dy, const Tensor& x, const Tensor& w, const Tensor& mean, const Tensor& rstd) {

@@ -101,10 +101,9 @@ Tensor mm(const Tensor& a, const Tensor& b, bool a_mn, bool b_mn, const Tensor& 
   tick(1);
   return out;
 }
-// dW[N, K] = dY^T[N, M] . X[M, K].  A parameter is reported only when every kernel of the backward pass that reads it has been
-// enqueued: its bucket's update may run on another stream, or in a peer's kernel, from that moment on.
-Tensor weight_grad(const Tensor& dy, const Tensor& x, const Target& t, bool& report) {
-  report = false;
+// dW[N, K] = dY^T[N, M] . X[M, K], called when every other kernel of the backward pass that reads the weight has been enqueued: a tagged parameter is
+// reported here, and its bucket's update may run on another stream, or in a peer's kernel, from that moment on.
+Tensor weight_grad(const Tensor& dy, const Tensor& x, const Target& t) {
   if (may_add(t)) {
     Tensor g = t->param.grad();
     if (g.defined() && g.scalar_type() == at::kBFloat16 && g.dim() == 2 && g.size(0) == dy.size(1) && g.size(1) == x.size(1) &&
@@ -112,18 +111,11 @@ Tensor weight_grad(const Tensor& dy, const Tensor& x, const Target& t, bool& rep
       check_storage(g);
       gemm(dy, x, g, true, true, c10::nullopt, 0, true, c10::nullopt);
       tick(1);
-      report = true;
+      t->report();
       return Tensor();
     }
   }
   return mm(dy, x, true, true);
-}
-// for a function whose last read of the weight has been enqueued
-Tensor weight_grad(const Tensor& dy, const Tensor& x, const Target& t) {
-  bool report;
-  Tensor dw = weight_grad(dy, x, t, report);
-  if (report) t->report();
-  return dw;
 }
 // where the gradient of a 1-D parameter goes: added to a tagged .grad, or a new tensor of the parameter's type
 struct VecGrad {
@@ -248,8 +240,8 @@ Tensor op_linear(const Tensor& x, const py::object& w_, const py::object& b_) {
 }
 
 // ------------------------------------------------------------------ norm / activation + linear
-// (x [+ residual]) -> RMSNorm -> linear, keeping the un-normalised stream and rstd; the normalised rows are recomputed in
-// backward.  Second output: x + residual.
+// (x [+ residual]) -> RMSNorm -> linear, keeping the un-normalised stream and rstd; the normalised rows are made again by the
+// norm's backward kernel.  Second output: x + residual.
 struct NormLinear : torch::autograd::Function<NormLinear> {
   static variable_list forward(AutogradContext* ctx, const Tensor& x, const OptTensor& res_, const Tensor& nw, const Tensor& w, CfgPtr c) {
     const Tensor res = get(res_);
@@ -272,13 +264,16 @@ struct NormLinear : torch::autograd::Function<NormLinear> {
     if (!grads[0].defined()) {   // only the residual stream was used
       dx = dr;
     } else {
-      Tensor dy = rows_of(grads[0]);
-      bool report = false;   // the weight is read once more, by d(normalised rows)
-      if (c->need[3]) dw = weight_grad(dy, rmsnorm_fwd(r, c10::nullopt, nw, c->eps, c->offset)[0], c->t[1], report);
-      auto b = rmsnorm_bwd_partial(mm(dy, w, false, true), r, nw, rstd, dr.defined() ? OptTensor(dr.contiguous()) : OptTensor(), c->offset);
+      Tensor dy = rows_of(grads[0]), yn;
+      auto b = rmsnorm_bwd_partial(mm(dy, w, false, true), r, nw, rstd, dr.defined() ? OptTensor(dr.contiguous()) : OptTensor(), c->offset,
+                                   c->need[3] ? &yn : nullptr);
       dx = b[0];
-      tick(2);
-      if (report) c->t[1]->report();
+      tick(1);
+      if (c->need[3]) {
+        if (!yn.defined()) { yn = rmsnorm_fwd(r, c10::nullopt, nw, c->eps, c->offset)[0]; tick(1); }
+        dw = weight_grad(dy, yn, c->t[1]);
+        yn.reset();
+      }
       if (c->need[2]) {
         VecGrad g(nw, c->t[0]);
         sum_rows(b[1].data_ptr<float>(), nullptr, b[1].size(1), b[1].size(0), b[1].size(1), g, nullptr);
@@ -305,7 +300,7 @@ py::object op_norm_linear(const Tensor& x, const py::object& res_, const py::obj
   });
 }
 
-// LayerNorm -> linear, the normalised rows recomputed in backward
+// LayerNorm -> linear, the normalised rows made again by the norm's backward kernel
 struct LnLinear : torch::autograd::Function<LnLinear> {
   static Tensor forward(AutogradContext* ctx, const Tensor& x, const Tensor& lw, const OptTensor& lb_, const Tensor& w, const OptTensor& b_, CfgPtr c) {
     const Tensor lb = get(lb_), b = get(b_);
@@ -327,12 +322,14 @@ struct LnLinear : torch::autograd::Function<LnLinear> {
     auto c = kept(ctx);
     const Tensor &x = saved[0], &lw = saved[1], &mean = saved[2], &rstd = saved[3], &w = saved[4];
     Tensor lb = c->n_q ? saved[5] : Tensor(), b = c->n_kv ? saved[5 + c->n_q] : Tensor();
-    Tensor dy = rows_of(grads[0]), dlw, dlb, dw, db;
-    bool report = false;   // the weight is read once more, by d(normalised rows)
-    if (c->need[3]) dw = weight_grad(dy, layernorm_fwd(x, lw, opt(lb), c->eps)[0], c->t[2], report);
-    auto r = layernorm_bwd_partial(mm(dy, w, false, true), x, lw, mean, rstd);
-    tick(2);
-    if (report) c->t[2]->report();
+    Tensor dy = rows_of(grads[0]), yn, dlw, dlb, dw, db;
+    auto r = layernorm_bwd_partial(mm(dy, w, false, true), x, lw, mean, rstd, opt(lb), c->need[3] ? &yn : nullptr);
+    tick(1);
+    if (c->need[3]) {
+      if (!yn.defined()) { yn = layernorm_fwd(x, lw, opt(lb), c->eps)[0]; tick(1); }
+      dw = weight_grad(dy, yn, c->t[2]);
+      yn.reset();
+    }
     if (c->need[1] || c->need[2]) {
       VecGrad gw(lw, c->need[1] ? c->t[0] : Target());
       const int rows = r[1].size(0), cols = r[1].size(1);

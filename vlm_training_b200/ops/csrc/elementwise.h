@@ -7,9 +7,11 @@ extern "C" {
 #endif
 int vlmt_norm_blocks(int rows);
 void vlmt_rmsnorm_fwd(const void* x, const void* res, const void* w, int w_fp32, void* y, void* r_out, float* rstd, int rows, int D, float eps, int offset, cudaStream_t st);
-int vlmt_rmsnorm_bwd(const void* dy, const void* x, const void* w, int w_fp32, const float* rstd, const void* dres, void* dx, float* dw_partial, int rows, int D, int offset, cudaStream_t st);
+// yn (null, a buffer, or dy, which they then replace): the normalised rows, only where vlmt_norm_rewrites(D)
+int vlmt_norm_rewrites(int D);
+int vlmt_rmsnorm_bwd(const void* dy, const void* x, const void* w, int w_fp32, const float* rstd, const void* dres, void* dx, void* yn, float* dw_partial, int rows, int D, int offset, cudaStream_t st);
 void vlmt_layernorm_fwd(const void* x, const void* w, const void* b, void* y, float* mean, float* rstd, int rows, int D, float eps, cudaStream_t st);
-int vlmt_layernorm_bwd(const void* dy, const void* x, const void* w, const float* mean, const float* rstd, void* dx, float* dw_partial, float* db_partial, int rows, int D, cudaStream_t st);
+int vlmt_layernorm_bwd(const void* dy, const void* x, const void* w, const void* b, const float* mean, const float* rstd, void* dx, void* yn, float* dw_partial, float* db_partial, int rows, int D, cudaStream_t st);
 void vlmt_rmsnorm_gated_fwd(const void* x, const void* z, const void* w, void* y, float* rstd, int rows, int D, float eps, cudaStream_t st);
 int vlmt_rmsnorm_gated_bwd(const void* dy, const void* x, const void* z, const void* w, const float* rstd, void* dx, void* dz, float* dw_partial, int rows, int D, cudaStream_t st);
 void vlmt_swiglu_fwd(const void* gu, void* out, long rows, int I, cudaStream_t st);

@@ -14,9 +14,11 @@ void gemm(const Tensor& a, const Tensor& b, Tensor& out, bool a_mn, bool b_mn, c
           const OptTensor& alpha, bool one_sum = false);   // one_sum: see vlmt_gemm_bf16
 std::vector<Tensor> rmsnorm_fwd(const Tensor& x, const OptTensor& res, const Tensor& w, double eps, bool offset);
 // *_partial: the weight gradients as per-block partial rows, to be summed by vlmt_sum_rows
-std::vector<Tensor> rmsnorm_bwd_partial(const Tensor& dy, const Tensor& x, const Tensor& w, const Tensor& rstd, const OptTensor& dres, bool offset);
+std::vector<Tensor> rmsnorm_bwd_partial(const Tensor& dy, const Tensor& x, const Tensor& w, const Tensor& rstd, const OptTensor& dres, bool offset,
+                                        Tensor* yn = nullptr);   // yn: rmsnorm_fwd(x) from the same pass, in the place of dy; left alone where the kernel has no such form
 std::vector<Tensor> layernorm_fwd(const Tensor& x, const Tensor& w, const OptTensor& b, double eps);
-std::vector<Tensor> layernorm_bwd_partial(const Tensor& dy, const Tensor& x, const Tensor& w, const Tensor& mean, const Tensor& rstd);
+std::vector<Tensor> layernorm_bwd_partial(const Tensor& dy, const Tensor& x, const Tensor& w, const Tensor& mean, const Tensor& rstd,
+                                          const OptTensor& b = c10::nullopt, Tensor* yn = nullptr);   // yn: layernorm_fwd(x) with bias b, as above
 std::vector<Tensor> rmsnorm_gated_fwd(const Tensor& x, const Tensor& z, const Tensor& w, double eps);
 std::vector<Tensor> rmsnorm_gated_bwd_partial(const Tensor& dy, const Tensor& x, const Tensor& z, const Tensor& w, const Tensor& rstd);
 Tensor swiglu_fwd(const Tensor& gu);
