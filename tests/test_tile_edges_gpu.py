@@ -515,3 +515,59 @@ def test_rope_tables_and_position_embedding_outside_the_kernels_forms():
     assert torch.equal(ops.pos_embed_add(x, table, plan, 2), ops.pos_embed_add(x, table, dataclasses.replace(plan, images=None), 2))
     with pytest.raises(ValueError):   # no patches: refused as on the host
         VisionPlan.build([[1, 0, 0]], VisionConfig(hidden_size=64, num_heads=2, num_position_embeddings=16), DEV)
+
+
+# whole blocks as one call of the extension against the same block run module by module (a hook on a module that the block calls forces it): the same
+# bits in outputs and gradients, with and without a graph; weights that take another path, and hooks, keep their say
+@pytest.mark.parametrize("preset,layer", [("tiny-qwen3-vl-gpu", 0), ("qwen3.5-dense", 3)])
+@pytest.mark.parametrize("block", ["decoder", "vision", "merger"])
+def test_blocks_in_one_call(preset, layer, block):
+    from vlm_training_b200.models import BatchPlan, ModelConfig
+    from vlm_training_b200.models.causal_lm import rotary_inv_freq, rotary_tables
+    from vlm_training_b200.models.layers import DecoderLayer, RowContext
+    from vlm_training_b200.models.vision import PatchMerger, VisionBlock, VisionPlan
+
+    cfg = ModelConfig.preset(preset)
+    if block != "decoder" and preset != "tiny-qwen3-vl-gpu":
+        pytest.skip("the vision tower of one preset is enough")
+    if block == "decoder":
+        cfg.text.hidden_size, cfg.text.intermediate_size = 512, 768
+        m, hooked = DecoderLayer(cfg.text, layer), "self_attn.o_proj"
+        bounds = [0, 100, 333]
+        plan = BatchPlan.build(cfg, torch.zeros(333, dtype=torch.int64).numpy(), torch.tensor(bounds, dtype=torch.int32), None, DEV)
+        ctx = RowContext(plan.cu_seqlens, plan.max_seqlen, *rotary_tables(cfg.text, plan.position_ids, rotary_inv_freq(cfg.text, torch.device(DEV)), torch.float32),
+                         plan.seq_idx, plan.extras)
+        x, args = _rand(333, 512), (ctx,)
+    else:
+        plan = VisionPlan.build([[1, 6, 10], [1, 4, 4]], cfg.vision, torch.device(DEV))
+        m, hooked, args = (VisionBlock(cfg.vision), "attn.proj", (plan,)) if block == "vision" else (PatchMerger(cfg.vision, layer == 0), "", ())
+        x = _rand(76, cfg.vision.hidden_size)
+    m = m.to(DEV, torch.bfloat16)
+    with torch.no_grad():
+        for p in m.parameters():
+            p.copy_(_rand(*p.shape, scale=0.05) + (1.0 if p.dim() == 1 else 0.0))
+
+    def run(grad):
+        with torch.set_grad_enabled(grad):
+            xi = x.clone().requires_grad_(grad)
+            y = m(xi, *args)
+            if not grad:
+                return [y]
+            g = torch.autograd.grad(y, [xi, *m.parameters()], torch.ones_like(y))
+            return [y.detach(), *g]
+
+    one = run(True), run(False)
+    calls = []
+    target = m.get_submodule(hooked)
+    if block == "merger":
+        handle = None
+        m.linear_fc1.weight._vlmt_resharded = True   # a weight that is gathered by the module that reads it
+    else:
+        handle = target.register_forward_hook(lambda *_: calls.append(1))
+    apart = run(True), run(False)
+    assert block == "merger" or len(calls) == 2
+    for a, b in zip(one, apart):
+        for s, t in zip(a, b):
+            assert torch.equal(s, t)
+    if handle is not None:
+        handle.remove()

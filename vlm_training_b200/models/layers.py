@@ -334,7 +334,31 @@ class DecoderLayer(nn.Module):
         return x + self.mlp(h)
 
     def forward(self, x, ctx: RowContext):
+        if type(self) is DecoderLayer and x.is_cuda:
+            out = self._in_one_call(x, ctx)
+            if out is not None:
+                return out
         return self.mlp_half(self.mixer_half(x, ctx), x)
+
+    def _in_one_call(self, x, ctx: RowContext):
+        """The whole layer as one call of the extension where it is dense, unsharded attention + SwiGLU; else ``None``."""
+        parts = self._modules
+        attn, mlp = parts.get("self_attn"), parts["mlp"]
+        if type(attn) is not SelfAttention or type(mlp) is not SwiGLUMLP:
+            return None
+        qkv, o_proj, q_norm, k_norm = (attn._modules[n] for n in ("qkv", "o_proj", "q_norm", "k_norm"))
+        gate_up, down = mlp._modules["gate_up"], mlp._modules["down_proj"]
+        cfg = attn.cfg
+        if (cfg.dsa or qkv.tp.enabled or o_proj.tp.enabled or gate_up.tp.enabled or down.tp.enabled or type(o_proj) is not Linear
+                or any(m.bias is not None for m in (qkv, o_proj, gate_up, down))):
+            return None
+        ext = ops.whole_blocks(x, attn, o_proj)
+        if ext is None:
+            return None
+        n1, n2 = parts["input_layernorm"], parts["post_attention_layernorm"]
+        w = tuple(m._parameters["weight"] for m in (n1, qkv, q_norm, k_norm, o_proj, n2, gate_up, down))
+        return ext.op_decoder_layer(x, w, ctx.cos, ctx.sin, ctx.cu_seqlens, int(ctx.max_seqlen), attn.n_q, attn.n_kv, attn.head_dim, n1.eps, n2.eps,
+                                    cfg.rms_norm_eps, n1.offset, n2.offset, cfg.offset_norm, attn.gated, float(attn.scale))
 
     def forward_sac(self, x, ctx: RowContext):
         """Selective activation checkpointing: the mixer half runs under plain autograd, so what its ops saved (the

@@ -135,8 +135,28 @@ class VisionBlock(nn.Module):
         self.mlp = VisionMLP(cfg)
 
     def forward(self, x, plan: VisionPlan):
+        if type(self) is VisionBlock and x.is_cuda:
+            out = self._in_one_call(x, plan)
+            if out is not None:
+                return out
         x = x + self.attn(x, plan, prenorm=self.norm1)
         return x + self.mlp(x, prenorm=self.norm2)
+
+    def _in_one_call(self, x, plan: VisionPlan):
+        """The whole block as one call of the extension, or ``None`` where its modules have to run one by one."""
+        parts = self._modules
+        attn, mlp, n1, n2 = parts["attn"], parts["mlp"], parts["norm1"], parts["norm2"]
+        if type(attn) is not VisionAttention or type(mlp) is not VisionMLP:
+            return None
+        qkv, proj, fc1, fc2 = attn._modules["qkv"], attn._modules["proj"], mlp._modules["linear_fc1"], mlp._modules["linear_fc2"]
+        if any(type(m) is not Linear or m.parallel is not None for m in (qkv, proj, fc1, fc2)):
+            return None
+        ext = ops.whole_blocks(x, attn, proj, mlp)
+        if ext is None:
+            return None
+        w = tuple(m._parameters.get(n) for m in (n1, qkv, proj, n2, fc1, fc2) for n in ("weight", "bias"))
+        return ext.op_vision_block(x, w, plan.cos, plan.sin, plan.cu_seqlens, int(plan.max_seqlen), attn.n_heads, attn.head_dim, n1.eps, n2.eps,
+                                   attn.head_dim ** -0.5, mlp.approx == "tanh")
 
 
 class PatchMerger(nn.Module):
@@ -153,6 +173,13 @@ class PatchMerger(nn.Module):
         self.linear_fc2 = Linear(self.merged, cfg.out_hidden_size, bias=True)
 
     def forward(self, x):
+        ext = ops.whole_blocks(x) if type(self) is PatchMerger else None
+        if ext is not None:
+            parts = self._modules
+            w = tuple(parts[m]._parameters.get(n) for m in ("norm", "linear_fc1", "linear_fc2") for n in ("weight", "bias"))
+            out = ext.op_patch_merger(x, w, self.merged, self.postshuffle, parts["norm"].eps)
+            if out is not None:
+                return out
         if self.postshuffle:
             x = ops.layer_norm(x.view(-1, self.merged), self.norm.weight, self.norm.bias, self.norm.eps)
         else:

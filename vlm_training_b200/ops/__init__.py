@@ -15,6 +15,7 @@ from __future__ import annotations
 import os
 
 import torch
+from torch.nn.modules.module import _has_any_global_hook as _any_global_hook
 
 from . import reference as ref
 
@@ -35,6 +36,18 @@ def _cu():
 
         _CUDA_MODULE = cuda
     return _CUDA_MODULE
+
+
+def whole_blocks(x, *modules):
+    """The binding calls that run a whole block (``op_decoder_layer``, ``op_vision_block``, ``op_patch_merger``), or ``None`` where the modules have
+    to run one by one: other devices, the library GEMM, and ``modules`` (those that the block calls) with hooks or a forward of their own."""
+    if not _use_cuda(x) or _cu()._GEMM_BACKEND == "cublas" or _any_global_hook():
+        return None
+    for m in modules:
+        d = m.__dict__
+        if d["_forward_pre_hooks"] or d["_forward_hooks"] or d["_backward_hooks"] or d["_backward_pre_hooks"] or "forward" in d:
+            return None
+    return _CUDA_MODULE._C
 
 
 # --- norms -------------------------------------------------------------------

@@ -478,7 +478,7 @@ class ShardedOptimizerEngine(torch.optim.Optimizer):
             if fuse_first_gemm and symmetric_shards and tp_size == 1:
                 self._pick_fused_weights()
             self._install_unit_hooks()
-        if self.is_cuda:
+        if self.is_cuda and (self.reshard or any(d.shard and d.size > 1 for d in self.domains)):   # else nothing is ever gathered
             self._install_forward_waits()
         if self.is_cuda and pdtype == torch.bfloat16:
             self._build_adamw_tables()
