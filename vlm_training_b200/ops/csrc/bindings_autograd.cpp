@@ -719,6 +719,48 @@ Tensor op_attention(const Tensor& q, const Tensor& k, const Tensor& v, const Ten
   });
 }
 
+// Bidirectional attention over a fused projection [S, 3 H D]: rotary on q and k, v read in place, and one gradient for the whole projection
+// instead of three that autograd would put together.
+struct RopeAttention : torch::autograd::Function<RopeAttention> {
+  static std::vector<Tensor> run(const Tensor& x, const Tensor& cosv, const Tensor& sinv, const Tensor& cu, const CfgPtr& c) {
+    c10::cuda::CUDAGuard guard(x.device());
+    const int64_t S = x.size(0), H = c->n_q, D = c->D;
+    Tensor q = torch::empty({S, H, D}, x.options()), k = torch::empty_like(q);
+    vlmt_rope_qkv_fwd(x.data_ptr(), x.stride(0), cosv.data_ptr<float>(), sinv.data_ptr<float>(), q.data_ptr(), k.data_ptr(), (int)S, (int)H, (int)D,
+                      cur_stream());
+    auto r = attn_fwd(q, k, x.view({S, 3, H, D}).select(1, 2), cu, c->max_seqlen, false, c->scale);
+    tick(2);
+    return {q, k, r[0], r[1]};
+  }
+  static Tensor forward(AutogradContext* ctx, const Tensor& qkv, const Tensor& cosv, const Tensor& sinv, const Tensor& cu, CfgPtr c) {
+    Tensor x = qkv.contiguous();
+    auto r = run(x, cosv, sinv, cu, c);
+    keep(ctx, c);
+    ctx->save_for_backward({x, cosv, sinv, cu, r[0], r[1], r[2], r[3]});
+    return r[2];
+  }
+  static variable_list backward(AutogradContext* ctx, variable_list grads) {
+    auto s = ctx->get_saved_variables();
+    auto c = kept(ctx);
+    const int64_t S = s[0].size(0), H = c->n_q, D = c->D;
+    auto r = attn_bwd(grads[0].contiguous(), s[4], s[5], s[0].view({S, 3, H, D}).select(1, 2), s[6], s[7], s[3], c->max_seqlen, false, c->scale);
+    c10::cuda::CUDAGuard guard(s[0].device());
+    Tensor dqkv = torch::empty_like(s[0]);
+    vlmt_rope_qkv_bwd(r[0].data_ptr(), r[1].data_ptr(), r[2].data_ptr(), s[1].data_ptr<float>(), s[2].data_ptr<float>(), dqkv.data_ptr(), (int)S, (int)H,
+                      (int)D, cur_stream());
+    tick(4);
+    return {dqkv, Tensor(), Tensor(), Tensor(), Tensor()};
+  }
+};
+Tensor rope_attention(const Tensor& qkv, const Tensor& cosv, const Tensor& sinv, const Tensor& cu, int64_t max_seqlen, int64_t H, int64_t D, double scale) {
+  return guarded([&] {
+    auto c = c10::make_intrusive<Cfg>();
+    c->max_seqlen = max_seqlen; c->scale = scale; c->n_q = H; c->D = D;
+    if (no_graph(qkv, cosv, sinv)) return RopeAttention::run(qkv.contiguous(), cosv, sinv, cu, c)[2];
+    return RopeAttention::apply(qkv, cosv, sinv, cu, c);
+  });
+}
+
 // ------------------------------------------------------------------ rows of a packed sequence
 struct RowsUpdate : torch::autograd::Function<RowsUpdate> {
   static Tensor forward(AutogradContext* ctx, const Tensor& x, const Tensor& index, const Tensor& src, bool add) {
@@ -830,7 +872,7 @@ bool plain_vector(const py::object& w, int64_t n, bool optional = false) {
   return t.is_cuda() && t.scalar_type() == at::kBFloat16 && t.dim() == 1 && t.size(0) == n;
 }
 bool plain_rows(const Tensor& x) { return x.is_cuda() && x.scalar_type() == at::kBFloat16 && x.dim() == 2 && x.size(0) > 0 && x.size(1) % 8 == 0; }
-bool plain_table(const Tensor& t) { return t.scalar_type() == at::kFloat && t.is_contiguous(); }
+bool plain_table(const Tensor& t) { return t.is_cuda() && t.scalar_type() == at::kFloat && t.is_contiguous() && reinterpret_cast<uintptr_t>(t.data_ptr()) % 16 == 0; }
 bool plain_heads(int64_t D) { return D == 256 || (D <= 128 && D % 8 == 0); }
 
 py::object op_decoder_layer(const Tensor& x, const py::tuple& w, const Tensor& cosv, const Tensor& sinv, const Tensor& cu, int64_t max_seqlen, int64_t n_q,
@@ -866,7 +908,8 @@ py::object op_decoder_layer(const Tensor& x, const py::tuple& w, const Tensor& c
 py::object op_vision_block(const Tensor& x, const py::tuple& w, const Tensor& cosv, const Tensor& sinv, const Tensor& cu, int64_t max_seqlen, int64_t heads,
                            int64_t D, double eps1, double eps2, double scale, bool tanh_approx) {
   const int64_t H = plain_rows(x) ? x.size(1) : 0;
-  if (H == 0 || H != heads * D || !plain_heads(D) || D > 128 || !plain_table(cosv) || !plain_table(sinv) || cu.scalar_type() != at::kInt ||
+  if (H == 0 || H != heads * D || D > 128 || !vlmt_rope_qkv_usable((int)D) || cosv.sizes() != sinv.sizes() || cosv.dim() != 2 || cosv.size(0) != x.size(0) ||
+      cosv.size(1) != D || cosv.requires_grad() || sinv.requires_grad() || !plain_table(cosv) || !plain_table(sinv) || cu.scalar_type() != at::kInt ||
       !plain_vector(w[0], H) || !plain_vector(w[1], H, true) || !plain_weight(w[2], H) || !plain_vector(w[3], 3 * H, true) || !plain_weight(w[4], H) ||
       !plain_vector(w[5], H, true) || !plain_vector(w[6], H) || !plain_vector(w[7], H, true) || !plain_weight(w[8], H))
     return py::none();
@@ -874,11 +917,8 @@ py::object op_vision_block(const Tensor& x, const py::tuple& w, const Tensor& co
   if (!plain_vector(w[9], inter, true) || !plain_weight(w[10], inter) || !plain_vector(w[11], H, true)) return py::none();
   const int64_t S = x.size(0);
   Tensor qkv = op_ln_linear(x, w[0], w[1], w[2], w[3], eps1);
-  auto parts = guarded([&] { return qkv.view({S, 3, heads, D}).unbind(1); });
+  Tensor o = rope_attention(qkv, cosv, sinv, cu, max_seqlen, heads, D, scale);
   qkv.reset();
-  Tensor q = op_rope(parts[0], cosv, sinv, D), k = op_rope(parts[1], cosv, sinv, D);
-  Tensor o = op_attention(q, k, parts[2], cu, max_seqlen, false, scale);
-  q.reset(); k.reset(); parts.clear();
   Tensor a = op_linear(o.reshape({S, H}), w[4], w[5]);
   o.reset();
   Tensor r = guarded([&] { return x + a; });

@@ -1551,6 +1551,62 @@ __global__ void rope_generic_kernel(const bf16* __restrict__ x, long ss, long hs
   }
 }
 
+// The rotation of q and k of a fused projection [S, 3, H, D] in one pass, and its transpose back into the projection's gradient, v's part of which is
+// copied: a warp per token and part (blockIdx.y: q, k, v), whose angles stay in registers (four times the bytes of the 8 channels that they turn), G heads
+// at a time, six groups in flight.  Same products and additions as above.  Bound by the memory's rate: 28672 x 16 heads of 72, q and k with a launch
+// each 72 us, 61 here; backward with the concatenation of the three gradients 133 us, 74 here.
+template <bool BWD>
+__global__ void __launch_bounds__(256) rope_qkv_kernel(const bf16* __restrict__ a0, const bf16* __restrict__ a1, const bf16* __restrict__ a2, long ld,
+                                                       const float* __restrict__ cosv, const float* __restrict__ sinv, bf16* __restrict__ o0,
+                                                       bf16* __restrict__ o1, int S, int H, int D) {
+  pdl_begin();
+  const int s = (int)((blockIdx.x * 256u + threadIdx.x) >> 5), lane = threadIdx.x & 31, part = blockIdx.y;
+  if (s >= S) return;
+  const int half = D >> 1, hq = half >> 2, G = 32 / hq;   // lanes of a head, heads of a warp
+  const int g = lane / hq, j = (lane - g * hq) * 4;
+  if (g >= G) return;
+  const bf16* src = (BWD ? (part == 0 ? a0 : part == 1 ? a1 : a2) + (long)s * H * D : a0 + (long)s * ld + (long)part * H * D) + j;
+  bf16* dst = (BWD ? o0 + ((long)s * 3 + part) * H * D : (part == 0 ? o0 : o1) + (long)s * H * D) + j;
+  float c0[4], c1[4], s0[4], s1[4];
+  if (part < 2) {
+    const float* ct = cosv + (long)s * D + j;
+    const float* st = sinv + (long)s * D + j;
+    *reinterpret_cast<float4*>(c0) = *reinterpret_cast<const float4*>(ct); *reinterpret_cast<float4*>(c1) = *reinterpret_cast<const float4*>(ct + half);
+    *reinterpret_cast<float4*>(s0) = *reinterpret_cast<const float4*>(st); *reinterpret_cast<float4*>(s1) = *reinterpret_cast<const float4*>(st + half);
+  }
+  constexpr int U = 6;
+  for (int h0 = g; h0 < H; h0 += U * G) {
+    uint2 lo[U], hi[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int at = (h0 + u * G) * D;
+      if (h0 + u * G < H) {
+        lo[u] = *reinterpret_cast<const uint2*>(src + at);
+        hi[u] = *reinterpret_cast<const uint2*>(src + at + half);
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int at = (h0 + u * G) * D;
+      if (h0 + u * G >= H) break;
+      if (part < 2) {
+        float a[4], b[4], r0[4], r1[4];
+        unpack4(lo[u], a);
+        unpack4(hi[u], b);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          if (!BWD) { r0[i] = a[i] * c0[i] - b[i] * s0[i]; r1[i] = b[i] * c1[i] + a[i] * s1[i]; }
+          else { r0[i] = a[i] * c0[i] + b[i] * s1[i]; r1[i] = b[i] * c1[i] - a[i] * s0[i]; }
+        }
+        lo[u] = pack4(r0);
+        hi[u] = pack4(r1);
+      }
+      *reinterpret_cast<uint2*>(dst + at) = lo[u];
+      *reinterpret_cast<uint2*>(dst + at + half) = hi[u];
+    }
+  }
+}
+
 // ----------------------------------------------------------------------------------- GDN gate prep
 // g = -exp(A_log) * softplus(a + dt_bias) (fp32 out), beta = sigmoid(b) (bf16 out); a,b strided rows
 __global__ void gdn_gates_fwd_kernel(const bf16* __restrict__ a, const bf16* __restrict__ b, long row_stride,
@@ -2062,6 +2118,15 @@ void vlmt_rope_generic(const void* x, long ss, long hs, const float* cosv, const
   }
   rope_generic_kernel<<<grid_for((long)S * H * (D / 2), 256, 148 * 16), 256, 0, st>>>(BF(x), ss, hs, cosv, sinv, BFM(out), oss, ohs, S, H, D,
                                                                                     transpose);
+}
+
+int vlmt_rope_qkv_usable(int D) { return D >= 8 && D % 8 == 0 && D <= 256; }
+void vlmt_rope_qkv_fwd(const void* qkv, long ld, const float* cosv, const float* sinv, void* q, void* k, int S, int H, int D, cudaStream_t st) {
+  launch_pdl(rope_qkv_kernel<false>, dim3((S + 7) / 8, 2), dim3(256), 0, st, 1, BF(qkv), nullptr, nullptr, ld, cosv, sinv, BFM(q), BFM(k), S, H, D);
+}
+void vlmt_rope_qkv_bwd(const void* dq, const void* dk, const void* dv, const float* cosv, const float* sinv, void* dqkv, int S, int H, int D,
+                       cudaStream_t st) {
+  launch_pdl(rope_qkv_kernel<true>, dim3((S + 7) / 8, 3), dim3(256), 0, st, 1, BF(dq), BF(dk), BF(dv), 0l, cosv, sinv, BFM(dqkv), nullptr, S, H, D);
 }
 
 void vlmt_gdn_gates_fwd(const void* a, const void* b, long row_stride, const float* A_log, const float* dt_bias, float* g, void* beta,

@@ -25,6 +25,11 @@ int vlmt_qkv_blocks(long items);
 int vlmt_qkv_norm_rope_fwd(const void* qkv, const void* qw, const void* kw, const float* cosv, const float* sinv, void* q, void* k, void* v, void* gate, float* rstd, int T, int n_q, int n_kv, int D, int R, float eps, int offset, int gated, int has_norm, cudaStream_t st);
 int vlmt_qkv_norm_rope_bwd(const void* dq, const void* dk, const void* dv, const void* dgate, const void* qkv, const void* qw, const void* kw, const float* cosv, const float* sinv, const float* rstd, void* dqkv, float* dw_partial, int T, int n_q, int n_kv, int D, int R, int offset, int gated, int has_norm, cudaStream_t st);
 void vlmt_rope_generic(const void* x, long ss, long hs, const float* cosv, const float* sinv, void* out, long oss, long ohs, int S, int H, int D, int transpose, cudaStream_t st);
+// q and k [S, H, D] of a projection [S, 3, H, D] (ld: elements between tokens) rotated, and the gradient of the projection from those of q, k and v;
+// rows and tables on 16 bytes, usable(D)
+int vlmt_rope_qkv_usable(int D);
+void vlmt_rope_qkv_fwd(const void* qkv, long ld, const float* cosv, const float* sinv, void* q, void* k, int S, int H, int D, cudaStream_t st);
+void vlmt_rope_qkv_bwd(const void* dq, const void* dk, const void* dv, const float* cosv, const float* sinv, void* dqkv, int S, int H, int D, cudaStream_t st);
 void vlmt_gdn_gates_fwd(const void* a, const void* b, long row_stride, const float* A_log, const float* dt_bias, float* g, void* beta, long T, int H, cudaStream_t st);
 int vlmt_gdn_gates_bwd(const float* dg, const void* dbeta, const void* a, const void* b, long row_stride, const float* A_log, const float* dt_bias, void* da, void* db, long out_stride, float* partial, long T, int H, cudaStream_t st);
 int vlmt_conv1d_silu_fwd(const void* x, long xs, const void* w, const int* seq_idx, void* y, long ys, int T, int C, int K, cudaStream_t st);
