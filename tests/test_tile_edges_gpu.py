@@ -54,6 +54,24 @@ def test_gemm_split_over_k(M, N, K, layout):
     cu.check_status()
 
 
+# gated RMS norm: rows of 128 and 256 in groups of four and two per warp (a last group that is not full), other widths and alignments in the general form
+@pytest.mark.parametrize("rows", [1, 3, 4, 5, 33, 4097])
+@pytest.mark.parametrize("D,shift", [(128, 0), (256, 0), (64, 0), (128, 1)])
+def test_gated_norm_rows(rows, D, shift):
+    def part():
+        return _rand(rows * D + shift)[shift:].view(rows, D).requires_grad_()
+
+    x, z, w, g = part(), part(), (_rand(D) + 1).requires_grad_(), _rand(rows, D)
+    y = ops.rms_norm_gated(x, z, w, 1e-6)
+    got = [y, *torch.autograd.grad(y, [x, z, w], g)]
+    xf, zf, wf = (t.detach().float().requires_grad_() for t in (x, z, w))
+    want = xf * torch.rsqrt(xf.pow(2).mean(-1, keepdim=True) + 1e-6) * wf * torch.nn.functional.silu(zf)
+    want = [want, *torch.autograd.grad(want, [xf, zf, wf], g.float())]
+    for name, a, b in zip(("y", "dx", "dz"), got, want):
+        _close(a, b, 1e-2, 8e-3, name)   # fp32 inside, one bf16 rounding (2^-9 of the value)
+    _close(got[3], want[3], 4e-3 * rows ** 0.5, 8e-3, "dw")
+
+
 # column sums: one cluster per 64 columns up to 2048 rows (a last block with fewer rows or none), slabs of 256 rows behind
 @pytest.mark.parametrize("rows", [1, 256, 257, 513, 1793, 2048, 2049])
 @pytest.mark.parametrize("cols", [8, 64, 72, 1160])

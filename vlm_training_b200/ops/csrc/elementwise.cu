@@ -816,6 +816,36 @@ __global__ void __launch_bounds__(kLnWarpsFwd * 32) layernorm_fwd_warp_kernel(co
   cp_wait<0>();
 }
 
+// E consecutive bf16 (E = 1, 2, 4, 8; the address is E*2-byte aligned) <-> floats, as one memory access
+template <int E> struct VecE;
+template <> struct VecE<1> { using T = unsigned short; };
+template <> struct VecE<2> { using T = uint32_t; };
+template <> struct VecE<4> { using T = uint2; };
+template <> struct VecE<8> { using T = uint4; };
+template <int E>
+__device__ __forceinline__ void ldE(const bf16* p, float (&f)[E]) {
+  const typename VecE<E>::T raw = *reinterpret_cast<const typename VecE<E>::T*>(p);
+  const bf16* h = reinterpret_cast<const bf16*>(&raw);
+#pragma unroll
+  for (int i = 0; i < E; ++i) f[i] = __bfloat162float(h[i]);
+}
+template <int E>
+__device__ __forceinline__ void stE(bf16* p, const float (&f)[E]) {
+  typename VecE<E>::T raw;
+  bf16* h = reinterpret_cast<bf16*>(&raw);
+#pragma unroll
+  for (int i = 0; i < E; ++i) h[i] = __float2bfloat16(f[i]);
+  *reinterpret_cast<typename VecE<E>::T*>(p) = raw;
+}
+__device__ __forceinline__ void unpack4(const uint2& u, float* f) {
+  f[0] = __uint_as_float(u.x << 16); f[1] = __uint_as_float(u.x & 0xffff0000u);
+  f[2] = __uint_as_float(u.y << 16); f[3] = __uint_as_float(u.y & 0xffff0000u);
+}
+__device__ __forceinline__ uint2 pack4(const float* f) {
+  bf162 a = __floats2bfloat162_rn(f[0], f[1]), b = __floats2bfloat162_rn(f[2], f[3]);
+  return make_uint2(*reinterpret_cast<uint32_t*>(&a), *reinterpret_cast<uint32_t*>(&b));
+}
+
 // ----------------------------------------------------------------------------------- gated RMSNorm (GDN output)
 // y = x * rstd * w * z * sigmoid(z), rows of D (<= 256), one warp per row
 __global__ void rmsnorm_gated_fwd_kernel(const bf16* __restrict__ x, const bf16* __restrict__ z, const bf16* __restrict__ w,
@@ -868,6 +898,126 @@ __global__ void rmsnorm_gated_bwd_kernel(const bf16* __restrict__ dy, const bf16
   for (int i = threadIdx.x; i < D; i += blockDim.x) {
     float s = 0.f;
 for (int wi = 0; wi < nwarps; ++wi) s += sm_dw[(size_t)wi * D + i];
+    dw_partial[(size_t)blockIdx.x * D + i] = s;
+  }
+}
+
+// The same for rows of 128 V channels: a lane holds four consecutive channels of every 128 as one 8-byte load per tensor, U rows in flight, and the weight
+// gradient of its channels in registers.  With 2-byte loads and sums in shared memory 524288 rows of 128 took 117 us forward and 273 us backward, now
+// 70 and 103; the memory's rate gives 62 and 104.
+template <int V>
+__global__ void __launch_bounds__(kThreads, 4) rmsnorm_gated_vec_fwd_kernel(const bf16* __restrict__ x, const bf16* __restrict__ z,
+                                                                           const bf16* __restrict__ w, bf16* __restrict__ y, float* __restrict__ rstd,
+                                                                           int rows, float eps) {
+  pdl_begin();
+  constexpr int D = 128 * V, U = V == 1 ? 4 : 2;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  float wv[V][4];
+#pragma unroll
+  for (int k = 0; k < V; ++k) ldE<4>(w + k * 128 + lane * 4, wv[k]);
+  for (long r0 = ((long)blockIdx.x * kWarpsPerBlock + warp) * U; r0 < rows; r0 += (long)gridDim.x * kWarpsPerBlock * U) {
+    uint2 xr[U][V], zr[U][V];
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+#pragma unroll
+      for (int k = 0; k < V; ++k) {
+        if (r0 + u >= rows) continue;
+        const size_t o = (size_t)(r0 + u) * D + k * 128 + lane * 4;
+        xr[u][k] = *reinterpret_cast<const uint2*>(x + o);
+        zr[u][k] = *reinterpret_cast<const uint2*>(z + o);
+      }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      if (r0 + u >= rows) continue;
+      float f[V][4], ss = 0.f;
+#pragma unroll
+      for (int k = 0; k < V; ++k) {
+        unpack4(xr[u][k], f[k]);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) ss += f[k][i] * f[k][i];
+      }
+      const float rs = rsqrtf(warp_sum(ss) / (float)D + eps);
+      if (lane == 0) rstd[r0 + u] = rs;
+#pragma unroll
+      for (int k = 0; k < V; ++k) {
+        float zz[4];
+        unpack4(zr[u][k], zz);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) f[k][i] = f[k][i] * rs * wv[k][i] * zz[i] * sigmoidf_(zz[i]);
+        *reinterpret_cast<uint2*>(y + (size_t)(r0 + u) * D + k * 128 + lane * 4) = pack4(f[k]);
+      }
+    }
+  }
+}
+template <int V>
+__global__ void __launch_bounds__(kThreads, 3) rmsnorm_gated_vec_bwd_kernel(const bf16* __restrict__ dy, const bf16* __restrict__ x,
+                                                                           const bf16* __restrict__ z, const bf16* __restrict__ w,
+                                                                           const float* __restrict__ rstd, bf16* __restrict__ dx, bf16* __restrict__ dz,
+                                                                           float* __restrict__ dw_partial, int rows) {
+  pdl_begin();
+  constexpr int D = 128 * V, U = V == 1 ? 4 : 2;
+  __shared__ float sm_dw[kWarpsPerBlock][D];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  float wv[V][4], dw[V][4];
+#pragma unroll
+  for (int k = 0; k < V; ++k) {
+    ldE<4>(w + k * 128 + lane * 4, wv[k]);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) dw[k][i] = 0.f;
+  }
+  for (long r0 = ((long)blockIdx.x * kWarpsPerBlock + warp) * U; r0 < rows; r0 += (long)gridDim.x * kWarpsPerBlock * U) {
+    uint2 xr[U][V], zr[U][V], gr[U][V];
+    float rs_[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      if (r0 + u >= rows) continue;
+      rs_[u] = rstd[r0 + u];
+#pragma unroll
+      for (int k = 0; k < V; ++k) {
+        const size_t o = (size_t)(r0 + u) * D + k * 128 + lane * 4;
+        xr[u][k] = *reinterpret_cast<const uint2*>(x + o);
+        zr[u][k] = *reinterpret_cast<const uint2*>(z + o);
+        gr[u][k] = *reinterpret_cast<const uint2*>(dy + o);
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      if (r0 + u >= rows) continue;
+      const float rs = rs_[u];
+      float xh[V][4], gw[V][4], dot = 0.f;
+#pragma unroll
+      for (int k = 0; k < V; ++k) {
+        float zz[4], g[4], d[4];
+        unpack4(xr[u][k], xh[k]);
+        unpack4(zr[u][k], zz);
+        unpack4(gr[u][k], g);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          xh[k][i] *= rs;
+          const float sg = sigmoidf_(zz[i]), act = zz[i] * sg, gn = g[i] * act;   // gn: gradient of normalised * weight
+          gw[k][i] = gn * wv[k][i];
+          dot += gw[k][i] * xh[k][i];
+          dw[k][i] += gn * xh[k][i];
+          d[i] = g[i] * xh[k][i] * wv[k][i] * (sg + act * (1.f - sg));
+        }
+        *reinterpret_cast<uint2*>(dz + (size_t)(r0 + u) * D + k * 128 + lane * 4) = pack4(d);
+      }
+      dot = warp_sum(dot) / (float)D;
+#pragma unroll
+      for (int k = 0; k < V; ++k) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) gw[k][i] = rs * (gw[k][i] - xh[k][i] * dot);
+        *reinterpret_cast<uint2*>(dx + (size_t)(r0 + u) * D + k * 128 + lane * 4) = pack4(gw[k]);
+      }
+    }
+  }
+#pragma unroll
+  for (int k = 0; k < V; ++k) *reinterpret_cast<float4*>(&sm_dw[warp][k * 128 + lane * 4]) = make_float4(dw[k][0], dw[k][1], dw[k][2], dw[k][3]);
+  __syncthreads();
+  for (int i = threadIdx.x; i < D; i += blockDim.x) {
+    float s = 0.f;
+#pragma unroll
+    for (int wi = 0; wi < kWarpsPerBlock; ++wi) s += sm_dw[wi][i];
     dw_partial[(size_t)blockIdx.x * D + i] = s;
   }
 }
@@ -1045,31 +1195,6 @@ __global__ void gelu_bwd_kernel(const bf16* dy, const bf16* __restrict__ x, bf16
 // One warp per (token, head slot).  Head slots: [0, n_q) q heads, [n_q, n_q+n_kv) k heads,
 // [n_q+n_kv, n_q+2 n_kv) v heads.  Lane owns E = D/32 consecutive channels; the rotate-half
 // partner of channel j (< R/2) is j + R/2, held by lane + (R/2)/E.
-// E consecutive bf16 (E = 1, 2, 4, 8; the address is E*2-byte aligned) <-> floats, as one memory access
-template <int E> struct VecE;
-template <> struct VecE<1> { using T = unsigned short; };
-template <> struct VecE<2> { using T = uint32_t; };
-template <> struct VecE<4> { using T = uint2; };
-template <> struct VecE<8> { using T = uint4; };
-template <int E>
-__device__ __forceinline__ void ldE(const bf16* p, float (&f)[E]) {
-  const typename VecE<E>::T raw = *reinterpret_cast<const typename VecE<E>::T*>(p);
-  const bf16* h = reinterpret_cast<const bf16*>(&raw);
-#pragma unroll
-  for (int i = 0; i < E; ++i) f[i] = __bfloat162float(h[i]);
-}
-template <int E>
-__device__ __forceinline__ void stE(bf16* p, const float (&f)[E]) {
-  typename VecE<E>::T raw;
-  bf16* h = reinterpret_cast<bf16*>(&raw);
-#pragma unroll
-  for (int i = 0; i < E; ++i) h[i] = __float2bfloat16(f[i]);
-  *reinterpret_cast<typename VecE<E>::T*>(p) = raw;
-}
-template <int E>
-__device__ __forceinline__ void cpE(bf16* dst, const bf16* src) {
-  *reinterpret_cast<typename VecE<E>::T*>(dst) = *reinterpret_cast<const typename VecE<E>::T*>(src);
-}
 // E consecutive floats starting at p[j] when the whole group lies below `limit`, else zeros (j, limit multiples of E
 // when `vec`; element-wise otherwise)
 template <int E>
@@ -1096,8 +1221,11 @@ __device__ __forceinline__ void ldF(const float* p, int j, int limit, bool vec, 
 
 constexpr int kQkvGroup = 12;   // heads of one token handled by one warp (the token's angles are loaded once per group)
 
+// Heads of 256 (eight channels per lane) want two blocks per SM: without the bound the compiler took 131 registers forward, which leaves one (16384
+// tokens of 16 + 2 x 4 heads with gates, 671 MB, forward 265 -> 164 us with four heads in flight; three blocks of three heads 199); backward, with the
+// loads of a head's pair first, 342 -> 184 (single heads in four blocks 221, loads where they are used 270).
 template <int E>
-__global__ void qkv_norm_rope_fwd_kernel(const bf16* __restrict__ qkv, const bf16* __restrict__ qw, const bf16* __restrict__ kw,
+__global__ void __launch_bounds__(kThreads, E == 8 ? 2 : 1) qkv_norm_rope_fwd_kernel(const bf16* __restrict__ qkv, const bf16* __restrict__ qw, const bf16* __restrict__ kw,
                                          const float* __restrict__ cosv, const float* __restrict__ sinv, bf16* __restrict__ q,
                                          bf16* __restrict__ k, bf16* __restrict__ v, bf16* __restrict__ gate,
                                          float* __restrict__ rstd, int T, int n_q, int n_kv, int R, float eps, int offset,
@@ -1187,7 +1315,7 @@ __global__ void qkv_norm_rope_fwd_kernel(const bf16* __restrict__ qkv, const bf1
 }
 
 template <int E>
-__global__ void qkv_norm_rope_bwd_kernel(const bf16* __restrict__ dq, const bf16* __restrict__ dk, const bf16* __restrict__ dv,
+__global__ void __launch_bounds__(kThreads, E == 8 ? 2 : 1) qkv_norm_rope_bwd_kernel(const bf16* __restrict__ dq, const bf16* __restrict__ dk, const bf16* __restrict__ dv,
                                          const bf16* __restrict__ dgate, const bf16* __restrict__ qkv, const bf16* __restrict__ qw,
                                          const bf16* __restrict__ kw, const float* __restrict__ cosv, const float* __restrict__ sinv,
                                          const float* __restrict__ rstd, bf16* __restrict__ dqkv, float* __restrict__ dw_partial,
@@ -1215,49 +1343,75 @@ __global__ void qkv_norm_rope_bwd_kernel(const bf16* __restrict__ dq, const bf16
     ldF<E>(sinv + (size_t)t * R, lane * E, R, vec_cs, sn);
     const bf16* row = qkv + (size_t)t * W;
     bf16* drow = dqkv + (size_t)t * W;
-#pragma unroll 4
-   for (int s = s_begin; s < s_end; ++s) {
-    int kind, off;
-    const bf16* g;
-    const bf16* wn = nullptr;
-    if (s < n_q) { kind = 0; off = s * qstride; g = dq + ((size_t)t * n_q + s) * D; wn = qw; }
-    else if (s < n_q + n_kv) { kind = 1; const int h = s - n_q; off = n_q * qstride + h * D; g = dk + ((size_t)t * n_kv + h) * D; wn = kw; }
-    else { kind = 2; const int h = s - n_q - n_kv; off = n_q * qstride + n_kv * D + h * D; g = dv + ((size_t)t * n_kv + h) * D; }
-    if (kind == 2) {
-      cpE<E>(drow + off + lane * E, g + lane * E);
-      continue;
-    }
-    if (kind == 0 && gated) cpE<E>(drow + off + D + lane * E, dgate + ((size_t)t * n_q + s) * D + lane * E);
-    // rotary transpose: dn[j] = do[j] c[j] + (j < half ? do[j+half] s[j+half] : -do[j-half] s[j-half])
-    float d[E], dn[E];
-    ldE<E>(g + lane * E, d);
+   // U heads per iteration, all loads first
+   constexpr int U = E == 8 ? 2 : 4;
+   using Raw = typename VecE<E>::T;
+   for (int s0 = s_begin; s0 < s_end; s0 += U) {
+    Raw graw[U], xraw[U], draw[U];
+    float rs_[U];
 #pragma unroll
-    for (int i = 0; i < E; ++i) {
-      const int j = lane * E + i;
-      const float ds = d[i] * sn[i];  // sn is zero beyond R
-      const float partner = __shfl_xor_sync(0xffffffffu, ds, plane);
-      dn[i] = j < R ? d[i] * c[i] + (j < half ? partner : -partner) : d[i];
+    for (int u = 0; u < U; ++u) {
+      const int s = s0 + u;
+      if (s >= s_end) continue;
+      const bool is_q = s < n_q, is_v = s >= n_q + n_kv;
+      const bf16* g = is_q ? dq + ((size_t)t * n_q + s) * D : is_v ? dv + ((size_t)t * n_kv + s - n_q - n_kv) * D : dk + ((size_t)t * n_kv + s - n_q) * D;
+      graw[u] = *reinterpret_cast<const Raw*>(g + lane * E);
+      if (is_q && gated) draw[u] = *reinterpret_cast<const Raw*>(dgate + ((size_t)t * n_q + s) * D + lane * E);
+      if (!is_v && has_norm) {
+        xraw[u] = *reinterpret_cast<const Raw*>(row + (is_q ? s * qstride : n_q * qstride + (s - n_q) * D) + lane * E);
+        rs_[u] = rstd[(size_t)t * (n_q + n_kv) + s];
+      }
     }
-    if (!has_norm) {
-      stE<E>(drow + off + lane * E, dn);
-      continue;
-    }
-    const float rs = rstd[(size_t)t * (n_q + n_kv) + s];
-    float xh[E], wv[E], dot = 0.f;
-    ldE<E>(row + off + lane * E, xh);
-    ldE<E>(wn + lane * E, wv);
 #pragma unroll
-    for (int i = 0; i < E; ++i) {
-      if (offset) wv[i] += 1.f;
-      xh[i] *= rs;
-      dot += dn[i] * wv[i] * xh[i];
-      if (kind == 0) acc_q[i] += dn[i] * xh[i]; else acc_k[i] += dn[i] * xh[i];
-    }
-    dot = warp_sum(dot) / (float)D;
-    float out[E];
+    for (int u = 0; u < U; ++u) {
+      const int s = s0 + u;
+      if (s >= s_end) continue;
+      const bool is_q = s < n_q, is_v = s >= n_q + n_kv;
+      bf16* dst = drow + (is_q ? s * qstride : n_q * qstride + (s - n_q) * D) + lane * E;
+      if (is_v) {
+        *reinterpret_cast<Raw*>(dst) = graw[u];
+        continue;
+      }
+      if (is_q && gated) *reinterpret_cast<Raw*>(dst + D) = draw[u];
+      // rotary transpose: dn[j] = do[j] c[j] + (j < half ? do[j+half] s[j+half] : -do[j-half] s[j-half])
+      float d[E], dn[E];
+      {
+        const bf16* h = reinterpret_cast<const bf16*>(&graw[u]);
 #pragma unroll
-    for (int i = 0; i < E; ++i) out[i] = rs * (dn[i] * wv[i] - xh[i] * dot);
-    stE<E>(drow + off + lane * E, out);
+        for (int i = 0; i < E; ++i) d[i] = __bfloat162float(h[i]);
+      }
+#pragma unroll
+      for (int i = 0; i < E; ++i) {
+        const int j = lane * E + i;
+        const float ds = d[i] * sn[i];  // sn is zero beyond R
+        const float partner = __shfl_xor_sync(0xffffffffu, ds, plane);
+        dn[i] = j < R ? d[i] * c[i] + (j < half ? partner : -partner) : d[i];
+      }
+      if (!has_norm) {
+        stE<E>(dst, dn);
+        continue;
+      }
+      const float rs = rs_[u];
+      float xh[E], wv[E], dot = 0.f;
+      {
+        const bf16* h = reinterpret_cast<const bf16*>(&xraw[u]);
+#pragma unroll
+        for (int i = 0; i < E; ++i) xh[i] = __bfloat162float(h[i]);
+      }
+      ldE<E>((is_q ? qw : kw) + lane * E, wv);
+#pragma unroll
+      for (int i = 0; i < E; ++i) {
+        if (offset) wv[i] += 1.f;
+        xh[i] *= rs;
+        dot += dn[i] * wv[i] * xh[i];
+        if (is_q) acc_q[i] += dn[i] * xh[i]; else acc_k[i] += dn[i] * xh[i];
+      }
+      dot = warp_sum(dot) / (float)D;
+      float out[E];
+#pragma unroll
+      for (int i = 0; i < E; ++i) out[i] = rs * (dn[i] * wv[i] - xh[i] * dot);
+      stE<E>(dst, out);
+    }
    }
   }
 #pragma unroll
@@ -1285,14 +1439,6 @@ __device__ __forceinline__ QkvSlot qkv_slot(int s, int s_end, int n_q, int n_kv,
   r.kind = s >= s_end ? -1 : s < n_q ? 0 : s < n_q + n_kv ? 1 : 2;
   r.off = s < n_q ? s * qstride : n_q * qstride + (s - n_q) * 128;
   return r;
-}
-__device__ __forceinline__ void unpack4(const uint2& u, float* f) {
-  f[0] = __uint_as_float(u.x << 16); f[1] = __uint_as_float(u.x & 0xffff0000u);
-  f[2] = __uint_as_float(u.y << 16); f[3] = __uint_as_float(u.y & 0xffff0000u);
-}
-__device__ __forceinline__ uint2 pack4(const float* f) {
-  bf162 a = __floats2bfloat162_rn(f[0], f[1]), b = __floats2bfloat162_rn(f[2], f[3]);
-  return make_uint2(*reinterpret_cast<uint32_t*>(&a), *reinterpret_cast<uint32_t*>(&b));
 }
 __device__ __forceinline__ void ld_angles(const float* p, int l, float (&f)[8]) {
   const float4 a = *reinterpret_cast<const float4*>(p + 4 * l), b = *reinterpret_cast<const float4*>(p + 64 + 4 * l);
@@ -2021,11 +2167,22 @@ int vlmt_layernorm_bwd(const void* dy, const void* x, const void* w, const void*
 }
 
 void vlmt_rmsnorm_gated_fwd(const void* x, const void* z, const void* w, void* y, float* rstd, int rows, int D, float eps, cudaStream_t st) {
+  if ((D == 128 || D == 256) && ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(z) | reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(y)) & 7) == 0) {
+    launch_pdl(D == 128 ? rmsnorm_gated_vec_fwd_kernel<1> : rmsnorm_gated_vec_fwd_kernel<2>, dim3(grid_for(rows, kWarpsPerBlock * (D == 128 ? 4 : 2), 148 * 8)),
+               dim3(kThreads), 0, st, 1, BF(x), BF(z), BF(w), BFM(y), rstd, rows, eps);
+    return;
+  }
   launch_pdl(rmsnorm_gated_fwd_kernel, dim3(grid_for(rows, kWarpsPerBlock, 148 * 16)), dim3(kThreads), 0, st, 1, BF(x), BF(z), BF(w), BFM(y), rstd, rows, D, eps);
 }
 int vlmt_rmsnorm_gated_bwd(const void* dy, const void* x, const void* z, const void* w, const float* rstd, void* dx, void* dz,
                            float* dw_partial, int rows, int D, cudaStream_t st) {
   const int grid = vlmt_norm_blocks(rows);
+  if ((D == 128 || D == 256) && ((reinterpret_cast<uintptr_t>(dy) | reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(z) | reinterpret_cast<uintptr_t>(w) |
+                                  reinterpret_cast<uintptr_t>(dx) | reinterpret_cast<uintptr_t>(dz)) & 7) == 0) {
+    launch_pdl(D == 128 ? rmsnorm_gated_vec_bwd_kernel<1> : rmsnorm_gated_vec_bwd_kernel<2>, dim3(grid), dim3(kThreads), 0, st, 1, BF(dy), BF(x), BF(z), BF(w), rstd,
+               BFM(dx), BFM(dz), dw_partial, rows);
+    return grid;
+  }
   launch_pdl(rmsnorm_gated_bwd_kernel, dim3(grid), dim3(kThreads), (size_t)kWarpsPerBlock * D * sizeof(float), st, 1, BF(dy), BF(x), BF(z), BF(w), rstd, BFM(dx),
              BFM(dz), dw_partial, rows, D);
   return grid;
