@@ -72,6 +72,24 @@ def test_gated_norm_rows(rows, D, shift):
     _close(got[3], want[3], 4e-3 * rows ** 0.5, 8e-3, "dw")
 
 
+# gate / up projection with its activation in one kernel: the bits of the product and the activation kernel behind one another, for few rows (one and
+# several parts of K, ragged K) and on CTA pairs (rows off the tile edges), gate and up kept or not; sizes without such a kernel are refused
+@pytest.mark.parametrize("M,I,K,there", [(1, 12288, 4096, True), (37, 12288, 4096, True), (17, 256, 1096, True), (100, 1536, 520, True), (128, 128, 64, True),
+                                         (451, 12288, 1032, True), (2049, 1280, 264, True), (1000, 9728, 512, True), (37, 192, 512, False), (300, 256, 512, False)])
+def test_gate_up_with_its_activation(M, I, K, there):
+    from vlm_training_b200.ops import cuda as cu
+
+    x, w = _rand(M, K, scale=0.5), _rand(2 * I, K, scale=0.5)
+    got = cu._C.gemm_glu(x, w, True)
+    assert (got is not None) == there
+    if there:
+        gu = cu._gemm(x, w)
+        assert torch.equal(got[1], gu) and torch.equal(got[0], cu._C.op_swiglu(gu))
+        alone = cu._C.gemm_glu(x, w, False)
+        assert torch.equal(alone[0], got[0]) and alone[1] is None
+    cu.check_status()
+
+
 # column sums: one cluster per 64 columns up to 2048 rows (a last block with fewer rows or none), slabs of 256 rows behind
 @pytest.mark.parametrize("rows", [1, 256, 257, 513, 1793, 2048, 2049])
 @pytest.mark.parametrize("cols", [8, 64, 72, 1160])

@@ -71,6 +71,21 @@ void gemm(const Tensor& a, const Tensor& b, Tensor& out, bool a_mn, bool b_mn, c
   TORCH_CHECK(r == 0, "vlmt_gemm_bf16 failed with code ", r);
 }
 
+// act = silu(gate) * up with [gate; up] = x w^T; false: nothing was done.  gu: null, or gets gate and up.
+bool gemm_glu(const Tensor& x, const Tensor& w, Tensor* gu, Tensor& act) {
+  check_bf16(x, "x"); check_bf16(w, "w");
+  TORCH_CHECK(x.dim() == 2 && w.dim() == 2 && x.stride(1) == 1 && w.stride(1) == 1 && x.size(1) == w.size(1) && w.size(0) % 2 == 0);
+  c10::cuda::CUDAGuard guard(x.device());
+  const int64_t M = x.size(0), I = w.size(0) / 2;
+  if (I % 128 != 0 || M == 0) return false;
+  act = torch::empty({M, I}, x.options());
+  if (gu != nullptr) *gu = torch::empty({M, 2 * I}, x.options());
+  const int r = vlmt_gemm_bf16_glu(x.data_ptr(), w.data_ptr(), gu != nullptr ? gu->data_ptr() : nullptr, act.data_ptr(), (int)M, (int)I, (int)x.size(1),
+                                   (int)x.stride(0), (int)w.stride(0), status_tensor().data_ptr<int>(), num_sms(), cur_stream());
+  TORCH_CHECK(r == 0 || r == 1, "vlmt_gemm_bf16_glu failed with code ", r);
+  return r == 0;
+}
+
 // y-partials of a row-parallel linear pushed to their owners: rows [o*R, (o+1)*R) of a @ b^T go to dst_ptrs[o]
 void gemm_rs_push(const Tensor& a, const Tensor& b, const std::vector<int64_t>& dst_ptrs, int64_t rows_per_rank, bool b_mn) {
   check_bf16(a, "a"); check_bf16(b, "b");
@@ -551,6 +566,12 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     c10::cuda::CUDAGuard guard(t.device());
     cudaError_t e = cudaMemsetAsync(t.data_ptr(), 0, (size_t)t.numel() * t.element_size(), cur_stream());
     TORCH_CHECK(e == cudaSuccess, "cudaMemsetAsync failed: ", cudaGetErrorString(e));
+  });
+  // (act, gate and up or None), or None where the sizes have no such kernel
+  m.def("gemm_glu", [](const Tensor& x, const Tensor& w, bool keep) -> py::object {
+    Tensor gu, act;
+    if (!gemm_glu(x, w, keep ? &gu : nullptr, act)) return py::none();
+    return py::make_tuple(act, keep ? py::cast(gu) : py::object(py::none()));
   });
   m.def("gemm_rs_push", &gemm_rs_push);
   m.def("gemm_ag", &gemm_ag);

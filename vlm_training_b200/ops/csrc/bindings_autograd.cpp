@@ -432,6 +432,79 @@ Tensor op_swiglu_linear(const Tensor& gu, const py::object& w_) {
   });
 }
 
+// x + residual -> RMSNorm -> gate / up -> silu(gate) * up -> down: the two functions above with the activation made by the gate / up product's kernel
+// where the sizes have one.  Second output: x + residual.
+struct NormMlp : torch::autograd::Function<NormMlp> {
+  // out, x + residual, rstd, gate and up (undefined where they are not kept)
+  static std::array<Tensor, 4> run(const Tensor& x, const Tensor& res, const Tensor& nw, const Tensor& wgu, const Tensor& wd, const Cfg& c, bool keep_gu) {
+    auto r = rmsnorm_fwd(x.contiguous(), OptTensor(res.contiguous()), nw, c.eps, c.offset);
+    check_storage(wgu);
+    Tensor gu, act;
+    if (gemm_glu(r[0], wgu, keep_gu ? &gu : nullptr, act)) {
+      tick(1);
+    } else {
+      gu = mm(r[0], wgu, false, false);
+      act = swiglu_fwd(gu);
+      tick(1);
+    }
+    tick(1);
+    r[0].reset();
+    return {mm(act, wd, false, false), r[2], r[1], gu};
+  }
+  static variable_list forward(AutogradContext* ctx, const Tensor& x, const Tensor& res, const Tensor& nw, const Tensor& wgu_, const Tensor& wd_, CfgPtr c) {
+    ctx->set_materialize_grads(false);
+    Tensor wgu = operand(wgu_), wd = operand(wd_);
+    auto r = run(x, res, nw, wgu, wd, *c, true);
+    c->need[2] = wants(nw); c->need[3] = wants(wgu_); c->need[4] = wants(wd_);
+    keep(ctx, c);
+    ctx->save_for_backward({r[1], nw, r[2], wgu, r[3], wd});
+    return {r[0], r[1]};
+  }
+  static variable_list backward(AutogradContext* ctx, variable_list grads) {
+    auto s = ctx->get_saved_variables();
+    auto c = kept(ctx);
+    const Tensor &r = s[0], &nw = s[1], &rstd = s[2], &wgu = s[3], &gu = s[4], &wd = s[5];
+    Tensor dr = grads[1], dx, dnw, dwgu, dwd;
+    if (!grads[0].defined()) {   // only the residual stream was used
+      dx = dr;
+    } else {
+      Tensor dy = rows_of(grads[0]), h, yn;
+      Tensor dgu = swiglu_bwd(mm(dy, wd, false, true), gu, c->need[4] ? &h : nullptr);
+      if (c->need[4]) dwd = weight_grad(dy, h, c->t[2]);
+      h.reset();
+      auto b = rmsnorm_bwd_partial(mm(dgu, wgu, false, true), r, nw, rstd, dr.defined() ? OptTensor(dr.contiguous()) : OptTensor(), c->offset,
+                                   c->need[3] ? &yn : nullptr);
+      dx = b[0];
+      tick(2);
+      if (c->need[3]) {
+        if (!yn.defined()) { yn = rmsnorm_fwd(r, c10::nullopt, nw, c->eps, c->offset)[0]; tick(1); }
+        dwgu = weight_grad(dgu, yn, c->t[1]);
+        yn.reset();
+      }
+      if (c->need[2]) {
+        VecGrad g(nw, c->t[0]);
+        sum_rows(b[1].data_ptr<float>(), nullptr, b[1].size(1), b[1].size(0), b[1].size(1), g, nullptr);
+        dnw = g.finish(nw, c->t[0]);
+      }
+    }
+    return {dx, dx, dnw, dwgu, dwd, Tensor()};
+  }
+};
+std::array<Tensor, 2> norm_mlp(const Tensor& x, const Tensor& res, const py::object& nw_, const py::object& wgu_, const py::object& wd_, double eps, bool offset) {
+  return guarded([&]() -> std::array<Tensor, 2> {
+    Tensor nw = nw_.cast<Tensor>(), wgu = wgu_.cast<Tensor>(), wd = wd_.cast<Tensor>();
+    auto c = c10::make_intrusive<Cfg>();
+    c->eps = eps; c->offset = offset;
+    if (no_graph(x, res, nw, wgu, wd)) {
+      auto r = NormMlp::run(x, res, nw, operand(wgu), operand(wd), *c, false);
+      return {r[0], r[1]};
+    }
+    c->t[0] = target_of(nw_); c->t[1] = target_of(wgu_); c->t[2] = target_of(wd_);
+    auto out = NormMlp::apply(x, res, nw, wgu, wd, c);
+    return {out[0], out[1]};
+  });
+}
+
 // ------------------------------------------------------------------ norms
 struct RmsNorm : torch::autograd::Function<RmsNorm> {
   static variable_list forward(AutogradContext* ctx, const Tensor& x, const OptTensor& res_, const Tensor& w, CfgPtr c) {
@@ -895,13 +968,9 @@ py::object op_decoder_layer(const Tensor& x, const py::tuple& w, const Tensor& c
   heads = py::tuple();
   Tensor h = op_linear(o, w_o, py::none());
   o.reset();
-  py::tuple gr = op_norm_linear(h, py::cast(x), norm2, w_gu, eps2, offset2).cast<py::tuple>();
+  auto mlp = norm_mlp(h, x, norm2, w_gu, w_down, eps2, offset2);
   h.reset();
-  Tensor gu = gr[0].cast<Tensor>(), r = gr[1].cast<Tensor>();
-  gr = py::tuple();
-  Tensor out = op_swiglu_linear(gu, w_down);
-  gu.reset();
-  return py::cast(guarded([&] { return r + out; }));
+  return py::cast(guarded([&] { return mlp[1] + mlp[0]; }));
 }
 
 // norm1 (weight, bias), qkv, proj, norm2, fc1, fc2 (each weight, bias)

@@ -23,6 +23,9 @@ __device__ __forceinline__ float gelu_tanh_f(float x) {
 }
 __device__ __forceinline__ float gelu_erf_f(float x) { return 0.5f * x * (1.f + erff(x * 0.7071067811865476f)); }
 
+// the operations of the activation kernels (elementwise.cu), on values that have been rounded to bf16
+__device__ __forceinline__ float swiglu_f(float g, float u) { return g * (1.f / (1.f + __expf(-g))) * u; }
+
 // 32 columns of a row, from column `col`: bias (or null) and activation (GemmEpilogue)
 __device__ __forceinline__ void bias_activation(float (&v)[32], const __nv_bfloat16* bias, int col, int N, int epilogue) {
   if (bias != nullptr) {

@@ -53,6 +53,7 @@ struct Params {
   const float* rec_a;           // FP8: rec[1] undoes the operand's scaling
   const float* rec_b;
   uint32_t idesc;               // FP8: carries the two formats
+  int store_gu;                 // GLU: D is written
   int* status;
 };
 
@@ -100,10 +101,12 @@ __device__ __forceinline__ void store_parts(const uint8_t* smem, const Params& p
   }
 }
 
-template <bool A_MN, bool B_MN, bool FP8>
+// GLU (K-major operands): B is [gate; up] of N / 2 rows each.  The leader loads 128 rows of gate, its peer the same rows of up, so an accumulator row
+// has 128 columns of both, and the epilogue writes silu(gate) * up of the rounded values besides them, or alone (store_gu 0).
+template <bool A_MN, bool B_MN, bool FP8, bool GLU>
 __global__ void __launch_bounds__(NUM_THREADS, 1)
 gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b, const __grid_constant__ CUtensorMap tmap_d,
-                 Params p) {
+                 const __grid_constant__ CUtensorMap tmap_act, Params p) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + kBarOffset);
@@ -163,7 +166,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
         int tile, kb_lo, kb_hi, tm, tn;
         k_range(item, tile, kb_lo, kb_hi);
         tile_coords(p.group_m, tile, tiles_m, tiles_n, tm, tn);
-        const int m0 = (tm * 2 + (int)rank) * BM, n0 = tn * BN + (int)rank * (BN / 2);
+        const int m0 = (tm * 2 + (int)rank) * BM, n0 = GLU ? tn * (BN / 2) + (int)rank * (p.N / 2) : tn * BN + (int)rank * (BN / 2);
         for (int kb = kb_lo; kb < kb_hi; ++kb) {
           if (!mbar_wait(&empty_bar[stage], phase ^ 1, abort_flag, p.status, kErrTimeoutEmpty)) { ok = false; break; }
           uint8_t* sa = smem + stage * kStageBytes;
@@ -247,6 +250,49 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
         }
         break;
       }
+      if (GLU) {
+        auto put = [&](const uint32_t (&w)[32], const CUtensorMap* map, int col) {
+          uint8_t* buf = out + (slab++ & 1) * 4096;
+          if (lane == 0) tma_store_wait_read<1>();
+          __syncwarp();
+#pragma unroll
+          for (int t = 0; t < 8; ++t)
+            *reinterpret_cast<uint4*>(buf + lane * 128 + ((t ^ (lane & 7)) << 4)) = make_uint4(w[4 * t], w[4 * t + 1], w[4 * t + 2], w[4 * t + 3]);
+          fence_async_proxy();
+          __syncwarp();
+          if (lane == 0) {
+            tma_store_2d(map, buf, col, row0);
+            tma_store_commit();
+          }
+        };
+#pragma unroll 1
+        for (int c = 0; c < BN / 128; ++c) {
+          if (row0 >= p.M) break;
+          const int col = tn * (BN / 2) + c * 64;
+          uint32_t g[32], u[32];
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            uint32_t r[32];
+            tmem_ld_32x32(taddr + c * 64 + h * 32, r);
+            tmem_ld_wait();
+#pragma unroll
+            for (int i = 0; i < 16; ++i) g[h * 16 + i] = pack_bf16x2(__uint_as_float(r[2 * i]), __uint_as_float(r[2 * i + 1]));
+            tmem_ld_32x32(taddr + BN / 2 + c * 64 + h * 32, r);
+            tmem_ld_wait();
+#pragma unroll
+            for (int i = 0; i < 16; ++i) u[h * 16 + i] = pack_bf16x2(__uint_as_float(r[2 * i]), __uint_as_float(r[2 * i + 1]));
+          }
+          if (p.store_gu) {
+            put(g, &tmap_d, col);
+            put(u, &tmap_d, p.N / 2 + col);
+          }
+#pragma unroll
+          for (int i = 0; i < 32; ++i)
+            g[i] = pack_bf16x2(swiglu_f(__uint_as_float(g[i] << 16), __uint_as_float(u[i] << 16)),
+                               swiglu_f(__uint_as_float(g[i] & 0xffff0000u), __uint_as_float(u[i] & 0xffff0000u)));
+          put(g, &tmap_act, col);
+        }
+      } else
 #pragma unroll 1
       for (int c = 0; c < BN / 64; ++c) {
         const int col0 = n0 + c * 64;
@@ -304,9 +350,9 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
   }
 }
 
-template <bool A_MN, bool B_MN, bool FP8 = false>
-int launch(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& td, const Params& p, cudaStream_t st) {
-  auto kern = gemm_pair_kernel<A_MN, B_MN, FP8>;
+template <bool A_MN, bool B_MN, bool FP8 = false, bool GLU = false>
+int launch(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& td, const CUtensorMap& tact, const Params& p, cudaStream_t st) {
+  auto kern = gemm_pair_kernel<A_MN, B_MN, FP8, GLU>;
   static int max_pairs = 0;
   static std::once_flag once;
   cudaLaunchConfig_t cfg = {};
@@ -324,10 +370,10 @@ int launch(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& td, 
   if (max_pairs <= 0) return -50;
   if (p.parts > 1) {
     const int tiles = ((p.M + 2 * BM - 1) / (2 * BM)) * ((p.N + BN - 1) / BN);
-    return launch_pdl(kern, dim3(2 * p.parts * tiles), dim3(NUM_THREADS), kSmem, st, 2 * p.parts, ta, tb, td, p);
+    return launch_pdl(kern, dim3(2 * p.parts * tiles), dim3(NUM_THREADS), kSmem, st, 2 * p.parts, ta, tb, td, tact, p);
   }
   const int items = ((p.M + 2 * BM - 1) / (2 * BM)) * ((p.N + BN - 1) / BN) * p.k_splits;
-  return launch_pdl(kern, dim3(2 * (items < max_pairs ? items : max_pairs)), dim3(NUM_THREADS), kSmem, st, 2, ta, tb, td, p);
+  return launch_pdl(kern, dim3(2 * (items < max_pairs ? items : max_pairs)), dim3(NUM_THREADS), kSmem, st, 2, ta, tb, td, tact, p);
 }
 }  // namespace
 
@@ -341,7 +387,7 @@ extern "C" int vlmt_gemm_pair_clusters() {
   static int cap = 0;
   static std::once_flag once;
   std::call_once(once, [] {
-    auto kern = gemm_pair_kernel<false, false, false>;
+    auto kern = gemm_pair_kernel<false, false, false, false>;
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute attr;
     attr.id = cudaLaunchAttributeClusterDimension;
@@ -374,8 +420,26 @@ extern "C" int vlmt_gemm_pair(const void* A, const void* B, void* D, const void*
   p.accumulate = accumulate; p.k_splits = k_splits; p.kb_per_split = kb_per_split; p.status = status;
   p.group_m = raster_group(2l * N * K, 2l * K);
   p.parts = parts; p.D = reinterpret_cast<__nv_bfloat16*>(D); p.ldd = ldd;
-  if (a_mn_major) return b_mn_major ? launch<true, true>(ta, tb, td, p, stream) : launch<true, false>(ta, tb, td, p, stream);
-  return b_mn_major ? launch<false, true>(ta, tb, td, p, stream) : launch<false, false>(ta, tb, td, p, stream);
+  if (a_mn_major) return b_mn_major ? launch<true, true>(ta, tb, td, td, p, stream) : launch<true, false>(ta, tb, td, td, p, stream);
+  return b_mn_major ? launch<false, true>(ta, tb, td, td, p, stream) : launch<false, false>(ta, tb, td, td, p, stream);
+}
+
+// act[M, I] = silu(gate) * up with [gate; up] = X(M,K) W(2 I,K)^T, I a multiple of 128; gu (or null) [M, 2 I]
+extern "C" int vlmt_gemm_pair_glu(const void* X, const void* W, void* gu, void* act, int M, int I, int K, int ldx, int ldw, int* status,
+                                  cudaStream_t stream) {
+  CUtensorMap ta, tb, td, tact;
+  int r;
+  if ((r = vlmt_make_tmap_2d_bf16(&ta, X, (uint64_t)K, (uint64_t)M, (uint64_t)ldx * 2, 64, 128))) return 1000 + r;
+  if ((r = vlmt_make_tmap_2d_bf16(&tb, W, (uint64_t)K, (uint64_t)2 * I, (uint64_t)ldw * 2, 64, 128))) return 2000 + r;
+  if ((r = vlmt_make_tmap_2d_bf16(&tact, act, (uint64_t)I, (uint64_t)M, (uint64_t)I * 2, 64, 32))) return 3000 + r;
+  td = tact;
+  if (gu != nullptr && (r = vlmt_make_tmap_2d_bf16(&td, gu, (uint64_t)2 * I, (uint64_t)M, (uint64_t)I * 4, 64, 32))) return 3000 + r;
+  Params p = {};
+  p.M = M; p.N = 2 * I; p.K = K;
+  p.k_splits = 1; p.kb_per_split = (K + BK - 1) / BK; p.parts = 1; p.status = status;
+  p.group_m = raster_group(4l * I * K, 2l * K);
+  p.store_gu = gu != nullptr;
+  return launch<false, false, false, true>(ta, tb, td, tact, p, stream);
 }
 
 extern "C" int vlmt_gemm_pair_fp8(const void* A, const void* B, void* D, int M, int N, int K, long lda, long ldb, long ldd, uint32_t idesc,
@@ -391,5 +455,5 @@ extern "C" int vlmt_gemm_pair_fp8(const void* A, const void* B, void* D, int M, 
   p.accumulate = accumulate; p.k_splits = k_splits; p.kb_per_split = kb_per_split; p.status = status;
   p.group_m = raster_group((long)N * K, K);
   p.parts = 1;
-  return launch<false, false, true>(ta, tb, td, p, stream);
+  return launch<false, false, true>(ta, tb, td, td, p, stream);
 }

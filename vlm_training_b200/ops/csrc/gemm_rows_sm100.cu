@@ -39,7 +39,8 @@ struct Params {
   int M, N, K, ldd;
   int splits, kb_per;      // blocks of a cluster that share a tile's K, 64-wide k-blocks of each
   int prefetch_blocks;     // blocks that may be launched ahead
-  __nv_bfloat16* D;
+  __nv_bfloat16* D;        // GLU: [M, N] gate and up, or null
+  __nv_bfloat16* act;      // GLU: [M, N / 2]
   const __nv_bfloat16* bias;
   const float* alpha;
   int epilogue;
@@ -59,7 +60,9 @@ __device__ __forceinline__ void st_cluster_f32(uint32_t addr, float v) {
   asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(addr), "f"(v) : "memory");
 }
 
-template <int NT>
+// GLU: W is [gate; up] of N / 2 rows each; a weight tile is 64 rows of gate and the same 64 of up, and the sum of the parts (one part also) writes
+// silu(gate) * up of the rounded values, and gate and up where D is given.
+template <int NT, bool GLU>
 __global__ void __launch_bounds__(NUM_THREADS, 2)
 gemm_rows_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_x, Params p) {
   using L = Layout<NT>;
@@ -74,7 +77,7 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int rank = p.splits > 1 ? (int)cluster_rank() : 0;
-  const int n0 = (blockIdx.x / p.splits) * BW;
+  const int n0 = (blockIdx.x / p.splits) * (GLU ? BW / 2 : BW), up0 = n0 + p.N / 2;
   const int num_kb = (p.K + BK - 1) / BK;
   const int kb_lo = rank * p.kb_per, kb_hi = min(num_kb, kb_lo + p.kb_per);
 
@@ -88,7 +91,10 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
     // The weight's rows on their way to L2 while the kernel before this one drains: L2 is where the GPU's memory is coherent, so a
     // line that is still to be written is the written one when the loads below ask for it.
     if ((int)blockIdx.x < p.prefetch_blocks)
-      for (int kb = kb_lo; kb < min(kb_hi, kb_lo + 16); ++kb) tma_prefetch_l2_2d(&tmap_w, kb * BK, n0);
+      for (int kb = kb_lo; kb < min(kb_hi, kb_lo + 16); ++kb) {
+        tma_prefetch_l2_2d(&tmap_w, kb * BK, n0);
+        if (GLU) tma_prefetch_l2_2d(&tmap_w, kb * BK, up0);
+      }
   }
   if (warp == 1) tmem_alloc<L::kCols>(tmem_slot);
   tc_fence_before();
@@ -104,7 +110,8 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
         if (!mbar_wait(&empty_bar[stage], phase ^ 1, abort_flag, p.status, kErrTimeoutEmpty)) break;
         uint8_t* sw = smem + stage * L::kStageBytes;
         mbar_expect_tx(&full_bar[stage], L::kStageBytes);
-        tma_load_2d(sw, &tmap_w, &full_bar[stage], kb * BK, n0);               // box {64 k, 128 rows of the weight}
+        tma_load_2d(sw, &tmap_w, &full_bar[stage], kb * BK, n0);               // box {64 k, 128 rows of the weight; GLU: 64}
+        if (GLU) tma_load_2d(sw + L::kWBytes / 2, &tmap_w, &full_bar[stage], kb * BK, up0);
         tma_load_2d(sw + L::kWBytes, &tmap_x, &full_bar[stage], kb * BK, 0);   // box {64 k, NT rows of X}
         if (++stage == STAGES) { stage = 0; phase ^= 1; }
       }
@@ -139,7 +146,7 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
   const float alpha = p.alpha != nullptr ? __ldg(p.alpha) : 1.f;
   const int q = warp & 3;
   const uint32_t taddr = tmem + ((uint32_t)(q * 32) << 16);
-  if (p.splits == 1) {
+  if (!GLU && p.splits == 1) {
     if (warp >= 2 && !*abort_flag) {
       const int n = n0 + q * 32 + lane;
       const float bias = p.bias != nullptr && n < p.N ? __bfloat162float(p.bias[n]) : 0.f;
@@ -169,7 +176,7 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
     }
   } else {
     const int share = (((p.M + p.splits - 1) / p.splits) + 7) & ~7;   // rows of X per block, whole groups of 8 columns of tensor memory
-    cluster_sync();   // every block's MMAs have completed: the stages of all of them are free
+    if (p.splits > 1) cluster_sync(); else __syncthreads();   // every block's MMAs have completed: the stages of all of them are free
     if (warp >= 2 && !*abort_flag) {
       // [rank of the part][row of the owner's share][128 features]
       const uint32_t mine = smem_u32(smem) + (uint32_t)(rank * share * BW + q * 32 + lane) * 4;
@@ -189,8 +196,35 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
       }
     }
     __syncwarp();
-    cluster_sync();   // the parts have arrived; nobody reads another block's memory from here on
-    if (!*abort_flag) {
+    if (p.splits > 1) cluster_sync(); else __syncthreads();   // the parts have arrived; nobody reads another block's memory from here on
+    if (GLU && !*abort_flag) {
+      const int rows = min(share, p.M - rank * share), half = p.N / 2;
+      const float4* parts = reinterpret_cast<const float4*>(smem);
+      for (int i = threadIdx.x; i < rows * (BW / 8); i += NUM_THREADS) {
+        const int row = i / (BW / 8), f = i % (BW / 8);
+        float g[4] = {0.f, 0.f, 0.f, 0.f}, u[4] = {0.f, 0.f, 0.f, 0.f};
+        for (int s = 0; s < p.splits; ++s) {
+          const float4 a = parts[(s * share + row) * (BW / 4) + f], b = parts[(s * share + row) * (BW / 4) + BW / 8 + f];
+          g[0] += a.x; g[1] += a.y; g[2] += a.z; g[3] += a.w;
+          u[0] += b.x; u[1] += b.y; u[2] += b.z; u[3] += b.w;
+        }
+        const uint2 gp = make_uint2(pack_bf16x2(g[0], g[1]), pack_bf16x2(g[2], g[3])), upk = make_uint2(pack_bf16x2(u[0], u[1]), pack_bf16x2(u[2], u[3]));
+        const size_t t = (size_t)(rank * share + row);
+        const int n = n0 + f * 4;   // N / 2 is a multiple of 64
+        if (p.D != nullptr) {
+          *reinterpret_cast<uint2*>(p.D + t * p.N + n) = gp;
+          *reinterpret_cast<uint2*>(p.D + t * p.N + half + n) = upk;
+        }
+        const uint32_t gw[2] = {gp.x, gp.y}, uw[2] = {upk.x, upk.y};
+        uint32_t o[2];
+#pragma unroll
+        for (int j = 0; j < 2; ++j)
+          o[j] = pack_bf16x2(swiglu_f(__uint_as_float(gw[j] << 16), __uint_as_float(uw[j] << 16)),
+                             swiglu_f(__uint_as_float(gw[j] & 0xffff0000u), __uint_as_float(uw[j] & 0xffff0000u)));
+        *reinterpret_cast<uint2*>(p.act + t * half + n) = make_uint2(o[0], o[1]);
+      }
+    }
+    if (!GLU && !*abort_flag) {
       const int rows = min(share, p.M - rank * share);   // none: a block beyond the last share
       const bool wide = (p.ldd & 3) == 0 && (reinterpret_cast<uintptr_t>(p.D) & 7) == 0;
       const float4* parts = reinterpret_cast<const float4*>(smem);
@@ -231,10 +265,10 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
   }
 }
 
-template <int NT>
+template <int NT, bool GLU>
 int launch(const void* X, const void* W, int lda, int ldb, const Params& p, cudaStream_t stream) {
   using L = Layout<NT>;
-  auto kern = gemm_rows_kernel<NT>;
+  auto kern = gemm_rows_kernel<NT, GLU>;
   static bool configured = false;
   if (!configured) {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kTotal);
@@ -244,7 +278,7 @@ int launch(const void* X, const void* W, int lda, int ldb, const Params& p, cuda
   CUtensorMap tw, tx;
   int r = vlmt_make_tmap_2d_bf16(&tx, X, (uint64_t)p.K, (uint64_t)p.M, (uint64_t)lda * 2, 64, NT);
   if (r) return 1000 + r;
-  r = vlmt_make_tmap_2d_bf16(&tw, W, (uint64_t)p.K, (uint64_t)p.N, (uint64_t)ldb * 2, 64, 128);
+  r = vlmt_make_tmap_2d_bf16(&tw, W, (uint64_t)p.K, (uint64_t)p.N, (uint64_t)ldb * 2, 64, GLU ? 64 : 128);
   if (r) return 2000 + r;
   const int tiles = (p.N + BW - 1) / BW;
   return launch_pdl(kern, dim3(tiles * p.splits), dim3(NUM_THREADS), L::kTotal, stream, p.splits, tw, tx, p);
@@ -274,21 +308,38 @@ extern "C" int vlmt_gemm_rows_splits(int M, int N, int K, int num_sms) {
   return (num_kb + kb_per - 1) / kb_per;   // every block has a part
 }
 
+namespace {
+template <bool GLU>
+int dispatch(const void* X, const void* W, int lda, int ldb, Params& p, int splits, int num_sms, cudaStream_t stream) {
+  const int num_kb = (p.K + BK - 1) / BK;
+  p.splits = splits; p.kb_per = (num_kb + splits - 1) / splits;
+  if (splits < 1 || splits > 8 || p.M < 1 || p.M > 128 || (splits - 1) * p.kb_per >= num_kb) return -50;   // every block has a part of K
+  p.prefetch_blocks = 2 * num_sms;
+  if (p.M <= 16) return launch<16, GLU>(X, W, lda, ldb, p, stream);
+  if (p.M <= 32) return launch<32, GLU>(X, W, lda, ldb, p, stream);
+  if (p.M <= 48) return launch<48, GLU>(X, W, lda, ldb, p, stream);
+  if (p.M <= 64) return launch<64, GLU>(X, W, lda, ldb, p, stream);
+  if (p.M <= 96) return launch<96, GLU>(X, W, lda, ldb, p, stream);
+  return launch<128, GLU>(X, W, lda, ldb, p, stream);
+}
+}  // namespace
+
 extern "C" int vlmt_gemm_rows(const void* X, const void* W, void* D, const void* bias, int M, int N, int K, int lda, int ldb, int ldd, int epilogue,
                               const float* alpha, int splits, int* status, int num_sms, cudaStream_t stream) {
-  const int num_kb = (K + BK - 1) / BK;
-  Params p;
+  Params p = {};
   p.M = M; p.N = N; p.K = K; p.ldd = ldd;
-  p.splits = splits; p.kb_per = (num_kb + splits - 1) / splits;
-  if (splits < 1 || splits > 8 || M < 1 || M > 128 || (splits - 1) * p.kb_per >= num_kb) return -50;   // every block has a part of K
-  p.prefetch_blocks = 2 * num_sms;
   p.D = reinterpret_cast<__nv_bfloat16*>(D);
   p.bias = reinterpret_cast<const __nv_bfloat16*>(bias);
   p.alpha = alpha; p.epilogue = epilogue; p.status = status;
-  if (M <= 16) return launch<16>(X, W, lda, ldb, p, stream);
-  if (M <= 32) return launch<32>(X, W, lda, ldb, p, stream);
-  if (M <= 48) return launch<48>(X, W, lda, ldb, p, stream);
-  if (M <= 64) return launch<64>(X, W, lda, ldb, p, stream);
-  if (M <= 96) return launch<96>(X, W, lda, ldb, p, stream);
-  return launch<128>(X, W, lda, ldb, p, stream);
+  return dispatch<false>(X, W, lda, ldb, p, splits, num_sms, stream);
+}
+
+extern "C" int vlmt_gemm_rows_glu(const void* X, const void* W, void* gu, void* act, int M, int I, int K, int lda, int ldb, int splits, int* status,
+                                  int num_sms, cudaStream_t stream) {
+  Params p = {};
+  p.M = M; p.N = 2 * I; p.K = K; p.ldd = 2 * I;
+  p.D = reinterpret_cast<__nv_bfloat16*>(gu);
+  p.act = reinterpret_cast<__nv_bfloat16*>(act);
+  p.status = status;
+  return dispatch<true>(X, W, lda, ldb, p, splits, num_sms, stream);
 }
