@@ -607,3 +607,59 @@ def test_blocks_in_one_call(preset, layer, block):
             assert torch.equal(s, t)
     if handle is not None:
         handle.remove()
+
+
+def test_expert_gradients_are_stored_only_over_zeros():
+    """The first gradient behind a clearing is stored, every other one is added: accumulation, a step, a clearing by hand, and gradients that
+    the caller has written into meanwhile."""
+    from vlm_training_b200.config import Config
+    from vlm_training_b200.parallel.mesh import get_mesh
+    from vlm_training_b200.train.optimizer import create_optimizer
+
+    T, H, I, E, k = 300, 256, 128, 8, 2
+    m = torch.nn.Module()
+    m.gate_up_proj, m.down_proj = (torch.nn.Parameter(_rand(*s, scale=0.05)) for s in ((E, 2 * I, H), (E, H, I)))
+    t = Config().training
+    t.lr_llm = t.lr_mlp = t.lr_vit = 1e-3
+    t.data_parallel = "fsdp"
+    engine = create_optimizer(m, t, get_mesh(1, torch.device(DEV)))
+    engine.set_requires_gradient_sync(False)   # no update under a backward pass that no step follows
+    x, dy = _rand(T, H), _rand(T, H)
+    w, chosen = ops.moe_router(_rand(T, E)[:, :E - 1].contiguous(), k)   # the last expert gets no token
+
+    def backward():
+        ops.moe_experts(x, m.gate_up_proj, m.down_proj, w.to(x.dtype), chosen).backward(dy)
+
+    ps = m.gate_up_proj, m.down_proj
+    alone = [torch.autograd.grad(ops.moe_experts(x, *ps, w.to(x.dtype), chosen), ps, dy)[i] for i in range(2)]
+    for p in ps:
+        assert not bool(p.grad.any())
+    backward()                                                # over the zeros of a new engine
+    for p, a in zip(ps, alone):
+        assert torch.equal(p.grad, a) and not bool(p.grad[-1].any())
+    backward()                                                # added
+    for p, a in zip(ps, alone):
+        assert torch.equal(p.grad, a + a)
+    engine.zero_grad()
+    for p in ps:
+        assert not bool(p.grad.any())
+        p.grad.add_(1.0)                                      # the caller's own part
+    backward()
+    for p, a in zip(ps, alone):
+        torch.testing.assert_close(p.grad.float(), a.float() + 1, atol=0, rtol=8e-3)   # one bf16 rounding of the sum
+    engine.zero_grad()
+    engine.set_requires_gradient_sync(True)
+    backward()
+    engine.step()
+    engine.set_requires_gradient_sync(False)
+    for p in ps:
+        assert not bool(p.grad.any())                         # cleared by the update
+    engine.zero_grad()
+    alone = torch.autograd.grad(ops.moe_experts(x, *ps, w.to(x.dtype), chosen), ps, dy)
+    backward()
+    for p, a in zip(ps, alone):
+        assert torch.equal(p.grad, a)
+    engine.zero_grad()
+    ps[0].grad = torch.full_like(ps[0], 2.0)                  # not the engine's buffer
+    backward()
+    torch.testing.assert_close(ps[0].grad.float(), alone[0].float() + 2, atol=0, rtol=8e-3)
