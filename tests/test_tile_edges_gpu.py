@@ -388,6 +388,25 @@ def test_grouped_weight_gradient_added_in_place(tiles, M, N):
     cu.check_status()
 
 
+# on CTA pairs: columns off the tile edges, groups of one 128-row tile and of none, long enough groups added
+@pytest.mark.parametrize("tiles,M,N", [([1, 0, 3, 2], 512, 264), ([0, 1], 256, 520), ([4, 6], 256, 256)])
+def test_grouped_weight_gradient_on_cta_pairs(tiles, M, N):
+    from vlm_training_b200.ops import cuda as cu
+
+    first = [sum(tiles[:i]) for i in range(len(tiles) + 1)]
+    prefix = torch.tensor(first, dtype=torch.int32, device=DEV)
+    a, b = _rand(first[-1] * 128, M, scale=0.5), _rand(first[-1] * 128, N, scale=0.5)
+    want = torch.cat([a[128 * s:128 * e].float().t() @ b[128 * s:128 * e].float() for s, e in zip(first[:-1], first[1:])])
+    out = torch.full((len(tiles) * M, N), 7.0, dtype=torch.bfloat16, device=DEV)
+    cu._C.gemm_grouped(a, b, out, prefix, 2, True, False)
+    torch.testing.assert_close(out.float(), want, atol=1e-3, rtol=8e-3)   # one bf16 rounding; a group without rows is zero
+    base = _rand(len(tiles) * M, N)
+    acc = base.clone()
+    cu._C.gemm_grouped(a, b, acc, prefix, 2, True, True)
+    assert torch.equal(acc, base + out)
+    cu.check_status()
+
+
 def _reference(fn):
     import vlm_training_b200.ops as O
 

@@ -961,6 +961,10 @@ int gemm_launch(const void* A, const void* B, void* D, float* Dacc32, const void
   p.M = M; p.N = N; p.K = K; p.ldd = ldd;
   p.grp_prefix = x.grp_prefix; p.grp_count = x.grp_count; p.grp_mode = x.grp_mode; p.grp_b_rows = x.grp_b_rows;
   if (p.grp_mode == 2 && !p.tma_store) return -30;  // grouped wgrad writes through the TMA-store epilogue only
+  // CTA pairs store a group's gradient faster; added to D they are the slower ones until groups have about 512 rows (256 groups, us, one block / pairs:
+  // 320 rows of 1024 x 2048 stored 371 / 359, added 451 / 558; 576 rows 580 / 525 and 646 / 582)
+  if (p.grp_mode == 2 && M % 256 == 0 && N >= 256 && (!accumulate || K >= 512l * x.grp_count) && vlmt_gemm_pair_enabled())
+    return vlmt_gemm_pair_grouped(A, B, D, x.grp_prefix, x.grp_count, M, N, K, lda, ldb, ldd, accumulate, status, stream);
   p.D = reinterpret_cast<__nv_bfloat16*>(D);
   p.bias = reinterpret_cast<const __nv_bfloat16*>(bias);
   p.Dacc32 = Dacc32;
