@@ -310,7 +310,35 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
                                swiglu_f(__uint_as_float(g[i] & 0xffff0000u), __uint_as_float(u[i] & 0xffff0000u)));
           put(g, &tmap_act, col);
         }
-      } else
+      } else if (!FP8 && alpha == 1.f && p.bias == nullptr && p.epilogue == GEMM_EPI_NONE && !empty) {
+        // the next slab's columns come out of tensor memory while this one is converted and staged
+        uint32_t r[2][2][32];
+        auto fetch = [&](int c) {
+          tmem_ld_32x32(taddr + c * 64, r[c & 1][0]);
+          tmem_ld_32x32(taddr + c * 64 + 32, r[c & 1][1]);
+        };
+        if (row0 < p.M) {
+          fetch(0);
+#pragma unroll
+          for (int c = 0; c < BN / 64; ++c) {
+            const int col0 = n0 + c * 64;
+            tmem_ld_wait();
+            if (col0 >= p.N) break;
+            if (c + 1 < BN / 64) fetch(c + 1);
+            uint8_t* buf = out + (slab++ & 1) * 4096;
+            if (lane == 0) tma_store_wait_read<1>();   // the store issued two slabs ago has finished reading this buffer
+            __syncwarp();
+            stage_slab(buf, lane, r[c & 1][0], r[c & 1][1]);
+            fence_async_proxy();
+            __syncwarp();
+            if (lane == 0) {
+              if (p.accumulate) tma_reduce_add_2d(&tmap_d, buf, col0, d_row0 + row0);
+              else tma_store_2d(&tmap_d, buf, col0, d_row0 + row0);
+              tma_store_commit();
+            }
+          }
+        }
+      } else {
 #pragma unroll 1
       for (int c = 0; c < BN / 64; ++c) {
         const int col0 = n0 + c * 64;
@@ -336,6 +364,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
           else tma_store_2d(&tmap_d, buf, col0, d_row0 + row0);
           tma_store_commit();
         }
+      }
       }
       tc_fence_before();
       __syncwarp();

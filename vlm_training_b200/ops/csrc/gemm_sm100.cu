@@ -501,6 +501,39 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
             for (int i = 0; i < 32; i += 4) *reinterpret_cast<uint4*>(part + c * 32 + i) = make_uint4(r[i], r[i + 1], r[i + 2], r[i + 3]);
           }
         }
+      } else if (p.tma_store && alpha == 1.f && p.bias == nullptr && p.epilogue == GEMM_EPI_NONE && !empty_group) {
+        // 64-column slabs: TMEM -> registers -> bf16 -> swizzled smem -> one TMA store per slab and warp; the next slab's columns are on their way meanwhile
+        uint8_t* stage = smem + L::kOutOffset + q * 8192;
+        uint32_t r[2][2][32];
+        auto fetch = [&](int c) {
+          tmem_ld_32x32(taddr + c * 64, r[c & 1][0]);
+          tmem_ld_32x32(taddr + c * 64 + 32, r[c & 1][1]);
+        };
+        fetch(0);
+#pragma unroll
+        for (int c = 0; c < BN / 64; ++c) {
+          const int col0 = n0 + c * 64;
+          tmem_ld_wait();
+          if (col0 >= p.N) break;
+          if (c + 1 < BN / 64) fetch(c + 1);
+          uint8_t* buf = stage + (slab++ & 1) * 4096;
+          if (lane == 0) tma_store_wait_read<1>();  // the store issued two slabs ago has finished reading this buffer
+          __syncwarp();
+          stage_slab(buf, lane, r[c & 1][0], r[c & 1][1]);
+          fence_async_proxy();
+          __syncwarp();
+          if (lane == 0) {
+            if (p.rs_world > 0) {  // the tile's rows belong to one owner (rs_rows is a multiple of the tile height)
+              const int owner = (tm * BM) / p.rs_rows;
+              tma_store_2d(&rs_maps.m[owner], buf, col0, tm * BM - owner * p.rs_rows + q * 32);
+            } else if (p.accumulate) {
+              tma_reduce_add_2d(&tmap_d, buf, col0, d_row0 + tm * BM + q * 32);
+            } else {
+              tma_store_2d(&tmap_d, buf, col0, d_row0 + tm * BM + q * 32);
+            }
+            tma_store_commit();
+          }
+        }
       } else if (p.tma_store) {
         // 64-column slabs: TMEM -> registers -> (bias / GELU) -> bf16 -> swizzled smem -> one TMA store per slab and warp
         uint8_t* stage = smem + L::kOutOffset + q * 8192;
