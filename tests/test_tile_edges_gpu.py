@@ -682,3 +682,34 @@ def test_expert_gradients_are_stored_only_over_zeros():
     ps[0].grad = torch.full_like(ps[0], 2.0)                  # not the engine's buffer
     backward()
     torch.testing.assert_close(ps[0].grad.float(), alone[0].float() + 2, atol=0, rtol=8e-3)
+
+
+# rows of one id in a block of 32 neighbours, over its edge, over several blocks, and all of them; a last block with one row; a second chunk of columns
+@pytest.mark.parametrize("counts", [(1,), (32, 1), (31, 2, 5), (33, 64, 96), (7, 500, 1, 1, 90), (1000,), ()])
+@pytest.mark.parametrize("D", [8, 1032])
+def test_embedding_gradient_in_place(counts, D):
+    n = sum(counts)
+    ids = torch.cat([torch.full((c,), 3 * i, device=DEV) for i, c in enumerate(counts)] + [torch.empty(0, dtype=torch.long, device=DEV)])
+    ids = ids[torch.randperm(n, device=DEV)]
+    w = torch.nn.Parameter(_rand(20, D))
+    w._vlmt_grad_in_place = True
+    start = _rand(20, D)
+    w.grad = start.clone()
+    seen = []
+    w._vlmt_grad_ready = seen.append
+    dy = _rand(n, D)
+    y = ops.embedding(ids, w, grad_in_place=True)
+    assert torch.equal(y, w.detach()[ids])
+    y.backward(dy)
+    want = start.double().index_add(0, ids, dy.double())
+    # fp32 sums of up to 1000 values of size 1, then one bf16 rounding of the sum
+    torch.testing.assert_close(w.grad.double(), want, atol=1e-4, rtol=4e-3)
+    assert len(seen) == 1 and seen[0] is w
+    first, w.grad = w.grad, start.clone()
+    ops.embedding(ids, w, grad_in_place=True).backward(dy)
+    assert torch.equal(w.grad, first)
+    # whoever asks for the gradient, or waits for it, gets the dense one
+    w.grad = start.clone()
+    dense, = torch.autograd.grad(ops.embedding(ids, w, grad_in_place=True), w, dy)
+    plain, = torch.autograd.grad(torch.nn.functional.embedding(ids, w), w, dy)
+    assert torch.equal(dense, plain) and torch.equal(w.grad, start)

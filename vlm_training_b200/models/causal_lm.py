@@ -190,7 +190,7 @@ class _CausalLMBase(nn.Module):
             if T % tp.size:
                 raise ValueError(f"sequence parallelism needs the row length ({T}) divisible by tp={tp.size}")
             lo, hi = tp.rank * (T // tp.size), (tp.rank + 1) * (T // tp.size)
-        x = ops.embedding(ids[lo:hi], dec.embed_tokens.weight)
+        x = ops.embedding(ids[lo:hi], dec.embed_tokens.weight, grad_in_place=not self.config.text.tie_word_embeddings)
         deepstack = None
         if pixel_values is not None and self.visual is not None:
             if tp is not None and tp.enabled:

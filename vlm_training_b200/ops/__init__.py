@@ -309,5 +309,9 @@ def pos_embed_add(x, table, plan, merge: int):
     return x + (pe.float() * weight.unsqueeze(-1)).sum(0).to(x.dtype)
 
 
-def embedding(ids, weight):
+def embedding(ids, weight, grad_in_place: bool = False):
+    """``grad_in_place``: nothing else of the forward pass reads the weight, so its gradient may be added to ``.grad`` where the optimizer engine allows it
+    (a tied output head's may not)."""
+    if grad_in_place and _use_cuda(weight) and ids.dtype == torch.int64:
+        return _cu()._C.op_embedding(ids, weight)
     return torch.nn.functional.embedding(ids, weight)

@@ -920,6 +920,51 @@ std::vector<Tensor> rope_tables(const Tensor& pos, const Tensor& inv_freq, int64
   return {c, s};
 }
 
+// ------------------------------------------------------------------ embedding
+// Rows of a table; the gradient of a tagged table is added to .grad row by row (loss_optim.cu) instead of as a dense tensor of the table's size.
+struct Embedding : torch::autograd::Function<Embedding> {
+  static Tensor forward(AutogradContext* ctx, const Tensor& ids, const Tensor& w, CfgPtr c) {
+    c->n_q = w.size(0);
+    keep(ctx, c);
+    ctx->save_for_backward({ids});
+    return at::embedding(w, ids);
+  }
+  static variable_list backward(AutogradContext* ctx, variable_list grads) {
+    auto c = kept(ctx);
+    Tensor ids = ctx->get_saved_variables()[0], dy = grads[0];
+    if (may_add(c->t[0])) {
+      Tensor g = c->t[0]->param.grad();
+      if (g.defined() && g.scalar_type() == at::kBFloat16 && dy.scalar_type() == at::kBFloat16 && g.dim() == 2 && g.size(0) == c->n_q &&
+          g.size(1) == dy.size(-1) && g.is_contiguous() && g.size(1) % 8 == 0 && reinterpret_cast<uintptr_t>(g.data_ptr()) % 16 == 0) {
+        check_storage(g);
+        c10::cuda::CUDAGuard guard(g.device());
+        const int64_t T = ids.numel(), D = g.size(1);
+        Tensor rows = dy.contiguous().view({T, D});
+        if (reinterpret_cast<uintptr_t>(rows.data_ptr()) % 16 != 0) rows = rows.clone();
+        auto sorted = ids.reshape({-1}).sort(/*stable=*/true, 0, false);
+        Tensor part = torch::empty({vlmt_embed_blocks((int)T), 2, D}, g.options().dtype(at::kFloat));
+        const int r = vlmt_embed_bwd(rows.data_ptr(), std::get<0>(sorted).data_ptr<int64_t>(), std::get<1>(sorted).data_ptr<int64_t>(), (int)T, (int)D,
+                                     g.data_ptr(), part.data_ptr<float>(), cur_stream());
+        TORCH_CHECK(r == 0, "vlmt_embed_bwd failed with code ", r);
+        tick(2);
+        c->t[0]->report();
+        return {Tensor(), Tensor(), Tensor()};
+      }
+    }
+    return {Tensor(), at::embedding_dense_backward(dy, ids, c->n_q, -1, false), Tensor()};
+  }
+};
+Tensor op_embedding(const Tensor& ids, const py::object& w_) {
+  return guarded([&] {
+    Tensor w = w_.cast<Tensor>();
+    if (no_graph(w)) return at::embedding(w, ids);
+    auto c = c10::make_intrusive<Cfg>();
+    c->t[0] = target_of(w_);
+    if (!c->t[0] || !w.requires_grad()) return at::embedding(w, ids);   // autograd's own
+    return Embedding::apply(ids, w, c);
+  });
+}
+
 // ------------------------------------------------------------------ whole blocks
 // A decoder layer and the blocks of the vision tower as one binding call each: the functions above in the order in which the modules call them one by
 // one, so graph, gradients and results are the same; what is saved is the interpreter between them (a step of the smallest vision model, bound by the
@@ -1049,6 +1094,7 @@ void bind_autograd(py::module_& m) {
     return guarded([&] { return RowsUpdate::apply(x, index, src, add); });
   });
   m.def("op_pos_embed", &op_pos_embed);
+  m.def("op_embedding", &op_embedding);
   m.def("op_decoder_layer", &op_decoder_layer);
   m.def("op_vision_block", &op_vision_block);
   m.def("op_patch_merger", &op_patch_merger);

@@ -392,6 +392,107 @@ __global__ void __launch_bounds__(256) sum_rows_kernel(const __grid_constant__ V
   }
 }
 
+// ------------------------------------------------------------------ gradient of an embedding table, added in place
+// Rows of dy that belong to one id are neighbours in the order `perm` of the sorted ids.  A block takes kEmbRows neighbours and 1024 columns and adds each
+// run of equal ids in fp32, in order: a run that lies inside goes to the table's gradient with one rounding, the part of one that began before (slot 0)
+// or goes on behind (slot 1) to `part` [blocks][2][D], and embed_join_kernel adds those in order for the run's first block.  An id may hold thousands of
+// rows (image placeholders), so runs are not walked by one block.  A dense gradient of the table, its fill, and its addition to .grad moved 1.2 GB three
+// times for 8192 rows of 67 MB: 151936 x 4096, 7600 of 8192 ids equal 1239 -> 187 us, 640 ids 890 -> 69 us, sorting the ids included.
+constexpr int kEmbRows = 32, kEmbThreads = 128, kEmbJoinThreads = 32;
+__device__ __forceinline__ void add_row8(bf16* g, const float (&a)[8]) {
+  uint4 o = *reinterpret_cast<const uint4*>(g);
+  uint32_t w[4] = {o.x, o.y, o.z, o.w};
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const __nv_bfloat162 b = __floats2bfloat162_rn(__uint_as_float(w[j] << 16) + a[2 * j], __uint_as_float(w[j] & 0xffff0000u) + a[2 * j + 1]);
+    w[j] = *reinterpret_cast<const uint32_t*>(&b);
+  }
+  *reinterpret_cast<uint4*>(g) = make_uint4(w[0], w[1], w[2], w[3]);
+}
+__device__ __forceinline__ void put_part8(float* p, const float (&a)[8]) {
+  reinterpret_cast<float4*>(p)[0] = make_float4(a[0], a[1], a[2], a[3]);
+  reinterpret_cast<float4*>(p)[1] = make_float4(a[4], a[5], a[6], a[7]);
+}
+__global__ void __launch_bounds__(kEmbThreads) embed_runs_kernel(const bf16* __restrict__ dy, const long* __restrict__ ids, const long* __restrict__ perm, int T,
+                                                                 int D, bf16* __restrict__ grad, float* __restrict__ part) {
+  pdl_begin();
+  __shared__ long id[kEmbRows + 2];   // the neighbours' ids on both sides too (-1: none)
+  __shared__ int row[kEmbRows];
+  const int p0 = blockIdx.x * kEmbRows, n = min(kEmbRows, T - p0);
+  for (int i = threadIdx.x; i < n + 2; i += kEmbThreads) {
+    const int p = p0 + i - 1;
+    id[i] = p >= 0 && p < T ? ids[p] : -1;
+    if (i < n) row[i] = (int)perm[p0 + i];
+  }
+  __syncthreads();
+  const int c = (blockIdx.y * kEmbThreads + threadIdx.x) * 8;
+  if (c >= D) return;
+  float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+  bool before = id[0] == id[1];        // the current run began in a block before
+  constexpr int U = 8;
+  for (int i0 = 0; i0 < n; i0 += U) {
+    uint4 v[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) if (i0 + u < n) v[u] = *reinterpret_cast<const uint4*>(dy + (size_t)row[i0 + u] * D + c);
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int i = i0 + u;
+      if (i >= n) break;
+      const uint32_t w4[4] = {v[u].x, v[u].y, v[u].z, v[u].w};
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        acc[2 * j] += __uint_as_float(w4[j] << 16);
+        acc[2 * j + 1] += __uint_as_float(w4[j] & 0xffff0000u);
+      }
+      const bool ends = id[i + 2] != id[i + 1];   // the run ends with this row
+      if (ends || i == n - 1) {
+        if (before) put_part8(part + ((size_t)blockIdx.x * 2) * D + c, acc);
+        else if (!ends) put_part8(part + ((size_t)blockIdx.x * 2 + 1) * D + c, acc);
+        else add_row8(grad + (size_t)id[i + 1] * D + c, acc);
+        before = false;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) acc[j] = 0.f;
+      }
+    }
+  }
+}
+// runs that go on behind the block in which they begin; one warp per block, since one long run is all that there is to do
+__global__ void __launch_bounds__(kEmbJoinThreads) embed_join_kernel(const long* __restrict__ ids, int T, int D, bf16* __restrict__ grad,
+                                                                 const float* __restrict__ part) {
+  pdl_begin();
+  const int p0 = blockIdx.x * kEmbRows, last = p0 + kEmbRows - 1;
+  if (last + 1 >= T) return;
+  const long id = ids[last];
+  if (ids[last + 1] != id || (p0 > 0 && ids[p0] == id && ids[p0 - 1] == id)) return;   // ends here, or began in a block before
+  const int c = (blockIdx.y * kEmbJoinThreads + threadIdx.x) * 8;
+  if (c >= D) return;
+  float acc[8];
+  const float* p = part + ((size_t)blockIdx.x * 2 + 1) * D + c;
+#pragma unroll
+  for (int j = 0; j < 8; ++j) acc[j] = p[j];
+  constexpr int U = 16;   // parts in flight: one at a time, by 128 threads a block, took 119 us for 7600 placeholders, now 47
+  bool more = true;
+  for (int b0 = blockIdx.x + 1; more; b0 += U) {
+    bool on[U];
+    float4 v[U][2];
+#pragma unroll
+    for (int u = 0; u < U; ++u) on[u] = (long)(b0 + u) * kEmbRows < T && ids[(b0 + u) * kEmbRows] == id;   // sorted: none follows the first that is not
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const float4* q = reinterpret_cast<const float4*>(part + (size_t)(b0 + u) * 2 * D + c);
+      v[u][0] = on[u] ? q[0] : make_float4(0.f, 0.f, 0.f, 0.f);
+      v[u][1] = on[u] ? q[1] : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      acc[0] += v[u][0].x; acc[1] += v[u][0].y; acc[2] += v[u][0].z; acc[3] += v[u][0].w;
+      acc[4] += v[u][1].x; acc[5] += v[u][1].y; acc[6] += v[u][1].z; acc[7] += v[u][1].w;
+    }
+    more = on[U - 1];
+  }
+  add_row8(grad + (size_t)id * D + c, acc);
+}
+
 // sum of squares of a flat bf16/fp32 range -> out[0] (atomic; used for gradient clipping)
 template <typename GT>
 __global__ void sumsq_kernel(const GT* __restrict__ x, long n, float* __restrict__ out) {
@@ -494,6 +595,16 @@ int vlmt_colsum(const void* x, long ld, int rows, int cols, float* partial, void
 void vlmt_sum_rows(const VlmtRowSums* a, int sums, int rows, int cols, cudaStream_t st) {
   if (cols <= 0 || sums <= 0) return;
   launch_pdl(sum_rows_kernel, dim3((cols + 15) / 16, sums), dim3(256), 0, st, 1, *a, rows, cols);
+}
+int vlmt_embed_blocks(int T) { return (T + kEmbRows - 1) / kEmbRows; }
+// grad[ids[i]] += dy[perm[i]] for the sorted ids; D a multiple of 8, rows on 16 bytes; part: 2 x vlmt_embed_blocks(T) x D floats
+int vlmt_embed_bwd(const void* dy, const long* ids, const long* perm, int T, int D, void* grad, float* part, cudaStream_t st) {
+  if (T <= 0) return 0;
+  const dim3 grid(vlmt_embed_blocks(T), (D / 8 + kEmbThreads - 1) / kEmbThreads);
+  int r = launch_pdl(embed_runs_kernel, grid, dim3(kEmbThreads), 0, st, 1, reinterpret_cast<const bf16*>(dy), ids, perm, T, D, reinterpret_cast<bf16*>(grad), part);
+  const dim3 jgrid(grid.x, (D / 8 + kEmbJoinThreads - 1) / kEmbJoinThreads);
+  if (r == 0) r = launch_pdl(embed_join_kernel, jgrid, dim3(kEmbJoinThreads), 0, st, 1, ids, T, D, reinterpret_cast<bf16*>(grad), part);
+  return r;
 }
 void vlmt_sumsq(const void* x, int fp32, long n, float* out, cudaStream_t st) {
   if (n <= 0) return;

@@ -27,6 +27,8 @@ int vlmt_adamw_bucket(void* grad, float* master, void* m, void* v, int state_bf1
 void vlmt_sum_rows(const struct VlmtRowSums* a, int sums, int rows, int cols, cudaStream_t st);
 int vlmt_colsum_slabs(int rows);   // 0: no partial sums in memory
 int vlmt_colsum(const void* x, long ld, int rows, int cols, float* partial, void* out, int mode, cudaStream_t st);
+int vlmt_embed_blocks(int T);
+int vlmt_embed_bwd(const void* dy, const long* ids, const long* perm, int T, int D, void* grad, float* part, cudaStream_t st);
 void vlmt_sumsq(const void* x, int fp32, long n, float* out, cudaStream_t st);
 #ifdef __cplusplus
 }
