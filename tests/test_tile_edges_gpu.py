@@ -713,3 +713,19 @@ def test_embedding_gradient_in_place(counts, D):
     dense, = torch.autograd.grad(ops.embedding(ids, w, grad_in_place=True), w, dy)
     plain, = torch.autograd.grad(torch.nn.functional.embedding(ids, w), w, dy)
     assert torch.equal(dense, plain) and torch.equal(w.grad, start)
+
+
+# tiles of 128 rows x 64 columns, patches of 4 rows x 8 columns: remainders of each, a gap between the rows, the transpose alone and not at all
+@pytest.mark.parametrize("rows", [1, 3, 16, 127, 129, 255])
+@pytest.mark.parametrize("cols,fmt", [(16, 0), (48, 1), (64, 0), (80, 1), (208, 0)])
+def test_cast_tiles(rows, cols, fmt):
+    from vlm_training_b200.ops import cuda as cu
+    from vlm_training_b200.ops.float8 import quantize_ref
+
+    x = _rand(rows, cols + 24)[:, :cols]
+    want = quantize_ref(x, fmt)[0].view(torch.uint8)
+    for rm, t in ((True, True), (False, True), (True, False)):
+        q, qt, rec = cu._C.fp8_quantize(x, fmt, rm, t)
+        assert float(rec[0]) == float(x.abs().max())
+        assert q.numel() == 0 if not rm else torch.equal(q, want)
+        assert qt.numel() == 0 if not t else torch.equal(qt, want.t())
