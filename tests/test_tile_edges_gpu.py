@@ -729,3 +729,22 @@ def test_cast_tiles(rows, cols, fmt):
         assert float(rec[0]) == float(x.abs().max())
         assert q.numel() == 0 if not rm else torch.equal(q, want)
         assert qt.numel() == 0 if not t else torch.equal(qt, want.t())
+
+
+# gradient of gate and up in the kernel of the down projection's input gradient: the bits of the product and the activation kernel behind one another;
+# rows and columns off the tile edges, a short contraction, an empty half tile of rows, the activation wanted or not; sizes without such a kernel
+@pytest.mark.parametrize("M,I,K,there", [(4000, 9728, 72, True), (8321, 4800, 520, True), (16130, 2496, 264, True), (8192, 12288, 1024, True),
+                                         (8192, 4680, 520, False), (2049, 4864, 520, False), (37, 12288, 4096, False), (300, 256, 512, False)])
+def test_gate_up_gradient_with_its_product(M, I, K, there):
+    from vlm_training_b200.ops import cuda as cu
+
+    dy, w, gu = _rand(M, K, scale=0.5), _rand(K, I, scale=0.05), _rand(M, 2 * I)
+    got = cu._C.gemm_glu_bwd(dy, w, gu, True)
+    assert (got is not None) == there
+    if there:
+        d = torch.empty(M, I, dtype=torch.bfloat16, device=DEV)
+        cu._C.gemm(dy, w, d, False, True, None, 0, False)
+        assert torch.equal(got[0], cu._C.swiglu_bwd(d, gu)) and torch.equal(got[1], cu._C.op_swiglu(gu))
+        alone = cu._C.gemm_glu_bwd(dy, w, gu, False)
+        assert torch.equal(alone[0], got[0]) and alone[1] is None
+    cu.check_status()

@@ -86,6 +86,25 @@ bool gemm_glu(const Tensor& x, const Tensor& w, Tensor* gu, Tensor& act) {
   return r == 0;
 }
 
+// Gradients of gate and up from dy w, the gradient of silu(gate) * up, and that itself if asked for; false: nothing was done.
+bool gemm_glu_bwd(const Tensor& dy, const Tensor& w, const Tensor& gu, Tensor& dgu, Tensor* act) {
+  check_bf16(dy, "dy"); check_bf16(w, "w"); check_bf16(gu, "gu"); check_contig(gu, "gu");
+  TORCH_CHECK(dy.dim() == 2 && w.dim() == 2 && dy.stride(1) == 1 && w.stride(1) == 1 && dy.size(1) == w.size(0));
+  const int64_t M = dy.size(0), I = w.size(1);
+  TORCH_CHECK(gu.size(-1) == 2 * I && gu.numel() == M * 2 * I);
+  c10::cuda::CUDAGuard guard(dy.device());
+  if (I % 64 != 0 || M == 0) return false;
+  Tensor d = torch::empty_like(gu), a;
+  if (act != nullptr) a = torch::empty({M, I}, dy.options());
+  const int r = vlmt_gemm_bf16_glu_bwd(dy.data_ptr(), w.data_ptr(), gu.data_ptr(), d.data_ptr(), act != nullptr ? a.data_ptr() : nullptr, (int)M, (int)I,
+                                       (int)dy.size(1), (int)dy.stride(0), (int)w.stride(0), status_tensor().data_ptr<int>(), num_sms(), cur_stream());
+  TORCH_CHECK(r == 0 || r == 1, "vlmt_gemm_bf16_glu_bwd failed with code ", r);
+  if (r != 0) return false;
+  dgu = d;
+  if (act != nullptr) *act = a;
+  return true;
+}
+
 // y-partials of a row-parallel linear pushed to their owners: rows [o*R, (o+1)*R) of a @ b^T go to dst_ptrs[o]
 void gemm_rs_push(const Tensor& a, const Tensor& b, const std::vector<int64_t>& dst_ptrs, int64_t rows_per_rank, bool b_mn) {
   check_bf16(a, "a"); check_bf16(b, "b");
@@ -572,6 +591,12 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     Tensor gu, act;
     if (!gemm_glu(x, w, keep ? &gu : nullptr, act)) return py::none();
     return py::make_tuple(act, keep ? py::cast(gu) : py::object(py::none()));
+  });
+  // (gradient of gate and up, act or None), or None
+  m.def("gemm_glu_bwd", [](const Tensor& dy, const Tensor& w, const Tensor& gu, bool want_act) -> py::object {
+    Tensor dgu, act;
+    if (!gemm_glu_bwd(dy, w, gu, dgu, want_act ? &act : nullptr)) return py::none();
+    return py::make_tuple(dgu, want_act ? py::cast(act) : py::object(py::none()));
   });
   m.def("gemm_rs_push", &gemm_rs_push);
   m.def("gemm_ag", &gemm_ag);

@@ -399,6 +399,14 @@ Tensor op_gelu_linear(const Tensor& pre, const py::object& w_, const py::object&
 }
 
 // silu(gate) * up -> linear for a fused [T, 2 I] input, only the input is kept
+// Gradient of [gate, up] behind y = (silu(gate) * up) w^T; h (or null) gets silu(gate) * up.
+Tensor glu_grad(const Tensor& dy, const Tensor& w, const Tensor& gu, Tensor* h) {
+  check_storage(w);
+  Tensor dgu;
+  if (!gemm_glu_bwd(dy, w, gu, dgu, h)) dgu = swiglu_bwd(mm(dy, w, false, true), gu, h);
+  tick(1);
+  return dgu;
+}
 struct SwigluLinear : torch::autograd::Function<SwigluLinear> {
   static Tensor forward(AutogradContext* ctx, const Tensor& gu, const Tensor& w, CfgPtr c) {
     Tensor g = gu.contiguous(), wc = operand(w);
@@ -413,9 +421,8 @@ struct SwigluLinear : torch::autograd::Function<SwigluLinear> {
     auto saved = ctx->get_saved_variables();
     auto c = kept(ctx);
     Tensor dy = rows_of(grads[0]), dw;
-    Tensor h, dgu = swiglu_bwd(mm(dy, saved[1], false, true), saved[0], c->need[1] ? &h : nullptr);
+    Tensor h, dgu = glu_grad(dy, saved[1], saved[0], c->need[1] ? &h : nullptr);
     if (c->need[1]) dw = weight_grad(dy, h, c->t[0]);
-    tick(1);
     return {dgu, dw, Tensor()};
   }
 };
@@ -469,13 +476,13 @@ struct NormMlp : torch::autograd::Function<NormMlp> {
       dx = dr;
     } else {
       Tensor dy = rows_of(grads[0]), h, yn;
-      Tensor dgu = swiglu_bwd(mm(dy, wd, false, true), gu, c->need[4] ? &h : nullptr);
+      Tensor dgu = glu_grad(dy, wd, gu, c->need[4] ? &h : nullptr);
       if (c->need[4]) dwd = weight_grad(dy, h, c->t[2]);
       h.reset();
       auto b = rmsnorm_bwd_partial(mm(dgu, wgu, false, true), r, nw, rstd, dr.defined() ? OptTensor(dr.contiguous()) : OptTensor(), c->offset,
                                    c->need[3] ? &yn : nullptr);
       dx = b[0];
-      tick(2);
+      tick(1);
       if (c->need[3]) {
         if (!yn.defined()) { yn = rmsnorm_fwd(r, c10::nullopt, nw, c->eps, c->offset)[0]; tick(1); }
         dwgu = weight_grad(dgu, yn, c->t[1]);

@@ -26,6 +26,15 @@ __device__ __forceinline__ float gelu_erf_f(float x) { return 0.5f * x * (1.f + 
 // the operations of the activation kernels (elementwise.cu), on values that have been rounded to bf16
 __device__ __forceinline__ float swiglu_f(float g, float u) { return g * (1.f / (1.f + __expf(-g))) * u; }
 
+// dg, du and the activation itself from its gradient
+__device__ __forceinline__ void swiglu_grad_f(float d, float g, float u, float& dg, float& du, float& act) {
+  const float s = 1.f / (1.f + __expf(-g));
+  const float silu = g * s;
+  du = d * silu;
+  dg = d * u * (s + silu * (1.f - s));
+  act = silu * u;
+}
+
 // 32 columns of a row, from column `col`: bias (or null) and activation (GemmEpilogue)
 __device__ __forceinline__ void bias_activation(float (&v)[32], const __nv_bfloat16* bias, int col, int N, int epilogue) {
   if (bias != nullptr) {

@@ -53,7 +53,7 @@ struct Params {
   const float* rec_a;           // FP8: rec[1] undoes the operand's scaling
   const float* rec_b;
   uint32_t idesc;               // FP8: carries the two formats
-  int store_gu;                 // GLU: D is written
+  int store_gu;                 // GLU 1: D is written; GLU 2: the activation is
   // grouped weight gradients (both operands MN-major, see gemm_sm100.cu): group g contracts over its own rows, 128-row tiles grp_prefix[g] to
   // grp_prefix[g + 1], into the block of M rows of D that starts at g * M
   const int* grp_prefix;
@@ -107,10 +107,14 @@ __device__ __forceinline__ void store_parts(const uint8_t* smem, const Params& p
 
 // GLU (K-major operands): B is [gate; up] of N / 2 rows each.  The leader loads 128 rows of gate, its peer the same rows of up, so an accumulator row
 // has 128 columns of both, and the epilogue writes silu(gate) * up of the rounded values besides them, or alone (store_gu 0).
-template <bool A_MN, bool B_MN, bool FP8, bool GLU>
+// GLU 2 (B MN-major): the product is the gradient of silu(gate) * up, [M, N].  The epilogue reads gate and up ([M, 2 N], loaded a slab ahead into what
+// is the last operand stage otherwise) and writes their gradients into D, [M, 2 N], and silu(gate) * up for the weight gradient that follows.
+constexpr int kGlu = 1, kGluBwd = 2;
+template <bool A_MN, bool B_MN, bool FP8, int GLU>
 __global__ void __launch_bounds__(NUM_THREADS, 1)
 gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b, const __grid_constant__ CUtensorMap tmap_d,
-                 const __grid_constant__ CUtensorMap tmap_act, Params p) {
+                 const __grid_constant__ CUtensorMap tmap_act, const __grid_constant__ CUtensorMap tmap_gu, Params p) {
+    constexpr int NST = GLU == kGluBwd ? STAGES - 1 : STAGES;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + kBarOffset);
@@ -119,6 +123,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
   uint64_t* tmem_empty = tmem_full + 2;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tmem_empty + 2);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+  uint64_t* gu_bar = reinterpret_cast<uint64_t*>(tmem_slot + 2);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t rank = cluster_rank() & 1, lead = cluster_rank() & ~1u;   // place in the pair; its leader's rank in the cluster
@@ -132,8 +137,9 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
   const int num_kb = (p.K + kStageK - 1) / kStageK;
 
   if (threadIdx.x == 0) {
-    for (int s = 0; s < STAGES; ++s) { mbar_init(&full_bar[s], 1); mbar_init(&empty_bar[s], 1); }
+    for (int s = 0; s < NST; ++s) { mbar_init(&full_bar[s], 1); mbar_init(&empty_bar[s], 1); }
     for (int a = 0; a < 2; ++a) { mbar_init(&tmem_full[a], 1); mbar_init(&tmem_empty[a], 8); }
+    if (GLU == kGluBwd) for (int q = 0; q < 4; ++q) mbar_init(&gu_bar[q], 1);
     *abort_flag = 0;
     fence_mbar_init();
     tma_prefetch_desc(&tmap_a);
@@ -178,7 +184,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
         int tile, kb_lo, kb_hi, tm, tn;
         k_range(item, tile, kb_lo, kb_hi);
         tile_coords(p.group_m, tile, tiles_m, tiles_n, tm, tn);
-        const int m0 = (tm * 2 + (int)rank) * BM, n0 = GLU ? tn * (BN / 2) + (int)rank * (p.N / 2) : tn * BN + (int)rank * (BN / 2);
+        const int m0 = (tm * 2 + (int)rank) * BM, n0 = GLU == kGlu ? tn * (BN / 2) + (int)rank * (p.N / 2) : tn * BN + (int)rank * (BN / 2);
         for (int kb = kb_lo; kb < kb_hi; ++kb) {
           if (!mbar_wait(&empty_bar[stage], phase ^ 1, abort_flag, p.status, kErrTimeoutEmpty)) { ok = false; break; }
           uint8_t* sa = smem + stage * kStageBytes;
@@ -196,7 +202,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
 #pragma unroll
             for (int j = 0; j < BN / 128; ++j) tma_load_2d_pair(sb + j * 8192, &tmap_b, bar, n0 + 64 * j, k0);   // boxes {64 n, 64 k}
           }
-          if (++stage == STAGES) { stage = 0; phase ^= 1; }
+          if (++stage == NST) { stage = 0; phase ^= 1; }
         }
       }
       pdl_trigger();
@@ -228,7 +234,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
             else umma_ss_pair<1, FP8>(d_tmem, ad, bd, idesc);
           }
           umma_commit_pair(&empty_bar[stage], both);
-          if (++stage == STAGES) { stage = 0; phase ^= 1; }
+          if (++stage == NST) { stage = 0; phase ^= 1; }
         }
         if (ok) umma_commit_pair(&tmem_full[acc], both);
       }
@@ -240,6 +246,13 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
     uint8_t* out = smem + kOutOffset + q * 8192;
     int it = 0;
     uint32_t slab = 0;   // runs across items (see gemm_sm100.cu)
+    uint8_t* in = smem + NST * kStageBytes + q * 8192;   // GLU 2: a slab of gate and of up
+    uint32_t in_phase = 0;
+    auto load_gu = [&](int col, int row) {
+      mbar_expect_tx(&gu_bar[q], 8192);
+      tma_load_2d(in, &tmap_gu, &gu_bar[q], col, row);
+      tma_load_2d(in + 4096, &tmap_gu, &gu_bar[q], p.N + col, row);
+    };
     for (int item = pair; item < num_items; item += pairs, ++it) {
       const int tile = grouped || p.k_splits > 1 ? item % num_tiles : item;
       int tm, tn, d_row0 = 0;
@@ -251,9 +264,10 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
         empty = p.grp_prefix[g + 1] == p.grp_prefix[g];
       }
       const int acc = it & 1;
+      const int row0 = (tm * 2 + (int)rank) * BM + q * 32, n0 = tn * BN;
+      if (GLU == kGluBwd && lane == 0 && row0 < p.M) load_gu(n0, row0);
       if (!mbar_wait(&tmem_full[acc], (it >> 1) & 1, abort_flag, p.status, kErrTimeoutTmemFull)) break;
       tc_fence_after();
-      const int row0 = (tm * 2 + (int)rank) * BM + q * 32, n0 = tn * BN;
       const uint32_t taddr = tmem_base + acc * BN + ((uint32_t)(q * 32) << 16);
       if (p.parts > 1) {
         // the operand stages are free: every MMA of the pair's only item has completed
@@ -268,21 +282,63 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
         }
         break;
       }
-      if (GLU) {
-        auto put = [&](const uint32_t (&w)[32], const CUtensorMap* map, int col) {
-          uint8_t* buf = out + (slab++ & 1) * 4096;
-          if (lane == 0) tma_store_wait_read<1>();
-          __syncwarp();
+      auto put = [&](const uint32_t (&w)[32], const CUtensorMap* map, int col) {
+        uint8_t* buf = out + (slab++ & 1) * 4096;
+        if (lane == 0) tma_store_wait_read<1>();
+        __syncwarp();
 #pragma unroll
-          for (int t = 0; t < 8; ++t)
-            *reinterpret_cast<uint4*>(buf + lane * 128 + ((t ^ (lane & 7)) << 4)) = make_uint4(w[4 * t], w[4 * t + 1], w[4 * t + 2], w[4 * t + 3]);
-          fence_async_proxy();
-          __syncwarp();
-          if (lane == 0) {
-            tma_store_2d(map, buf, col, row0);
-            tma_store_commit();
+        for (int t = 0; t < 8; ++t)
+          *reinterpret_cast<uint4*>(buf + lane * 128 + ((t ^ (lane & 7)) << 4)) = make_uint4(w[4 * t], w[4 * t + 1], w[4 * t + 2], w[4 * t + 3]);
+        fence_async_proxy();
+        __syncwarp();
+        if (lane == 0) {
+          tma_store_2d(map, buf, col, row0);
+          tma_store_commit();
+        }
+      };
+      if (GLU == kGluBwd) {
+        bool ok = true;
+#pragma unroll 1
+        for (int c = 0; c < BN / 64; ++c) {
+          const int col = n0 + c * 64;   // N is a multiple of 64
+          if (row0 >= p.M || col >= p.N) break;
+          if (!mbar_wait(&gu_bar[q], in_phase, abort_flag, p.status, kErrTimeoutFull)) { ok = false; break; }
+          in_phase ^= 1;
+          uint32_t g[32], u[32], a[32];
+#pragma unroll
+          for (int t = 0; t < 8; ++t) {
+            const uint4 x = *reinterpret_cast<const uint4*>(in + lane * 128 + ((t ^ (lane & 7)) << 4));
+            const uint4 y = *reinterpret_cast<const uint4*>(in + 4096 + lane * 128 + ((t ^ (lane & 7)) << 4));
+            g[4 * t] = x.x; g[4 * t + 1] = x.y; g[4 * t + 2] = x.z; g[4 * t + 3] = x.w;
+            u[4 * t] = y.x; u[4 * t + 1] = y.y; u[4 * t + 2] = y.z; u[4 * t + 3] = y.w;
           }
-        };
+          fence_async_proxy();   // the loads above have returned before the next slab may be written: a converged warp's barrier does not wait for them
+          __syncwarp();
+          if (lane == 0 && c + 1 < BN / 64 && col + 64 < p.N) load_gu(col + 64, row0);
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            uint32_t r[32];
+            tmem_ld_32x32(taddr + c * 64 + h * 32, r);
+            tmem_ld_wait();
+#pragma unroll
+            for (int i = 0; i < 16; ++i) {   // the product is rounded to bf16 as if it were stored
+              const int j = h * 16 + i;
+              const uint32_t d = pack_bf16x2(__uint_as_float(r[2 * i]), __uint_as_float(r[2 * i + 1]));
+              float dg[2], du[2], act[2];
+              swiglu_grad_f(__uint_as_float(d << 16), __uint_as_float(g[j] << 16), __uint_as_float(u[j] << 16), dg[0], du[0], act[0]);
+              swiglu_grad_f(__uint_as_float(d & 0xffff0000u), __uint_as_float(g[j] & 0xffff0000u), __uint_as_float(u[j] & 0xffff0000u), dg[1], du[1],
+                            act[1]);
+              g[j] = pack_bf16x2(dg[0], dg[1]);
+              u[j] = pack_bf16x2(du[0], du[1]);
+              a[j] = pack_bf16x2(act[0], act[1]);
+            }
+          }
+          put(g, &tmap_d, col);
+          put(u, &tmap_d, p.N + col);
+          if (p.store_gu) put(a, &tmap_act, col);
+        }
+        if (!ok) break;
+      } else if (GLU == kGlu) {
 #pragma unroll 1
         for (int c = 0; c < BN / 128; ++c) {
           if (row0 >= p.M) break;
@@ -397,8 +453,10 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
   }
 }
 
-template <bool A_MN, bool B_MN, bool FP8 = false, bool GLU = false>
-int launch(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& td, const CUtensorMap& tact, const Params& p, cudaStream_t st) {
+template <bool A_MN, bool B_MN, bool FP8 = false, int GLU = 0>
+int launch(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& td, const CUtensorMap& tact, const Params& p, cudaStream_t st,
+           const CUtensorMap* tgu = nullptr) {
+  const CUtensorMap& tg = tgu != nullptr ? *tgu : td;
   auto kern = gemm_pair_kernel<A_MN, B_MN, FP8, GLU>;
   static int max_pairs = 0;
   static std::once_flag once;
@@ -417,10 +475,10 @@ int launch(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& td, 
   if (max_pairs <= 0) return -50;
   if (p.parts > 1) {
     const int tiles = ((p.M + 2 * BM - 1) / (2 * BM)) * ((p.N + BN - 1) / BN);
-    return launch_pdl(kern, dim3(2 * p.parts * tiles), dim3(NUM_THREADS), kSmem, st, 2 * p.parts, ta, tb, td, tact, p);
+    return launch_pdl(kern, dim3(2 * p.parts * tiles), dim3(NUM_THREADS), kSmem, st, 2 * p.parts, ta, tb, td, tact, tg, p);
   }
   const int items = ((p.M + 2 * BM - 1) / (2 * BM)) * ((p.N + BN - 1) / BN) * (p.grp_prefix != nullptr ? p.grp_count : p.k_splits);
-  return launch_pdl(kern, dim3(2 * (items < max_pairs ? items : max_pairs)), dim3(NUM_THREADS), kSmem, st, 2, ta, tb, td, tact, p);
+  return launch_pdl(kern, dim3(2 * (items < max_pairs ? items : max_pairs)), dim3(NUM_THREADS), kSmem, st, 2, ta, tb, td, tact, tg, p);
 }
 }  // namespace
 
@@ -434,7 +492,7 @@ extern "C" int vlmt_gemm_pair_clusters() {
   static int cap = 0;
   static std::once_flag once;
   std::call_once(once, [] {
-    auto kern = gemm_pair_kernel<false, false, false, false>;
+    auto kern = gemm_pair_kernel<false, false, false, 0>;
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute attr;
     attr.id = cudaLaunchAttributeClusterDimension;
@@ -504,7 +562,26 @@ extern "C" int vlmt_gemm_pair_glu(const void* X, const void* W, void* gu, void* 
   p.k_splits = 1; p.kb_per_split = (K + BK - 1) / BK; p.parts = 1; p.status = status;
   p.group_m = raster_group(4l * I * K, 2l * K);
   p.store_gu = gu != nullptr;
-  return launch<false, false, false, true>(ta, tb, td, tact, p, stream);
+  return launch<false, false, false, kGlu>(ta, tb, td, tact, p, stream);
+}
+
+// dgu[M, 2 I] and, if act is given, act[M, I] from dY(M,K) W(K,I) and gu[M, 2 I], I a multiple of 64
+extern "C" int vlmt_gemm_pair_glu_bwd(const void* dY, const void* W, const void* gu, void* dgu, void* act, int M, int I, int K, int ldy, int ldw,
+                                      int* status, cudaStream_t stream) {
+  CUtensorMap ta, tb, td, tact, tgu;
+  int r;
+  if ((r = vlmt_make_tmap_2d_bf16(&ta, dY, (uint64_t)K, (uint64_t)M, (uint64_t)ldy * 2, 64, 128))) return 1000 + r;
+  if ((r = vlmt_make_tmap_2d_bf16(&tb, W, (uint64_t)I, (uint64_t)K, (uint64_t)ldw * 2, 64, 64))) return 2000 + r;
+  if ((r = vlmt_make_tmap_2d_bf16(&td, dgu, (uint64_t)2 * I, (uint64_t)M, (uint64_t)I * 4, 64, 32))) return 3000 + r;
+  if ((r = vlmt_make_tmap_2d_bf16(&tgu, gu, (uint64_t)2 * I, (uint64_t)M, (uint64_t)I * 4, 64, 32))) return 4000 + r;
+  tact = td;
+  if (act != nullptr && (r = vlmt_make_tmap_2d_bf16(&tact, act, (uint64_t)I, (uint64_t)M, (uint64_t)I * 2, 64, 32))) return 3000 + r;
+  Params p = {};
+  p.M = M; p.N = I; p.K = K;
+  p.k_splits = 1; p.kb_per_split = (K + BK - 1) / BK; p.parts = 1; p.status = status;
+  p.group_m = raster_group(2l * I * K, 2l * K);
+  p.store_gu = act != nullptr;
+  return launch<false, true, false, kGluBwd>(ta, tb, td, tact, p, stream, &tgu);
 }
 
 extern "C" int vlmt_gemm_pair_fp8(const void* A, const void* B, void* D, int M, int N, int K, long lda, long ldb, long ldd, uint32_t idesc,

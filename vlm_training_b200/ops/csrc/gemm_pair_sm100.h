@@ -14,6 +14,8 @@ int vlmt_gemm_pair(const void* A, const void* B, void* D, const void* bias, int 
 int vlmt_gemm_pair_clusters();
 int vlmt_gemm_pair_grouped(const void* A, const void* B, void* D, const int* prefix, int groups, int M, int N, int rows, int lda, int ldb, int ldd,
                            int accumulate, int* status, cudaStream_t stream);
+int vlmt_gemm_pair_glu_bwd(const void* dY, const void* W, const void* gu, void* dgu, void* act, int M, int I, int K, int ldy, int ldw, int* status,
+                           cudaStream_t stream);
 int vlmt_gemm_pair_glu(const void* X, const void* W, void* gu, void* act, int M, int I, int K, int ldx, int ldw, int* status, cudaStream_t stream);
 // D (+)= rec_a[1] * rec_b[1] * A(M,K) * B(N,K)^T, one byte per element, arguments checked by vlmt_gemm_fp8; idesc: instruction
 // descriptor of kind::f8f6f4 for M = 256, N = 256.  k_splits as above in parts of kb_per_split 128-wide blocks.

@@ -1081,6 +1081,21 @@ extern "C" int vlmt_gemm_bf16_glu(const void* X, const void* W, void* gu, void* 
   return vlmt_gemm_pair_glu(X, W, gu, act, M, I, K, ldx, ldw, status, stream);
 }
 
+// Gradients of gate and up, and their activation (or null), from the gradient dY(M,K) W(K,I) of the activation; 1: no such kernel for these sizes, nothing
+// was done.  The activation kernel's two passes over the product go away, and the rest of its memory traffic runs beside the contraction, but the epilogue
+// of a tile takes three times as long, and the last one is in the open: from 4 tiles of 256 x 256 per SM on (8 for each pair).  Product and
+// activation kernel / this one: 8192 x 12288 x 4096 650 / 594 us, K = 2048 500 / 423, 4096 x 12288 x 2048 255 / 230, 16384 x 17408 x 5120 2366 / 2224,
+// 16384 x 6144 x 512 260 / 244, 8192 x 4864 x 1024 (608 tiles) 152 / 152, 142 / 138; with fewer 2048 x 12288 x 4096 175 / 174, 1024 x 9728 x 2560 67 / 72.
+extern "C" int vlmt_gemm_bf16_glu_bwd(const void* dY, const void* W, const void* gu, void* dgu, void* act, int M, int I, int K, int ldy, int ldw,
+                                      int* status, int num_sms, cudaStream_t stream) {
+  if (M <= BM || K <= 0 || I <= 0 || I % 64 != 0 || (ldy & 7) || (ldw & 7)) return 1;
+  if ((reinterpret_cast<uintptr_t>(dY) | reinterpret_cast<uintptr_t>(W) | reinterpret_cast<uintptr_t>(gu) | reinterpret_cast<uintptr_t>(dgu) |
+       reinterpret_cast<uintptr_t>(act)) & 15) return 1;
+  const GemmForm form = gemm_form(M, I, K, true, true, false, num_sms, cluster_capacity(), vlmt_gemm_pair_clusters());
+  if (!form.pairs || form.parts > 1 || form.k_splits > 1 || (long)((M + 255) / 256) * ((I + 255) / 256) < 4l * num_sms) return 1;
+  return vlmt_gemm_pair_glu_bwd(dY, W, gu, dgu, act, M, I, K, ldy, ldw, status, stream);
+}
+
 // D rows [o * rows_per_rank, (o + 1) * rows_per_rank) are written to dst[o] (row stride ldd) instead of a local D:
 // the producer half of a tensor-parallel GEMM -> reduce-scatter (the consumer sums the `world` partial blocks it received).
 // B is K-major (a row-parallel forward linear) or MN-major (the input gradient of a column-parallel linear).
