@@ -748,3 +748,20 @@ def test_gate_up_gradient_with_its_product(M, I, K, there):
         alone = cu._C.gemm_glu_bwd(dy, w, gu, False)
         assert torch.equal(alone[0], got[0]) and alone[1] is None
     cu.check_status()
+
+
+# the same for a GELU, whose columns may end inside a slab
+@pytest.mark.parametrize("M,N,K,tanh,there", [(10240, 4304, 1152, True, True), (8321, 4808, 520, False, True), (16130, 2504, 264, True, True), (37, 4304, 1152, True, False)])
+def test_gelu_gradient_with_its_product(M, N, K, tanh, there):
+    from vlm_training_b200.ops import cuda as cu
+
+    dy, w, x = _rand(M, K, scale=0.5), _rand(K, N, scale=0.05), _rand(M, N, scale=2.0)
+    got = cu._C.gemm_gelu_bwd(dy, w, x, tanh, True)
+    assert (got is not None) == there
+    if there:
+        d = torch.empty(M, N, dtype=torch.bfloat16, device=DEV)
+        cu._C.gemm(dy, w, d, False, True, None, 0, False)
+        assert torch.equal(got[0], cu._C.gelu_bwd(d, x, tanh)) and torch.equal(got[1], cu._C.op_gelu(x, tanh))
+        alone = cu._C.gemm_gelu_bwd(dy, w, x, tanh, False)
+        assert torch.equal(alone[0], got[0]) and alone[1] is None
+    cu.check_status()

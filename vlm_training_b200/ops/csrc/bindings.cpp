@@ -93,7 +93,7 @@ bool gemm_glu_bwd(const Tensor& dy, const Tensor& w, const Tensor& gu, Tensor& d
   const int64_t M = dy.size(0), I = w.size(1);
   TORCH_CHECK(gu.size(-1) == 2 * I && gu.numel() == M * 2 * I);
   c10::cuda::CUDAGuard guard(dy.device());
-  if (I % 64 != 0 || M == 0) return false;
+  if (I % 64 != 0 || M <= 128) return false;
   Tensor d = torch::empty_like(gu), a;
   if (act != nullptr) a = torch::empty({M, I}, dy.options());
   const int r = vlmt_gemm_bf16_glu_bwd(dy.data_ptr(), w.data_ptr(), gu.data_ptr(), d.data_ptr(), act != nullptr ? a.data_ptr() : nullptr, (int)M, (int)I,
@@ -102,6 +102,26 @@ bool gemm_glu_bwd(const Tensor& dy, const Tensor& w, const Tensor& gu, Tensor& d
   if (r != 0) return false;
   dgu = d;
   if (act != nullptr) *act = a;
+  return true;
+}
+
+// Gradient of x from dy w, the gradient of gelu(x), and that itself if asked for; false: nothing was done.
+bool gemm_gelu_bwd(const Tensor& dy, const Tensor& w, const Tensor& x, bool tanh_approx, Tensor& dx, Tensor* y) {
+  check_bf16(dy, "dy"); check_bf16(w, "w"); check_bf16(x, "x"); check_contig(x, "x");
+  TORCH_CHECK(dy.dim() == 2 && w.dim() == 2 && dy.stride(1) == 1 && w.stride(1) == 1 && dy.size(1) == w.size(0));
+  const int64_t M = dy.size(0), N = w.size(1);
+  TORCH_CHECK(x.size(-1) == N && x.numel() == M * N);
+  c10::cuda::CUDAGuard guard(dy.device());
+  if (N % 8 != 0 || M <= 128) return false;
+  Tensor d = torch::empty_like(x), a;
+  if (y != nullptr) a = torch::empty({M, N}, dy.options());
+  const int r = vlmt_gemm_bf16_gelu_bwd(dy.data_ptr(), w.data_ptr(), x.data_ptr(), d.data_ptr(), y != nullptr ? a.data_ptr() : nullptr, (int)M, (int)N,
+                                        (int)dy.size(1), (int)dy.stride(0), (int)w.stride(0), tanh_approx, status_tensor().data_ptr<int>(), num_sms(),
+                                        cur_stream());
+  TORCH_CHECK(r == 0 || r == 1, "vlmt_gemm_bf16_gelu_bwd failed with code ", r);
+  if (r != 0) return false;
+  dx = d;
+  if (y != nullptr) *y = a;
   return true;
 }
 
@@ -597,6 +617,12 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     Tensor dgu, act;
     if (!gemm_glu_bwd(dy, w, gu, dgu, want_act ? &act : nullptr)) return py::none();
     return py::make_tuple(dgu, want_act ? py::cast(act) : py::object(py::none()));
+  });
+  // (dx, gelu(x) or None), or None
+  m.def("gemm_gelu_bwd", [](const Tensor& dy, const Tensor& w, const Tensor& x, bool tanh_approx, bool want_act) -> py::object {
+    Tensor dx, act;
+    if (!gemm_gelu_bwd(dy, w, x, tanh_approx, dx, want_act ? &act : nullptr)) return py::none();
+    return py::make_tuple(dx, want_act ? py::cast(act) : py::object(py::none()));
   });
   m.def("gemm_rs_push", &gemm_rs_push);
   m.def("gemm_ag", &gemm_ag);

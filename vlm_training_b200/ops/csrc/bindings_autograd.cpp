@@ -377,9 +377,12 @@ struct GeluLinear : torch::autograd::Function<GeluLinear> {
     auto c = kept(ctx);
     const Tensor &pre = saved[0], &w = saved[1];
     Tensor dy = rows_of(grads[0]), dw, db;
-    Tensor act, dpre = gelu_bwd(mm(dy, w, false, true), pre, c->tanh, c->need[1] ? &act : nullptr);
-    if (c->need[1]) dw = weight_grad(dy, act, c->t[0]);
+    Tensor act, dpre;
+    check_storage(w);
+    if (!gemm_gelu_bwd(dy, w, pre, c->tanh, dpre, c->need[1] ? &act : nullptr))
+      dpre = gelu_bwd(mm(dy, w, false, true), pre, c->tanh, c->need[1] ? &act : nullptr);
     tick(1);
+    if (c->need[1]) dw = weight_grad(dy, act, c->t[0]);
     if (c->need[2]) db = bias_grad(dy, saved[2], c->t[1]);
     return {dpre, dw, db, Tensor()};
   }
@@ -398,7 +401,6 @@ Tensor op_gelu_linear(const Tensor& pre, const py::object& w_, const py::object&
   });
 }
 
-// silu(gate) * up -> linear for a fused [T, 2 I] input, only the input is kept
 // Gradient of [gate, up] behind y = (silu(gate) * up) w^T; h (or null) gets silu(gate) * up.
 Tensor glu_grad(const Tensor& dy, const Tensor& w, const Tensor& gu, Tensor* h) {
   check_storage(w);
@@ -407,6 +409,7 @@ Tensor glu_grad(const Tensor& dy, const Tensor& w, const Tensor& gu, Tensor* h) 
   tick(1);
   return dgu;
 }
+// silu(gate) * up -> linear for a fused [T, 2 I] input, only the input is kept
 struct SwigluLinear : torch::autograd::Function<SwigluLinear> {
   static Tensor forward(AutogradContext* ctx, const Tensor& gu, const Tensor& w, CfgPtr c) {
     Tensor g = gu.contiguous(), wc = operand(w);

@@ -26,6 +26,16 @@ __device__ __forceinline__ float gelu_erf_f(float x) { return 0.5f * x * (1.f + 
 // the operations of the activation kernels (elementwise.cu), on values that have been rounded to bf16
 __device__ __forceinline__ float swiglu_f(float g, float u) { return g * (1.f / (1.f + __expf(-g))) * u; }
 
+__device__ __forceinline__ float gelu_tanh_grad_f(float x) {
+  const float u = 0.7978845608028654f * (x + 0.044715f * x * x * x);
+  const float t = tanhf(u);
+  const float du = 0.7978845608028654f * (1.f + 3.f * 0.044715f * x * x);
+  return 0.5f * (1.f + t) + 0.5f * x * (1.f - t * t) * du;
+}
+__device__ __forceinline__ float gelu_erf_grad_f(float x) {
+  const float cdf = 0.5f * (1.f + erff(x * 0.7071067811865476f));
+  return cdf + x * 0.3989422804014327f * __expf(-0.5f * x * x);
+}
 // dg, du and the activation itself from its gradient
 __device__ __forceinline__ void swiglu_grad_f(float d, float g, float u, float& dg, float& du, float& act) {
   const float s = 1.f / (1.f + __expf(-g));

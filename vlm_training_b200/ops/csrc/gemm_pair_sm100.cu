@@ -53,7 +53,7 @@ struct Params {
   const float* rec_a;           // FP8: rec[1] undoes the operand's scaling
   const float* rec_b;
   uint32_t idesc;               // FP8: carries the two formats
-  int store_gu;                 // GLU 1: D is written; GLU 2: the activation is
+  int store_gu;                 // GLU 1: D is written; GLU 2, 3: the activation is
   // grouped weight gradients (both operands MN-major, see gemm_sm100.cu): group g contracts over its own rows, 128-row tiles grp_prefix[g] to
   // grp_prefix[g + 1], into the block of M rows of D that starts at g * M
   const int* grp_prefix;
@@ -109,12 +109,14 @@ __device__ __forceinline__ void store_parts(const uint8_t* smem, const Params& p
 // has 128 columns of both, and the epilogue writes silu(gate) * up of the rounded values besides them, or alone (store_gu 0).
 // GLU 2 (B MN-major): the product is the gradient of silu(gate) * up, [M, N].  The epilogue reads gate and up ([M, 2 N], loaded a slab ahead into what
 // is the last operand stage otherwise) and writes their gradients into D, [M, 2 N], and silu(gate) * up for the weight gradient that follows.
-constexpr int kGlu = 1, kGluBwd = 2;
+// GLU 3: the same for gelu(x), x and its gradient [M, N].
+constexpr int kGlu = 1, kGluBwd = 2, kGeluBwd = 3;
 template <bool A_MN, bool B_MN, bool FP8, int GLU>
 __global__ void __launch_bounds__(NUM_THREADS, 1)
 gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b, const __grid_constant__ CUtensorMap tmap_d,
                  const __grid_constant__ CUtensorMap tmap_act, const __grid_constant__ CUtensorMap tmap_gu, Params p) {
-    constexpr int NST = GLU == kGluBwd ? STAGES - 1 : STAGES;
+    constexpr bool BWD = GLU == kGluBwd || GLU == kGeluBwd;
+  constexpr int NST = BWD ? STAGES - 1 : STAGES;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + kBarOffset);
@@ -139,7 +141,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
   if (threadIdx.x == 0) {
     for (int s = 0; s < NST; ++s) { mbar_init(&full_bar[s], 1); mbar_init(&empty_bar[s], 1); }
     for (int a = 0; a < 2; ++a) { mbar_init(&tmem_full[a], 1); mbar_init(&tmem_empty[a], 8); }
-    if (GLU == kGluBwd) for (int q = 0; q < 4; ++q) mbar_init(&gu_bar[q], 1);
+    if (BWD) for (int q = 0; q < 4; ++q) mbar_init(&gu_bar[q], 1);
     *abort_flag = 0;
     fence_mbar_init();
     tma_prefetch_desc(&tmap_a);
@@ -246,12 +248,12 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
     uint8_t* out = smem + kOutOffset + q * 8192;
     int it = 0;
     uint32_t slab = 0;   // runs across items (see gemm_sm100.cu)
-    uint8_t* in = smem + NST * kStageBytes + q * 8192;   // GLU 2: a slab of gate and of up
+    uint8_t* in = smem + NST * kStageBytes + q * 8192;   // BWD: a slab of x, or of gate and of up
     uint32_t in_phase = 0;
     auto load_gu = [&](int col, int row) {
-      mbar_expect_tx(&gu_bar[q], 8192);
+      mbar_expect_tx(&gu_bar[q], GLU == kGluBwd ? 8192 : 4096);
       tma_load_2d(in, &tmap_gu, &gu_bar[q], col, row);
-      tma_load_2d(in + 4096, &tmap_gu, &gu_bar[q], p.N + col, row);
+      if (GLU == kGluBwd) tma_load_2d(in + 4096, &tmap_gu, &gu_bar[q], p.N + col, row);
     };
     for (int item = pair; item < num_items; item += pairs, ++it) {
       const int tile = grouped || p.k_splits > 1 ? item % num_tiles : item;
@@ -265,7 +267,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
       }
       const int acc = it & 1;
       const int row0 = (tm * 2 + (int)rank) * BM + q * 32, n0 = tn * BN;
-      if (GLU == kGluBwd && lane == 0 && row0 < p.M) load_gu(n0, row0);
+      if (BWD && lane == 0 && row0 < p.M) load_gu(n0, row0);
       if (!mbar_wait(&tmem_full[acc], (it >> 1) & 1, abort_flag, p.status, kErrTimeoutTmemFull)) break;
       tc_fence_after();
       const uint32_t taddr = tmem_base + acc * BN + ((uint32_t)(q * 32) << 16);
@@ -296,11 +298,11 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
           tma_store_commit();
         }
       };
-      if (GLU == kGluBwd) {
+      if (BWD) {
         bool ok = true;
 #pragma unroll 1
         for (int c = 0; c < BN / 64; ++c) {
-          const int col = n0 + c * 64;   // N is a multiple of 64
+          const int col = n0 + c * 64;   // GLU 2: N is a multiple of 64
           if (row0 >= p.M || col >= p.N) break;
           if (!mbar_wait(&gu_bar[q], in_phase, abort_flag, p.status, kErrTimeoutFull)) { ok = false; break; }
           in_phase ^= 1;
@@ -308,9 +310,11 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
 #pragma unroll
           for (int t = 0; t < 8; ++t) {
             const uint4 x = *reinterpret_cast<const uint4*>(in + lane * 128 + ((t ^ (lane & 7)) << 4));
-            const uint4 y = *reinterpret_cast<const uint4*>(in + 4096 + lane * 128 + ((t ^ (lane & 7)) << 4));
             g[4 * t] = x.x; g[4 * t + 1] = x.y; g[4 * t + 2] = x.z; g[4 * t + 3] = x.w;
-            u[4 * t] = y.x; u[4 * t + 1] = y.y; u[4 * t + 2] = y.z; u[4 * t + 3] = y.w;
+            if (GLU == kGluBwd) {
+              const uint4 y = *reinterpret_cast<const uint4*>(in + 4096 + lane * 128 + ((t ^ (lane & 7)) << 4));
+              u[4 * t] = y.x; u[4 * t + 1] = y.y; u[4 * t + 2] = y.z; u[4 * t + 3] = y.w;
+            }
           }
           fence_async_proxy();   // the loads above have returned before the next slab may be written: a converged warp's barrier does not wait for them
           __syncwarp();
@@ -320,8 +324,23 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
             uint32_t r[32];
             tmem_ld_32x32(taddr + c * 64 + h * 32, r);
             tmem_ld_wait();
+            if (GLU == kGeluBwd) {   // the product is rounded to bf16 as if it were stored
+              auto grad = [&](auto f, auto df) {
 #pragma unroll
-            for (int i = 0; i < 16; ++i) {   // the product is rounded to bf16 as if it were stored
+                for (int i = 0; i < 16; ++i) {
+                  const int j = h * 16 + i;
+                  const uint32_t d = pack_bf16x2(__uint_as_float(r[2 * i]), __uint_as_float(r[2 * i + 1]));
+                  const float x0 = __uint_as_float(g[j] << 16), x1 = __uint_as_float(g[j] & 0xffff0000u);
+                  g[j] = pack_bf16x2(__uint_as_float(d << 16) * df(x0), __uint_as_float(d & 0xffff0000u) * df(x1));
+                  a[j] = pack_bf16x2(f(x0), f(x1));
+                }
+              };
+              if (p.epilogue == GEMM_EPI_GELU_TANH) grad([](float x) { return gelu_tanh_f(x); }, [](float x) { return gelu_tanh_grad_f(x); });
+              else grad([](float x) { return gelu_erf_f(x); }, [](float x) { return gelu_erf_grad_f(x); });
+              continue;
+            }
+#pragma unroll
+            for (int i = 0; i < 16; ++i) {
               const int j = h * 16 + i;
               const uint32_t d = pack_bf16x2(__uint_as_float(r[2 * i]), __uint_as_float(r[2 * i + 1]));
               float dg[2], du[2], act[2];
@@ -334,7 +353,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
             }
           }
           put(g, &tmap_d, col);
-          put(u, &tmap_d, p.N + col);
+          if (GLU == kGluBwd) put(u, &tmap_d, p.N + col);
           if (p.store_gu) put(a, &tmap_act, col);
         }
         if (!ok) break;
@@ -582,6 +601,25 @@ extern "C" int vlmt_gemm_pair_glu_bwd(const void* dY, const void* W, const void*
   p.group_m = raster_group(2l * I * K, 2l * K);
   p.store_gu = act != nullptr;
   return launch<false, true, false, kGluBwd>(ta, tb, td, tact, p, stream, &tgu);
+}
+
+// dx[M, N] and, if y is given, y[M, N] = gelu(x) from dY(M,K) W(K,N) and x[M, N]; epilogue: one of the two GELUs
+extern "C" int vlmt_gemm_pair_gelu_bwd(const void* dY, const void* W, const void* x, void* dx, void* y, int M, int N, int K, int ldy, int ldw, int epilogue,
+                                       int* status, cudaStream_t stream) {
+  CUtensorMap ta, tb, td, tact, tx;
+  int r;
+  if ((r = vlmt_make_tmap_2d_bf16(&ta, dY, (uint64_t)K, (uint64_t)M, (uint64_t)ldy * 2, 64, 128))) return 1000 + r;
+  if ((r = vlmt_make_tmap_2d_bf16(&tb, W, (uint64_t)N, (uint64_t)K, (uint64_t)ldw * 2, 64, 64))) return 2000 + r;
+  if ((r = vlmt_make_tmap_2d_bf16(&td, dx, (uint64_t)N, (uint64_t)M, (uint64_t)N * 2, 64, 32))) return 3000 + r;
+  if ((r = vlmt_make_tmap_2d_bf16(&tx, x, (uint64_t)N, (uint64_t)M, (uint64_t)N * 2, 64, 32))) return 4000 + r;
+  tact = td;
+  if (y != nullptr && (r = vlmt_make_tmap_2d_bf16(&tact, y, (uint64_t)N, (uint64_t)M, (uint64_t)N * 2, 64, 32))) return 3000 + r;
+  Params p = {};
+  p.M = M; p.N = N; p.K = K; p.epilogue = epilogue;
+  p.k_splits = 1; p.kb_per_split = (K + BK - 1) / BK; p.parts = 1; p.status = status;
+  p.group_m = raster_group(2l * N * K, 2l * K);
+  p.store_gu = y != nullptr;
+  return launch<false, true, false, kGeluBwd>(ta, tb, td, tact, p, stream, &tx);
 }
 
 extern "C" int vlmt_gemm_pair_fp8(const void* A, const void* B, void* D, int M, int N, int K, long lda, long ldb, long ldd, uint32_t idesc,

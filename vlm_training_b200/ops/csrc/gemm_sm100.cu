@@ -1096,6 +1096,21 @@ extern "C" int vlmt_gemm_bf16_glu_bwd(const void* dY, const void* W, const void*
   return vlmt_gemm_pair_glu_bwd(dY, W, gu, dgu, act, M, I, K, ldy, ldw, status, stream);
 }
 
+// Gradient of x and gelu(x) (or null) from the gradient dY(M,K) W(K,N) of the latter, N a multiple of 8; 1: no such kernel for these sizes, nothing was
+// done.  The product is neither written nor read again, and the activation kernel's other traffic runs beside the contraction; with one slab of input
+// the epilogue stays short enough for any number of tiles.  Product and activation kernel / this one: 28672 x 4304 x 1152 333 / 276 us, 10240 128 / 112,
+// 4096 60.4 / 55.2, 2304 46 / 43; 7168 x 4608 x 4096 202 / 186, 2560 x 4608 x 2560 66.6 / 63.5.  The choice of the GELU stands outside the loop over a
+// slab's values: inside it the epilogue took three times as long (28672 rows 522 us).
+extern "C" int vlmt_gemm_bf16_gelu_bwd(const void* dY, const void* W, const void* x, void* dx, void* y, int M, int N, int K, int ldy, int ldw,
+                                       int tanh_approx, int* status, int num_sms, cudaStream_t stream) {
+  if (M <= BM || K <= 0 || N <= 0 || (N & 7) || (ldy & 7) || (ldw & 7)) return 1;
+  if ((reinterpret_cast<uintptr_t>(dY) | reinterpret_cast<uintptr_t>(W) | reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(dx) |
+       reinterpret_cast<uintptr_t>(y)) & 15) return 1;
+  const GemmForm form = gemm_form(M, N, K, true, true, false, num_sms, cluster_capacity(), vlmt_gemm_pair_clusters());
+  if (!form.pairs || form.parts > 1 || form.k_splits > 1) return 1;
+  return vlmt_gemm_pair_gelu_bwd(dY, W, x, dx, y, M, N, K, ldy, ldw, tanh_approx ? GEMM_EPI_GELU_TANH : GEMM_EPI_GELU_ERF, status, stream);
+}
+
 // D rows [o * rows_per_rank, (o + 1) * rows_per_rank) are written to dst[o] (row stride ldd) instead of a local D:
 // the producer half of a tensor-parallel GEMM -> reduce-scatter (the consumer sums the `world` partial blocks it received).
 // B is K-major (a row-parallel forward linear) or MN-major (the input gradient of a column-parallel linear).
