@@ -765,3 +765,20 @@ def test_gelu_gradient_with_its_product(M, N, K, tanh, there):
         alone = cu._C.gemm_gelu_bwd(dy, w, x, tanh, False)
         assert torch.equal(alone[0], got[0]) and alone[1] is None
     cu.check_status()
+
+
+# first linear of a vision MLP with its activation: the bits of the product and the activation kernel behind one another
+@pytest.mark.parametrize("M,N,K,tanh,bias,there", [(10240, 4304, 1152, True, True, True), (2049, 1288, 520, False, True, True), (4001, 2504, 72, True, False, True),
+                                                   (37, 4304, 1152, True, True, False), (300, 256, 512, True, True, False)])
+def test_linear_with_its_gelu(M, N, K, tanh, bias, there):
+    from vlm_training_b200.ops import cuda as cu
+
+    x, w, b = _rand(M, K, scale=0.5), _rand(N, K, scale=0.1), _rand(N) if bias else None
+    got = cu._C.gemm_gelu(x, w, b, tanh, True)
+    assert (got is not None) == there
+    if there:
+        pre = cu._gemm(x, w, bias=b)
+        assert torch.equal(got[1], pre) and torch.equal(got[0], cu._C.op_gelu(pre, tanh))
+        alone = cu._C.gemm_gelu(x, w, b, tanh, False)
+        assert torch.equal(alone[0], got[0]) and alone[1] is None
+    cu.check_status()

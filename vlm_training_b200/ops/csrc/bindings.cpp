@@ -105,6 +105,25 @@ bool gemm_glu_bwd(const Tensor& dy, const Tensor& w, const Tensor& gu, Tensor& d
   return true;
 }
 
+// act = gelu(pre), pre = x w^T + bias; false: nothing was done.  pre: null, or gets it.
+bool gemm_gelu(const Tensor& x, const Tensor& w, const OptTensor& bias, bool tanh_approx, Tensor* pre, Tensor& act) {
+  check_bf16(x, "x"); check_bf16(w, "w");
+  TORCH_CHECK(x.dim() == 2 && w.dim() == 2 && x.stride(1) == 1 && w.stride(1) == 1 && x.size(1) == w.size(1));
+  const int64_t M = x.size(0), N = w.size(0);
+  if (bias.has_value()) { check_bf16(*bias, "bias"); check_contig(*bias, "bias"); TORCH_CHECK(bias->numel() == N); }
+  c10::cuda::CUDAGuard guard(x.device());
+  if (N % 8 != 0 || M <= 128) return false;
+  Tensor a = torch::empty({M, N}, x.options()), p;
+  if (pre != nullptr) p = torch::empty({M, N}, x.options());
+  const int r = vlmt_gemm_bf16_gelu(x.data_ptr(), w.data_ptr(), optptr(bias), pre != nullptr ? p.data_ptr() : nullptr, a.data_ptr(), (int)M, (int)N,
+                                    (int)x.size(1), (int)x.stride(0), (int)w.stride(0), tanh_approx, status_tensor().data_ptr<int>(), num_sms(), cur_stream());
+  TORCH_CHECK(r == 0 || r == 1, "vlmt_gemm_bf16_gelu failed with code ", r);
+  if (r != 0) return false;
+  act = a;
+  if (pre != nullptr) *pre = p;
+  return true;
+}
+
 // Gradient of x from dy w, the gradient of gelu(x), and that itself if asked for; false: nothing was done.
 bool gemm_gelu_bwd(const Tensor& dy, const Tensor& w, const Tensor& x, bool tanh_approx, Tensor& dx, Tensor* y) {
   check_bf16(dy, "dy"); check_bf16(w, "w"); check_bf16(x, "x"); check_contig(x, "x");
@@ -617,6 +636,12 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     Tensor dgu, act;
     if (!gemm_glu_bwd(dy, w, gu, dgu, want_act ? &act : nullptr)) return py::none();
     return py::make_tuple(dgu, want_act ? py::cast(act) : py::object(py::none()));
+  });
+  // (act, pre or None), or None
+  m.def("gemm_gelu", [](const Tensor& x, const Tensor& w, const c10::optional<Tensor>& bias, bool tanh_approx, bool keep) -> py::object {
+    Tensor pre, act;
+    if (!gemm_gelu(x, w, bias, tanh_approx, keep ? &pre : nullptr, act)) return py::none();
+    return py::make_tuple(act, keep ? py::cast(pre) : py::object(py::none()));
   });
   // (dx, gelu(x) or None), or None
   m.def("gemm_gelu_bwd", [](const Tensor& dy, const Tensor& w, const Tensor& x, bool tanh_approx, bool want_act) -> py::object {

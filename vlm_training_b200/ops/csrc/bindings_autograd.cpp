@@ -173,6 +173,8 @@ struct Cfg : torch::CustomClassHolder {
   int64_t n_q = 0, n_kv = 0, D = 0, max_seqlen = 0;
   std::vector<int64_t> shape;
   Target t[4];
+  bool want_act = false;   // LnLinear: gelu of the output too, into `act`; GeluLinear takes it from there
+  Tensor act;
 };
 using CfgPtr = c10::intrusive_ptr<Cfg>;
 void keep(AutogradContext* ctx, const CfgPtr& c) { ctx->saved_data["cfg"] = c10::IValue::make_capsule(c); }
@@ -306,7 +308,10 @@ struct LnLinear : torch::autograd::Function<LnLinear> {
     const Tensor lb = get(lb_), b = get(b_);
     Tensor xc = x.contiguous();
     auto r = layernorm_fwd(xc, lw, opt(lb), c->eps);
-    Tensor wc = operand(w), y = mm(r[0], wc, false, false, b);
+    Tensor wc = operand(w), y;
+    check_storage(wc);
+    if (c->want_act && gemm_gelu(r[0], wc, opt(b), c->tanh, &y, c->act)) tick(1);
+    else y = mm(r[0], wc, false, false, b);
     tick(1);
     c->need[1] = wants(lw); c->need[2] = wants(lb); c->need[3] = wants(w); c->need[4] = wants(b);
     keep(ctx, c);
@@ -346,18 +351,33 @@ struct LnLinear : torch::autograd::Function<LnLinear> {
     return {r[0], dlw, dlb, dw, db, Tensor()};
   }
 };
-Tensor op_ln_linear(const Tensor& x, const py::object& lw_, const py::object& lb_, const py::object& w_, const py::object& b_, double eps) {
+// gelu_kind: 0 no activation, 1 gelu(output) in `act` too, 2 the tanh form of it; undefined where the sizes have no such kernel.  Without a graph the
+// output itself is undefined where `act` is not.
+Tensor ln_linear(const Tensor& x, const py::object& lw_, const py::object& lb_, const py::object& w_, const py::object& b_, double eps, int gelu_kind,
+                 Tensor* act) {
   return guarded([&] {
     Tensor lw = lw_.cast<Tensor>(), lb = as_tensor(lb_), w = w_.cast<Tensor>(), b = as_tensor(b_);
     if (no_graph(x, lw, lb, w, b)) {
       tick(1);
-      return mm(layernorm_fwd(x.contiguous(), lw, opt(lb), eps)[0], operand(w), false, false, b);
+      Tensor h = layernorm_fwd(x.contiguous(), lw, opt(lb), eps)[0], wc = operand(w);
+      check_storage(wc);
+      if (gelu_kind != 0 && gemm_gelu(h, wc, opt(b), gelu_kind == 2, nullptr, *act)) {
+        tick(1);
+        return Tensor();
+      }
+      return mm(h, wc, false, false, b);
     }
     auto c = c10::make_intrusive<Cfg>();
     c->eps = eps;
+    c->want_act = gelu_kind != 0; c->tanh = gelu_kind == 2;
     c->t[0] = target_of(lw_); c->t[1] = target_of(lb_); c->t[2] = target_of(w_); c->t[3] = target_of(b_);
-    return LnLinear::apply(x, lw, opt(lb), w, opt(b), c);
+    Tensor y = LnLinear::apply(x, lw, opt(lb), w, opt(b), c);
+    if (act != nullptr) *act = std::move(c->act);
+    return y;
   });
+}
+Tensor op_ln_linear(const Tensor& x, const py::object& lw_, const py::object& lb_, const py::object& w_, const py::object& b_, double eps) {
+  return ln_linear(x, lw_, lb_, w_, b_, eps, 0, nullptr);
 }
 
 // gelu(pre) -> linear, only `pre` is kept
@@ -365,8 +385,9 @@ struct GeluLinear : torch::autograd::Function<GeluLinear> {
   static Tensor forward(AutogradContext* ctx, const Tensor& pre, const Tensor& w, const OptTensor& b_, CfgPtr c) {
     const Tensor b = get(b_);
     Tensor pc = pre.contiguous(), wc = operand(w);
-    Tensor y = mm(gelu_fwd(pc, c->tanh), wc, false, false, b);
-    tick(1);
+    Tensor act = std::move(c->act);
+    if (!act.defined()) { act = gelu_fwd(pc, c->tanh); tick(1); }
+    Tensor y = mm(act, wc, false, false, b);
     c->need[1] = wants(w); c->need[2] = wants(b);
     keep(ctx, c);
     ctx->save_for_backward(b.defined() ? variable_list{pc, wc, b} : variable_list{pc, wc});
@@ -387,18 +408,23 @@ struct GeluLinear : torch::autograd::Function<GeluLinear> {
     return {dpre, dw, db, Tensor()};
   }
 };
-Tensor op_gelu_linear(const Tensor& pre, const py::object& w_, const py::object& b_, bool tanh_approx) {
+// `act`: gelu(pre) where its kernel has made it
+Tensor gelu_linear(const Tensor& pre, const py::object& w_, const py::object& b_, bool tanh_approx, Tensor act) {
   return guarded([&] {
     Tensor w = w_.cast<Tensor>(), b = as_tensor(b_);
     if (no_graph(pre, w, b)) {
-      tick(1);
-      return mm(gelu_fwd(pre.contiguous(), tanh_approx), operand(w), false, false, b);
+      if (!act.defined()) { act = gelu_fwd(pre.contiguous(), tanh_approx); tick(1); }
+      return mm(act, operand(w), false, false, b);
     }
     auto c = c10::make_intrusive<Cfg>();
     c->tanh = tanh_approx;
+    c->act = std::move(act);
     c->t[0] = target_of(w_); c->t[1] = target_of(b_);
     return GeluLinear::apply(pre, w, opt(b), c);
   });
+}
+Tensor op_gelu_linear(const Tensor& pre, const py::object& w_, const py::object& b_, bool tanh_approx) {
+  return gelu_linear(pre, w_, b_, tanh_approx, Tensor());
 }
 
 // Gradient of [gate, up] behind y = (silu(gate) * up) w^T; h (or null) gets silu(gate) * up.
@@ -1047,8 +1073,8 @@ py::object op_vision_block(const Tensor& x, const py::tuple& w, const Tensor& co
   o.reset();
   Tensor r = guarded([&] { return x + a; });
   a.reset();
-  Tensor pre = op_ln_linear(r, w[6], w[7], w[8], w[9], eps2);
-  Tensor out = op_gelu_linear(pre, w[10], w[11], tanh_approx);
+  Tensor act, pre = ln_linear(r, w[6], w[7], w[8], w[9], eps2, tanh_approx ? 2 : 1, &act);
+  Tensor out = gelu_linear(pre, w[10], w[11], tanh_approx, std::move(act));
   pre.reset();
   return py::cast(guarded([&] { return r + out; }));
 }

@@ -53,7 +53,7 @@ struct Params {
   const float* rec_a;           // FP8: rec[1] undoes the operand's scaling
   const float* rec_b;
   uint32_t idesc;               // FP8: carries the two formats
-  int store_gu;                 // GLU 1: D is written; GLU 2, 3: the activation is
+  int store_gu;                 // GLU 1, 4: D is written; GLU 2, 3: the activation is
   // grouped weight gradients (both operands MN-major, see gemm_sm100.cu): group g contracts over its own rows, 128-row tiles grp_prefix[g] to
   // grp_prefix[g + 1], into the block of M rows of D that starts at g * M
   const int* grp_prefix;
@@ -110,7 +110,8 @@ __device__ __forceinline__ void store_parts(const uint8_t* smem, const Params& p
 // GLU 2 (B MN-major): the product is the gradient of silu(gate) * up, [M, N].  The epilogue reads gate and up ([M, 2 N], loaded a slab ahead into what
 // is the last operand stage otherwise) and writes their gradients into D, [M, 2 N], and silu(gate) * up for the weight gradient that follows.
 // GLU 3: the same for gelu(x), x and its gradient [M, N].
-constexpr int kGlu = 1, kGluBwd = 2, kGeluBwd = 3;
+// GLU 4 (K-major operands): x = product + bias into D and gelu of the rounded value besides it, or alone (store_gu 0).
+constexpr int kGlu = 1, kGluBwd = 2, kGeluBwd = 3, kGelu = 4;
 template <bool A_MN, bool B_MN, bool FP8, int GLU>
 __global__ void __launch_bounds__(NUM_THREADS, 1)
 gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b, const __grid_constant__ CUtensorMap tmap_d,
@@ -385,6 +386,33 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
                                swiglu_f(__uint_as_float(g[i] & 0xffff0000u), __uint_as_float(u[i] & 0xffff0000u)));
           put(g, &tmap_act, col);
         }
+      } else if (GLU == kGelu) {
+#pragma unroll 1
+        for (int c = 0; c < BN / 64; ++c) {
+          const int col = n0 + c * 64;
+          if (row0 >= p.M || col >= p.N) break;
+          uint32_t g[32];
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            uint32_t r[32];
+            tmem_ld_32x32(taddr + c * 64 + h * 32, r);
+            tmem_ld_wait();
+            float v[32];
+#pragma unroll
+            for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]);
+            bias_activation(v, p.bias, col + h * 32, p.N, GEMM_EPI_NONE);
+#pragma unroll
+            for (int i = 0; i < 16; ++i) g[h * 16 + i] = pack_bf16x2(v[2 * i], v[2 * i + 1]);
+          }
+          if (p.store_gu) put(g, &tmap_d, col);
+          auto activate = [&](auto f) {
+#pragma unroll
+            for (int i = 0; i < 32; ++i) g[i] = pack_bf16x2(f(__uint_as_float(g[i] << 16)), f(__uint_as_float(g[i] & 0xffff0000u)));
+          };
+          if (p.epilogue == GEMM_EPI_GELU_TANH) activate([](float x) { return gelu_tanh_f(x); });
+          else activate([](float x) { return gelu_erf_f(x); });
+          put(g, &tmap_act, col);
+        }
       } else if (!FP8 && alpha == 1.f && p.bias == nullptr && p.epilogue == GEMM_EPI_NONE && !empty) {
         // the next slab's columns come out of tensor memory while this one is converted and staged
         uint32_t r[2][2][32];
@@ -601,6 +629,24 @@ extern "C" int vlmt_gemm_pair_glu_bwd(const void* dY, const void* W, const void*
   p.group_m = raster_group(2l * I * K, 2l * K);
   p.store_gu = act != nullptr;
   return launch<false, true, false, kGluBwd>(ta, tb, td, tact, p, stream, &tgu);
+}
+
+// y[M, N] = gelu(x), x = X(M,K) W(N,K)^T + bias, and x itself if given; epilogue: one of the two GELUs
+extern "C" int vlmt_gemm_pair_gelu(const void* X, const void* W, const void* bias, void* x, void* y, int M, int N, int K, int ldx, int ldw, int epilogue,
+                                   int* status, cudaStream_t stream) {
+  CUtensorMap ta, tb, td, tact;
+  int r;
+  if ((r = vlmt_make_tmap_2d_bf16(&ta, X, (uint64_t)K, (uint64_t)M, (uint64_t)ldx * 2, 64, 128))) return 1000 + r;
+  if ((r = vlmt_make_tmap_2d_bf16(&tb, W, (uint64_t)K, (uint64_t)N, (uint64_t)ldw * 2, 64, 128))) return 2000 + r;
+  if ((r = vlmt_make_tmap_2d_bf16(&tact, y, (uint64_t)N, (uint64_t)M, (uint64_t)N * 2, 64, 32))) return 3000 + r;
+  td = tact;
+  if (x != nullptr && (r = vlmt_make_tmap_2d_bf16(&td, x, (uint64_t)N, (uint64_t)M, (uint64_t)N * 2, 64, 32))) return 3000 + r;
+  Params p = {};
+  p.M = M; p.N = N; p.K = K; p.epilogue = epilogue; p.bias = reinterpret_cast<const __nv_bfloat16*>(bias);
+  p.k_splits = 1; p.kb_per_split = (K + BK - 1) / BK; p.parts = 1; p.status = status;
+  p.group_m = raster_group(2l * N * K, 2l * K);
+  p.store_gu = x != nullptr;
+  return launch<false, false, false, kGelu>(ta, tb, td, tact, p, stream);
 }
 
 // dx[M, N] and, if y is given, y[M, N] = gelu(x) from dY(M,K) W(K,N) and x[M, N]; epilogue: one of the two GELUs

@@ -14,6 +14,8 @@ int vlmt_gemm_pair(const void* A, const void* B, void* D, const void* bias, int 
 int vlmt_gemm_pair_clusters();
 int vlmt_gemm_pair_grouped(const void* A, const void* B, void* D, const int* prefix, int groups, int M, int N, int rows, int lda, int ldb, int ldd,
                            int accumulate, int* status, cudaStream_t stream);
+int vlmt_gemm_pair_gelu(const void* X, const void* W, const void* bias, void* x, void* y, int M, int N, int K, int ldx, int ldw, int epilogue,
+                        int* status, cudaStream_t stream);
 int vlmt_gemm_pair_gelu_bwd(const void* dY, const void* W, const void* x, void* dx, void* y, int M, int N, int K, int ldy, int ldw, int epilogue,
                             int* status, cudaStream_t stream);
 int vlmt_gemm_pair_glu_bwd(const void* dY, const void* W, const void* gu, void* dgu, void* act, int M, int I, int K, int ldy, int ldw, int* status,

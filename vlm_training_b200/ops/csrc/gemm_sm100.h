@@ -19,6 +19,8 @@ int vlmt_gemm_bf16(const void* A, const void* B, void* D, float* Dacc32, const v
                    int ldb, int ldd, int a_mn_major, int b_mn_major, int epilogue, int accumulate, const float* alpha, int one_sum,
                    int* status, int num_sms, cudaStream_t stream);
 // act = silu(gate) * up of a gate / up projection, see gemm_sm100.cu; 1: not for these sizes
+int vlmt_gemm_bf16_gelu(const void* X, const void* W, const void* bias, void* x, void* y, int M, int N, int K, int ldx, int ldw, int tanh_approx,
+                        int* status, int num_sms, cudaStream_t stream);
 int vlmt_gemm_bf16_gelu_bwd(const void* dY, const void* W, const void* x, void* dx, void* y, int M, int N, int K, int ldy, int ldw, int tanh_approx,
                             int* status, int num_sms, cudaStream_t stream);
 int vlmt_gemm_bf16_glu_bwd(const void* dY, const void* W, const void* gu, void* dgu, void* act, int M, int I, int K, int ldy, int ldw, int* status,

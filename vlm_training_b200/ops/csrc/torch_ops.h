@@ -12,6 +12,7 @@ using OptTensor = c10::optional<Tensor>;
 int num_sms();
 void gemm(const Tensor& a, const Tensor& b, Tensor& out, bool a_mn, bool b_mn, const OptTensor& bias, int64_t epilogue, bool accumulate,
           const OptTensor& alpha, bool one_sum = false);   // one_sum: see vlmt_gemm_bf16
+bool gemm_gelu(const Tensor& x, const Tensor& w, const OptTensor& bias, bool tanh_approx, Tensor* pre, Tensor& act);
 bool gemm_gelu_bwd(const Tensor& dy, const Tensor& w, const Tensor& x, bool tanh_approx, Tensor& dx, Tensor* y);   // gradient of x from dy w
 bool gemm_glu_bwd(const Tensor& dy, const Tensor& w, const Tensor& gu, Tensor& dgu, Tensor* act);   // gradient of gate and up from dy w
 bool gemm_glu(const Tensor& x, const Tensor& w, Tensor* gu, Tensor& act);   // silu(gate) * up of a gate / up projection; false: not for these sizes
