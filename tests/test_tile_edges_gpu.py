@@ -782,3 +782,19 @@ def test_linear_with_its_gelu(M, N, K, tanh, bias, there):
         alone = cu._C.gemm_gelu(x, w, b, tanh, False)
         assert torch.equal(alone[0], got[0]) and alone[1] is None
     cu.check_status()
+
+
+# a bias read as vectors (columns that end inside a slab, and between two) and one that is not (off 16 bytes, columns not in eights), on one block and on pairs:
+# the bits do not depend on how it is read
+@pytest.mark.parametrize("M,N,K", [(300, 264, 72), (450, 1160, 1152), (10240, 1160, 520), (2305, 3456, 264), (450, 1156, 136)])
+def test_bias_of_the_common_epilogue(M, N, K):
+    from vlm_training_b200.ops import cuda as cu
+
+    x, w, b = _rand(M, K, scale=0.5), _rand(N, K, scale=0.5), _rand(N + 1)
+    y = cu._gemm(x, w, bias=b[:N])
+    # fp32 accumulation of K products of size about 0.25, then one bf16 rounding (2^-8 of the value)
+    torch.testing.assert_close(y.float(), x.float() @ w.float().t() + b[:N].float(), atol=2e-2 * (K / 4096) ** 0.5, rtol=8e-3)
+    off = torch.empty(N + 1, dtype=b.dtype, device=DEV)[1:]
+    off.copy_(b[:N])
+    assert torch.equal(cu._gemm(x, w, bias=off), y)
+    cu.check_status()

@@ -391,19 +391,18 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
         for (int c = 0; c < BN / 64; ++c) {
           const int col = n0 + c * 64;
           if (row0 >= p.M || col >= p.N) break;
-          uint32_t g[32];
-#pragma unroll
-          for (int h = 0; h < 2; ++h) {
-            uint32_t r[32];
-            tmem_ld_32x32(taddr + c * 64 + h * 32, r);
-            tmem_ld_wait();
-            float v[32];
-#pragma unroll
-            for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]);
-            bias_activation(v, p.bias, col + h * 32, p.N, GEMM_EPI_NONE);
-#pragma unroll
-            for (int i = 0; i < 16; ++i) g[h * 16 + i] = pack_bf16x2(v[2 * i], v[2 * i + 1]);
+          uint32_t g[32], r[2][32];
+          uint4 b[8];
+          if (p.bias != nullptr) load_bias(b, p.bias, col, p.N);
+          tmem_ld_32x32(taddr + c * 64, r[0]);
+          tmem_ld_32x32(taddr + c * 64 + 32, r[1]);
+          tmem_ld_wait();
+          if (p.bias != nullptr) {
+            add_bias<0>(r[0], b);
+            add_bias<32>(r[1], b);
           }
+#pragma unroll
+          for (int i = 0; i < 32; ++i) g[i] = pack_bf16x2(__uint_as_float(r[i >> 4][2 * (i & 15)]), __uint_as_float(r[i >> 4][2 * (i & 15) + 1]));
           if (p.store_gu) put(g, &tmap_d, col);
           auto activate = [&](auto f) {
 #pragma unroll
@@ -413,7 +412,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
           else activate([](float x) { return gelu_erf_f(x); });
           put(g, &tmap_act, col);
         }
-      } else if (!FP8 && alpha == 1.f && p.bias == nullptr && p.epilogue == GEMM_EPI_NONE && !empty) {
+      } else if (!FP8 && alpha == 1.f && (p.bias == nullptr || bias_vectors(p.bias, p.N)) && p.epilogue == GEMM_EPI_NONE && !empty) {
         // the next slab's columns come out of tensor memory while this one is converted and staged
         uint32_t r[2][2][32];
         auto fetch = [&](int c) {
@@ -425,9 +424,15 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
 #pragma unroll
           for (int c = 0; c < BN / 64; ++c) {
             const int col0 = n0 + c * 64;
+            uint4 b[8];
+            if (p.bias != nullptr) load_bias(b, p.bias, col0, p.N);
             tmem_ld_wait();
             if (col0 >= p.N) break;
             if (c + 1 < BN / 64) fetch(c + 1);
+            if (p.bias != nullptr) {
+              add_bias<0>(r[c & 1][0], b);
+              add_bias<32>(r[c & 1][1], b);
+            }
             uint8_t* buf = out + (slab++ & 1) * 4096;
             if (lane == 0) tma_store_wait_read<1>();   // the store issued two slabs ago has finished reading this buffer
             __syncwarp();

@@ -501,7 +501,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
             for (int i = 0; i < 32; i += 4) *reinterpret_cast<uint4*>(part + c * 32 + i) = make_uint4(r[i], r[i + 1], r[i + 2], r[i + 3]);
           }
         }
-      } else if (p.tma_store && alpha == 1.f && p.bias == nullptr && p.epilogue == GEMM_EPI_NONE && !empty_group) {
+      } else if (p.tma_store && alpha == 1.f && (p.bias == nullptr || bias_vectors(p.bias, p.N)) && p.epilogue == GEMM_EPI_NONE && !empty_group) {
         // 64-column slabs: TMEM -> registers -> bf16 -> swizzled smem -> one TMA store per slab and warp; the next slab's columns are on their way meanwhile
         uint8_t* stage = smem + L::kOutOffset + q * 8192;
         uint32_t r[2][2][32];
@@ -513,9 +513,15 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
 #pragma unroll
         for (int c = 0; c < BN / 64; ++c) {
           const int col0 = n0 + c * 64;
+          uint4 b[8];
+          if (p.bias != nullptr) load_bias(b, p.bias, col0, p.N);
           tmem_ld_wait();
           if (col0 >= p.N) break;
           if (c + 1 < BN / 64) fetch(c + 1);
+          if (p.bias != nullptr) {
+            add_bias<0>(r[c & 1][0], b);
+            add_bias<32>(r[c & 1][1], b);
+          }
           uint8_t* buf = stage + (slab++ & 1) * 4096;
           if (lane == 0) tma_store_wait_read<1>();  // the store issued two slabs ago has finished reading this buffer
           __syncwarp();
@@ -1097,12 +1103,13 @@ extern "C" int vlmt_gemm_bf16_glu_bwd(const void* dY, const void* W, const void*
 }
 
 // y = gelu(x), x = X(M,K) W(N,K)^T + bias (or null), and x itself or null, N a multiple of 8; 1: no such kernel for these sizes, nothing was
-// done.  Saves the pass over x.  Product and activation kernel / this one / without x: 28672 x 4304 x 1152 292 / 247 / 227 us, 10240 136 / 122 / 112, 4096
-// 58 / 54 / 50, 1024 27.6 / 25.6 / 25.6; 7168 x 4608 x 4096 187 / 177 / 174.
+// done.  Saves the pass over x.  Product and activation kernel / this one / without x: 28672 x 4304 x 1152 265 / 219 / 208 us, 10240 103 / 90 / 86, 4096
+// 48 / 45 / 44, 1024 25.6 / 23.5 / 22.5; 7168 x 4608 x 4096 183 / 174 / 170.
 extern "C" int vlmt_gemm_bf16_gelu(const void* X, const void* W, const void* bias, void* x, void* y, int M, int N, int K, int ldx, int ldw,
                                    int tanh_approx, int* status, int num_sms, cudaStream_t stream) {
   if (M <= BM || K <= 0 || N <= 0 || (N & 7) || (ldx & 7) || (ldw & 7)) return 1;
-  if ((reinterpret_cast<uintptr_t>(X) | reinterpret_cast<uintptr_t>(W) | reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(y)) & 15) return 1;
+  if ((reinterpret_cast<uintptr_t>(X) | reinterpret_cast<uintptr_t>(W) | reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(y) |
+       reinterpret_cast<uintptr_t>(bias)) & 15) return 1;
   const GemmForm form = gemm_form(M, N, K, true, true, false, num_sms, cluster_capacity(), vlmt_gemm_pair_clusters());
   if (!form.pairs || form.parts > 1 || form.k_splits > 1) return 1;
   return vlmt_gemm_pair_gelu(X, W, bias, x, y, M, N, K, ldx, ldw, tanh_approx ? GEMM_EPI_GELU_TANH : GEMM_EPI_GELU_ERF, status, stream);
