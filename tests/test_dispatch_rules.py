@@ -78,3 +78,16 @@ def test_tensor_memory_is_allocated_before_the_next_kernel_may_start():
                 allocating.add(m.group(1))
                 assert "pdl_begin" not in body and "pdl_trigger" not in body[:at], m.group(1)
     assert {"gemm_kernel", "gemm_pair_kernel", "gdn_scan_kernel", "gdn_prepare_fwd_kernel", "dsa_index_scores_kernel", "attn256_fwd_kernel"} <= allocating
+
+
+def test_the_selections_result_is_not_read_from_words_that_are_counted_in():
+    """Top-k selection: warps leave the search for the threshold without a barrier and begin to count in `warp_cnt`."""
+    import pathlib
+    import re
+
+    import vlm_training_b200.ops as ops
+
+    src = (pathlib.Path(ops.__file__).parent / "csrc" / "dsa_indexer_sm100.cu").read_text()
+    reads = re.findall(r"out\[\d\] = \(uint32_t\)sh_i\[(\d+)\];", src)
+    counted, = re.findall(r"warp_cnt = sh_res \+ (\d+);", src)
+    assert len(reads) == 3 and max(map(int, reads)) < int(counted)

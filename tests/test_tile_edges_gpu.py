@@ -233,7 +233,6 @@ def test_adamw_bucket_matches_segment_launches(lens, state):
         assert torch.equal(a, b)
 
 
-# documents below, at and beyond the number of selected keys; ends on and off the 64- / 128-row tiles; one token; 1, 2 and 8 query heads per kv head
 # the selection where it can go wrong: integer scores, so the oracle's are the same to the last bit; a bin of equal steps between smallest and largest
 # score holds few keys ("spread"), a few hundred of them equal ("equal"), nearly all ("clustered": one far outlier), infinite scores, one value only
 @pytest.mark.parametrize("kind", ["spread", "equal", "clustered", "infinite", "constant"])
@@ -268,6 +267,37 @@ def test_dsa_selection_of_integer_scores(kind, L, topk):
     assert torch.equal(listed, got[b0:])
 
 
+# a threshold that several keys share, of which only some are kept: the rows whose warps go on counting behind the search, on every SM and many times over
+@pytest.mark.parametrize("L,topk", [(2300, 700), (1100, 130)])
+def test_dsa_selection_with_a_shared_threshold(L, topk):
+    from vlm_training_b200.ops import cuda as cu
+
+    # a key's score is its level for every query; half of the keys share one level
+    level = torch.randint(0, 400, (L,), device=DEV)
+    level[torch.rand(L, device=DEV) < 0.5] = 200
+    iq, ik, w = torch.zeros(L, 4, 64, device=DEV), torch.zeros(L, 64, device=DEV), torch.zeros(L, 4, device=DEV)
+    iq[..., 0], iq[..., 1], w[:, 0] = 1.0, 16.0, 1.0
+    ik[:, 0], ik[:, 1] = level % 16, level // 16
+    iq, ik = iq.to(torch.bfloat16), ik.to(torch.bfloat16)
+    pos = torch.arange(L, device=DEV)
+    causal = pos[None, :] <= pos[:, None]
+    order = torch.where(causal, level[None, :].expand(L, L), -1).sort(dim=1, descending=True, stable=True).indices[:, :topk]
+    want = torch.zeros(L, L, dtype=torch.bool, device=DEV).scatter_(1, order, True) & causal
+    kept = torch.where(want, level[None, :], 1 << 20).amin(1)
+    shared = ((level[None, :] == kept[:, None]) & causal & ~want).any(1)
+    assert int(shared.sum()) > L // 4   # rows that go through the counting
+    b0 = max(0, L - 1024)
+    for _ in range(30):
+        bits = cu._C.dsa_select_bits(iq, ik, w, [0, L], topk)
+        got = ((bits[: (L + 63) // 64].t()[:, pos // 64] >> (pos % 64)) & 1).bool() & (pos[None, :] <= (pos[:, None] | 127))
+        assert torch.equal(got, want)
+        rows = cu._C.dsa_select(iq, ik, w, b0, b0, 0, L - b0, topk).long()
+        assert bool(((rows >= -1) & (rows <= pos[b0:, None])).all())   # -1: a row with fewer keys
+        assert torch.equal(torch.zeros(L - b0, L + 1, dtype=torch.bool, device=DEV).scatter_(1, torch.where(rows < 0, L, rows), True)[:, :L], want[b0:])
+    cu.check_status()
+
+
+# documents below, at and beyond the number of selected keys; ends on and off the 64- / 128-row tiles; one token; 1, 2 and 8 query heads per kv head
 @pytest.mark.parametrize("lens,topk,Hq,Hkv", [([700, 64, 1, 129, 300], 64, 16, 2), ([128, 1024, 257], 128, 8, 1), ([2100, 90], 512, 4, 4), ([1090], 1000, 4, 2)])
 def test_dsa_masked_dense_attention(lens, topk, Hq, Hkv):
     """Bit masks hold exactly the keys of the list form, and attention under them (forward, all gradients) matches the float32

@@ -221,6 +221,8 @@ constexpr int kBins = 2048, kMaxCand = 1024;
 // rank among the keys of that bin, a handful: the digits of a float put most scores of a row into a few exponents, whose counters a warp's
 // additions then queue for, and take three passes (12301 tokens in four documents, 2048 keys each: 247 us, now 91).  `out`: threshold, keys equal to it that are still wanted, keys equal to it.
 // False (the same in every thread) where scores are not finite, all equal, or more than kMaxCand fall into that bin.
+// Words of sh_i (the block's scratch): 0 to 2 hold the bin, then, behind the barrier that follows its last read, the result; 3 counts candidates; 8 to 15
+// hold the warps' counts.  A warp returns while another one still reads the result, and the caller's compaction counts in words 4 to 19 from there on.
 __device__ __forceinline__ bool select_by_value(const uint32_t* keys, int n, int want, float lo, float hi, bool bad, uint32_t* hist, float* sh_f,
                                                 int* sh_i, uint32_t (&out)[3]) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -278,10 +280,10 @@ __device__ __forceinline__ bool select_by_value(const uint32_t* keys, int n, int
     const uint32_t k = cand[t];
     int gt = 0, ge = 0;
     for (int i = 0; i < count; ++i) { gt += cand[i] > k; ge += cand[i] >= k; }
-    if (gt < want && want <= ge) { sh_i[4] = (int)k; sh_i[5] = want - gt; sh_i[6] = ge - gt; }   // equal keys write the same
+    if (gt < want && want <= ge) { sh_i[0] = (int)k; sh_i[1] = want - gt; sh_i[2] = ge - gt; }   // equal keys write the same
   }
   __syncthreads();
-  out[0] = (uint32_t)sh_i[4]; out[1] = (uint32_t)sh_i[5]; out[2] = (uint32_t)sh_i[6];
+  out[0] = (uint32_t)sh_i[0]; out[1] = (uint32_t)sh_i[1]; out[2] = (uint32_t)sh_i[2];   // no barrier behind: the caller leaves these words alone
   return true;
 }
 
@@ -310,7 +312,7 @@ __global__ void __launch_bounds__(TOPK_THREADS) dsa_topk_kernel(const __grid_con
   }
   uint32_t* hist = keys + ((n + 3) & ~3);
   int* sh_res = reinterpret_cast<int*>(hist + kBins);
-  int* warp_cnt = sh_res + 4;                   // [2][8]
+  int* warp_cnt = sh_res + 4;                   // [2][8]: behind the words from which select_by_value's result is read
   float* sh_f = reinterpret_cast<float*>(sh_res + 20);
   const float4* row = reinterpret_cast<const float4*>(p.scores + qb.off + (size_t)b * qb.ld);
   float lo = INFINITY, hi = -INFINITY;
