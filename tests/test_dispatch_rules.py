@@ -91,3 +91,21 @@ def test_the_selections_result_is_not_read_from_words_that_are_counted_in():
     reads = re.findall(r"out\[\d\] = \(uint32_t\)sh_i\[(\d+)\];", src)
     counted, = re.findall(r"warp_cnt = sh_res \+ (\d+);", src)
     assert len(reads) == 3 and max(map(int, reads)) < int(counted)
+
+
+def test_a_refusal_with_a_number_in_its_message_is_an_exception():
+    import os
+    import subprocess
+    import sys
+
+    code = """
+from vlm_training_b200.ops import cuda as cu
+try:
+    cu._C.gemm_set_flag_wait_ms(1000)
+except RuntimeError as e:
+    assert str(e).startswith("vlmt_gemm_set_flag_wait_ms failed with code "), e   # no device
+    print("raised")
+"""
+    # a process of its own, which a second C++ library would end, and without a GPU
+    r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, env={**os.environ, "CUDA_VISIBLE_DEVICES": ""})
+    assert r.returncode == 0 and r.stdout.strip() == "raised", (r.returncode, r.stdout, r.stderr)

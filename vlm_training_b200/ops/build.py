@@ -80,6 +80,16 @@ def _torch_flags():
     return inc, defs, libs
 
 
+def _shared_runtime(cxx: str) -> list[str]:
+    """The shared C++ library, by its path.  A compiler that ships only ``libstdc++.a`` would link a second copy beside torch's, and a stream of one
+    copy that meets a locale of the other ends the process: every error message with a number in it did."""
+    for name in ("libstdc++.so", "libstdc++.so.6"):
+        path = subprocess.run([cxx, f"-print-file-name={name}"], capture_output=True, text=True).stdout.strip()
+        if os.path.isabs(path):
+            return [path]
+    return []
+
+
 def _compile_one(src: str, verbose: bool, force: bool) -> tuple[str, str]:
     is_cu = src.endswith(".cu")
     inc, defs, _ = _torch_flags() if not is_cu else ([], [], [])
@@ -113,12 +123,13 @@ def build(force: bool = False, verbose: bool = False) -> str:
         results = list(pool.map(lambda s: _compile_one(s, verbose, force), srcs))
     objs = [o for o, _ in results]
     out = ext_path()
-    stamp = hashlib.sha256(" ".join(sorted(objs)).encode()).hexdigest()
+    cxx = os.environ.get("CXX", "g++")
+    libs = _torch_flags()[2] + _shared_runtime(cxx)
+    stamp = hashlib.sha256(" ".join(sorted(objs) + libs).encode()).hexdigest()
     stamp_file = os.path.join(BUILD, "link.stamp")
     if not force and os.path.exists(out) and os.path.exists(stamp_file) and open(stamp_file).read() == stamp:
         return out
-    _, _, libs = _torch_flags()
-    cmd = [os.environ.get("CXX", "g++"), "-shared", "-o", out] + objs + libs
+    cmd = [cxx, "-shared", "-o", out] + objs + libs
     res = subprocess.run(cmd, capture_output=True, text=True)
     if res.returncode != 0:
         raise RuntimeError(f"link failed: {' '.join(cmd)}\n{res.stdout}{res.stderr}")
