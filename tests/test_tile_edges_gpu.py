@@ -297,6 +297,26 @@ def test_dsa_selection_with_a_shared_threshold(L, topk):
     cu.check_status()
 
 
+# as many keys as a block's shared memory holds, and one more, which is refused
+def test_dsa_selection_from_the_longest_document():
+    from vlm_training_b200.ops import cuda as cu
+
+    L, B, topk = 56044, 3, 2048
+    level = torch.randint(0, 4000, (L + 1,), device=DEV)
+    iq, ik, w = torch.zeros(L + 1, 4, 64, device=DEV), torch.zeros(L + 1, 64, device=DEV), torch.zeros(L + 1, 4, device=DEV)
+    iq[..., 0], iq[..., 1], w[:, 0] = 1.0, 64.0, 1.0
+    ik[:, 0], ik[:, 1] = level % 64, level // 64
+    iq, ik = iq.to(torch.bfloat16), ik.to(torch.bfloat16)
+    rows = cu._C.dsa_select(iq, ik, w, L - B, L - B, 0, B, topk).long()
+    for b in range(B):
+        n = L - B + b + 1
+        want = level[:n].sort(descending=True, stable=True).indices[:topk].sort().values
+        assert torch.equal(rows[b].sort().values, want)
+    with pytest.raises(RuntimeError, match="code -3"):
+        cu._C.dsa_select(iq, ik, w, L + 1 - B, L + 1 - B, 0, B, topk)
+    cu.check_status()
+
+
 # documents below, at and beyond the number of selected keys; ends on and off the 64- / 128-row tiles; one token; 1, 2 and 8 query heads per kv head
 @pytest.mark.parametrize("lens,topk,Hq,Hkv", [([700, 64, 1, 129, 300], 64, 16, 2), ([128, 1024, 257], 128, 8, 1), ([2100, 90], 512, 4, 4), ([1090], 1000, 4, 2)])
 def test_dsa_masked_dense_attention(lens, topk, Hq, Hkv):

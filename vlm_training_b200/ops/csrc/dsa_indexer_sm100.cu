@@ -221,11 +221,12 @@ constexpr int kBins = 2048, kMaxCand = 1024;
 // rank among the keys of that bin, a handful: the digits of a float put most scores of a row into a few exponents, whose counters a warp's
 // additions then queue for, and take three passes (12301 tokens in four documents, 2048 keys each: 247 us, now 91).  `out`: threshold, keys equal to it that are still wanted, keys equal to it.
 // False (the same in every thread) where scores are not finite, all equal, or more than kMaxCand fall into that bin.
-// Words of sh_i (the block's scratch): 0 to 2 hold the bin, then, behind the barrier that follows its last read, the result; 3 counts candidates; 8 to 15
-// hold the warps' counts.  A warp returns while another one still reads the result, and the caller's compaction counts in words 4 to 19 from there on.
-__device__ __forceinline__ bool select_by_value(const uint32_t* keys, int n, int want, float lo, float hi, bool bad, uint32_t* hist, float* sh_f,
-                                                int* sh_i, uint32_t (&out)[3]) {
+// Words of sh_i (the block's scratch of 20): 0 to 2 hold the bin, then, behind the barrier that follows its last read, the result; 3 counts candidates; 4 to
+// 19 hold the warps' smallest and largest scores, and behind the barrier that follows their reads 8 to 15 the warps' counts.  A warp returns while another one still reads the result, and the caller's compaction counts in words 4 to 19 from there on.
+__device__ __forceinline__ bool select_by_value(const uint32_t* keys, int n, int want, float lo, float hi, bool bad, uint32_t* hist, int* sh_i,
+                                                uint32_t (&out)[3]) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  float* sh_f = reinterpret_cast<float*>(sh_i + 4);
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {
     lo = fminf(lo, __shfl_xor_sync(0xffffffffu, lo, o));
@@ -313,7 +314,6 @@ __global__ void __launch_bounds__(TOPK_THREADS) dsa_topk_kernel(const __grid_con
   uint32_t* hist = keys + ((n + 3) & ~3);
   int* sh_res = reinterpret_cast<int*>(hist + kBins);
   int* warp_cnt = sh_res + 4;                   // [2][8]: behind the words from which select_by_value's result is read
-  float* sh_f = reinterpret_cast<float*>(sh_res + 20);
   const float4* row = reinterpret_cast<const float4*>(p.scores + qb.off + (size_t)b * qb.ld);
   float lo = INFINITY, hi = -INFINITY;
   bool bad = false;
@@ -333,7 +333,7 @@ __global__ void __launch_bounds__(TOPK_THREADS) dsa_topk_kernel(const __grid_con
     *reinterpret_cast<uint4*>(keys + 4 * i) = make_uint4(k[0], k[1], k[2], k[3]);
   }
   uint32_t found[3];
-  if (!select_by_value(keys, n, p.kk, lo, hi, bad, hist, sh_f, sh_res, found)) {
+  if (!select_by_value(keys, n, p.kk, lo, hi, bad, hist, sh_res, found)) {
     __syncthreads();
     int bin, above, want = p.kk;
     uint32_t prefix = 0, mask = 0;
@@ -416,7 +416,7 @@ int launch_topk(QueryBlocks blocks, const TopkParams& p, cudaStream_t st) {
     n_max = n_max > b.q_pos0 + b.B ? n_max : b.q_pos0 + b.B;
   }
   if (grid <= 0 || p.kk <= 0) return 0;
-  const int smem = (((n_max + 3) & ~3) + kBins + 4 + 16 + 16) * 4;
+  const int smem = (((n_max + 3) & ~3) + kBins + 4 + 16) * 4;   // 56044 keys at most
   if (smem > 227 * 1024) return -3;
   if (cudaFuncSetAttribute(dsa_topk_kernel<BITS>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return -4;
   launch_pdl(dsa_topk_kernel<BITS>, dim3(grid), dim3(TOPK_THREADS), smem, st, 1, blocks, p);
