@@ -109,3 +109,49 @@ except RuntimeError as e:
     # a process of its own, which a second C++ library would end, and without a GPU
     r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, env={**os.environ, "CUDA_VISIBLE_DEVICES": ""})
     assert r.returncode == 0 and r.stdout.strip() == "raised", (r.returncode, r.stdout, r.stderr)
+
+
+class _Extension:
+    """Stands for the binding calls that run a whole block: remembers the weights that it gets."""
+
+    def __init__(self):
+        self.w = None
+
+    def __getattr__(self, name):
+        def call(x, w, *_):
+            self.w = w
+            return x
+        return call
+
+
+def test_vision_blocks_in_one_call_get_pruned_and_parametrised_tensors(monkeypatch):
+    import types
+
+    import torch
+    from torch.nn.utils import parametrize, prune
+
+    from vlm_training_b200 import ops
+    from vlm_training_b200.models import ModelConfig
+    from vlm_training_b200.models.vision import PatchMerger, VisionBlock
+
+    class Twice(torch.nn.Module):
+        def forward(self, t):
+            return 2 * t
+
+    ext = _Extension()
+    monkeypatch.setattr(ops, "whole_blocks", lambda x, *modules: ext)
+    cfg = ModelConfig.preset("tiny-qwen3-vl").vision
+    plan = types.SimpleNamespace(cos=None, sin=None, cu_seqlens=None, max_seqlen=1)
+    block, merger = VisionBlock(cfg), PatchMerger(cfg, False)
+    for p in (*block.parameters(), *merger.parameters()):
+        torch.nn.init.normal_(p)
+    prune.random_unstructured(block.norm1, "bias", 0.5)
+    prune.random_unstructured(block.mlp.linear_fc1, "bias", 0.5)
+    prune.random_unstructured(block.attn.proj, "weight", 0.5)
+    parametrize.register_parametrization(block.norm2, "bias", Twice())
+    prune.random_unstructured(merger.linear_fc2, "bias", 0.5)
+    x = torch.zeros(4, cfg.hidden_size)
+    for call, modules in ((lambda: block._in_one_call(x, plan), (block.norm1, block.attn.qkv, block.attn.proj, block.norm2, block.mlp.linear_fc1, block.mlp.linear_fc2)),
+                          (lambda: merger(x), (merger.norm, merger.linear_fc1, merger.linear_fc2))):
+        assert call() is x
+        assert all(torch.equal(w, t) for w, t in zip(ext.w, (t for m in modules for t in (m.weight, m.bias)))) and len(ext.w) == 2 * len(modules)

@@ -127,6 +127,12 @@ def expose_fused(parent: nn.Module, attr: str):
     parent._register_load_state_dict_pre_hook(load_hook, with_module=True)
 
 
+def tensor_of(module, name: str):
+    """``module.name`` without the lookup of ``nn.Module`` where it is a parameter; pruned, parametrised and replaced ones are not."""
+    own = module._parameters
+    return own[name] if name in own else getattr(module, name)
+
+
 # ----------------------------------------------------------------------------- MLP
 class SwiGLUMLP(nn.Module):
     def __init__(self, hidden: int, intermediate: int):
