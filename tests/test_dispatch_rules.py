@@ -155,3 +155,34 @@ def test_vision_blocks_in_one_call_get_pruned_and_parametrised_tensors(monkeypat
                           (lambda: merger(x), (merger.norm, merger.linear_fc1, merger.linear_fc2))):
         assert call() is x
         assert all(torch.equal(w, t) for w, t in zip(ext.w, (t for m in modules for t in (m.weight, m.bias)))) and len(ext.w) == 2 * len(modules)
+
+
+def test_decoder_layers_in_one_call_get_pruned_and_parametrised_weights(monkeypatch):
+    import types
+
+    import torch
+    from torch.nn.utils import parametrize, prune
+
+    from vlm_training_b200 import ops
+    from vlm_training_b200.models import ModelConfig
+    from vlm_training_b200.models.layers import DecoderLayer
+
+    class Twice(torch.nn.Module):
+        def forward(self, t):
+            return 2 * t
+
+    ext = _Extension()
+    monkeypatch.setattr(ops, "whole_blocks", lambda x, *modules: ext)
+    cfg = ModelConfig.preset("tiny-qwen3-vl").text
+    layer = DecoderLayer(cfg, 0)
+    for p in layer.parameters():
+        torch.nn.init.normal_(p)
+    attn, mlp = layer.self_attn, layer.mlp
+    prune.random_unstructured(attn.qkv, "weight", 0.5)
+    parametrize.register_parametrization(mlp.gate_up, "weight", Twice())
+    parametrize.register_parametrization(attn.k_norm, "weight", Twice())
+    prune.random_unstructured(mlp.down_proj, "weight", 0.5)
+    x, ctx = torch.zeros(4, cfg.hidden_size), types.SimpleNamespace(cos=None, sin=None, cu_seqlens=None, max_seqlen=1)
+    assert layer._in_one_call(x, ctx) is x
+    modules = (layer.input_layernorm, attn.qkv, attn.q_norm, attn.k_norm, attn.o_proj, layer.post_attention_layernorm, mlp.gate_up, mlp.down_proj)
+    assert len(ext.w) == len(modules) and all(torch.equal(w, m.weight) for w, m in zip(ext.w, modules))

@@ -362,7 +362,7 @@ class DecoderLayer(nn.Module):
         if ext is None:
             return None
         n1, n2 = parts["input_layernorm"], parts["post_attention_layernorm"]
-        w = tuple(m._parameters["weight"] for m in (n1, qkv, q_norm, k_norm, o_proj, n2, gate_up, down))
+        w = tuple(tensor_of(m, "weight") for m in (n1, qkv, q_norm, k_norm, o_proj, n2, gate_up, down))
         return ext.op_decoder_layer(x, w, ctx.cos, ctx.sin, ctx.cu_seqlens, int(ctx.max_seqlen), attn.n_q, attn.n_kv, attn.head_dim, n1.eps, n2.eps,
                                     cfg.rms_norm_eps, n1.offset, n2.offset, cfg.offset_norm, attn.gated, float(attn.scale))
 
