@@ -186,3 +186,24 @@ def test_decoder_layers_in_one_call_get_pruned_and_parametrised_weights(monkeypa
     assert layer._in_one_call(x, ctx) is x
     modules = (layer.input_layernorm, attn.qkv, attn.q_norm, attn.k_norm, attn.o_proj, layer.post_attention_layernorm, mlp.gate_up, mlp.down_proj)
     assert len(ext.w) == len(modules) and all(torch.equal(w, m.weight) for w, m in zip(ext.w, modules))
+
+
+@pytest.mark.parametrize("replaced", ["self_attn.o_proj", "mlp.down_proj"])
+def test_a_layer_with_a_replaced_projection_runs_module_by_module(monkeypatch, replaced):
+    import types
+
+    import torch
+
+    from vlm_training_b200 import ops
+    from vlm_training_b200.models import ModelConfig
+    from vlm_training_b200.models.layers import DecoderLayer
+
+    ext = _Extension()
+    monkeypatch.setattr(ops, "whole_blocks", lambda x, *modules: ext)
+    cfg = ModelConfig.preset("tiny-qwen3-vl").text
+    layer = DecoderLayer(cfg, 0)
+    x, ctx = torch.zeros(4, cfg.hidden_size), types.SimpleNamespace(cos=None, sin=None, cu_seqlens=None, max_seqlen=1)
+    assert layer._in_one_call(x, ctx) is x
+    old = layer.get_submodule(replaced)
+    layer.set_submodule(replaced, torch.nn.Linear(old.weight.shape[1], old.weight.shape[0], bias=False))   # without `tp` and `parallel`
+    assert layer._in_one_call(x, ctx) is None

@@ -355,7 +355,10 @@ class DecoderLayer(nn.Module):
         qkv, o_proj, q_norm, k_norm = (attn._modules[n] for n in ("qkv", "o_proj", "q_norm", "k_norm"))
         gate_up, down = mlp._modules["gate_up"], mlp._modules["down_proj"]
         cfg = attn.cfg
-        if (cfg.dsa or qkv.tp.enabled or o_proj.tp.enabled or gate_up.tp.enabled or down.tp.enabled or type(o_proj) is not Linear
+        # modules put in the place of these may have no more in common with them than what the halves below use
+        if type(o_proj) is not Linear or not all(isinstance(m, Linear) for m in (qkv, gate_up, down)):
+            return None
+        if (cfg.dsa or qkv.tp.enabled or o_proj.tp.enabled or gate_up.tp.enabled or down.tp.enabled
                 or any(m.bias is not None for m in (qkv, o_proj, gate_up, down))):
             return None
         ext = ops.whole_blocks(x, attn, o_proj)
