@@ -207,3 +207,22 @@ def test_a_layer_with_a_replaced_projection_runs_module_by_module(monkeypatch, r
     old = layer.get_submodule(replaced)
     layer.set_submodule(replaced, torch.nn.Linear(old.weight.shape[1], old.weight.shape[0], bias=False))   # without `tp` and `parallel`
     assert layer._in_one_call(x, ctx) is None
+
+
+@pytest.mark.parametrize("owner,method", [("", "mixer_half"), ("", "mlp_half"), ("mlp", "forward_prenorm")])
+def test_a_layer_with_a_half_of_its_own_runs_it(monkeypatch, owner, method):
+    import types
+
+    import torch
+
+    from vlm_training_b200 import ops
+    from vlm_training_b200.models import ModelConfig
+    from vlm_training_b200.models.layers import DecoderLayer
+
+    monkeypatch.setattr(ops, "whole_blocks", lambda x, *modules: _Extension())
+    cfg = ModelConfig.preset("tiny-qwen3-vl").text
+    layer = DecoderLayer(cfg, 0)
+    x, ctx = torch.zeros(4, cfg.hidden_size), types.SimpleNamespace(cos=None, sin=None, cu_seqlens=None, max_seqlen=1)
+    module = layer.get_submodule(owner)
+    setattr(module, method, getattr(module, method))   # what a wrapper around a method leaves on the instance
+    assert layer._in_one_call(x, ctx) is None

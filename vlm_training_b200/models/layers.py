@@ -352,6 +352,9 @@ class DecoderLayer(nn.Module):
         attn, mlp = parts.get("self_attn"), parts["mlp"]
         if type(attn) is not SelfAttention or type(mlp) is not SwiGLUMLP:
             return None
+        own = self.__dict__   # halves of its own, as `ops.whole_blocks` asks of `forward`
+        if "mixer_half" in own or "mlp_half" in own or "forward_prenorm" in mlp.__dict__:
+            return None
         qkv, o_proj, q_norm, k_norm = (attn._modules[n] for n in ("qkv", "o_proj", "q_norm", "k_norm"))
         gate_up, down = mlp._modules["gate_up"], mlp._modules["down_proj"]
         cfg = attn.cfg
