@@ -226,3 +226,22 @@ def test_a_layer_with_a_half_of_its_own_runs_it(monkeypatch, owner, method):
     module = layer.get_submodule(owner)
     setattr(module, method, getattr(module, method))   # what a wrapper around a method leaves on the instance
     assert layer._in_one_call(x, ctx) is None
+
+
+def test_a_saved_parameter_does_not_take_the_optimizer_along():
+    import io
+
+    import torch
+
+    from vlm_training_b200.config import Config
+    from vlm_training_b200.parallel.mesh import get_mesh
+    from vlm_training_b200.train.optimizer import create_optimizer
+
+    m = torch.nn.Linear(256, 256, bias=False)
+    t = Config().training
+    t.data_parallel = "fsdp"
+    engine = create_optimizer(m, t, get_mesh(1, torch.device("cpu")))
+    file = io.BytesIO()
+    torch.save(m.weight, file)
+    state = sum(x.numel() * x.element_size() for d in engine.domains for x in (*d.master, *d.exp_avg, *d.exp_avg_sq))
+    assert file.tell() < m.weight.numel() * m.weight.element_size() + state // 2

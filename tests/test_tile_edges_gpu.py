@@ -848,3 +848,47 @@ def test_bias_of_the_common_epilogue(M, N, K):
     off.copy_(b[:N])
     assert torch.equal(cu._gemm(x, w, bias=off), y)
     cu.check_status()
+
+
+def test_expert_gradients_are_added_to_what_the_caller_has_left_in_the_buffer():
+    """Writes that a tensor's version does not show: through `.data`, and by the replay of a captured pass."""
+    from vlm_training_b200.config import Config
+    from vlm_training_b200.parallel.mesh import get_mesh
+    from vlm_training_b200.train.optimizer import create_optimizer
+
+    T, H, I, E, k = 300, 256, 128, 8, 2
+    m = torch.nn.Module()
+    m.gate_up_proj, m.down_proj = ps = [torch.nn.Parameter(_rand(*s, scale=0.05)) for s in ((E, 2 * I, H), (E, H, I))]
+    t = Config().training
+    t.lr_llm = t.lr_mlp = t.lr_vit = 1e-3
+    t.data_parallel = "fsdp"
+    engine = create_optimizer(m, t, get_mesh(1, torch.device(DEV)))
+    engine.set_requires_gradient_sync(False)   # no update under a backward pass that no step follows
+    x, dy = _rand(T, H), _rand(T, H)
+    w, chosen = ops.moe_router(_rand(T, E), k)
+    alone = torch.autograd.grad(ops.moe_experts(x, *ps, w.to(x.dtype), chosen), ps, dy)
+
+    def backward():
+        ops.moe_experts(x, *ps, w.to(x.dtype), chosen).backward(dy)
+
+    engine.zero_grad()
+    for p, a in zip(ps, alone):
+        p.grad.data.copy_(a)                   # a gradient that was kept from before
+    backward()
+    for p, a in zip(ps, alone):
+        assert torch.equal(p.grad, a + a)
+    engine.zero_grad()
+    torch.cuda.synchronize()
+    side = torch.cuda.Stream()
+    with torch.cuda.stream(side):
+        backward()                             # workspaces of the first pass
+        side.synchronize()
+        engine.zero_grad()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=side):
+            backward()
+        graph.replay()
+        graph.replay()
+    side.synchronize()
+    for p, a in zip(ps, alone):
+        assert torch.equal(p.grad, a + a)

@@ -56,9 +56,7 @@ class _GroupedLinear(torch.autograd.Function):
                 g = param.grad.view(E * N, K)
             else:
                 dw = torch.empty(E * N, K, dtype=w.dtype, device=w.device)
-            # a gradient that the optimizer has just cleared is stored: adding it reads 1.6 GB of zeros for 256 experts of 3 x 2048 x 512
-            zero = getattr(param, "_vlmt_take_zero_grad", None) if g is not None else None
-            cu._C.gemm_grouped(dy, x, dw if g is None else g, prefix, 2, True, g is not None and not (zero is not None and zero(param.grad)))
+            cu._C.gemm_grouped(dy, x, dw if g is None else g, prefix, 2, True, g is not None)
             cu._tick()
             if g is None:
                 dw = dw.view(E, N, K)

@@ -38,7 +38,6 @@ from __future__ import annotations
 import math
 import os
 from dataclasses import dataclass, field
-from functools import partial
 
 import torch
 import torch.distributed as dist
@@ -179,10 +178,6 @@ class _Domain:
                 # (ops/cuda.py:_wgrad, csrc/bindings_autograd.cpp); valid because every such parameter enters exactly one op per
                 # forward pass.  Parameters with tensor hooks get their gradients through autograd.
                 p._vlmt_grad_in_place = True
-                p._vlmt_take_zero_grad = partial(self.take_zero_grad, p, o)
-        # every gradient is zero since generation `zero_gen` but for those that a kernel has taken since (`take_zero_grad`), as long as nobody has
-        # written into the buffer through autograd or a tensor operation (its version, which all views share)
-        self.zero_gen, self.zero_version, self.taken = 1, self.flat_grad._version, {}
         # ---- optimizer state on the local shard of every bucket
         self.master, self.exp_avg, self.exp_avg_sq = [], [], []
         for b in self.buckets:
@@ -190,19 +185,6 @@ class _Domain:
             self.master.append(self.flat_param[lo:hi].float().clone())
             self.exp_avg.append(torch.zeros(hi - lo, dtype=state_dtype, device=device))
             self.exp_avg_sq.append(torch.zeros(hi - lo, dtype=state_dtype, device=device))
-
-    def mark_zero(self):
-        """The gradient buffer has been cleared as a whole (ordered before what the current stream is given next)."""
-        if not self.reshard:
-            self.zero_gen, self.zero_version = self.zero_gen + 1, self.flat_grad._version
-
-    def take_zero_grad(self, p, offset, g) -> bool:
-        """Whether ``g`` (``p.grad``) is known to be zero, so that a kernel may store into it what it would add; once per clearing."""
-        if (self.taken.get(p) == self.zero_gen or g._version != self.zero_version
-                or g.data_ptr() != self.flat_grad.data_ptr() + offset * self.flat_grad.element_size()):
-            return False
-        self.taken[p] = self.zero_gen
-        return True
 
     # ------------------------------------------------------------------ sharded parameters and gradients (ZeRO-3)
     def _init_resharded(self, param_dtype, state_dtype, symmetric):
@@ -531,7 +513,6 @@ class ShardedOptimizerEngine(torch.optim.Optimizer):
                 from ..ops import cuda as cu
 
                 cu.memset_zero_(d.flat_grad)
-                d.mark_zero()
             else:
                 d.flat_grad.zero_()
             for b in d.buckets:
@@ -820,8 +801,6 @@ class ShardedOptimizerEngine(torch.optim.Optimizer):
             # on this path every rank's kernel clears the gradients it consumed; when each rank consumes the whole
             # buffer (one rank, or unsharded data parallelism) the next zero_grad() has nothing left to do
             d.grads_clean = self.is_cuda and d.flat_param.dtype == torch.bfloat16 and (d.size == 1 or not d.shard)
-            if d.grads_clean:
-                d.mark_zero()
         if self.reshard:
             self.release_all()
             self._bwd_phase, self._prefetched = False, -1
