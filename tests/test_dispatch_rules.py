@@ -245,3 +245,50 @@ def test_a_saved_parameter_does_not_take_the_optimizer_along():
     torch.save(m.weight, file)
     state = sum(x.numel() * x.element_size() for d in engine.domains for x in (*d.master, *d.exp_avg, *d.exp_avg_sq))
     assert file.tell() < m.weight.numel() * m.weight.element_size() + state // 2
+
+
+@pytest.mark.parametrize("owner,method", [("layers.SelfAttention", "forward"), ("layers.Linear", "forward"), ("layers.SwiGLUMLP", "forward_prenorm"),
+                                          ("layers.DecoderLayer", "mixer_half"), ("layers.DecoderLayer", "mlp_half"),
+                                          ("vision.VisionAttention", "forward"), ("vision.VisionMLP", "forward")])
+def test_a_class_whose_method_is_replaced_runs_it(monkeypatch, owner, method):
+    import importlib
+    import types
+
+    import torch
+
+    from vlm_training_b200 import ops
+    from vlm_training_b200.models import ModelConfig
+    from vlm_training_b200.models.layers import DecoderLayer
+    from vlm_training_b200.models.vision import VisionBlock
+
+    monkeypatch.setattr(ops, "whole_blocks", lambda x, *modules: _Extension())
+    cfg = ModelConfig.preset("tiny-qwen3-vl")
+    ctx = types.SimpleNamespace(cos=None, sin=None, cu_seqlens=None, max_seqlen=1)
+    layer, block = DecoderLayer(cfg.text, 0), VisionBlock(cfg.vision)
+    x, patches = torch.zeros(4, cfg.text.hidden_size), torch.zeros(4, cfg.vision.hidden_size)
+    assert layer._in_one_call(x, ctx) is x and block._in_one_call(patches, ctx) is patches
+    module, cls = owner.split(".")
+    cls = getattr(importlib.import_module(f"vlm_training_b200.models.{module}"), cls)
+    old = getattr(cls, method)
+    monkeypatch.setattr(cls, method, lambda *args, **kwargs: old(*args, **kwargs))
+    one, passed_by = (layer, x) if module == "layers" else (block, patches)
+    assert one._in_one_call(passed_by, ctx) is None
+
+
+@pytest.mark.parametrize("name", ["attention_varlen", "linear", "gelu_linear", "qkv_norm_rope"])
+def test_blocks_with_a_replaced_op_run_module_by_module(monkeypatch, name):
+    import types
+
+    import torch
+
+    from vlm_training_b200 import ops
+
+    cuda = types.SimpleNamespace(_GEMM_BACKEND="tcgen05", _C=object())
+    monkeypatch.setattr(ops, "_use_cuda", lambda x: True)
+    monkeypatch.setattr(ops, "_cu", lambda: cuda)
+    monkeypatch.setattr(ops, "_CUDA_MODULE", cuda)
+    x = torch.zeros(4, 64)
+    assert ops.whole_blocks(x) is cuda._C
+    old = getattr(ops, name)
+    monkeypatch.setattr(ops, name, lambda *args, **kwargs: old(*args, **kwargs))
+    assert ops.whole_blocks(x) is None

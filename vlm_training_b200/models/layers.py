@@ -352,8 +352,8 @@ class DecoderLayer(nn.Module):
         attn, mlp = parts.get("self_attn"), parts["mlp"]
         if type(attn) is not SelfAttention or type(mlp) is not SwiGLUMLP:
             return None
-        own = self.__dict__   # halves of its own, as `ops.whole_blocks` asks of `forward`
-        if "mixer_half" in own or "mlp_half" in own or "forward_prenorm" in mlp.__dict__:
+        own = self.__dict__   # halves of its own, as `ops.whole_blocks` asks of `forward`, or of its class
+        if _layer_methods() != _LAYER_METHODS or "mixer_half" in own or "mlp_half" in own or "forward_prenorm" in mlp.__dict__:
             return None
         qkv, o_proj, q_norm, k_norm = (attn._modules[n] for n in ("qkv", "o_proj", "q_norm", "k_norm"))
         gate_up, down = mlp._modules["gate_up"], mlp._modules["down_proj"]
@@ -383,6 +383,13 @@ class DecoderLayer(nn.Module):
 
         h = self.mixer_half(x, ctx)
         return checkpoint(self.mlp_half, h, x, use_reentrant=False)
+
+
+def _layer_methods():
+    return SelfAttention.forward, Linear.forward, SwiGLUMLP.forward_prenorm, DecoderLayer.mixer_half, DecoderLayer.mlp_half
+
+
+_LAYER_METHODS = _layer_methods()   # what `DecoderLayer._in_one_call` stands for; a class whose method is replaced later runs that
 
 
 class Decoder(nn.Module):

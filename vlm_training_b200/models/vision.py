@@ -146,7 +146,7 @@ class VisionBlock(nn.Module):
         """The whole block as one call of the extension, or ``None`` where its modules have to run one by one."""
         parts = self._modules
         attn, mlp, n1, n2 = parts["attn"], parts["mlp"], parts["norm1"], parts["norm2"]
-        if type(attn) is not VisionAttention or type(mlp) is not VisionMLP:
+        if type(attn) is not VisionAttention or type(mlp) is not VisionMLP or _block_methods() != _BLOCK_METHODS:
             return None
         qkv, proj, fc1, fc2 = attn._modules["qkv"], attn._modules["proj"], mlp._modules["linear_fc1"], mlp._modules["linear_fc2"]
         if any(type(m) is not Linear or m.parallel is not None for m in (qkv, proj, fc1, fc2)):
@@ -157,6 +157,13 @@ class VisionBlock(nn.Module):
         w = tuple(tensor_of(m, n) for m in (n1, qkv, proj, n2, fc1, fc2) for n in ("weight", "bias"))
         return ext.op_vision_block(x, w, plan.cos, plan.sin, plan.cu_seqlens, int(plan.max_seqlen), attn.n_heads, attn.head_dim, n1.eps, n2.eps,
                                    attn.head_dim ** -0.5, mlp.approx == "tanh")
+
+
+def _block_methods():
+    return VisionAttention.forward, VisionMLP.forward, Linear.forward
+
+
+_BLOCK_METHODS = _block_methods()   # what `VisionBlock._in_one_call` stands for; a class whose method is replaced later runs that
 
 
 class PatchMerger(nn.Module):

@@ -12,6 +12,7 @@ Set ``VLMT_FORCE_REFERENCE=1`` to run the PyTorch statements on CUDA tensors
 """
 from __future__ import annotations
 
+import operator
 import os
 
 import torch
@@ -40,8 +41,9 @@ def _cu():
 
 def whole_blocks(x, *modules):
     """The binding calls that run a whole block (``op_decoder_layer``, ``op_vision_block``, ``op_patch_merger``), or ``None`` where the modules have
-    to run one by one: other devices, the library GEMM, and ``modules`` (those that the block calls) with hooks or a forward of their own."""
-    if not _use_cuda(x) or _cu()._GEMM_BACKEND == "cublas" or _any_global_hook():
+    to run one by one: other devices, the library GEMM, ``modules`` (those that the block calls) with hooks or a forward of their own, and an op
+    of this package that has been replaced (a wrapper that counts or traces it, another attention)."""
+    if not _use_cuda(x) or _cu()._GEMM_BACKEND == "cublas" or _any_global_hook() or _block_ops(globals()) != _BLOCK_OPS:
         return None
     for m in modules:
         d = m.__dict__
@@ -315,3 +317,9 @@ def embedding(ids, weight, grad_in_place: bool = False):
     if grad_in_place and _use_cuda(weight) and ids.dtype == torch.int64:
         return _cu()._C.op_embedding(ids, weight)
     return torch.nn.functional.embedding(ids, weight)
+
+
+# the ops that the modules of a whole block call one by one
+_block_ops = operator.itemgetter("linear", "rms_norm_linear", "layer_norm", "layer_norm_linear", "gelu_linear", "swiglu_linear", "sigmoid_mul",
+                                 "qkv_norm_rope", "rope_vision", "attention_varlen")
+_BLOCK_OPS = _block_ops(globals())
