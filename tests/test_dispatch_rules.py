@@ -292,3 +292,14 @@ def test_blocks_with_a_replaced_op_run_module_by_module(monkeypatch, name):
     old = getattr(ops, name)
     monkeypatch.setattr(ops, name, lambda *args, **kwargs: old(*args, **kwargs))
     assert ops.whole_blocks(x) is None
+
+
+def test_products_of_few_rows_ask_for_their_shared_memory_on_every_device():
+    """The attribute belongs to a device: a flag of the process would leave it out on the second one."""
+    import pathlib
+
+    import vlm_training_b200.ops as ops
+
+    src = (pathlib.Path(ops.__file__).parent / "csrc" / "gemm_rows_sm100.cu").read_text()
+    launch = src[src.index("int launch("):]
+    assert "static bool" not in launch and launch.index("cudaGetDevice") < launch.index("cudaFuncSetAttribute") < launch.index("launch_pdl(")

@@ -17,6 +17,7 @@
 #include "pdl.cuh"
 #include "sm100.cuh"
 
+#include <atomic>
 #include <cuda_runtime.h>
 
 namespace {
@@ -269,11 +270,14 @@ template <int NT, bool GLU>
 int launch(const void* X, const void* W, int lda, int ldb, const Params& p, cudaStream_t stream) {
   using L = Layout<NT>;
   auto kern = gemm_rows_kernel<NT, GLU>;
-  static bool configured = false;
-  if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kTotal);
-    if (e != cudaSuccess) return (int)e;
-    configured = true;
+  static std::atomic<uint64_t> configured{0};   // devices (beyond the 64th: set on every launch) that allow the shared memory
+  int device;
+  cudaError_t e = cudaGetDevice(&device);
+  if (e != cudaSuccess) return (int)e;
+  const uint64_t bit = device < 64 ? 1ull << device : 0;
+  if ((configured.load(std::memory_order_relaxed) & bit) == 0) {
+    if ((e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kTotal)) != cudaSuccess) return (int)e;
+    configured.fetch_or(bit, std::memory_order_relaxed);
   }
   CUtensorMap tw, tx;
   int r = vlmt_make_tmap_2d_bf16(&tx, X, (uint64_t)p.K, (uint64_t)p.M, (uint64_t)lda * 2, 64, NT);
