@@ -303,3 +303,20 @@ def test_products_of_few_rows_ask_for_their_shared_memory_on_every_device():
     src = (pathlib.Path(ops.__file__).parent / "csrc" / "gemm_rows_sm100.cu").read_text()
     launch = src[src.index("int launch("):]
     assert "static bool" not in launch and launch.index("cudaGetDevice") < launch.index("cudaFuncSetAttribute") < launch.index("launch_pdl(")
+
+
+def test_shared_arrays_that_are_accessed_as_vectors_are_aligned():
+    import pathlib
+    import re
+
+    import vlm_training_b200.ops as ops
+
+    src = (pathlib.Path(ops.__file__).parent / "csrc" / "elementwise.cu").read_text()
+    found = 0
+    for body in src.split("__global__")[1:]:
+        for name in set(re.findall(r"reinterpret_cast<(?:const )?(?:float|uint)4\*>\(&(\w+)\[", body)):
+            declared = re.search(rf"__shared__ ([^;]*?)\b{name}\[", body)
+            if declared is not None:
+                found += 1
+                assert "__align__(16)" in declared.group(1), name
+    assert found > 0

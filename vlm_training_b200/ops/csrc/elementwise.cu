@@ -956,7 +956,7 @@ __global__ void __launch_bounds__(kThreads, 3) rmsnorm_gated_vec_bwd_kernel(cons
                                                                            float* __restrict__ dw_partial, int rows) {
   pdl_begin();
   constexpr int D = 128 * V, U = V == 1 ? 4 : 2;
-  __shared__ float sm_dw[kWarpsPerBlock][D];
+  __shared__ __align__(16) float sm_dw[kWarpsPerBlock][D];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   float wv[V][4], dw[V][4];
 #pragma unroll
