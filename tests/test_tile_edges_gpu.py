@@ -892,3 +892,18 @@ def test_expert_gradients_are_added_to_what_the_caller_has_left_in_the_buffer():
     side.synchronize()
     for p, a in zip(ps, alone):
         assert torch.equal(p.grad, a + a)
+
+
+def test_launches_are_counted_where_they_are_made():
+    from vlm_training_b200.ops import cuda as cu
+
+    def launched(fn):
+        before = cu.LAUNCHES["count"]
+        fn()
+        return cu.LAUNCHES["count"] - before
+
+    assert launched(lambda: cu._colsum(_rand(2048, 64))) == 1   # one launch, then slabs and their sum
+    assert launched(lambda: cu._colsum(_rand(2049, 64))) == 2
+    iq, ik, w = _rand(40 * 129, 4, 64), _rand(40 * 129, 64), _rand(40 * 129, 4).float()
+    for docs, times in ((1, 1), (32, 1), (33, 2), (40, 2)):     # 32 blocks of queries per pair of launches
+        assert launched(lambda: cu._C.dsa_select_bits(iq, ik, w, [129 * i for i in range(docs + 1)], 128)) == 2 * times

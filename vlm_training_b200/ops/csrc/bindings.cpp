@@ -593,6 +593,7 @@ void colsum_into(const Tensor& x, void* out, int mode) {
   if (slabs > 0) partial = torch::empty({slabs, cols}, x.options().dtype(torch::kFloat));
   const int r = vlmt_colsum(x.data_ptr(), x.stride(0), rows, cols, slabs > 0 ? partial.data_ptr<float>() : nullptr, out, mode, cur_stream());
   TORCH_CHECK(r == 0, "vlmt_colsum failed with code ", r);
+  count_launches(slabs > 0 ? 2 : 1);
 }
 Tensor colsum(const Tensor& x) {
   Tensor out = torch::empty({x.size(1)}, x.options().dtype(torch::kFloat));

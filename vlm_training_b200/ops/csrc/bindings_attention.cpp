@@ -152,9 +152,11 @@ static Tensor dsa_select_bits(const Tensor& iq, const Tensor& ik, const Tensor& 
   Tensor bits = torch::empty({(longest + 127) / 128 * 2, T}, iq.options().dtype(torch::kLong));
   Tensor st = vlmt_status_tensor();
   const std::vector<long> b(bounds.begin(), bounds.end());
+  int launches;
   int r = vlmt_dsa_select_bits(iq.data_ptr(), ik.data_ptr(), w.data_ptr<float>(), (int)T, b.data(), (int)b.size() - 1, (int)topk, (int)kBlock,
-                               scores.data_ptr<float>(), (long)room, bits.data_ptr(), st.data_ptr<int>(), at::cuda::getCurrentCUDAStream().stream());
+                               scores.data_ptr<float>(), (long)room, bits.data_ptr(), st.data_ptr<int>(), &launches, at::cuda::getCurrentCUDAStream().stream());
   TORCH_CHECK(r == 0, "vlmt_dsa_select_bits failed with code ", r);
+  vlmt::count_launches(launches);
   return bits;
 }
 

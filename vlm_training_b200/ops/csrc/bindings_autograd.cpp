@@ -161,7 +161,6 @@ Tensor bias_grad(const Tensor& dy, const Tensor& b, const Target& t) {
     return dy.to(at::kFloat).sum(0).to(b.scalar_type());
   VecGrad g(b, t);
   colsum_into(dy, g.out.data_ptr(), g.mode);
-  tick(2);
   return g.finish(b, t);
 }
 
@@ -1108,6 +1107,7 @@ std::vector<Tensor> vision_plan(const Tensor& images, const Tensor& trig, int64_
   return {c, s, index, weight};
 }
 }  // namespace
+void count_launches(int n) { tick(n); }
 }  // namespace vlmt
 
 void bind_autograd(py::module_& m) {

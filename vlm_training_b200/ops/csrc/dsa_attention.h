@@ -22,9 +22,9 @@ int vlmt_dsa_index_scores(const void* iq, const void* ik, const float* w, int T,
                           int* status, cudaStream_t st);
 int vlmt_dsa_topk(const float* scores, int B, int ld, int q_pos0, int kk, int* sel, cudaStream_t st);
 // both for the documents of a row that are longer than kk, the selection as a bit mask for the dense kernels (attention256_sm100.cu):
-// [ceil(L / 64)][T] 64-bit words; scores: `room` floats, at least `rows` x the longest document rounded up to 4
+// [ceil(L / 64)][T] 64-bit words; scores: `room` floats, at least `rows` x the longest document rounded up to 4; launches: set to their number
 int vlmt_dsa_select_bits(const void* iq, const void* ik, const float* w, int T, const long* bounds, int n_docs, int kk, int rows, float* scores,
-                         long room, void* bits, int* status, cudaStream_t st);
+                         long room, void* bits, int* status, int* launches, cudaStream_t st);
 #ifdef __cplusplus
 }
 #endif

@@ -452,7 +452,8 @@ extern "C" int vlmt_dsa_topk(const float* scores, int B, int ld, int q_pos0, int
 // The same selection as bits for every document longer than kk: word [kt][t] of `bits` ([key tiles][T] 64-bit words) holds keys 64 kt .. of token t.
 // Blocks of `rows` queries are scored and selected a buffer full (`room` floats, at least rows x the longest document rounded up to 4) at a time.
 extern "C" int vlmt_dsa_select_bits(const void* iq, const void* ik, const float* w, int T, const long* bounds, int n_docs, int kk, int rows, float* scores,
-                                    long room, void* bits, int* status, cudaStream_t st) {
+                                    long room, void* bits, int* status, int* launches, cudaStream_t st) {
+  *launches = 0;
   QueryBlocks blocks;
   blocks.count = 0;
   long used = 0;
@@ -463,6 +464,7 @@ extern "C" int vlmt_dsa_select_bits(const void* iq, const void* ik, const float*
     if (blocks.count == 0) return 0;
     int r = launch_scores(iq, ik, w, T, blocks, scores, status, st);
     if (r == 0) r = launch_topk<true>(blocks, p, st);
+    *launches += 2;
     blocks.count = 0;
     used = 0;
     return r;

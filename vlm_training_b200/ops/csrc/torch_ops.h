@@ -10,6 +10,7 @@ using torch::Tensor;
 using OptTensor = c10::optional<Tensor>;
 
 int num_sms();
+void count_launches(int n);   // of this package's kernels, see op_launches
 void gemm(const Tensor& a, const Tensor& b, Tensor& out, bool a_mn, bool b_mn, const OptTensor& bias, int64_t epilogue, bool accumulate,
           const OptTensor& alpha, bool one_sum = false);   // one_sum: see vlmt_gemm_bf16
 bool gemm_gelu(const Tensor& x, const Tensor& w, const OptTensor& bias, bool tanh_approx, Tensor* pre, Tensor& act);

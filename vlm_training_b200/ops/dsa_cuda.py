@@ -140,7 +140,6 @@ def dsa_attention_cuda(q, k, v, idx_q, idx_k, idx_w, cu_seqlens, topk, scale=Non
     # the masked kernels take the row maximum before the scale and mask by -inf: a scale that is not positive goes to the gathered form
     if D == 256 and fused_select and longest <= _DENSE_TIMES * topk and scale > 0:
         bits = cu._C.dsa_select_bits(iq_c, ik_c, iw_c, bounds, int(topk))
-        cu._tick(2)
         on_device = _device_bounds(cu_seqlens, bounds, q.device)
         if n == T:   # a slice of everything would still cost a zero fill and a copy per gradient
             return _MaskedAttention.apply(q, k, v, on_device, bits, int(topk), float(scale))
