@@ -907,3 +907,95 @@ def test_launches_are_counted_where_they_are_made():
     iq, ik, w = _rand(40 * 129, 4, 64), _rand(40 * 129, 64), _rand(40 * 129, 4).float()
     for docs, times in ((1, 1), (32, 1), (33, 2), (40, 2)):     # 32 blocks of queries per pair of launches
         assert launched(lambda: cu._C.dsa_select_bits(iq, ik, w, [129 * i for i in range(docs + 1)], 128)) == 2 * times
+
+
+# the same comparison, with both routes shown to be the ones that are meant, and enough rows for the activations in the products' epilogues
+@pytest.mark.parametrize("block,preset,layer,rows", [("decoder", "tiny-qwen3-vl-gpu", 0, 333), ("decoder", "tiny-qwen3-vl-gpu", 0, 8192), ("decoder", "qwen3.5-dense", 3, 1500),
+                                                     ("vision", "tiny-qwen3-vl-gpu", 0, 76), ("vision", "tiny-qwen3-vl-gpu", 0, 4096), ("merger", "tiny-qwen3-vl-gpu", 0, 76),
+                                                     ("merger", "tiny-qwen3-vl-gpu", 1, 4096)])
+def test_blocks_go_the_way_that_they_are_meant_to(block, preset, layer, rows):
+    from vlm_training_b200.models import BatchPlan, ModelConfig
+    from vlm_training_b200.models.causal_lm import rotary_inv_freq, rotary_tables
+    from vlm_training_b200.models.layers import DecoderLayer, RowContext
+    from vlm_training_b200.models.vision import PatchMerger, VisionBlock, VisionPlan
+    from vlm_training_b200.ops import cuda as cu
+
+    cfg = ModelConfig.preset(preset)
+    if block == "decoder":
+        cfg.text.hidden_size, cfg.text.intermediate_size = 512, 4864
+        m, hooked = DecoderLayer(cfg.text, layer), "self_attn.o_proj"
+        plan = BatchPlan.build(cfg, torch.zeros(rows, dtype=torch.int64).numpy(), torch.tensor([0, rows // 3, rows], dtype=torch.int32), None, DEV)
+        args = (RowContext(plan.cu_seqlens, plan.max_seqlen, *rotary_tables(cfg.text, plan.position_ids, rotary_inv_freq(cfg.text, torch.device(DEV)), torch.float32),
+                           plan.seq_idx, plan.extras),)
+        x = _rand(rows, 512)
+        if rows == 8192:   # SwiGLU and its gradient in the epilogues
+            gu, act = cu._C.gemm_glu(x, _rand(2 * 4864, 512), True)[::-1]
+            assert cu._C.gemm_glu_bwd(x, _rand(512, 4864), gu, True) is not None
+    else:
+        cfg.vision.hidden_size, cfg.vision.num_heads, cfg.vision.intermediate_size = 512, 8, 1280
+        grid = [[1, 64, 64]] if rows == 4096 else [[1, 6, 10], [1, 4, 4]]
+        plan = VisionPlan.build(grid, cfg.vision, torch.device(DEV))
+        m, hooked, args = (VisionBlock(cfg.vision), "attn.proj", (plan,)) if block == "vision" else (PatchMerger(cfg.vision, layer == 0), "", ())
+        x = _rand(rows, 512)
+        if block == "vision" and rows == 4096:   # GELU and its gradient in the epilogues
+            act, pre = cu._C.gemm_gelu(x, _rand(1280, 512), _rand(1280), True, True)
+            assert cu._C.gemm_gelu_bwd(x, _rand(512, 1280), pre, True, True) is not None
+    m = m.to(DEV, torch.bfloat16)
+    with torch.no_grad():
+        for p in m.parameters():
+            p.copy_(_rand(*p.shape, scale=0.05) + (1.0 if p.dim() == 1 else 0.0))
+
+    def in_one_call():
+        if block != "merger":
+            return m._in_one_call(x, *args) is not None
+        w = tuple(t for n in ("norm", "linear_fc1", "linear_fc2") for t in (m.get_submodule(n).weight, m.get_submodule(n).bias))
+        return ops.whole_blocks(x).op_patch_merger(x, w, m.merged, m.postshuffle, m.norm.eps) is not None
+
+    dy = None
+
+    def run(grad):
+        nonlocal dy
+        with torch.set_grad_enabled(grad):
+            xi = x.clone().requires_grad_(grad)
+            y = m(xi, *args)
+            if not grad:
+                return [y]
+            dy = _rand(*y.shape) if dy is None else dy
+            return [y.detach(), *torch.autograd.grad(y, [xi, *m.parameters()], dy)]
+
+    assert in_one_call()
+    one = run(True), run(False)
+    if block == "merger":
+        m.linear_fc1.weight._vlmt_resharded = True   # a weight that is gathered by the module that reads it
+    else:
+        m.get_submodule(hooked).register_forward_hook(lambda *_: None)
+    assert not in_one_call()
+    apart = run(True), run(False)
+    for a, b in zip(one, apart):
+        for s, t in zip(a, b):
+            assert torch.equal(s, t)
+    cu.check_status()
+
+
+# the score buffer filled more than once: by 32 blocks of queries, and by its 64 MB, in the middle of a document
+@pytest.mark.parametrize("lens,topk", [([129] * 40, 128), ([4100, 20, 3300], 512)])
+def test_dsa_selection_fills_its_buffer_again(lens, topk):
+    from vlm_training_b200.ops import cuda as cu
+
+    T = sum(lens)
+    level = torch.randint(0, 400, (T,), device=DEV)   # a key's score, for every query
+    iq, ik, w = torch.zeros(T, 4, 64, device=DEV), torch.zeros(T, 64, device=DEV), torch.zeros(T, 4, device=DEV)
+    iq[..., 0], iq[..., 1], w[:, 0] = 1.0, 16.0, 1.0
+    ik[:, 0], ik[:, 1] = level % 16, level // 16
+    bounds = [sum(lens[:i]) for i in range(len(lens) + 1)]
+    bits = cu._C.dsa_select_bits(iq.to(torch.bfloat16), ik.to(torch.bfloat16), w, bounds, topk)
+    for s, L in zip(bounds, lens):
+        if L <= topk:
+            continue
+        pos = torch.arange(L, device=DEV)
+        causal = pos[None, :] <= pos[:, None]
+        order = torch.where(causal, level[None, s:s + L].expand(L, L), -1).sort(dim=1, descending=True, stable=True).indices[:, :topk]
+        want = torch.zeros(L, L, dtype=torch.bool, device=DEV).scatter_(1, order, True) & causal
+        got = ((bits[: (L + 63) // 64, s:s + L].t()[:, pos // 64] >> (pos % 64)) & 1).bool() & (pos[None, :] <= (pos[:, None] | 127))
+        assert torch.equal(got, want)
+    cu.check_status()
