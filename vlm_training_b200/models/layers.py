@@ -127,10 +127,12 @@ def expose_fused(parent: nn.Module, attr: str):
     parent._register_load_state_dict_pre_hook(load_hook, with_module=True)
 
 
-def tensor_of(module, name: str):
-    """``module.name`` without the lookup of ``nn.Module`` where it is a parameter; pruned, parametrised and replaced ones are not."""
-    own = module._parameters
-    return own[name] if name in own else getattr(module, name)
+def tensors_of(modules, names):
+    """``module.name`` of all, without the lookup of ``nn.Module`` where they are parameters; pruned, parametrised and replaced ones are not."""
+    try:
+        return tuple([m._parameters[n] for m in modules for n in names])
+    except KeyError:
+        return tuple([getattr(m, n) for m in modules for n in names])
 
 
 # ----------------------------------------------------------------------------- MLP
@@ -368,7 +370,7 @@ class DecoderLayer(nn.Module):
         if ext is None:
             return None
         n1, n2 = parts["input_layernorm"], parts["post_attention_layernorm"]
-        w = tuple(tensor_of(m, "weight") for m in (n1, qkv, q_norm, k_norm, o_proj, n2, gate_up, down))
+        w = tensors_of((n1, qkv, q_norm, k_norm, o_proj, n2, gate_up, down), ("weight",))
         return ext.op_decoder_layer(x, w, ctx.cos, ctx.sin, ctx.cu_seqlens, int(ctx.max_seqlen), attn.n_q, attn.n_kv, attn.head_dim, n1.eps, n2.eps,
                                     cfg.rms_norm_eps, n1.offset, n2.offset, cfg.offset_norm, attn.gated, float(attn.scale))
 

@@ -14,7 +14,7 @@ import torch.nn as nn
 from .. import ops
 from . import positions
 from .config import VisionConfig
-from .layers import Linear, tensor_of
+from .layers import Linear, tensors_of
 
 
 def _inv_freq(half):
@@ -154,7 +154,7 @@ class VisionBlock(nn.Module):
         ext = ops.whole_blocks(x, attn, proj, mlp)
         if ext is None:
             return None
-        w = tuple(tensor_of(m, n) for m in (n1, qkv, proj, n2, fc1, fc2) for n in ("weight", "bias"))
+        w = tensors_of((n1, qkv, proj, n2, fc1, fc2), ("weight", "bias"))
         return ext.op_vision_block(x, w, plan.cos, plan.sin, plan.cu_seqlens, int(plan.max_seqlen), attn.n_heads, attn.head_dim, n1.eps, n2.eps,
                                    attn.head_dim ** -0.5, mlp.approx == "tanh")
 
@@ -183,7 +183,7 @@ class PatchMerger(nn.Module):
         ext = ops.whole_blocks(x) if type(self) is PatchMerger else None
         if ext is not None:
             parts = self._modules
-            w = tuple(tensor_of(parts[m], n) for m in ("norm", "linear_fc1", "linear_fc2") for n in ("weight", "bias"))
+            w = tensors_of((parts["norm"], parts["linear_fc1"], parts["linear_fc2"]), ("weight", "bias"))
             out = ext.op_patch_merger(x, w, self.merged, self.postshuffle, parts["norm"].eps)
             if out is not None:
                 return out
