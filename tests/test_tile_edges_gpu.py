@@ -999,3 +999,16 @@ def test_dsa_selection_fills_its_buffer_again(lens, topk):
         got = ((bits[: (L + 63) // 64, s:s + L].t()[:, pos // 64] >> (pos % 64)) & 1).bool() & (pos[None, :] <= (pos[:, None] | 127))
         assert torch.equal(got, want)
     cu.check_status()
+
+
+# no rows: the weight's gradient is a sum of nothing, whatever the memory held before
+@pytest.mark.parametrize("form", ["linear", "layer_norm_linear", "rms_norm_linear", "gelu_linear", "swiglu_linear"])
+def test_gradients_of_no_rows_are_zero(form):
+    w = _rand(64, 128).requires_grad_()
+    n = [_rand(128).requires_grad_() for _ in range(2)]
+    x = torch.empty(0, 256 if form == "swiglu_linear" else 128, dtype=torch.bfloat16, device=DEV, requires_grad=True)
+    y = {"linear": lambda: ops.linear(x, w), "layer_norm_linear": lambda: ops.layer_norm_linear(x, *n, w), "rms_norm_linear": lambda: ops.rms_norm_linear(x, n[0], w),
+         "gelu_linear": lambda: ops.gelu_linear(x, w), "swiglu_linear": lambda: ops.swiglu_linear(x, w)}[form]()
+    held = [torch.full((64, 128), float("nan"), dtype=torch.bfloat16, device=DEV) for _ in range(64)]
+    del held   # what the gradient's memory holds
+    assert torch.equal(torch.autograd.grad(y, w, torch.empty_like(y))[0], torch.zeros_like(w))

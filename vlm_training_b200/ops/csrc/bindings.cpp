@@ -64,6 +64,11 @@ void gemm(const Tensor& a, const Tensor& b, Tensor& out, bool a_mn, bool b_mn, c
     TORCH_CHECK(alpha->is_cuda() && alpha->scalar_type() == at::kFloat && alpha->numel() == 1, "alpha must be one fp32 value on the device");
     alpha_p = alpha->data_ptr<float>();
   }
+  if (K == 0 && !accumulate && epilogue == GEMM_EPI_NONE) {   // a sum of nothing, for which no kernel runs
+    out.zero_();
+    if (bias.has_value()) out.add_(*bias);
+    return;
+  }
   Tensor st = status_tensor();
   int r = vlmt_gemm_bf16(a.data_ptr(), b.data_ptr(), d_bf16, d_f32, optptr(bias), M, N, K, (int)a.stride(0), (int)b.stride(0),
                          (int)out.stride(0), a_mn, b_mn, (int)epilogue, accumulate, alpha_p, one_sum, st.data_ptr<int>(), num_sms(),
