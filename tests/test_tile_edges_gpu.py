@@ -233,6 +233,7 @@ def test_adamw_bucket_matches_segment_launches(lens, state):
         assert torch.equal(a, b)
 
 
+# documents below, at and beyond the number of selected keys; ends on and off the 64- / 128-row tiles; one token; 1, 2 and 8 query heads per kv head
 # the selection where it can go wrong: integer scores, so the oracle's are the same to the last bit; a bin of equal steps between smallest and largest
 # score holds few keys ("spread"), a few hundred of them equal ("equal"), nearly all ("clustered": one far outlier), infinite scores, one value only
 @pytest.mark.parametrize("kind", ["spread", "equal", "clustered", "infinite", "constant"])
@@ -317,7 +318,6 @@ def test_dsa_selection_from_the_longest_document():
     cu.check_status()
 
 
-# documents below, at and beyond the number of selected keys; ends on and off the 64- / 128-row tiles; one token; 1, 2 and 8 query heads per kv head
 @pytest.mark.parametrize("lens,topk,Hq,Hkv", [([700, 64, 1, 129, 300], 64, 16, 2), ([128, 1024, 257], 128, 8, 1), ([2100, 90], 512, 4, 4), ([1090], 1000, 4, 2)])
 def test_dsa_masked_dense_attention(lens, topk, Hq, Hkv):
     """Bit masks hold exactly the keys of the list form, and attention under them (forward, all gradients) matches the float32

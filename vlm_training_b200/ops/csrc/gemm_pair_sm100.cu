@@ -116,7 +116,7 @@ template <bool A_MN, bool B_MN, bool FP8, int GLU>
 __global__ void __launch_bounds__(NUM_THREADS, 1)
 gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b, const __grid_constant__ CUtensorMap tmap_d,
                  const __grid_constant__ CUtensorMap tmap_act, const __grid_constant__ CUtensorMap tmap_gu, Params p) {
-    constexpr bool BWD = GLU == kGluBwd || GLU == kGeluBwd;
+  constexpr bool BWD = GLU == kGluBwd || GLU == kGeluBwd;
   constexpr int NST = BWD ? STAGES - 1 : STAGES;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));

@@ -1,7 +1,8 @@
 """DSA sparse attention on CUDA.
 
 Indexer scores -> per-query top-k key selection -> attention restricted to the selected keys.  The documents are walked from the
-host copy of the boundaries (no device read), the scores in query blocks of 1024 so they are never larger than ``block x L``.
+host copy of the boundaries (no device read).  Scores are made for blocks of 1024 queries, so they are never larger than ``1024 x L``
+or, where the selection becomes bits, than the larger of that and 64 MB, which hold as many blocks as fit.
 
 Head size 256 and documents up to ``_DENSE_TIMES x topk`` tokens: the selection becomes one bit per query and causal key, and the
 dense kernels of ``csrc/attention256_sm100.cu`` compute every tile up to the diagonal with the bits as a mask, one launch per pass
@@ -11,7 +12,7 @@ tensor cores: 12301 tokens in documents of 1303 to 5015, 16 heads, forward and b
 Longer documents and other head sizes go block by block:
 
 * selection: ``csrc/dsa_indexer_sm100.cu`` (indexer heads' products on the tensor cores folded into fp32 scores, then a
-  radix-select top-k; -1 in unused slots) for 4 indexer heads of 64 channels in bf16, else ``einsum`` / ``topk`` under
+  top-k by steps of the score's value; -1 in unused slots) for 4 indexer heads of 64 channels in bf16, else ``einsum`` / ``topk`` under
   ``no_grad`` — the selection is an index set, nothing of it is kept for backward;
 * attention over the selected keys: the tcgen05 kernels of ``csrc/dsa_attention_sm100.cu`` (head size 256, 8 query heads
   per kv head), else the CUDA-core kernels of ``csrc/dsa_attention.cu`` (one CTA per query and kv head reads each selected
@@ -162,7 +163,7 @@ def dsa_attention_cuda(q, k, v, idx_q, idx_k, idx_w, cu_seqlens, topk, scale=Non
             b1 = min(L, b0 + _QBLOCK)
             n_keys = b1  # causal: keys [0, b1)
             if fused_select:
-                # scores on the tensor cores and a radix-select top-k, two launches per block, -1 in unused slots
+                # scores on the tensor cores and the top-k of their rows, two launches per block, -1 in unused slots
                 sel32 = cu._C.dsa_select(iq_c, ik_c, iw_c, s + b0, b0, s, b1 - b0, min(topk, n_keys))
                 cu._tick(2)
                 doc_out.append(_SelectedAttention.apply(q[s + b0:s + b1], kd, vd, sel32, scale))
